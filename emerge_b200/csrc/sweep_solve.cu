@@ -85,8 +85,15 @@ __device__ __forceinline__ double nrm2(T a) { return (double)a.x * a.x + (double
 
 enum DotMode { DOT_NONE = 0, DOT_XY = 1, DOT_CONJW_Y = 2, DOT_CONJY_W_YY = 3 };
 
+// DOF pairs (i, i + n/2) per block of the kernels below.  Every dot product is summed block by block, so
+// these depend on the batch size only: a mesh's groups of pairs (multiples of 256) are cut alike alone and
+// inside a grouped solve.
+__host__ __device__ constexpr int spmv_pairs(int S) { return S >= 16 ? 16 : 8; }
+__host__ __device__ constexpr int vec_pairs(int S) { return S >= 16 ? 512 / S : VB / S; }
+
 // Block-level fixed-order tree reduction of up to three components per thread (two complex, one
-// real); thread s < S stores component c of this block at partial[(c * nblocks + block) * S + s].
+// real); thread s < S stores component c of this block at partial[(c * S + s) * nblocks + block], so the
+// partials of one system are contiguous.
 __device__ __forceinline__ void block_store3(double2 v0, double2 v1, double v2, int ncomp, int S, double2* partial) {
     __shared__ double2 r0[VB], r1[VB];
     __shared__ double r2[VB];
@@ -103,167 +110,357 @@ __device__ __forceinline__ void block_store3(double2 v0, double2 v1, double v2, 
         __syncthreads();
     }
     if (threadIdx.x < S) {
-        partial[(long long)blockIdx.x * S + threadIdx.x] = r0[threadIdx.x];
-        if (ncomp > 1) partial[((long long)gridDim.x + blockIdx.x) * S + threadIdx.x] = r1[threadIdx.x];
-        if (ncomp > 2) partial[(2LL * gridDim.x + blockIdx.x) * S + threadIdx.x] = make_double2(r2[threadIdx.x], 0.0);
+        const long long nb = gridDim.x;
+        partial[threadIdx.x * nb + blockIdx.x] = r0[threadIdx.x];
+        if (ncomp > 1) partial[(S + threadIdx.x) * nb + blockIdx.x] = r1[threadIdx.x];
+        if (ncomp > 2) partial[(2 * S + threadIdx.x) * nb + blockIdx.x] = make_double2(r2[threadIdx.x], 0.0);
     }
 }
 __device__ __forceinline__ void block_store2(double2 v0, double2 v1, int ncomp, int S, double2* partial) {
     block_store3(v0, v1, 0.0, ncomp, S, partial);
 }
 
-// y = A x for all systems, one thread per (row, system); optional dot-product epilogue (DotMode).
+// y = A x for all systems, a warp per DOF pair (rows i and i + n/2); optional dot-product epilogue (DotMode).
 // The operator values (E, B, Robin patch) are always FP64 and every row is accumulated in FP64;
 // R is the precision of the Krylov vectors only (FP32 in the mixed-precision inner solve), so the
 // inner iterations see the exact operator and only the vectors are rounded.  Rounding E and B to
 // FP32 separately would lose the cancellation in E - k0^2 B near resonances.
-template <typename R>
-__global__ void __launch_bounds__(VB) spmv_kernel(OpArgs a, const typename V2<R>::T* __restrict__ x,
-                                                   typename V2<R>::T* __restrict__ y, double2* __restrict__ partial,
-                                                   int dotmode, const typename V2<R>::T* __restrict__ w) {
-    typedef typename V2<R>::T T;
-    const int S = a.S;
-    long long g = (long long)blockIdx.x * VB + threadIdx.x;
-    long long i = g / S;
-    int s = (int)(g % S);
-    double2 c0 = make_double2(0.0, 0.0), c1 = c0;
-    double c2 = 0.0;
-    const int sy = i < a.n ? sys_of_row(a.pg, a.hh, i, S, s) : 0;
-    bool act = i < a.n && (!a.skip || sys_active(a.skip, sy));
-    // S >= 32: the 32 lanes of a warp are 32 systems of one row and stage that row's entries together
-    // (warp-synchronous below), so the warp skips the row only when none of its systems is active.
-    // Every lane reaches this vote, and the row index is the same for the whole warp.
-    if (S >= 32) act = __any_sync(0xffffffffu, act);
-    if (act) {
-        double yr = 0, yi = 0;
-        if (a.mask[i]) {
-            const double2* Ev = (const double2*)a.E;
-            const double2* Bv = (const double2*)a.B;
-            double er = 0, ei = 0, br = 0, bi = 0;
-            int jb = a.indptr[i], je = a.indptr[i + 1];
-            int j = jb;
-            if (S >= 32) {
-                // a warp holds 32 systems of one row: it stages 32 consecutive (column, E, B) entries
-                // with one coalesced load per lane and reads them back as shared-memory broadcasts;
-                // the products are summed in column order as below
-                __shared__ int s_c[VB / 32][32];
-                __shared__ double2 s_e[VB / 32][32], s_b[VB / 32][32];
-                const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
-                for (int base = jb; base < je; base += 32) {
-                    int jj = base + lane;
-                    if (jj < je) {
-                        s_c[wl][lane] = a.indices[jj];
-                        s_e[wl][lane] = Ev[jj];
-                        s_b[wl][lane] = Bv ? Bv[jj] : make_double2(0.0, 0.0);
-                    }
-                    __syncwarp();
-                    const int cnt = min(32, je - base);
-                    int u = 0;
-                    for (; u + 4 <= cnt; u += 4) {
-                        T xv[4];
+//
+// The latency of the gathers of x bounds it (16 S bytes per nonzero against 36 of the matrix).  The rows of a
+// pair have the same columns (they belong to one mesh entity), so the warp gathers each x once for both (a
+// CSR without that structure gathers the second row's too).  L lanes hold different systems, NR of them
+// per lane, and the 32 / L groups of lanes take every (32 / L)-th entry, so that a read of a matrix entry
+// serves NR systems and a batch of one system still has 32 entries in flight.  Entries travel by asynchronous
+// copies, DEPTH stages of 32 / L entries deep: as many bytes in flight held in registers leave too few
+// warps (115 against 75 us at S = 32 below; depths 3 to 5 are alike, 8 costs the second block of an SM, and
+// one system, whose row is three stages, is fastest with 2).  E - k0^2 B is formed per entry (2 + 4
+// multiply-adds per system instead of 8).
+// Measured (one launch, us, before: a thread per row and system): 6 000-tet guide, S = 1 / 4 / 16 / 32:
+// 37 / 30 / 69 / 98 -> 14 / 23 / 51 / 75; 82 944-tet cavity: 283 / 379 / 1058 / 1340 -> 205 / 290 / 613 / 921
+// (the last at 0.9 TB/s of matrix and 6.4 TB/s of gathered x; FP64 multiply-adds are half of its time).
+// Sum over the lane groups, halving the values a lane holds while it can: afterwards a lane holds row
+// (lane & 16) and max(1, 2 NR L / 32) systems of the lane, the first of them the returned one.
+template <int L, int NR>
+__device__ __forceinline__ int pair_reduce(double2* v, int lane) {
+    int r0 = 0;
+    int cnt = 2 * NR;
 #pragma unroll
-                        for (int t = 0; t < 4; t++) xv[t] = x[(long long)s_c[wl][u + t] * S + s];
+    for (int off = 16; off >= L; off >>= 1) {
+        if (cnt > 1) {
+            const int half = cnt / 2;
+            const bool up = lane & off;
 #pragma unroll
-                        for (int t = 0; t < 4; t++) {
-                            double2 e = s_e[wl][u + t], b = s_b[wl][u + t];
-                            double xr = xv[t].x, xi = xv[t].y;
-                            er += e.x * xr - e.y * xi;
-                            ei += e.x * xi + e.y * xr;
-                            if (Bv) {
-                                br += b.x * xr - b.y * xi;
-                                bi += b.x * xi + b.y * xr;
-                            }
-                        }
-                    }
-                    for (; u < cnt; u++) {
-                        T xv = x[(long long)s_c[wl][u] * S + s];
-                        double2 e = s_e[wl][u], b = s_b[wl][u];
-                        double xr = xv.x, xi = xv.y;
-                        er += e.x * xr - e.y * xi;
-                        ei += e.x * xi + e.y * xr;
-                        if (Bv) {
-                            br += b.x * xr - b.y * xi;
-                            bi += b.x * xi + b.y * xr;
-                        }
-                    }
-                    __syncwarp();
+            for (int i = 0; i < NR; i++)
+                if (i < half) {
+                    double2 send = up ? v[i] : v[i + half], keep = up ? v[i + half] : v[i];
+                    keep.x += __shfl_xor_sync(0xffffffffu, send.x, off);
+                    keep.y += __shfl_xor_sync(0xffffffffu, send.y, off);
+                    v[i] = keep;
                 }
-                j = je;
-            }
-            // four entries' loads are issued before their products are summed (in column order, so
-            // the sums are the same as the one-at-a-time loop): the row walk is latency-bound
-            for (; j + 4 <= je; j += 4) {
-                int cc[4];
-                T xv[4];
-                double2 e[4], b[4];
-#pragma unroll
-                for (int u = 0; u < 4; u++) cc[u] = a.indices[j + u];
-#pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    xv[u] = x[(long long)cc[u] * S + s];
-                    e[u] = Ev[j + u];
-                    b[u] = Bv ? Bv[j + u] : make_double2(0.0, 0.0);
-                }
-#pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    double xr = xv[u].x, xi = xv[u].y;
-                    er += e[u].x * xr - e[u].y * xi;
-                    ei += e[u].x * xi + e[u].y * xr;
-                    if (Bv) {
-                        br += b[u].x * xr - b[u].y * xi;
-                        bi += b[u].x * xi + b[u].y * xr;
-                    }
-                }
-            }
-            for (; j < je; j++) {
-                int c = a.indices[j];
-                T xv = x[(long long)c * S + s];
-                double xr = xv.x, xi = xv.y;
-                double2 e = Ev[j];
-                er += e.x * xr - e.y * xi;
-                ei += e.x * xi + e.y * xr;
-                if (Bv) {
-                    double2 b = Bv[j];
-                    br += b.x * xr - b.y * xi;
-                    bi += b.x * xi + b.y * xr;
-                }
-            }
-            double k2 = a.k0sq[sy];
-            yr = er - k2 * br;
-            yi = ei - k2 * bi;
-            int pr = a.patch_of_row ? a.patch_of_row[i] : -1;
-            if (pr >= 0) {
-                const double2* Pv = (const double2*)a.patch_vals;
-                for (int q = 0; q < a.n_ports; q++) {
-                    double pr_ = 0, pi_ = 0;
-                    for (int j = a.patch_rowptr[pr]; j < a.patch_rowptr[pr + 1]; j++) {
-                        if (a.patch_port[j] != q) continue;
-                        T xv = x[(long long)a.patch_cols[j] * S + s];
-                        double2 v = Pv[j];
-                        pr_ += v.x * xv.x - v.y * xv.y;
-                        pi_ += v.x * xv.y + v.y * xv.x;
-                    }
-                    double gr = a.gamma[2 * (sy * a.n_ports + q)], gi = a.gamma[2 * (sy * a.n_ports + q) + 1];
-                    yr += gr * pr_ - gi * pi_;
-                    yi += gr * pi_ + gi * pr_;
-                }
-            }
-        }
-        y[i * S + s] = mk2<R>((R)yr, (R)yi);
-        if (dotmode == DOT_XY) {
-            T xi = x[i * S + s];
-            c0 = make_double2((double)xi.x * yr - (double)xi.y * yi, (double)xi.x * yi + (double)xi.y * yr);
-        } else if (dotmode == DOT_CONJW_Y) {
-            T wi = w[i * S + s];
-            c0 = make_double2((double)wi.x * yr + (double)wi.y * yi, (double)wi.x * yi - (double)wi.y * yr);
-        } else if (dotmode == DOT_CONJY_W_YY) {
-            T wi = w[i * S + s];
-            c0 = make_double2(yr * wi.x + yi * wi.y, yr * wi.y - yi * wi.x);
-            c1 = make_double2(yr * yr + yi * yi, 0.0);
-            c2 = nrm2(wi);
+            if (off < 16 && up) r0 += half;
+            cnt = half;
+        } else {
+            v[0].x += __shfl_xor_sync(0xffffffffu, v[0].x, off);
+            v[0].y += __shfl_xor_sync(0xffffffffu, v[0].y, off);
         }
     }
-    if (dotmode != DOT_NONE) block_store3(c0, c1, c2, dotmode == DOT_CONJY_W_YY ? 3 : 1, S, partial);
+    return r0;
+}
+
+__device__ __forceinline__ void cp_async16z(void* dst, const void* src, bool ok) {   // zero fill when !ok
+    unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    int n = ok ? 16 : 0;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ void cp_async8z(void* dst, const void* src, bool ok) {
+    unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    int n = ok ? 8 : 0;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src), "r"(n) : "memory");
+}
+
+// Pipeline stages of a warp: 32 / L entries each, their x values and the two rows' E and B.
+template <typename R, int L, int NR, bool HASB>
+struct SpmvStage {
+    static constexpr int DEPTH = L == 1 ? 2 : 4;
+    typename V2<R>::T x[32 / L][L * NR];
+    double2 eb[HASB ? 4 : 2][32 / L];        // E row 0, E row 1, B row 0, B row 1
+};
+
+template <typename R, int L, int NR, bool HASB>
+__global__ void __launch_bounds__(VB, NR == 1 ? 4 : NR == 2 ? 3 : 2) spmv_kernel(
+    OpArgs a, const typename V2<R>::T* __restrict__ x, typename V2<R>::T* __restrict__ y, double2* __restrict__ partial,
+    int dotmode, const typename V2<R>::T* __restrict__ w) {
+    typedef typename V2<R>::T T;
+    typedef SpmvStage<R, L, NR, HASB> Stage;
+    constexpr int G = 32 / L;                       // entry groups of a warp
+    constexpr int NV = 2 * NR > G ? 2 * NR / G : 1; // values of a lane after the reduction
+    constexpr int D = Stage::DEPTH;
+    constexpr int XC = L * NR * (int)sizeof(T) / 16;      // 16-byte chunks of an entry's x values (0: 8 bytes)
+    extern __shared__ __align__(16) unsigned char spmv_sm[];
+    const int S = a.S;
+    const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
+    Stage* st = reinterpret_cast<Stage*>(spmv_sm) + wl * D;
+    const int g = lane / L, sl = lane % L, sb = blockIdx.y * (L * NR), s0 = sb + sl;
+    const long long hh = (a.n + 1) / 2;
+    const int ppb = spmv_pairs(S);
+    const double2* __restrict__ Ev = (const double2*)a.E;
+    const double2* __restrict__ Bv = (const double2*)a.B;
+    double2 c0[NV];
+    double c1[NV], c2[NV];
+#pragma unroll
+    for (int q = 0; q < NV; q++) { c0[q] = make_double2(0.0, 0.0); c1[q] = c2[q] = 0.0; }
+    for (int pw = wl; pw < ppb; pw += VB / 32) {
+        const long long i = (long long)blockIdx.x * ppb + pw;
+        if (i >= hh) break;
+        const int base = a.pg ? a.pg[i] * S : 0;
+        if (a.skip) {
+            bool act = false;
+#pragma unroll
+            for (int r = 0; r < NR; r++) act |= sys_active(a.skip, base + s0 + r * L);
+            if (!__any_sync(0xffffffffu, act)) continue;
+        }
+        const long long i1 = i + hh < a.n ? i + hh : i;      // odd n: the last pair has one row
+        const bool two = i1 != i;
+        const bool f0 = a.mask[i] != 0, f1 = two && a.mask[i1] != 0;
+        const int j0 = a.indptr[i], j1 = a.indptr[i1];
+        const int n0 = f0 ? a.indptr[i + 1] - j0 : 0, n1 = f1 ? a.indptr[i1 + 1] - j1 : 0;
+        double k2[NR];
+        if (HASB) {
+#pragma unroll
+            for (int r = 0; r < NR; r++) k2[r] = a.k0sq[base + s0 + r * L];
+        }
+        double2 acc[2 * NR];
+#pragma unroll
+        for (int q = 0; q < 2 * NR; q++) acc[q] = make_double2(0.0, 0.0);
+        const int nm = n0 > n1 ? n0 : n1;
+        const int nst = (nm + G - 1) / G;
+        // 32 column indices of each row per coalesced load, the next ones in flight while these are used
+        int ia = -1, ib = -1;
+        int ia2 = lane < n0 ? a.indices[j0 + lane] : -1, ib2 = lane < n1 ? a.indices[j1 + lane] : -1;
+        bool paired = true;                          // the rows' columns agree so far
+        auto issue = [&](int t) {
+            if (t < nst) {
+                if (t % L == 0) {
+                    ia = ia2; ib = ib2;
+                    const int kn = t * G + 32 + lane;
+                    ia2 = kn < n0 ? a.indices[j0 + kn] : -1;
+                    ib2 = kn < n1 ? a.indices[j1 + kn] : -1;
+                    paired = paired && __all_sync(0xffffffffu, ia == ib);
+                }
+                Stage& sg = st[t % D];
+                const int kc = (t % L) * G;          // first entry of the stage inside the 32 of the chunk
+                if (XC > 0) {
+#pragma unroll
+                    for (int q = 0; q < (G * XC + 31) / 32; q++) {
+                        const int ch = lane + 32 * q, en = ch / (XC > 0 ? XC : 1), c = __shfl_sync(0xffffffffu, ia, (kc + en) & 31);
+                        if (G * XC >= 32 || ch < G * XC)
+                            cp_async16z(reinterpret_cast<char*>(&sg.x[0][0]) + 16 * ch,
+                                        reinterpret_cast<const char*>(x + (long long)(c < 0 ? 0 : c) * S + sb) + 16 * (ch % (XC > 0 ? XC : 1)), c >= 0);
+                    }
+                } else {
+                    const int c = __shfl_sync(0xffffffffu, ia, (kc + lane) & 31);
+                    if (lane < G) cp_async8z(&sg.x[lane][0], x + (long long)(c < 0 ? 0 : c) * S, c >= 0);
+                }
+                constexpr int NE = (HASB ? 4 : 2) * G;
+#pragma unroll
+                for (int q = 0; q < (NE + 31) / 32; q++) {
+                    const int e = lane + 32 * q, which = e / G, kk = t * G + e % G;
+                    if (NE % 32 == 0 || e < NE) {
+                        const bool second = which & 1;
+                        const bool ok = kk < (second ? n1 : n0);
+                        const double2* src = (which & 2 ? Bv : Ev) + (second ? j1 : j0) + (ok ? kk : 0);
+                        cp_async16z(&sg.eb[which][e % G], src, ok);
+                    }
+                }
+            }
+            asm volatile("cp.async.commit_group;\n" ::: "memory");
+        };
+#pragma unroll
+        for (int t = 0; t < D - 1; t++) issue(t);
+        for (int t = 0; t < nst; t++) {
+            issue(t + D - 1);
+            asm volatile("cp.async.wait_group %0;\n" ::"n"(D - 1) : "memory");
+            __syncwarp();
+            const Stage& sg = st[t % D];
+            T xa[NR];
+#pragma unroll
+            for (int r = 0; r < NR; r++) xa[r] = sg.x[g][sl + r * L];
+            const double2 e0 = sg.eb[0][g], e1 = sg.eb[1][g];
+            double2 b0, b1;
+            if (HASB) { b0 = sg.eb[2][g]; b1 = sg.eb[3][g]; }
+#pragma unroll
+            for (int r = 0; r < NR; r++) {
+                const double xr = xa[r].x, xi = xa[r].y;
+                const double kr = HASB ? fma(-k2[r], b0.x, e0.x) : e0.x;
+                const double ki = HASB ? fma(-k2[r], b0.y, e0.y) : e0.y;
+                acc[r].x = fma(kr, xr, fma(-ki, xi, acc[r].x));
+                acc[r].y = fma(kr, xi, fma(ki, xr, acc[r].y));
+            }
+            if (!paired) {                           // the second row's own columns
+                const int kk = t * G + g;
+                const int cb = kk < n1 ? a.indices[j1 + kk] : -1;
+                const T* xc = x + (long long)(cb >= 0 ? cb : 0) * S + s0;
+#pragma unroll
+                for (int r = 0; r < NR; r++) xa[r] = cb >= 0 ? xc[r * L] : mk2<R>(0, 0);
+            }
+#pragma unroll
+            for (int r = 0; r < NR; r++) {
+                const double xr = xa[r].x, xi = xa[r].y;
+                const double kr = HASB ? fma(-k2[r], b1.x, e1.x) : e1.x;
+                const double ki = HASB ? fma(-k2[r], b1.y, e1.y) : e1.y;
+                acc[NR + r].x = fma(kr, xr, fma(-ki, xi, acc[NR + r].x));
+                acc[NR + r].y = fma(kr, xi, fma(ki, xr, acc[NR + r].y));
+            }
+            __syncwarp();
+        }
+        if (a.patch_of_row) {
+            const double2* Pv = (const double2*)a.patch_vals;
+#pragma unroll
+            for (int half = 0; half < 2; half++) {
+                const int pr = (half ? f1 : f0) ? a.patch_of_row[half ? i1 : i] : -1;
+                if (pr < 0) continue;
+                const int je = a.patch_rowptr[pr + 1];
+                for (int j = a.patch_rowptr[pr] + g; j < je; j += G) {
+                    const int q = a.patch_port[j];
+                    const double2 v = Pv[j];
+                    const T* xc = x + (long long)a.patch_cols[j] * S + s0;
+#pragma unroll
+                    for (int r = 0; r < NR; r++) {
+                        const T xv = xc[r * L];
+                        const double* gm = a.gamma + 2 * ((base + s0 + r * L) * a.n_ports + q);
+                        const double kr = gm[0] * v.x - gm[1] * v.y, ki = gm[0] * v.y + gm[1] * v.x;
+                        acc[half * NR + r].x += kr * xv.x - ki * xv.y;
+                        acc[half * NR + r].y += kr * xv.y + ki * xv.x;
+                    }
+                }
+            }
+        }
+        const int r0 = pair_reduce<L, NR>(acc, lane);
+        const bool hi = lane & 16;
+        // lane groups that hold copies of a value already written by another group have a bit of L..8 set
+        const bool own = NR > 1 || (lane & 15 & ~(L - 1)) == 0;
+        if (own && (two || !hi)) {
+            const long long row = hi ? i1 : i;
+#pragma unroll
+            for (int q = 0; q < NV; q++) {
+                const long long o = row * S + s0 + (r0 + q) * L;
+                const double yr = acc[q].x, yi = acc[q].y;
+                y[o] = mk2<R>((R)yr, (R)yi);
+                if (dotmode == DOT_XY) {
+                    T xi = x[o];
+                    c0[q].x += (double)xi.x * yr - (double)xi.y * yi;
+                    c0[q].y += (double)xi.x * yi + (double)xi.y * yr;
+                } else if (dotmode == DOT_CONJW_Y) {
+                    T wi = w[o];
+                    c0[q].x += (double)wi.x * yr + (double)wi.y * yi;
+                    c0[q].y += (double)wi.x * yi - (double)wi.y * yr;
+                } else if (dotmode == DOT_CONJY_W_YY) {
+                    T wi = w[o];
+                    c0[q].x += yr * wi.x + yi * wi.y;
+                    c0[q].y += yr * wi.y - yi * wi.x;
+                    c1[q] += yr * yr + yi * yi;
+                    c2[q] += nrm2(wi);
+                }
+            }
+        }
+    }
+    if (dotmode == DOT_NONE) return;
+    // per warp and system: row 0 + row 1, then the warps in order
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    __syncthreads();                                 // the stages are free: the warps' sums take their place
+    typedef double2 WarpSums[L * NR];
+    WarpSums* r0s = reinterpret_cast<WarpSums*>(spmv_sm);
+    WarpSums* r1s = r0s + VB / 32;
+    const int rr0 = NR > 1 && L == 8 && (lane & 8) ? NR / 2 : 0;
+#pragma unroll
+    for (int q = 0; q < NV; q++) {
+        c0[q].x += __shfl_xor_sync(0xffffffffu, c0[q].x, 16);
+        c0[q].y += __shfl_xor_sync(0xffffffffu, c0[q].y, 16);
+        c1[q] += __shfl_xor_sync(0xffffffffu, c1[q], 16);
+        c2[q] += __shfl_xor_sync(0xffffffffu, c2[q], 16);
+        if ((NR > 1 || (lane & 15 & ~(L - 1)) == 0) && !(lane & 16)) {
+            r0s[wl][lane % L + (rr0 + q) * L] = c0[q];
+            r1s[wl][lane % L + (rr0 + q) * L] = make_double2(c1[q], c2[q]);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < L * NR) {
+        double2 t0 = make_double2(0.0, 0.0), t1 = t0;
+#pragma unroll
+        for (int q = 0; q < VB / 32; q++) {
+            t0.x += r0s[q][threadIdx.x].x; t0.y += r0s[q][threadIdx.x].y;
+            t1.x += r1s[q][threadIdx.x].x; t1.y += r1s[q][threadIdx.x].y;
+        }
+        const long long nb = gridDim.x;
+        const int s = blockIdx.y * (L * NR) + threadIdx.x;
+        partial[s * nb + blockIdx.x] = t0;
+        if (dotmode == DOT_CONJY_W_YY) {
+            partial[(S + s) * nb + blockIdx.x] = make_double2(t1.x, 0.0);
+            partial[(2 * S + s) * nb + blockIdx.x] = make_double2(t1.y, 0.0);
+        }
+    }
+}
+
+static unsigned spmv_blocks(long long n, int S) { return grid_for((n + 1) / 2, spmv_pairs(S)); }
+static unsigned vec_blocks(long long h, int S) { return grid_for(h, vec_pairs(S)); }
+
+template <typename R, bool HASB>
+static void launch_spmv_b(const OpArgs& a, const typename V2<R>::T* x, typename V2<R>::T* y, double2* partial, int dotmode,
+                          const typename V2<R>::T* w, cudaStream_t s) {
+    dim3 grid(spmv_blocks(a.n, a.S), a.S > 32 ? a.S / 32 : 1);
+#define EMFEM_SPMV(L, NR)                                                                                      \
+    do {                                                                                                       \
+        constexpr size_t sm = sizeof(SpmvStage<R, L, NR, HASB>) * SpmvStage<R, L, NR, HASB>::DEPTH * (VB / 32);                                                  \
+        if (sm > 48 * 1024)                                                                                    \
+            cudaFuncSetAttribute(spmv_kernel<R, L, NR, HASB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm); \
+        spmv_kernel<R, L, NR, HASB><<<grid, VB, sm, s>>>(a, x, y, partial, dotmode, w);                        \
+    } while (0)
+    switch (a.S) {
+    case 1: EMFEM_SPMV(1, 1); break;
+    case 2: EMFEM_SPMV(2, 1); break;
+    case 4: EMFEM_SPMV(4, 1); break;
+    case 8: EMFEM_SPMV(8, 1); break;
+    case 16: EMFEM_SPMV(8, 2); break;
+    default: EMFEM_SPMV(8, 4); break;
+    }
+#undef EMFEM_SPMV
+}
+template <typename R>
+static void launch_spmv(const OpArgs& a, const typename V2<R>::T* x, typename V2<R>::T* y, double2* partial, int dotmode,
+                        const typename V2<R>::T* w, cudaStream_t s) {
+    if (a.B) launch_spmv_b<R, true>(a, x, y, partial, dotmode, w, s);
+    else launch_spmv_b<R, false>(a, x, y, partial, dotmode, w, s);
+}
+
+// y[row] += sum_q gamma_q R_q x on the patch rows (a warp per patch row, lanes over (entry group, system)):
+// the Robin terms of an SpMV that keeps no row -> patch row map.
+__global__ void __launch_bounds__(VB) patch_rows_kernel(long long np, const int* __restrict__ rows, OpArgs a,
+                                                        const double2* __restrict__ x, double2* __restrict__ y) {
+    const int lane = threadIdx.x & 31;
+    const long long p = ((long long)blockIdx.x * VB + threadIdx.x) >> 5;
+    if (p >= np) return;
+    const long long row = rows[p];
+    if (!a.mask[row]) return;
+    const int S = a.S, L = S < 32 ? S : 32, g = lane / L, G = 32 / L;
+    const double2* Pv = (const double2*)a.patch_vals;
+    for (int s = lane % L; s < S; s += L) {
+        double2 acc = make_double2(0.0, 0.0);
+        for (int j = a.patch_rowptr[p] + g; j < a.patch_rowptr[p + 1]; j += G) {
+            const double2 v = Pv[j], xv = x[(long long)a.patch_cols[j] * S + s];
+            const double* gm = a.gamma + 2 * (s * a.n_ports + a.patch_port[j]);
+            const double kr = gm[0] * v.x - gm[1] * v.y, ki = gm[0] * v.y + gm[1] * v.x;
+            acc.x += kr * xv.x - ki * xv.y;
+            acc.y += kr * xv.y + ki * xv.x;
+        }
+        for (int off = 16; off >= L; off >>= 1) {
+            acc.x += __shfl_xor_sync(0xffffffffu, acc.x, off);
+            acc.y += __shfl_xor_sync(0xffffffffu, acc.y, off);
+        }
+        if (g == 0) {
+            double2 v = y[row * S + s];
+            y[row * S + s] = make_double2(v.x + acc.x, v.y + acc.y);
+        }
+    }
 }
 
 // Solver state per system (device).
@@ -304,39 +501,48 @@ __device__ void stop(SysState& q, int status) {
     q.alpha = make_double2(0, 0); q.omega = make_double2(0, 0); q.beta = make_double2(0, 0);
 }
 
-// One block per system: fixed-order sum of the block partials, then the scalar recurrences.
-// Grouped systems (G > 1): block sys = g S + s sums only group g's blocks, gblk[g] .. gblk[g + 1] of
-// a DOF-pair launch (nbh blocks), and for a launch over all rows also the same range in the second
-// half (two_halves).
+// One block per system: fixed-order sum of the block partials (contiguous per component and system), then
+// the scalar recurrences.  Grouped systems (G > 1): block sys = g S + s sums only group g's blocks, those
+// of the pairs gpair[g] .. gpair[g + 1] (ppb pairs per block of the launch that wrote the partials).
 __global__ void reduce_update_kernel(const double2* __restrict__ partial, int nblocks, int S, int ncomp,
-                                     SysState* st, int mode, int maxit, double tol, int nsys, int G = 1,
-                                     const int* __restrict__ gblk = nullptr, int two_halves = 0, int nbh = 0) {
-    __shared__ double2 red[VB];
+                                     SysState* st, int mode, int maxit, double tol, int nsys, int G, int ppb,
+                                     const int* __restrict__ gpair) {
+    __shared__ double2 red[VB / 32][3];
     __shared__ double2 sums[3];
     const int sys = blockIdx.x;
     const int s = G > 1 ? sys % S : sys;
-    int b0 = 0, cnt = nblocks, total = nblocks;
+    int b0 = 0, b1 = nblocks;
     if (G > 1) {
-        b0 = gblk[sys / S];
-        cnt = gblk[sys / S + 1] - b0;
-        total = two_halves ? 2 * cnt : cnt;
+        b0 = gpair[sys / S] / ppb;
+        b1 = gpair[sys / S + 1] / ppb;
     }
-    for (int comp = 0; comp < ncomp; comp++) {
-        double2 acc = make_double2(0, 0);
-        for (int k = threadIdx.x; k < total; k += VB) {
-            int b = k < cnt ? b0 + k : nbh + b0 + (k - cnt);
-            double2 v = partial[((long long)comp * nblocks + b) * S + s];
-            acc.x += v.x; acc.y += v.y;
-        }
-        red[threadIdx.x] = acc;
-        __syncthreads();
-        for (int off = VB / 2; off > 0; off >>= 1) {
-            if (threadIdx.x < off) { red[threadIdx.x].x += red[threadIdx.x + off].x; red[threadIdx.x].y += red[threadIdx.x + off].y; }
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) sums[comp] = red[0];
-        __syncthreads();
+    double2 acc[3];
+#pragma unroll
+    for (int comp = 0; comp < 3; comp++) acc[comp] = make_double2(0, 0);
+    for (int k = b0 + threadIdx.x; k < b1; k += VB) {
+#pragma unroll
+        for (int comp = 0; comp < 3; comp++)
+            if (comp < ncomp) {
+                double2 v = partial[((long long)comp * S + s) * nblocks + k];
+                acc[comp].x += v.x; acc[comp].y += v.y;
+            }
     }
+#pragma unroll
+    for (int comp = 0; comp < 3; comp++) {
+        if (comp < ncomp)
+            for (int off = 16; off > 0; off >>= 1) {
+                acc[comp].x += __shfl_down_sync(0xffffffffu, acc[comp].x, off);
+                acc[comp].y += __shfl_down_sync(0xffffffffu, acc[comp].y, off);
+            }
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][comp] = acc[comp];
+    }
+    __syncthreads();
+    if (threadIdx.x < ncomp) {
+        double2 t = make_double2(0, 0);
+        for (int q = 0; q < VB / 32; q++) { t.x += red[q][threadIdx.x].x; t.y += red[q][threadIdx.x].y; }
+        sums[threadIdx.x] = t;
+    }
+    __syncthreads();
     if (threadIdx.x != 0) return;
     SysState& q = st[sys];
     double2 c0 = sums[0], c1 = ncomp > 1 ? sums[1] : make_double2(0, 0);
@@ -432,17 +638,17 @@ __global__ void __launch_bounds__(VB) cocg_init_kernel(long long h, int S, int p
                                                        typename V2<R>::T* __restrict__ z, typename V2<R>::T* __restrict__ p,
                                                        const typename V2<R>::T* __restrict__ minv, double2* __restrict__ partial) {
     typedef typename V2<R>::T T;
-    long long g = (long long)blockIdx.x * VB + threadIdx.x;
-    long long i = g / S;
-    int s = (int)(g % S);
+    const int s = threadIdx.x % S;
     double2 rz = make_double2(0, 0);
-    if (i < h) {
+    for (int q = threadIdx.x / S; q < vec_pairs(S); q += VB / S) {
+        const long long i = (long long)blockIdx.x * vec_pairs(S) + q;
+        if (i >= h) break;
         T rl = r[i * S + s], rh = r[(i + h) * S + s], zl, zh;
         apply_pair<R>(precond, minv, S, i, s, rl, rh, zl, zh);
         z[i * S + s] = zl; z[(i + h) * S + s] = zh;
         p[i * S + s] = zl; p[(i + h) * S + s] = zh;
         double2 a = dotu(rl, zl), b = dotu(rh, zh);
-        rz = make_double2(a.x + b.x, a.y + b.y);
+        rz.x += a.x + b.x; rz.y += a.y + b.y;
     }
     block_store2(rz, rz, 1, S, partial);
 }
@@ -455,12 +661,14 @@ __global__ void __launch_bounds__(VB) cocg_update_kernel(long long h, int S, int
                                                          const typename V2<R>::T* __restrict__ q, const typename V2<R>::T* __restrict__ minv,
                                                          double2* __restrict__ partial) {
     typedef typename V2<R>::T T;
-    long long g = (long long)blockIdx.x * VB + threadIdx.x;
-    long long i = g / S;
-    int s = (int)(g % S);
+    const int s = threadIdx.x % S;
     double2 rz = make_double2(0, 0), rr = make_double2(0, 0);
-    if (i < h && st[sys_of_row(pg, h, i, S, s)].active) {
-        double2 al = st[sys_of_row(pg, h, i, S, s)].alpha;
+    for (int qp = threadIdx.x / S; qp < vec_pairs(S); qp += VB / S) {
+        const long long i = (long long)blockIdx.x * vec_pairs(S) + qp;
+        if (i >= h) break;
+        const int sy = sys_of_row(pg, h, i, S, s);
+        if (!st[sy].active) continue;
+        double2 al = st[sy].alpha;
         R ar = (R)al.x, ai = (R)al.y;
         T rv2[2];
 #pragma unroll
@@ -475,8 +683,8 @@ __global__ void __launch_bounds__(VB) cocg_update_kernel(long long h, int S, int
         apply_pair<R>(precond, minv, S, i, s, rv2[0], rv2[1], zl, zh);
         z[i * S + s] = zl; z[(i + h) * S + s] = zh;
         double2 a = dotu(rv2[0], zl), b = dotu(rv2[1], zh);
-        rz = make_double2(a.x + b.x, a.y + b.y);
-        rr.x = nrm2(rv2[0]) + nrm2(rv2[1]);
+        rz.x += a.x + b.x; rz.y += a.y + b.y;
+        rr.x += nrm2(rv2[0]) + nrm2(rv2[1]);
     }
     block_store2(rz, rr, 2, S, partial);
 }
@@ -497,17 +705,23 @@ __global__ void cocg_pupdate_kernel(long long n, int S, const int* __restrict__ 
 // ---- BiCGStab vector kernels ----
 // r_hat = r, p = v = 0, partial (r_hat, r) = ||r||^2
 template <typename R>
-__global__ void __launch_bounds__(VB) bicg_init_kernel(long long n, int S, const typename V2<R>::T* __restrict__ r,
+__global__ void __launch_bounds__(VB) bicg_init_kernel(long long h, int S, const typename V2<R>::T* __restrict__ r,
                                                        typename V2<R>::T* __restrict__ rh, typename V2<R>::T* __restrict__ p,
                                                        typename V2<R>::T* __restrict__ v, double2* __restrict__ partial) {
-    long long g = (long long)blockIdx.x * VB + threadIdx.x;
+    const int s = threadIdx.x % S;
     double2 c = make_double2(0, 0);
-    if (g < n * S) {
-        typename V2<R>::T rv = r[g];
-        rh[g] = rv;
-        p[g] = mk2<R>(0, 0);
-        v[g] = mk2<R>(0, 0);
-        c.x = nrm2(rv);
+    for (int q = threadIdx.x / S; q < vec_pairs(S); q += VB / S) {
+        const long long i = (long long)blockIdx.x * vec_pairs(S) + q;
+        if (i >= h) break;
+#pragma unroll
+        for (int half = 0; half < 2; half++) {
+            const long long g = (i + half * h) * S + s;
+            typename V2<R>::T rv = r[g];
+            rh[g] = rv;
+            p[g] = mk2<R>(0, 0);
+            v[g] = mk2<R>(0, 0);
+            c.x += nrm2(rv);
+        }
     }
     block_store2(c, c, 1, S, partial);
 }
@@ -577,28 +791,36 @@ __global__ void __launch_bounds__(VB) bicg_s_kernel(long long h, int S, int prec
 
 // x += alpha p_hat + omega s_hat; r = s - omega t; partial (r_hat, r) and ||r||^2
 template <typename R>
-__global__ void __launch_bounds__(VB) bicg_x_kernel(long long n, int S, const int* __restrict__ pg,
+__global__ void __launch_bounds__(VB) bicg_x_kernel(long long h, int S, const int* __restrict__ pg,
                                                     const SysState* __restrict__ st,
                                                     typename V2<R>::T* __restrict__ x, typename V2<R>::T* __restrict__ r,
                                                     const typename V2<R>::T* __restrict__ ph, const typename V2<R>::T* __restrict__ sh,
                                                     const typename V2<R>::T* __restrict__ t, const typename V2<R>::T* __restrict__ rh,
                                                     double2* __restrict__ partial) {
     typedef typename V2<R>::T T;
-    long long g = (long long)blockIdx.x * VB + threadIdx.x;
+    const int s = threadIdx.x % S;
     double2 c0 = make_double2(0, 0), c1 = c0;
-    const int sy = g < n * S ? sys_of_row(pg, n / 2, g / S, S, (int)(g % S)) : 0;
-    if (g < n * S && st[sy].active) {
+    for (int q = threadIdx.x / S; q < vec_pairs(S); q += VB / S) {
+        const long long i = (long long)blockIdx.x * vec_pairs(S) + q;
+        if (i >= h) break;
+        const int sy = sys_of_row(pg, h, i, S, s);
+        if (!st[sy].active) continue;
         double2 a = st[sy].alpha, w = st[sy].omega;
         R ar = (R)a.x, ai = (R)a.y, wr = (R)w.x, wi = (R)w.y;
-        T xv = x[g], pv = ph[g], sv = sh[g], rv = r[g], tv = t[g];
-        xv.x += ar * pv.x - ai * pv.y + wr * sv.x - wi * sv.y;
-        xv.y += ar * pv.y + ai * pv.x + wr * sv.y + wi * sv.x;
-        rv.x -= wr * tv.x - wi * tv.y;
-        rv.y -= wr * tv.y + wi * tv.x;
-        x[g] = xv;
-        r[g] = rv;
-        c0 = dotc(rh[g], rv);
-        c1.x = nrm2(rv);
+#pragma unroll
+        for (int half = 0; half < 2; half++) {
+            const long long g = (i + half * h) * S + s;
+            T xv = x[g], pv = ph[g], sv = sh[g], rv = r[g], tv = t[g];
+            xv.x += ar * pv.x - ai * pv.y + wr * sv.x - wi * sv.y;
+            xv.y += ar * pv.y + ai * pv.x + wr * sv.y + wi * sv.x;
+            rv.x -= wr * tv.x - wi * tv.y;
+            rv.y -= wr * tv.y + wi * tv.x;
+            x[g] = xv;
+            r[g] = rv;
+            double2 d = dotc(rh[g], rv);
+            c0.x += d.x; c0.y += d.y;
+            c1.x += nrm2(rv);
+        }
     }
     block_store2(c0, c1, 2, S, partial);
 }
@@ -611,21 +833,26 @@ __global__ void mask_vec_kernel(long long n, int S, const uint8_t* mask, double2
 }
 
 // r = b - Ax on free DOFs; partials ||b||^2 and ||r||^2
-__global__ void __launch_bounds__(VB) residual_kernel(long long n, int S, const uint8_t* __restrict__ mask,
+__global__ void __launch_bounds__(VB) residual_kernel(long long h, int S, const uint8_t* __restrict__ mask,
                                                        const double2* __restrict__ b, const double2* __restrict__ Ax,
                                                        double2* __restrict__ r, double2* __restrict__ partial) {
-    long long g = (long long)blockIdx.x * VB + threadIdx.x;
+    const int s = threadIdx.x % S;
     double2 cb = make_double2(0, 0), cr = cb;
-    if (g < n * S) {
-        long long i = g / S;
-        double2 res = make_double2(0, 0);
-        if (mask[i]) {
-            double2 bv = b[g], av = Ax[g];
-            res = make_double2(bv.x - av.x, bv.y - av.y);
-            cb.x = bv.x * bv.x + bv.y * bv.y;
-            cr.x = res.x * res.x + res.y * res.y;
+    for (int q = threadIdx.x / S; q < vec_pairs(S); q += VB / S) {
+        const long long i = (long long)blockIdx.x * vec_pairs(S) + q;
+        if (i >= h) break;
+#pragma unroll
+        for (int half = 0; half < 2; half++) {
+            const long long row = i + half * h, g = row * S + s;
+            double2 res = make_double2(0, 0);
+            if (mask[row]) {
+                double2 bv = b[g], av = Ax[g];
+                res = make_double2(bv.x - av.x, bv.y - av.y);
+                cb.x += bv.x * bv.x + bv.y * bv.y;
+                cr.x += res.x * res.x + res.y * res.y;
+            }
+            r[g] = res;
         }
-        r[g] = res;
     }
     block_store2(cb, cr, 2, S, partial);
 }
@@ -801,7 +1028,7 @@ static int pow2_at_least(int v) {
 
 // ---- workspace layout ----------------------------------------------------------------------
 struct Layout {
-    size_t off_state, off_gamma, off_k0, off_partial, off_patchmap, off_scale, off_gblk;
+    size_t off_state, off_gamma, off_k0, off_partial, off_patchmap, off_scale, off_gpair;
     size_t off_x, off_b, off_r64, off_Ax;                  // FP64 vectors (n, S)
     size_t off_v[8];                                       // Krylov vectors of the inner precision
     size_t off_minv;
@@ -813,7 +1040,7 @@ static size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 static Layout make_layout(long long n, long long nnz, long long npatch, int S, int nports, int precision, int G = 1) {
     Layout L;
     size_t o = 0;
-    long long nb = (n * S + VB - 1) / VB + 1;
+    long long nb = n / 16 + 2;          // spmv_pairs >= 8 and vec_pairs >= 8 pairs per block
     size_t vec64 = (size_t)n * S * sizeof(double2);
     size_t vecw = (size_t)n * S * (precision ? sizeof(float2) : sizeof(double2));
     L.off_state = o; o = align256(o + sizeof(SysState) * 2 * S * G);
@@ -822,7 +1049,7 @@ static Layout make_layout(long long n, long long nnz, long long npatch, int S, i
     L.off_partial = o; o = align256(o + sizeof(double2) * 3 * nb * S);
     L.off_patchmap = o; o = align256(o + sizeof(int) * n);
     L.off_scale = o; o = align256(o + sizeof(double) * S * G);
-    L.off_gblk = o; o = align256(o + sizeof(int) * (G + 1));
+    L.off_gpair = o; o = align256(o + sizeof(int) * (G + 1));
     L.off_x = o; o = align256(o + vec64);
     L.off_b = o; o = align256(o + vec64);
     L.off_r64 = o; o = align256(o + vec64);
@@ -848,10 +1075,10 @@ struct Krylov {
     double2* partial = nullptr;
     SysState* st = nullptr;
     cudaStream_t s = nullptr;
-    // grouped systems: G groups of S systems, group of every DOF pair, group block ranges
+    // grouped systems: G groups of S systems, group of every DOF pair, group pair ranges
     int G = 1;
     const int* pg = nullptr;
-    const int* gblk = nullptr;
+    const int* gpair = nullptr;
     // auxiliary-space correction (precond 3: aux Jacobi, 4: learned network); BiCGStab only
     const emfem_aux_s* aux = nullptr;
     T* adinv = nullptr;
@@ -866,20 +1093,23 @@ struct Krylov {
     // vectors' precision (the dots accumulate in FP64); a looser FP32 threshold restarts so often
     // that the Krylov memory is lost
     double restart_eps = sizeof(R) == 8 ? 1e-9 : 1e-6;
-    void reduce(int ncomp, unsigned nblocks, int mode) {
+    void reduce(int ncomp, unsigned nblocks, int ppb, int mode) {
         reduce_update_kernel<<<G * S, VB, 0, s>>>(partial, (int)nblocks, S, ncomp, st, mode, maxit, restart_eps, nsys, G,
-                                                  gblk, nblocks != nb_pair() ? 1 : 0, (int)nb_pair());
+                                                  ppb, gpair);
     }
+    void reduce_spmv(int ncomp, int mode) { reduce(ncomp, spmv_blocks(n, S), spmv_pairs(S), mode); }
+    void reduce_vec(int ncomp, int mode) { reduce(ncomp, vec_blocks(h, S), vec_pairs(S), mode); }
+    void spmv(const T* in, T* out, int dotmode, const T* w) { launch_spmv<R>(op, in, out, partial, dotmode, w, s); }
 
     int start() {
         if (method == 0) {
             T *z = v[0], *p = v[1];
-            cocg_init_kernel<R><<<nb_pair(), VB, 0, s>>>(h, S, precond, r, z, p, minv, partial);
-            reduce(1, nb_pair(), UPD_SET_RHO);
+            cocg_init_kernel<R><<<vec_blocks(h, S), VB, 0, s>>>(h, S, precond, r, z, p, minv, partial);
+            reduce_vec(1, UPD_SET_RHO);
         } else {
             T *rh = v[0], *p = v[1], *vv = v[2];
-            bicg_init_kernel<R><<<nb_all(), VB, 0, s>>>(n, S, r, rh, p, vv, partial);
-            reduce(1, nb_all(), UPD_SET_RHO);
+            bicg_init_kernel<R><<<vec_blocks(h, S), VB, 0, s>>>(h, S, r, rh, p, vv, partial);
+            reduce_vec(1, UPD_SET_RHO);
         }
         return check_cuda(cudaGetLastError(), "krylov start");
     }
@@ -887,10 +1117,10 @@ struct Krylov {
     int iteration() {
         if (method == 0) {
             T *z = v[0], *p = v[1], *q = v[2];
-            spmv_kernel<R><<<nb_all(), VB, 0, s>>>(op, p, q, partial, DOT_XY, nullptr);
-            reduce(1, nb_all(), UPD_COCG_ALPHA);
-            cocg_update_kernel<R><<<nb_pair(), VB, 0, s>>>(h, S, precond, pg, st, x, r, z, p, q, minv, partial);
-            reduce(2, nb_pair(), UPD_COCG_BETA);
+            spmv(p, q, DOT_XY, nullptr);
+            reduce_spmv(1, UPD_COCG_ALPHA);
+            cocg_update_kernel<R><<<vec_blocks(h, S), VB, 0, s>>>(h, S, precond, pg, st, x, r, z, p, q, minv, partial);
+            reduce_vec(2, UPD_COCG_BETA);
             cocg_pupdate_kernel<R><<<nb_all(), VB, 0, s>>>(n, S, pg, st, z, p);
         } else {
             T *rh = v[0], *p = v[1], *vv = v[2], *ph = v[3], *sh = v[4], *t = v[5];
@@ -899,17 +1129,17 @@ struct Krylov {
             if constexpr (sizeof(R) == 8) {
                 if (mf) EMFEM_TRY(mf_apply(mf, S, (const double2*)p, (double2*)ph, s));
             }
-            spmv_kernel<R><<<nb_all(), VB, 0, s>>>(op, ph, vv, partial, DOT_CONJW_Y, rh);
-            reduce(1, nb_all(), UPD_BICG_ALPHA);
+            spmv(ph, vv, DOT_CONJW_Y, rh);
+            reduce_spmv(1, UPD_BICG_ALPHA);
             bicg_s_kernel<R><<<nb_pair(), VB, 0, s>>>(h, S, bj(), pg, st, r, vv, sh, minv);
             if (aux) EMFEM_TRY(aux_correct<T>(aux, S, precond == 4, adinv, r, op.mask, sh, s));
             if constexpr (sizeof(R) == 8) {
                 if (mf) EMFEM_TRY(mf_apply(mf, S, (const double2*)r, (double2*)sh, s));
             }
-            spmv_kernel<R><<<nb_all(), VB, 0, s>>>(op, sh, t, partial, DOT_CONJY_W_YY, r);
-            reduce(3, nb_all(), UPD_BICG_OMEGA);
-            bicg_x_kernel<R><<<nb_all(), VB, 0, s>>>(n, S, pg, st, x, r, ph, sh, t, rh, partial);
-            reduce(2, nb_all(), UPD_BICG_RHO);
+            spmv(sh, t, DOT_CONJY_W_YY, r);
+            reduce_spmv(3, UPD_BICG_OMEGA);
+            bicg_x_kernel<R><<<vec_blocks(h, S), VB, 0, s>>>(h, S, pg, st, x, r, ph, sh, t, rh, partial);
+            reduce_vec(2, UPD_BICG_RHO);
         }
         return check_cuda(cudaGetLastError(), "krylov iteration");
     }
@@ -997,20 +1227,16 @@ int emfem_sweep_spmv(emfem_handle h, int64_t n, const int32_t* indptr, const int
                   "emfem_sweep_spmv: nsys must be a power of two <= 256");
     EMFEM_REQUIRE(n_patch_rows == 0 || (patch_rows && patch_rowptr && patch_cols && patch_vals && patch_port && gamma_dev),
                   "emfem_sweep_spmv: patch arrays missing");
-    int* pmap = nullptr;
-    if (n_patch_rows > 0) {
-        EMFEM_CUDA(cudaMallocAsync(&pmap, sizeof(int) * n, h->h.stream));
-        EMFEM_CUDA(cudaMemsetAsync(pmap, 0xff, sizeof(int) * n, h->h.stream));
-        patch_map_kernel<<<grid_for(n_patch_rows, VB), VB, 0, h->h.stream>>>(n_patch_rows, patch_rows, pmap);
-        EMFEM_LAUNCH("patch_map_kernel");
-    }
     OpArgs a;
-    build_op(a, n, nsys, indptr, indices, E_vals, B_vals, k0sq_dev, pmap, patch_rowptr, patch_cols, patch_vals,
+    build_op(a, n, nsys, indptr, indices, E_vals, B_vals, k0sq_dev, nullptr, patch_rowptr, patch_cols, patch_vals,
              patch_port, n_ports, gamma_dev, free_mask);
-    spmv_kernel<double><<<grid_for(n * nsys, VB), VB, 0, h->h.stream>>>(a, (const double2*)x, (double2*)y, nullptr,
-                                                                          DOT_NONE, nullptr);
+    launch_spmv<double>(a, (const double2*)x, (double2*)y, nullptr, DOT_NONE, nullptr, h->h.stream);
     EMFEM_LAUNCH("spmv_kernel");
-    if (pmap) EMFEM_CUDA(cudaFreeAsync(pmap, h->h.stream));
+    if (n_patch_rows > 0) {
+        patch_rows_kernel<<<grid_for(n_patch_rows * 32, VB), VB, 0, h->h.stream>>>(n_patch_rows, patch_rows, a,
+                                                                                    (const double2*)x, (double2*)y);
+        EMFEM_LAUNCH("patch_rows_kernel");
+    }
     return EMFEM_OK;
 }
 
@@ -1058,7 +1284,7 @@ static int krylov_impl(emfem_handle hd, int method, int64_t n, int64_t nnz, cons
                   "emfem_krylov_solve_lu: call emfem_mf_reserve with at least the padded batch size first");
     EMFEM_REQUIRE(precond < 3 || precond == 5 || aux->kbuf_bytes >= aux_solve_bytes(aux, S),
                   "emfem_krylov_solve: call emfem_aux_reserve with at least nsys systems first");
-    std::vector<int> hgblk(G + 1, 0);
+    std::vector<int> hgpair(G + 1, 0);
     if (G > 1) {
         EMFEM_REQUIRE(pair_group, "emfem_krylov_solve_grouped: pair_group required");
         EMFEM_REQUIRE((n / 2) % VB == 0, "emfem_krylov_solve_grouped: n/2 must be a multiple of 256");
@@ -1072,11 +1298,11 @@ static int krylov_impl(emfem_handle hd, int method, int64_t n, int64_t nnz, cons
             EMFEM_REQUIRE(v == prev + 1 && v < G && i % VB == 0,
                           "emfem_krylov_solve_grouped: pair_group must run through 0..G-1 in order, each group "
                           "starting at a multiple of 256 pairs");
-            hgblk[v] = (int)(i * S / VB);
+            hgpair[v] = (int)i;
             prev = v;
         }
         EMFEM_REQUIRE(prev == G - 1, "emfem_krylov_solve_grouped: every group needs at least one DOF pair");
-        hgblk[G] = (int)((n / 2) * S / VB);
+        hgpair[G] = (int)(n / 2);
     }
     Layout L = make_layout(n, nnz, npatch, S, n_ports, precision, G);
     size_t need = make_layout(n, nnz, nnz, S, 8, precision, G).total;
@@ -1095,8 +1321,8 @@ static int krylov_impl(emfem_handle hd, int method, int64_t n, int64_t nnz, cons
     }
     SysState* st = (SysState*)(ws + L.off_state);
     SysState* st_outer = st + (size_t)G * S;
-    int* gblk = (int*)(ws + L.off_gblk);
-    const int nbh = (int)grid_for((n / 2) * (long long)S, VB);
+    int* gpair = (int*)(ws + L.off_gpair);
+    const unsigned nbv = vec_blocks(n / 2, S);
     double* gdev = (double*)(ws + L.off_gamma);
     double* k0dev = (double*)(ws + L.off_k0);
     double2* partial = (double2*)(ws + L.off_partial);
@@ -1123,7 +1349,7 @@ static int krylov_impl(emfem_handle hd, int method, int64_t n, int64_t nnz, cons
     STRY(check_cuda(cudaEventRecord(ev, h->stream), "event"));
     STRY(check_cuda(cudaStreamWaitEvent(s, ev, 0), "wait"));
     STRY(check_cuda(cudaMemcpyAsync(k0dev, hk0.data(), sizeof(double) * hk0.size(), cudaMemcpyHostToDevice, s), "copy k0"));
-    STRY(check_cuda(cudaMemcpyAsync(gblk, hgblk.data(), sizeof(int) * (G + 1), cudaMemcpyHostToDevice, s), "copy gblk"));
+    STRY(check_cuda(cudaMemcpyAsync(gpair, hgpair.data(), sizeof(int) * (G + 1), cudaMemcpyHostToDevice, s), "copy gpair"));
     STRY(check_cuda(cudaMemcpyAsync(gdev, hg.data(), sizeof(double) * hg.size(), cudaMemcpyHostToDevice, s), "copy gamma"));
     STRY(check_cuda(cudaMemsetAsync(pmap, 0xff, sizeof(int) * n, s), "memset"));
     if (n_patch_rows > 0) {
@@ -1139,9 +1365,10 @@ static int krylov_impl(emfem_handle hd, int method, int64_t n, int64_t nnz, cons
              patch_cols, patch_vals, patch_port, n_ports, gdev, free_mask);
     if (G > 1) op64.pg = pair_group;
     // initial residual r64 = b - A x0 and the outer state (||b||, tolerance, active)
-    spmv_kernel<double><<<gv, VB, 0, s>>>(op64, x64, Ax, nullptr, DOT_NONE, nullptr);
-    residual_kernel<<<gv, VB, 0, s>>>(n, S, free_mask, b64, Ax, r64, partial);
-    reduce_update_kernel<<<G * S, VB, 0, s>>>(partial, (int)gv, S, 2, st_outer, UPD_INIT, maxit, tol, nsys, G, gblk, 1, nbh);
+    launch_spmv<double>(op64, x64, Ax, nullptr, DOT_NONE, nullptr, s);
+    residual_kernel<<<nbv, VB, 0, s>>>(n / 2, S, free_mask, b64, Ax, r64, partial);
+    reduce_update_kernel<<<G * S, VB, 0, s>>>(partial, (int)nbv, S, 2, st_outer, UPD_INIT, maxit, tol, nsys, G,
+                                              vec_pairs(S), gpair);
     STRY(check_cuda(cudaGetLastError(), "initial residual"));
 
     if (precision == 0) {
@@ -1151,7 +1378,7 @@ static int krylov_impl(emfem_handle hd, int method, int64_t n, int64_t nnz, cons
         for (int q = 0; q < 7; q++) k.v[q] = (double2*)(ws + L.off_v[q]);
         k.partial = partial; k.st = st; k.s = s;
         k.op.skip = st;
-        k.G = G; k.pg = G > 1 ? pair_group : nullptr; k.gblk = gblk;
+        k.G = G; k.pg = G > 1 ? pair_group : nullptr; k.gpair = gpair;
         if (k.bj()) {
             precond_setup_kernel<double><<<grid_for((n / 2) * (long long)S, VB), VB, 0, s>>>(op64, k.bj(), k.minv);
             STRY(check_cuda(cudaGetLastError(), "precond_setup"));
@@ -1163,8 +1390,8 @@ static int krylov_impl(emfem_handle hd, int method, int64_t n, int64_t nnz, cons
         }
         k.mf = mf;
         // the recurrence tolerance is half the requested one so the FP64 true residual meets it
-        reduce_update_kernel<<<G * S, VB, 0, s>>>(partial, (int)gv, S, 2, st, UPD_INIT, maxit, 0.5 * tol, nsys, G, gblk, 1,
-                                                  nbh);
+        reduce_update_kernel<<<G * S, VB, 0, s>>>(partial, (int)nbv, S, 2, st, UPD_INIT, maxit, 0.5 * tol, nsys, G,
+                                              vec_pairs(S), gpair);
         STRY(check_cuda(cudaGetLastError(), "init state"));
         STRY(k.start());
         STRY(k.run(mf ? 2 : 16));     // an LU application is ~1000 launches: short captured chunks
@@ -1178,7 +1405,7 @@ static int krylov_impl(emfem_handle hd, int method, int64_t n, int64_t nnz, cons
         for (int q = 0; q < 6; q++) k.v[q] = (float2*)(ws + L.off_v[q]);
         k.partial = partial; k.st = st; k.s = s;
         k.op.skip = st;
-        k.G = G; k.pg = G > 1 ? pair_group : nullptr; k.gblk = gblk;
+        k.G = G; k.pg = G > 1 ? pair_group : nullptr; k.gpair = gpair;
         const int* pgk = k.pg;
         const size_t GSm = (size_t)G * S;
         if (precond) {
@@ -1212,10 +1439,11 @@ static int krylov_impl(emfem_handle hd, int method, int64_t n, int64_t nnz, cons
             for (size_t q = 0; q < GSm; q++) if (ho[q].active) mx = std::max(mx, hin[q].iters);
             used += mx;
             add_scaled_f32_kernel<<<gv, VB, 0, s>>>(n, S, pgk, d32, scale, st_outer, x64);
-            spmv_kernel<double><<<gv, VB, 0, s>>>(op64, x64, Ax, nullptr, DOT_NONE, nullptr);
-            residual_kernel<<<gv, VB, 0, s>>>(n, S, free_mask, b64, Ax, r64, partial);
+            launch_spmv<double>(op64, x64, Ax, nullptr, DOT_NONE, nullptr, s);
+            residual_kernel<<<nbv, VB, 0, s>>>(n / 2, S, free_mask, b64, Ax, r64, partial);
             // the inner state array is free now: reuse it to reduce ||b||^2, ||r||^2 of the new residual
-            reduce_update_kernel<<<G * S, VB, 0, s>>>(partial, (int)gv, S, 2, st, UPD_INIT, maxit, 1.0, S, G, gblk, 1, nbh);
+            reduce_update_kernel<<<G * S, VB, 0, s>>>(partial, (int)nbv, S, 2, st, UPD_INIT, maxit, 1.0, S, G,
+                                              vec_pairs(S), gpair);
             STRY(check_cuda(cudaGetLastError(), "refinement"));
             std::vector<SysState> hr(GSm);
             STRY(check_cuda(cudaMemcpyAsync(hr.data(), st, sizeof(SysState) * GSm, cudaMemcpyDeviceToHost, s), "copy"));
@@ -1254,9 +1482,10 @@ static int krylov_impl(emfem_handle hd, int method, int64_t n, int64_t nnz, cons
         const size_t GS = (size_t)G * S;
         std::vector<SysState> hs(GS);
         STRY(check_cuda(cudaMemcpyAsync(hs.data(), st, sizeof(SysState) * GS, cudaMemcpyDeviceToHost, s), "copy"));
-        spmv_kernel<double><<<gv, VB, 0, s>>>(op64, x64, Ax, nullptr, DOT_NONE, nullptr);
-        residual_kernel<<<gv, VB, 0, s>>>(n, S, free_mask, b64, Ax, r64, partial);
-        reduce_update_kernel<<<G * S, VB, 0, s>>>(partial, (int)gv, S, 2, st_outer, UPD_INIT, maxit, tol, S, G, gblk, 1, nbh);
+        launch_spmv<double>(op64, x64, Ax, nullptr, DOT_NONE, nullptr, s);
+        residual_kernel<<<nbv, VB, 0, s>>>(n / 2, S, free_mask, b64, Ax, r64, partial);
+        reduce_update_kernel<<<G * S, VB, 0, s>>>(partial, (int)nbv, S, 2, st_outer, UPD_INIT, maxit, tol, S, G,
+                                              vec_pairs(S), gpair);
         unpad_copy_kernel<<<grid_for(n * (long long)nsys, VB), VB, 0, s>>>(n, nsys, S, x64, (double2*)x);
         STRY(check_cuda(cudaGetLastError(), "final residual"));
         std::vector<SysState> hf(GS);
@@ -1445,8 +1674,7 @@ extern "C" int emfem_sweep_spmv_noalloc(emfem_handle h, int64_t n, const int32_t
         OpArgs a;
         build_op(a, n, nsys, indptr, indices, E_vals, B_vals, k0sq_dev, pmap, patch_rowptr, patch_cols, patch_vals,
                  patch_port, n_ports, gamma_dev, free_mask);
-        spmv_kernel<double><<<grid_for(n * nsys, VB), VB, 0, h->h.stream>>>(a, (const double2*)x, (double2*)y, nullptr,
-                                                                              DOT_NONE, nullptr);
+        launch_spmv<double>(a, (const double2*)x, (double2*)y, nullptr, DOT_NONE, nullptr, h->h.stream);
         rc = check_cuda(cudaGetLastError(), "spmv_kernel");
     }
     if (prev != h->h.device) cudaSetDevice(prev);
