@@ -16,16 +16,18 @@
 //      4 x 4 complex register tiles per thread), every kernel batched over the level's fronts;
 //   3. the factor columns, the U block row and the Schur complement are copied out of the level
 //      workspace (compact_kernel): factors to the factor store (rounded to complex64), the Schur
-//      complement to the update store (front precision) until the parent's level consumes it.
+//      complement to the update store (front precision) until the parent's level consumes it;
+//   4. the 256 x 256 diagonal blocks of the factor store are replaced by the blocks of their L and U
+//      inverses (block_inverse_kernel), so that the solves have no 32-step chains.
 // Pivoting stays inside each 32-row diagonal block (rows are never exchanged across blocks), so row swaps
 // touch only the block row; the solves apply them step by step.  A pivot smaller than 1e-6 of its block's
 // largest entry is raised to that floor and counted: the factorization is a preconditioner under an FP64
 // Krylov iteration, which removes such perturbations.
 //
 // Solves (M^-1 r for S right-hand sides, FP64 in and out, FP32 inside, scaled by D^-1/2 on the way in
-// and out) run the same tree: forward in level order (gather, children's update vectors, blocked L solve
-// with 256-row blocks, update vector for the parent), backward in reverse (gather of the solved boundary,
-// U12 product, blocked U solve).
+// and out) run the same tree: forward in level order (gather of the right-hand side and the children's
+// update rows, then per 256 own rows the product with the block inverse and the update of the rows below),
+// backward in reverse (U12 product with the solved boundary, then per 256 own rows, from the last).
 #include "emfem_internal.cuh"
 
 #include <algorithm>
@@ -111,7 +113,7 @@ struct FrontMeta {        // per front, device
     long long fdof, ea, asm0, asm1;   // offsets into fdof / ea / asm arrays
     long long fact, inv, piv;         // factor store offsets (float2 / float2 / int)
     long long ws, upd;                // level workspace (float2) / update store (float2) offsets
-    long long wv, uv, y;              // solve buffers: level w (rows), update vectors (rows), own solution (rows)
+    long long wv, y;                  // solve buffers: the front's rows of w, its own rows of y
 };
 
 // ---------------------------------------------------------------- factorization kernels
@@ -459,6 +461,83 @@ __global__ void mf_compact_kernel(const int* __restrict__ lst, const FrontMeta* 
     }
 }
 
+// Inverses of the 256 x 256 diagonal blocks of L and U, written over the factor store's copy of those blocks.
+// With the step's inverses A_j = Linv_j P_j (mf_diag_kernel) on the diagonal, block column j of the inverse
+// of the block-lower L is G_jj = A_j, G_ij = -A_i sum_{j <= t < i} L_it G_tj; that of U is H_jj = Uinv_j,
+// H_ij = -Uinv_i sum_{i < t <= j} U_it H_tj.  One CTA per (block column, L or U, 256-block, front): the
+// columns are independent, so nothing is serial but the at most 8 steps of one column.  Computed in the
+// front's precision from the workspace; the diagonal 32 x 32 blocks stay in the inverse store.
+constexpr int MF_NBB = MF_SB / MF_NB;
+template <typename T>
+struct MfInvSmem {
+    T x[MF_NBB][MF_NB][MF_NB + 1];       // the column's blocks, [block][row][column]
+    T a[MF_NB][MF_NB + 1];
+    T s[MF_NB][MF_NB + 1];
+};
+template <typename T>
+__global__ void __launch_bounds__(256) mf_block_inverse_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm,
+                                                               const T* __restrict__ ws, const T* __restrict__ invc,
+                                                               float2* __restrict__ fact) {
+    extern __shared__ __align__(16) unsigned char mf_smem[];
+    MfInvSmem<T>& sm = *reinterpret_cast<MfInvSmem<T>*>(mf_smem);
+    const FrontMeta& f = fm[lst[blockIdx.z]];
+    const int k0 = blockIdx.y * MF_SB;
+    if (k0 >= f.e) return;
+    const int rows = min(MF_SB, f.e - k0), ns = (rows + MF_NB - 1) / MF_NB;
+    const int j = blockIdx.x >> 1;
+    const bool upper = blockIdx.x & 1;
+    if (j >= ns || (upper ? j == 0 : j == ns - 1)) return;       // no off-diagonal block in this column
+    const long long n = f.n;
+    const T* W = ws + f.ws + k0 + (long long)k0 * n;
+    const T* I = invc + f.inv + (long long)(k0 / MF_NB) * 2 * MF_NB * MF_NB;
+    float2* F = fact + f.fact + k0 + (long long)k0 * n;
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;   // thread: rows tx, tx + 16, columns ty, ty + 16
+    const T zero = CxT<T>::make(0.0, 0.0);
+    for (int t = tid; t < MF_NB * MF_NB; t += 256)
+        sm.x[j][t % MF_NB][t / MF_NB] = I[(long long)j * 2 * MF_NB * MF_NB + (upper ? MF_NB * MF_NB : 0) + t];
+    __syncthreads();
+    const int step = upper ? -1 : 1;
+    for (int i = j + step; upper ? i >= 0 : i < ns; i += step) {
+        T acc[2][2] = {{zero, zero}, {zero, zero}};
+        for (int t = j; t != i; t += step) {
+            for (int q = tid; q < MF_NB * MF_NB; q += 256) {
+                const int r = q % MF_NB, c = q / MF_NB;
+                sm.a[r][c] = (i * MF_NB + r < rows && t * MF_NB + c < rows) ? W[i * MF_NB + r + (long long)(t * MF_NB + c) * n] : zero;
+            }
+            __syncthreads();
+#pragma unroll 8
+            for (int k = 0; k < MF_NB; k++) {
+                const T a0 = sm.a[tx][k], a1 = sm.a[tx + 16][k], b0 = sm.x[t][k][ty], b1 = sm.x[t][k][ty + 16];
+                cfma(acc[0][0], a0, b0); cfma(acc[0][1], a0, b1); cfma(acc[1][0], a1, b0); cfma(acc[1][1], a1, b1);
+            }
+            __syncthreads();
+        }
+#pragma unroll
+        for (int p = 0; p < 2; p++)
+#pragma unroll
+            for (int q = 0; q < 2; q++) sm.s[tx + 16 * p][ty + 16 * q] = acc[p][q];
+        for (int q = tid; q < MF_NB * MF_NB; q += 256)
+            sm.a[q % MF_NB][q / MF_NB] = I[(long long)i * 2 * MF_NB * MF_NB + (upper ? MF_NB * MF_NB : 0) + q];
+        __syncthreads();
+        T o[2][2] = {{zero, zero}, {zero, zero}};
+#pragma unroll 8
+        for (int k = 0; k < MF_NB; k++) {
+            const T a0 = sm.a[tx][k], a1 = sm.a[tx + 16][k], b0 = sm.s[k][ty], b1 = sm.s[k][ty + 16];
+            cfms(o[0][0], a0, b0); cfms(o[0][1], a0, b1); cfms(o[1][0], a1, b0); cfms(o[1][1], a1, b1);
+        }
+#pragma unroll
+        for (int p = 0; p < 2; p++)
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                const int r = tx + 16 * p, c = ty + 16 * q;
+                sm.x[i][r][c] = o[p][q];
+                if (i * MF_NB + r < rows && j * MF_NB + c < rows)
+                    F[i * MF_NB + r + (long long)(j * MF_NB + c) * n] = to_c64(o[p][q]);
+            }
+        __syncthreads();
+    }
+}
+
 // ---------------------------------------------------------------- assembly lists on the device
 // Every CSR entry (r, c) of the free rows and columns belongs to the front that eliminates the earlier of
 // r and c; its local row/column is the DOF's own index there, or e + its index among the front's boundary
@@ -519,433 +598,252 @@ __global__ void mf_list_fill_kernel(long long n, const int* __restrict__ indptr,
 }
 
 // ---------------------------------------------------------------- solve kernels
-// w (rows of the level's fronts, S per row): own rows from the right-hand side, boundary rows zero
+// Rows of the two children's fronts that each front row receives (absolute rows of w, -1: none), built once:
+// the children's boundary rows are their update vectors.
+__global__ void mf_child_rows_kernel(int v0, int nf, const FrontMeta* __restrict__ fm, const int* __restrict__ ea,
+                                     int* __restrict__ cmap, long long rows) {
+    const int v = v0 + blockIdx.y;
+    if (v >= nf) return;
+    const FrontMeta& g = fm[v];
+    if (g.parent < 0) return;
+    const FrontMeta& f = fm[g.parent];
+    int* M = cmap + (f.child[0] == v ? 0 : rows) + f.wv;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < g.b; i += gridDim.x * blockDim.x)
+        M[ea[g.ea + i]] = (int)(g.wv + g.e + i);
+}
+
+// w (the front's rows, S per row): own rows from the right-hand side, plus both children's update rows
 __global__ void mf_fwd_gather_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm, int S,
                                      const int* __restrict__ fdof, const double* __restrict__ scale,
-                                     const double2* __restrict__ rhs, float2* __restrict__ w) {
+                                     const int* __restrict__ cmap, long long rows, const double2* __restrict__ rhs,
+                                     float2* __restrict__ w) {
     const FrontMeta& f = fm[lst[blockIdx.y]];
-    long long tot = (long long)f.n * S;
-    long long i0 = (long long)blockIdx.x * MF_CHUNK;
-    if (i0 >= tot) return;
-    long long i1 = min(i0 + MF_CHUNK, tot);
-    float2* W = w + f.wv * S;
-    const int* d = fdof + f.fdof;
-    for (long long idx = i0 + threadIdx.x; idx < i1; idx += blockDim.x) {
-        long long i = idx / S;
-        int s = (int)(idx % S);
-        float2 v = make_float2(0.f, 0.f);
-        if (i < f.e) {
-            double2 r = rhs[(long long)d[i] * S + s];
-            double sc = scale[d[i]];
-            v = make_float2((float)(r.x * sc), (float)(r.y * sc));
-        }
-        W[idx] = v;
+    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx >= (long long)f.n * S) return;
+    const int i = (int)(idx / S), s = (int)(idx % S);
+    const int a = cmap[f.wv + i], b = cmap[rows + f.wv + i];
+    float2 v = make_float2(0.f, 0.f);
+    if (i < f.e) {
+        const int d = fdof[f.fdof + i];
+        const double2 r = rhs[(long long)d * S + s];
+        const double sc = scale[d];
+        v = make_float2((float)(r.x * sc), (float)(r.y * sc));
     }
+    if (a >= 0) { const float2 u = w[(long long)a * S + s]; v.x += u.x; v.y += u.y; }
+    if (b >= 0) { const float2 u = w[(long long)b * S + s]; v.x += u.x; v.y += u.y; }
+    w[f.wv * S + idx] = v;
 }
 
-__global__ void mf_fwd_ea_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm, int S, int cslot,
-                                 const int* __restrict__ ea, const float2* __restrict__ uvec, float2* __restrict__ w) {
-    const FrontMeta& f = fm[lst[blockIdx.y]];
-    int c = f.child[cslot];
-    if (c < 0) return;
-    const FrontMeta& g = fm[c];
-    long long tot = (long long)g.b * S;
-    long long i0 = (long long)blockIdx.x * MF_CHUNK;
-    if (i0 >= tot) return;
-    long long i1 = min(i0 + MF_CHUNK, tot);
-    const int* map = ea + g.ea;
-    const float2* U = uvec + g.uv * S;
-    float2* W = w + f.wv * S;
-    for (long long idx = i0 + threadIdx.x; idx < i1; idx += blockDim.x) {
-        long long i = idx / S;
-        int s = (int)(idx % S);
-        float2 u = U[idx];
-        float2* p = W + (long long)map[i] * S + s;
-        p->x += u.x;
-        p->y += u.y;
-    }
-}
-
-// Forward solve inside the 256-row block [k0, k1) of the own rows, held in shared memory: for each
-// 32-step y = (Linv P) w_step, then the block's remaining rows.  One CTA per front, 16 right-hand sides
-// at a time.  Each step's inverse block and L panel (the block's rows below the step, 32 columns) are
-// first staged in shared memory with coalesced loads, so a step costs one global round trip.
-constexpr int MF_SC = 16;
-constexpr int MF_PAN = MF_SB - MF_NB;     // panel rows below a step inside the block
-template <int NBUF>
-struct MfBlockSmem {
-    float2 wb[MF_SB][MF_SC];
-    float2 y[MF_NB][MF_SC];
-    float2 li[NBUF][MF_NB * MF_NB];
-    float2 pan[NBUF][MF_PAN][MF_NB + 1];
+// One product of a solve: t[r] = sum_{c in [c0, c1)} M[r, c] x[c] for a tile of 32 RPL rows and NS right-hand
+// sides.  Each of the 8 warps takes every 8th column, lane rl holding rows rl + 32 i, so that a warp reads
+// 256 RPL contiguous bytes of a column; the columns' x values (S per row) are staged in shared memory, 256
+// columns at a time, and the warps' sums meet there in a fixed order.  It streams the factors once; what
+// bounds it is how many of a stage's columns are in flight (the loop is unrolled 8 deep).
+constexpr int MF_KC = MF_SB;
+template <int NS>
+struct MfProdSmem {
+    float2 x[MF_KC][NS];
+    float2 red[8][NS < 4 ? NS : 4][64];
 };
-constexpr size_t MF_BLOCK_SMEM = sizeof(MfBlockSmem<1>);
-constexpr size_t MF_BLOCK_SMEM2 = sizeof(MfBlockSmem<2>);
 
-// Stage step st's inverse block and panel (forward: rows below the step inside the block; backward: rows
-// above it) into buffer slot, as one committed group of asynchronous copies.
-__device__ __forceinline__ void mf_stage_step(float2* li, float2 (*pan)[MF_NB + 1], const float2* Ib,
-                                              const float2* F, long long n, int rbase, int pr, int kcol, int kb) {
-    for (int t = threadIdx.x; t < MF_NB * MF_NB; t += blockDim.x) cp_async8(&li[t], &Ib[t]);
-    for (int t = threadIdx.x; t < pr * kb; t += blockDim.x) {
-        int c = t / pr, r = t - c * pr;          // consecutive threads: consecutive rows of one column
-        cp_async8(&pan[r][c], &F[(rbase + r) + (long long)(kcol + c) * n]);
-    }
-    cp_async_commit();
-}
-
-// NT threads: 256 on levels of many fronts (several CTAs per SM), 1024 on levels of few fronts, where the
-// block chain of one front is serial and a step's items (rows x right-hand sides) spread over more threads.
-constexpr int MF_BLOCK_NT_FEW = 1024;
-template <int NBUF, int NT>
-__global__ void __launch_bounds__(NT) mf_fwd_block_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm,
-                                                           int S, int k0, const float2* __restrict__ fact,
-                                                           const float2* __restrict__ inv, float2* __restrict__ w) {
-    extern __shared__ __align__(16) unsigned char mf_smem[];
-    MfBlockSmem<NBUF>& sm = *reinterpret_cast<MfBlockSmem<NBUF>*>(mf_smem);
-    const FrontMeta& f = fm[lst[blockIdx.x]];
-    if (k0 >= f.e) return;
-    const int k1 = min(k0 + MF_SB, f.e);
-    const int rows = k1 - k0;
-    const int nsteps = (rows + MF_NB - 1) / MF_NB;
-    const long long n = f.n;
-    float2* W = w + f.wv * S;
-    const float2* F = fact + f.fact;
-    const int tid = threadIdx.x;
-    auto stage = [&](int st) {
-        const int k = k0 + st * MF_NB, kb = min(MF_NB, f.e - k);
-        mf_stage_step(sm.li[st % NBUF], sm.pan[st % NBUF], inv + f.inv + (long long)(k / MF_NB) * 2 * MF_NB * MF_NB,
-                      F, n, k + kb, k1 - k - kb, k, kb);
-    };
-    for (int sc = 0; sc < S; sc += MF_SC) {
-        const int ns = min(MF_SC, S - sc);
-        for (int t = tid; t < rows * ns; t += blockDim.x)
-            cp_async8(&sm.wb[t / ns][t % ns], &W[(long long)(k0 + t / ns) * S + sc + t % ns]);
-        stage(0);
-        for (int st = 0; st < nsteps; st++) {
-            const int k = k0 + st * MF_NB, kb = min(MF_NB, f.e - k), pr = k1 - k - kb;
-            if (NBUF == 2 && st + 1 < nsteps) {
-                stage(st + 1);                   // the next step's copies fly while this step computes
-                cp_async_wait_1();
-            } else {
-                cp_async_wait_all();
-            }
-            __syncthreads();
-            const float2* li = sm.li[st % NBUF];
-            for (int t = tid; t < kb * ns; t += blockDim.x) {
-                int i = t / ns, sj = t % ns;
-                float2 acc = make_float2(0.f, 0.f);
-                for (int c = 0; c < kb; c++) cfma(acc, li[i + c * MF_NB], sm.wb[k - k0 + c][sj]);
-                sm.y[i][sj] = acc;
-            }
-            __syncthreads();
-            for (int t = tid; t < kb * ns; t += blockDim.x) sm.wb[k - k0 + t / ns][t % ns] = sm.y[t / ns][t % ns];
-            for (int t = tid; t < pr * ns; t += blockDim.x) {
-                int r = t / ns, sj = t % ns;
-                float2 acc = sm.wb[k + kb - k0 + r][sj];
-                for (int c = 0; c < kb; c++) cfms(acc, sm.pan[st % NBUF][r][c], sm.y[c][sj]);
-                sm.wb[k + kb - k0 + r][sj] = acc;
-            }
-            __syncthreads();
-            if (NBUF == 1 && st + 1 < nsteps) stage(st + 1);
-        }
-        for (int t = tid; t < rows * ns; t += blockDim.x) W[(long long)(k0 + t / ns) * S + sc + t % ns] = sm.wb[t / ns][t % ns];
-        __syncthreads();
-    }
-}
-
-// w[r] -= sum_{c in [c0, c1)} M[r, c] x[c] for the rows [r0, r1) of a front, M column-major with leading
-// dimension ldm, x = rows c of w (or of xsrc).  A CTA owns 32 rows; its 8 warps take every 8th column
-// and their sums meet in shared memory.  8 right-hand sides per CTA (grid.z).
-// RPL row sets per lane: lane rl of warp g holds rows rb + rl + 32 i (i < RPL), so a warp streams
-// 32 * RPL consecutive rows (256 * RPL contiguous bytes) of every column it visits, with RPL loads in
-// flight per column.  Each row sums its columns in the same order as with one row set (bit-identical).
-constexpr int MF_RPL = 2;
-template <int RPL>
-__device__ __forceinline__ void mf_gemv_rowsets(float2* W, int S, long long rb, int rl, int g, long long rlim,
-                                                const float2* M, long long ldm, long long c0, long long c1,
-                                                const float2* X, long long xrow0, int s0, int ns,
-                                                float2 (*red)[32 * RPL][8]) {
-    float2 acc[RPL][8];
+// XOf(c): pointer to the NS values of column c;  MAt(i, c): entry (row rl + 32 i of the tile, column c);
+// Out(row of the tile, q, value)
+template <int NS, int RPL, typename XOf, typename MAt, typename Out>
+__device__ __forceinline__ void mf_product(MfProdSmem<NS>& sm, int c0, int c1, int ns, XOf xof, MAt mat, Out out) {
+    const int rl = threadIdx.x & 31, g = threadIdx.x >> 5;
+    float2 acc[RPL][NS];
 #pragma unroll
     for (int i = 0; i < RPL; i++)
 #pragma unroll
-        for (int q = 0; q < 8; q++) acc[i][q] = make_float2(0.f, 0.f);
-    bool live[RPL];
-#pragma unroll
-    for (int i = 0; i < RPL; i++) live[i] = rb + rl + 32 * i < rlim;
-    if (live[0]) {
-#pragma unroll 4
-        for (long long c = c0 + g; c < c1; c += 8) {
+        for (int q = 0; q < NS; q++) acc[i][q] = make_float2(0.f, 0.f);
+    for (int cb = c0; cb < c1; cb += MF_KC) {
+        const int nc = min(MF_KC, c1 - cb);
+        if (cb > c0) __syncthreads();
+        for (int t = threadIdx.x; t < nc * NS; t += 256) {
+            const int c = t / NS, q = t % NS;
+            sm.x[c][q] = q < ns ? xof(cb + c)[q] : make_float2(0.f, 0.f);
+        }
+        __syncthreads();
+#pragma unroll 8
+        for (int c = g; c < nc; c += 8) {
             float2 mv[RPL];
 #pragma unroll
-            for (int i = 0; i < RPL; i++) mv[i] = live[i] ? M[rb + rl + 32 * i + c * ldm] : make_float2(0.f, 0.f);
-            const float2* xc = X + (xrow0 + c - c0) * S + s0;
+            for (int i = 0; i < RPL; i++) mv[i] = mat(i, cb + c);
 #pragma unroll
-            for (int q = 0; q < 8; q++)
-                if (q < ns) {
-                    const float2 xv = xc[q];
+            for (int q = 0; q < NS; q++) {
+                const float2 xv = sm.x[c][q];
 #pragma unroll
-                    for (int i = 0; i < RPL; i++) cfma(acc[i][q], mv[i], xv);
-                }
+                for (int i = 0; i < RPL; i++) cfma(acc[i][q], mv[i], xv);
+            }
         }
     }
+    constexpr int QB = NS < 4 ? NS : 4;
 #pragma unroll
-    for (int i = 0; i < RPL; i++)
+    for (int q0 = 0; q0 < NS; q0 += QB) {
+        if (q0) __syncthreads();
 #pragma unroll
-        for (int q = 0; q < 8; q++) red[g][rl + 32 * i][q] = acc[i][q];
-    __syncthreads();
-    if (g < RPL && live[g]) {
-        const long long r = rb + rl + 32 * g;
-        for (int q = 0; q < ns; q++) {
-            float2 t = make_float2(0.f, 0.f);
+        for (int i = 0; i < RPL; i++)
 #pragma unroll
-            for (int gg = 0; gg < 8; gg++) { t.x += red[gg][rl + 32 * g][q].x; t.y += red[gg][rl + 32 * g][q].y; }
-            float2* p = W + r * S + s0 + q;
-            p->x -= t.x;
-            p->y -= t.y;
+            for (int q = 0; q < QB; q++) sm.red[g][q][rl + 32 * i] = acc[i][q0 + q];
+        __syncthreads();
+        for (int t = threadIdx.x; t < 32 * RPL * QB; t += 256) {
+            const int q = t / (32 * RPL), r = t % (32 * RPL);
+            if (q0 + q >= ns) continue;
+            float2 v = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int gg = 0; gg < 8; gg++) { v.x += sm.red[gg][q][r].x; v.y += sm.red[gg][q][r].y; }
+            out(r, q0 + q, v);
         }
     }
 }
 
-// Rows [k1, n) of every front: w[r] -= L[r, k0:k1] y[k0:k1]
+// y[k0 .. k1) = G w[k0 .. k1), G the inverse of the 256-block of L: 32 rows per CTA, off-diagonal blocks from
+// the factor store, the diagonal one from the inverse store
+template <int NS>
+__global__ void __launch_bounds__(256) mf_fwd_tri_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm,
+                                                         int S, int k0, const float2* __restrict__ fact,
+                                                         const float2* __restrict__ inv, const float2* __restrict__ w,
+                                                         float2* __restrict__ y) {
+    __shared__ MfProdSmem<NS> sm;
+    const FrontMeta& f = fm[lst[blockIdx.y]];
+    const int r0 = k0 + blockIdx.x * MF_NB;
+    if (r0 >= f.e) return;
+    const int s0 = blockIdx.z * NS, ns = min(NS, S - s0), r = r0 + (threadIdx.x & 31);
+    const float2* F = fact + f.fact + r;
+    const float2* D = inv + f.inv + (long long)(r0 / MF_NB) * 2 * MF_NB * MF_NB + (threadIdx.x & 31);
+    const float2* X = w + f.wv * S + s0;
+    float2* Y = y + f.y * S + s0;
+    const bool live = r < f.e;
+    const long long n = f.n;
+    mf_product<NS, 1>(sm, k0, min(r0 + MF_NB, f.e), ns, [&](int c) { return X + (long long)c * S; },
+                      [&](int, int c) {
+                          if (!live) return make_float2(0.f, 0.f);
+                          return c < r0 ? F[c * n] : D[(c - r0) * MF_NB];
+                      },
+                      [&](int t, int q, float2 v) { if (r0 + t < f.e) Y[(long long)(r0 + t) * S + q] = v; });
+}
+
+// rows [k1, n): w[r] -= L[r, k0:k1] y[k0:k1]
+template <int NS, int RPL>
 __global__ void __launch_bounds__(256) mf_fwd_update_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm,
                                                             int S, int k0, const float2* __restrict__ fact,
-                                                            float2* __restrict__ w) {
-    __shared__ float2 red[8][32 * MF_RPL][8];
+                                                            const float2* __restrict__ y, float2* __restrict__ w) {
+    __shared__ MfProdSmem<NS> sm;
     const FrontMeta& f = fm[lst[blockIdx.y]];
     if (k0 >= f.e) return;
     const int k1 = min(k0 + MF_SB, f.e);
-    const long long r0 = k1 + (long long)blockIdx.x * 32 * MF_RPL;
+    const int r0 = k1 + blockIdx.x * 32 * RPL;
     if (r0 >= f.n) return;
-    const int s0 = blockIdx.z * 8, ns = min(8, S - s0);
-    const int rl = threadIdx.x % 32, g = threadIdx.x / 32;
-    float2* W = w + f.wv * S;
-    mf_gemv_rowsets<MF_RPL>(W, S, r0, rl, g, f.n, fact + f.fact, f.n, k0, k1, W, k0, s0, ns, red);
+    const int s0 = blockIdx.z * NS, ns = min(NS, S - s0), r = r0 + (threadIdx.x & 31);
+    const float2* F = fact + f.fact + r;
+    const float2* X = y + f.y * S + s0;
+    float2* W = w + f.wv * S + s0;
+    const long long n = f.n;
+    mf_product<NS, RPL>(sm, k0, k1, ns, [&](int c) { return X + (long long)c * S; },
+                        [&](int i, int c) { return r + 32 * i < n ? F[32 * i + c * n] : make_float2(0.f, 0.f); },
+                        [&](int t, int q, float2 v) {
+                            if (r0 + t >= n) return;
+                            float2* p = W + (long long)(r0 + t) * S + q;
+                            p->x -= v.x;
+                            p->y -= v.y;
+                        });
 }
 
-// own rows -> y store, boundary rows -> update vector for the parent
-__global__ void mf_fwd_finish_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm, int S,
-                                     const float2* __restrict__ w, float2* __restrict__ ystore, float2* __restrict__ uvec) {
+// own rows: y[r] -= U12[r, :] x_bnd (U12 is e x b, column-major with ld e; x_bnd = the solved x of the boundary
+// DOFs).  Levels of few fronts split the columns over nsplit CTAs of cw columns; their sums go to part and
+// mf_bwd_bnd_sum_kernel subtracts them in order.
+template <int NS, int RPL>
+__global__ void __launch_bounds__(256) mf_bwd_bnd_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm, int S,
+                                                         int nrt, int nsplit, int cw, long long y0, long long yl,
+                                                         const float2* __restrict__ fact, const int* __restrict__ fdof,
+                                                         const float2* __restrict__ xs, float2* __restrict__ y,
+                                                         float2* __restrict__ part) {
+    __shared__ MfProdSmem<NS> sm;
     const FrontMeta& f = fm[lst[blockIdx.y]];
-    long long tot = (long long)f.n * S;
-    long long i0 = (long long)blockIdx.x * MF_CHUNK;
-    if (i0 >= tot) return;
-    long long i1 = min(i0 + MF_CHUNK, tot);
-    const float2* W = w + f.wv * S;
-    for (long long idx = i0 + threadIdx.x; idx < i1; idx += blockDim.x) {
-        long long i = idx / S;
-        if (i < f.e) ystore[f.y * S + idx] = W[idx];
-        else uvec[f.uv * S + (idx - (long long)f.e * S)] = W[idx];
-    }
-}
-
-// backward: own rows from y, boundary rows from the solved x (FP32, DOF order)
-__global__ void mf_bwd_gather_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm, int S,
-                                     const int* __restrict__ fdof, const float2* __restrict__ ystore,
-                                     const float2* __restrict__ xs, float2* __restrict__ w) {
-    const FrontMeta& f = fm[lst[blockIdx.y]];
-    long long tot = (long long)f.n * S;
-    long long i0 = (long long)blockIdx.x * MF_CHUNK;
-    if (i0 >= tot) return;
-    long long i1 = min(i0 + MF_CHUNK, tot);
-    float2* W = w + f.wv * S;
-    const int* d = fdof + f.fdof;
-    for (long long idx = i0 + threadIdx.x; idx < i1; idx += blockDim.x) {
-        long long i = idx / S;
-        int s = (int)(idx % S);
-        W[idx] = i < f.e ? ystore[f.y * S + idx] : xs[(long long)d[i] * S + s];
-    }
-}
-
-// own rows: w[r] -= U12[r, :] x_bnd   (U12 is e x b, column-major with ld e; x_bnd = rows e.. of w)
-// The same U12 product split over the boundary columns for fronts with long boundaries: CTA (row group,
-// column chunk of MF_CW) writes its partial sums to part[chunk][level row][S]; mf_bwd_bnd_sum_kernel
-// then subtracts the chunks in ascending order (deterministic).  A front's own rows [0, e) of its
-// level rows f.wv .. f.wv + n index the partials; chunks past the front's boundary write zeros.
-constexpr int MF_CW = 512;
-__global__ void __launch_bounds__(256) mf_bwd_bnd_split_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm,
-                                                               int S, int nrg, long long wvl,
-                                                               const float2* __restrict__ fact,
-                                                               const float2* __restrict__ w, float2* __restrict__ part) {
-    __shared__ float2 red[8][32 * MF_RPL][8];
-    const FrontMeta& f = fm[lst[blockIdx.y]];
-    if (f.b == 0) return;
-    const int rg = blockIdx.x % nrg, sp = blockIdx.x / nrg;
-    const long long r0 = (long long)rg * 32 * MF_RPL;
-    if (r0 >= f.e) return;
-    const int s0 = blockIdx.z * 8, ns = min(8, S - s0);
-    const int rl = threadIdx.x % 32, g = threadIdx.x / 32;
-    const float2* W = w + f.wv * S;
-    const float2* M = fact + f.fact + (long long)f.n * f.e;
-    const long long c0 = min((long long)sp * MF_CW, (long long)f.b), c1 = min(c0 + MF_CW, (long long)f.b);
-    float2 acc[MF_RPL][8];
-    bool live[MF_RPL];
-#pragma unroll
-    for (int i = 0; i < MF_RPL; i++) {
-        live[i] = r0 + rl + 32 * i < f.e;
-#pragma unroll
-        for (int q = 0; q < 8; q++) acc[i][q] = make_float2(0.f, 0.f);
-    }
-    if (live[0]) {
-#pragma unroll 4
-        for (long long c = c0 + g; c < c1; c += 8) {
-            float2 mv[MF_RPL];
-#pragma unroll
-            for (int i = 0; i < MF_RPL; i++) mv[i] = live[i] ? M[r0 + rl + 32 * i + c * f.e] : make_float2(0.f, 0.f);
-            const float2* xc = W + (f.e + c) * S + s0;
-#pragma unroll
-            for (int q = 0; q < 8; q++)
-                if (q < ns) {
-                    const float2 xv = xc[q];
-#pragma unroll
-                    for (int i = 0; i < MF_RPL; i++) cfma(acc[i][q], mv[i], xv);
-                }
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < MF_RPL; i++)
-#pragma unroll
-        for (int q = 0; q < 8; q++) red[g][rl + 32 * i][q] = acc[i][q];
-    __syncthreads();
-    if (g < MF_RPL && live[g]) {
-        const long long r = r0 + rl + 32 * g;
-        float2* P = part + ((long long)sp * wvl + f.wv + r) * S + s0;
-        for (int q = 0; q < ns; q++) {
-            float2 t = make_float2(0.f, 0.f);
-#pragma unroll
-            for (int gg = 0; gg < 8; gg++) { t.x += red[gg][rl + 32 * g][q].x; t.y += red[gg][rl + 32 * g][q].y; }
-            P[q] = t;
-        }
-    }
+    const int r0 = (blockIdx.x % nrt) * 32 * RPL, sp = blockIdx.x / nrt;
+    if (f.b == 0 || r0 >= f.e) return;
+    const int s0 = blockIdx.z * NS, ns = min(NS, S - s0), r = r0 + (threadIdx.x & 31);
+    const long long e = f.e;
+    const float2* M = fact + f.fact + (long long)f.n * e + r;
+    const int* d = fdof + f.fdof + e;
+    const float2* X = xs + s0;
+    const int c0 = min(sp * cw, f.b), c1 = nsplit > 1 ? min(c0 + cw, f.b) : f.b;
+    float2* Y = nsplit > 1 ? part + ((long long)sp * yl + f.y - y0) * S + s0 : y + f.y * S + s0;
+    mf_product<NS, RPL>(sm, c0, c1, ns, [&](int c) { return X + (long long)d[c] * S; },
+                        [&](int i, int c) { return r + 32 * i < e ? M[32 * i + c * e] : make_float2(0.f, 0.f); },
+                        [&](int t, int q, float2 v) {
+                            if (r0 + t >= e) return;
+                            float2* p = Y + (long long)(r0 + t) * S + q;
+                            if (nsplit > 1) { *p = v; return; }
+                            p->x -= v.x;
+                            p->y -= v.y;
+                        });
 }
 
 __global__ void mf_bwd_bnd_sum_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm, int S, int nsplit,
-                                      long long wvl, const float2* __restrict__ part, float2* __restrict__ w) {
+                                      long long y0, long long yl, const float2* __restrict__ part, float2* __restrict__ y) {
     const FrontMeta& f = fm[lst[blockIdx.y]];
-    if (f.b == 0) return;
-    const long long tot = (long long)f.e * S;
-    const long long i0 = (long long)blockIdx.x * MF_CHUNK;
-    if (i0 >= tot) return;
-    const long long i1 = min(i0 + MF_CHUNK, tot);
-    float2* W = w + f.wv * S;
-    for (long long idx = i0 + threadIdx.x; idx < i1; idx += blockDim.x) {
-        float2 t = make_float2(0.f, 0.f);
-        for (int sp = 0; sp < nsplit; sp++) {
-            float2 v = part[((long long)sp * wvl + f.wv) * S + idx];
-            t.x += v.x;
-            t.y += v.y;
-        }
-        W[idx].x -= t.x;
-        W[idx].y -= t.y;
+    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (f.b == 0 || idx >= (long long)f.e * S) return;
+    float2 t = make_float2(0.f, 0.f);
+    for (int sp = 0; sp < nsplit; sp++) {
+        const float2 v = part[((long long)sp * yl + f.y - y0) * S + idx];
+        t.x += v.x;
+        t.y += v.y;
     }
+    float2* p = y + f.y * S + idx;
+    p->x -= t.x;
+    p->y -= t.y;
 }
 
-__global__ void __launch_bounds__(256) mf_bwd_bnd_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm,
-                                                         int S, const float2* __restrict__ fact, float2* __restrict__ w) {
-    __shared__ float2 red[8][32 * MF_RPL][8];
+// x[k0 .. k1) = H y[k0 .. k1), H the inverse of the 256-block of U, into the solution (DOF order)
+template <int NS>
+__global__ void __launch_bounds__(256) mf_bwd_tri_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm,
+                                                         int S, int k0, const float2* __restrict__ fact,
+                                                         const float2* __restrict__ inv, const int* __restrict__ fdof,
+                                                         const float2* __restrict__ y, float2* __restrict__ xs) {
+    __shared__ MfProdSmem<NS> sm;
     const FrontMeta& f = fm[lst[blockIdx.y]];
-    if (f.b == 0) return;
-    const long long r0 = (long long)blockIdx.x * 32 * MF_RPL;
+    const int r0 = k0 + blockIdx.x * MF_NB;
     if (r0 >= f.e) return;
-    const int s0 = blockIdx.z * 8, ns = min(8, S - s0);
-    const int rl = threadIdx.x % 32, g = threadIdx.x / 32;
-    float2* W = w + f.wv * S;
-    mf_gemv_rowsets<MF_RPL>(W, S, r0, rl, g, f.e, fact + f.fact + (long long)f.n * f.e, f.e, 0, f.b, W, f.e, s0, ns,
-                            red);
-}
-
-// Backward solve inside the block [k0, k1), held in shared memory: 32-steps from the last,
-// x_k = Uinv (w_k), then the block's earlier rows.  One CTA per front, 16 right-hand sides at a time;
-// each step's Uinv block and U panel (the block's rows above the step) staged in shared memory first.
-template <int NBUF, int NT>
-__global__ void __launch_bounds__(NT) mf_bwd_block_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm,
-                                                           int S, int k0, const float2* __restrict__ fact,
-                                                           const float2* __restrict__ inv, float2* __restrict__ w) {
-    extern __shared__ __align__(16) unsigned char mf_smem[];
-    MfBlockSmem<NBUF>& sm = *reinterpret_cast<MfBlockSmem<NBUF>*>(mf_smem);
-    const FrontMeta& f = fm[lst[blockIdx.x]];
-    if (k0 >= f.e) return;
-    const int k1 = min(k0 + MF_SB, f.e);
-    const int rows = k1 - k0;
+    const int s0 = blockIdx.z * NS, ns = min(NS, S - s0), r = r0 + (threadIdx.x & 31);
+    const float2* F = fact + f.fact + r;
+    const float2* D = inv + f.inv + (long long)(r0 / MF_NB) * 2 * MF_NB * MF_NB + MF_NB * MF_NB + (threadIdx.x & 31);
+    const float2* X = y + f.y * S + s0;
+    const int* d = fdof + f.fdof;
+    const bool live = r < f.e;
     const long long n = f.n;
-    float2* W = w + f.wv * S;
-    const float2* F = fact + f.fact;
-    const int tid = threadIdx.x;
-    const int nsteps = (rows + MF_NB - 1) / MF_NB;
-    // processing order j = 0.. runs the steps from the last (st = nsteps - 1 - j); buffers follow j
-    auto stage = [&](int j) {
-        const int k = k0 + (nsteps - 1 - j) * MF_NB, kb = min(MF_NB, f.e - k);
-        mf_stage_step(sm.li[j % NBUF], sm.pan[j % NBUF],
-                      inv + f.inv + (long long)(k / MF_NB) * 2 * MF_NB * MF_NB + MF_NB * MF_NB, F, n, k0, k - k0, k, kb);
-    };
-    for (int sc = 0; sc < S; sc += MF_SC) {
-        const int ns = min(MF_SC, S - sc);
-        for (int t = tid; t < rows * ns; t += blockDim.x)
-            cp_async8(&sm.wb[t / ns][t % ns], &W[(long long)(k0 + t / ns) * S + sc + t % ns]);
-        stage(0);
-        for (int j = 0; j < nsteps; j++) {
-            const int k = k0 + (nsteps - 1 - j) * MF_NB, kb = min(MF_NB, f.e - k), pr = k - k0;
-            if (NBUF == 2 && j + 1 < nsteps) {
-                stage(j + 1);
-                cp_async_wait_1();
-            } else {
-                cp_async_wait_all();
-            }
-            __syncthreads();
-            const float2* ui = sm.li[j % NBUF];
-            for (int t = tid; t < kb * ns; t += blockDim.x) {
-                int i = t / ns, sj = t % ns;
-                float2 acc = make_float2(0.f, 0.f);
-                for (int c = i; c < kb; c++) cfma(acc, ui[i + c * MF_NB], sm.wb[k - k0 + c][sj]);
-                sm.y[i][sj] = acc;
-            }
-            __syncthreads();
-            for (int t = tid; t < kb * ns; t += blockDim.x) sm.wb[k - k0 + t / ns][t % ns] = sm.y[t / ns][t % ns];
-            for (int t = tid; t < pr * ns; t += blockDim.x) {
-                int r = t / ns, sj = t % ns;
-                float2 acc = sm.wb[r][sj];
-                for (int c = 0; c < kb; c++) cfms(acc, sm.pan[j % NBUF][r][c], sm.y[c][sj]);
-                sm.wb[r][sj] = acc;
-            }
-            __syncthreads();
-            if (NBUF == 1 && j + 1 < nsteps) stage(j + 1);
-        }
-        for (int t = tid; t < rows * ns; t += blockDim.x) W[(long long)(k0 + t / ns) * S + sc + t % ns] = sm.wb[t / ns][t % ns];
-        __syncthreads();
-    }
+    mf_product<NS, 1>(sm, r0, min(k0 + MF_SB, f.e), ns, [&](int c) { return X + (long long)c * S; },
+                      [&](int, int c) {
+                          if (!live) return make_float2(0.f, 0.f);
+                          return c < r0 + MF_NB ? D[(c - r0) * MF_NB] : F[c * n];
+                      },
+                      [&](int t, int q, float2 v) { if (r0 + t < f.e) xs[(long long)d[r0 + t] * S + s0 + q] = v; });
 }
 
-// rows [0, k0): w[r] -= U[r, k0:k1] x[k0:k1]
+// rows [0, k0): y[r] -= U[r, k0:k1] x[k0:k1]
+template <int NS, int RPL>
 __global__ void __launch_bounds__(256) mf_bwd_update_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm,
                                                             int S, int k0, const float2* __restrict__ fact,
-                                                            float2* __restrict__ w) {
-    __shared__ float2 red[8][32 * MF_RPL][8];
+                                                            const int* __restrict__ fdof, const float2* __restrict__ xs,
+                                                            float2* __restrict__ y) {
+    __shared__ MfProdSmem<NS> sm;
     const FrontMeta& f = fm[lst[blockIdx.y]];
     if (k0 >= f.e) return;
-    const int k1 = min(k0 + MF_SB, f.e);
-    const long long r0 = (long long)blockIdx.x * 32 * MF_RPL;
-    if (r0 >= k0) return;
-    const int s0 = blockIdx.z * 8, ns = min(8, S - s0);
-    const int rl = threadIdx.x % 32, g = threadIdx.x / 32;
-    float2* W = w + f.wv * S;
-    mf_gemv_rowsets<MF_RPL>(W, S, r0, rl, g, k0, fact + f.fact, f.n, k0, k1, W, k0, s0, ns, red);
-}
-
-__global__ void mf_bwd_finish_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm, int S,
-                                     const int* __restrict__ fdof, const float2* __restrict__ w, float2* __restrict__ xs) {
-    const FrontMeta& f = fm[lst[blockIdx.y]];
-    long long tot = (long long)f.e * S;
-    long long i0 = (long long)blockIdx.x * MF_CHUNK;
-    if (i0 >= tot) return;
-    long long i1 = min(i0 + MF_CHUNK, tot);
-    const float2* W = w + f.wv * S;
+    const int k1 = min(k0 + MF_SB, f.e), r0 = blockIdx.x * 32 * RPL;      // k0 is a multiple of 256: whole tiles
+    const int s0 = blockIdx.z * NS, ns = min(NS, S - s0), r = r0 + (threadIdx.x & 31);
+    const float2* F = fact + f.fact + r;
+    const float2* X = xs + s0;
     const int* d = fdof + f.fdof;
-    for (long long idx = i0 + threadIdx.x; idx < i1; idx += blockDim.x) {
-        long long i = idx / S;
-        int s = (int)(idx % S);
-        xs[(long long)d[i] * S + s] = W[idx];
-    }
+    float2* Y = y + f.y * S + s0;
+    const long long n = f.n;
+    mf_product<NS, RPL>(sm, k0, k1, ns, [&](int c) { return X + (long long)d[c] * S; },
+                        [&](int i, int c) { return F[32 * i + c * n]; },
+                        [&](int t, int q, float2 v) {
+                            float2* p = Y + (long long)(r0 + t) * S + q;
+                            p->x -= v.x;
+                            p->y -= v.y;
+                        });
 }
 
 __global__ void mf_fill_kernel(long long n, double v, double* __restrict__ x) {
@@ -958,9 +856,10 @@ __global__ void mf_out_kernel(long long n, int S, const uint8_t* __restrict__ fr
                               const float2* __restrict__ xs, double2* __restrict__ x) {
     long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= n * S) return;
-    float2 v = xs[g];
+    const bool in = freed[g / S];
+    const float2 v = in ? xs[g] : make_float2(0.f, 0.f);
     const double sc = scale[g / S];
-    x[g] = freed[g / S] ? make_double2((double)v.x * sc, (double)v.y * sc) : make_double2(0.0, 0.0);
+    x[g] = in ? make_double2((double)v.x * sc, (double)v.y * sc) : make_double2(0.0, 0.0);
 }
 
 }  // namespace emfem
@@ -993,13 +892,16 @@ struct emfem_mf_s {
     bool wide = false;                            // fronts factored in complex128
     int* d_npert = nullptr;
     long long fact_n = 0, inv_n = 0, piv_n = 0, ws_n = 0, upd_n = 0;
-    long long wv_n = 0, uv_n = 0, y_n = 0;        // solve buffer rows
-    std::vector<long long> lvl_wv, lvl_max_ob;    // per level: its fronts' rows (sum of n), largest own boundary
-    long long part_n = 0;                         // split U12 partials: max over levels of chunks x level rows
+    long long wv_n = 0, y_n = 0;                  // solve buffer rows
+    std::vector<long long> lvl_y0, lvl_yl;        // per level: first row of y and rows of y (its fronts' own rows)
+    std::vector<int> lvl_max_ob;                  // per level: largest boundary
+    std::vector<int> lvl_split;                   // per level: CTAs that share a boundary product
+    long long part_n = 0;                         // split U12 partials: max over levels of CTAs x own rows
+    int* d_cmap = nullptr;                        // children's update row of every front row, two slots
     float2* spart = nullptr;                      // (part_n, S) partial sums of the split backward products
     // solve buffers for the current S
     int S = 0;
-    float2 *sw = nullptr, *suv = nullptr, *sy = nullptr, *sx = nullptr;
+    float2 *sw = nullptr, *sy = nullptr, *sx = nullptr;
     double flops = 0.0;
     bool factored = false;
     bool lists = false;                           // assembly lists present (given or built)
@@ -1009,7 +911,7 @@ struct emfem_mf_s {
 
 static void mf_free(emfem_mf_s* m) {
     void* ps[] = {m->d_meta, m->d_lst, m->d_fdof, m->d_ea, m->d_slot, m->d_off, m->d_free, m->d_scale, m->fact, m->inv, m->piv,
-                  m->ws, m->upd, m->invc, m->d_npert, m->sw, m->suv, m->sy, m->sx, m->spart};
+                  m->ws, m->upd, m->invc, m->d_npert, m->d_cmap, m->sw, m->sy, m->sx, m->spart};
     for (void* p : ps)
         if (p) cudaFree(p);
 }
@@ -1021,14 +923,13 @@ static inline unsigned nblk(long long items, long long per) {
 
 static int mf_reserve(emfem_mf_s* m, int S) {
     if (m->S >= S) return EMFEM_OK;
-    void* ps[] = {m->sw, m->suv, m->sy, m->sx, m->spart};
+    void* ps[] = {m->sw, m->sy, m->sx, m->spart};
     for (void* p : ps)
         if (p) cudaFree(p);
-    m->sw = m->suv = m->sy = m->sx = m->spart = nullptr;
+    m->sw = m->sy = m->sx = m->spart = nullptr;
     m->S = 0;
     if (m->part_n > 0) EMFEM_CUDA(cudaMalloc(&m->spart, sizeof(float2) * m->part_n * S));
     EMFEM_CUDA(cudaMalloc(&m->sw, sizeof(float2) * std::max(1LL, m->wv_n) * S));
-    EMFEM_CUDA(cudaMalloc(&m->suv, sizeof(float2) * std::max(1LL, m->uv_n) * S));
     EMFEM_CUDA(cudaMalloc(&m->sy, sizeof(float2) * std::max(1LL, m->y_n) * S));
     EMFEM_CUDA(cudaMalloc(&m->sx, sizeof(float2) * m->n * S));
     m->S = S;
@@ -1038,6 +939,76 @@ static int mf_reserve(emfem_mf_s* m, int S) {
 namespace emfem {
 int mf_reserved(const emfem_mf_s* m) { return m ? m->S : 0; }
 
+// Tiles of 64 rows where they give every SM four CTAs, else of 32.
+static bool mf_wide_tiles(long long rows, int ny, unsigned sz) { return (rows + 63) / 64 * ny * sz >= 4 * 148; }
+
+// Forward and backward pass over the tree, NS right-hand sides per CTA.
+template <int NS>
+static int mf_sweep_tree(emfem_mf_s* m, int S, const double2* r, cudaStream_t s) {
+    const int nl = (int)m->levels.size();
+    const unsigned sz = (unsigned)((S + NS - 1) / NS);
+    for (int L = 0; L < nl; L++) {
+        const int nfl = (int)m->levels[L].size();
+        const long long maxn = m->lvl_max_n[L];
+        const int maxe = m->lvl_max_e[L];
+        for (int y0 = 0; y0 < nfl; y0 += 65535) {
+            const int ny = std::min(65535, nfl - y0);
+            const int* lst = m->d_lst + m->lvl_off[L] + y0;
+            mf_fwd_gather_kernel<<<dim3(nblk(maxn * S, 256), ny), 256, 0, s>>>(lst, m->d_meta, S, m->d_fdof, m->d_scale,
+                                                                              m->d_cmap, m->wv_n, r, m->sw);
+            for (int k0 = 0; k0 < maxe; k0 += MF_SB) {
+                const unsigned nt = nblk(std::min(MF_SB, maxe - k0), MF_NB);
+                mf_fwd_tri_kernel<NS><<<dim3(nt, ny, sz), 256, 0, s>>>(lst, m->d_meta, S, k0, m->fact, m->inv, m->sw, m->sy);
+                const long long rows = maxn - k0;            // rows [k1, n) of a front: at most n - k0
+                if (mf_wide_tiles(rows, ny, sz))
+                    mf_fwd_update_kernel<NS, 2><<<dim3(nblk(rows, 64), ny, sz), 256, 0, s>>>(lst, m->d_meta, S, k0, m->fact,
+                                                                                         m->sy, m->sw);
+                else
+                    mf_fwd_update_kernel<NS, 1><<<dim3(nblk(rows, 32), ny, sz), 256, 0, s>>>(lst, m->d_meta, S, k0, m->fact,
+                                                                                         m->sy, m->sw);
+            }
+        }
+        EMFEM_LAUNCH("multifrontal forward");
+    }
+    for (int L = nl - 1; L >= 0; L--) {
+        const int nfl = (int)m->levels[L].size();
+        const int maxe = m->lvl_max_e[L], nsplit = m->lvl_split[L];
+        const int cw = (int)nblk(nblk(m->lvl_max_ob[L], nsplit), MF_KC) * MF_KC;
+        for (int y0 = 0; y0 < nfl; y0 += 65535) {
+            const int ny = std::min(65535, nfl - y0);
+            const int* lst = m->d_lst + m->lvl_off[L] + y0;
+            if (m->lvl_max_ob[L] > 0) {
+                if (mf_wide_tiles(maxe, ny * nsplit, sz)) {
+                    const int nrt = (int)nblk(maxe, 64);
+                    mf_bwd_bnd_kernel<NS, 2><<<dim3(nrt * nsplit, ny, sz), 256, 0, s>>>(
+                        lst, m->d_meta, S, nrt, nsplit, cw, m->lvl_y0[L], m->lvl_yl[L], m->fact, m->d_fdof, m->sx, m->sy, m->spart);
+                } else {
+                    const int nrt = (int)nblk(maxe, 32);
+                    mf_bwd_bnd_kernel<NS, 1><<<dim3(nrt * nsplit, ny, sz), 256, 0, s>>>(
+                        lst, m->d_meta, S, nrt, nsplit, cw, m->lvl_y0[L], m->lvl_yl[L], m->fact, m->d_fdof, m->sx, m->sy, m->spart);
+                }
+                if (nsplit > 1)
+                    mf_bwd_bnd_sum_kernel<<<dim3(nblk((long long)maxe * S, 256), ny), 256, 0, s>>>(
+                        lst, m->d_meta, S, nsplit, m->lvl_y0[L], m->lvl_yl[L], m->spart, m->sy);
+            }
+            for (int k0 = (maxe - 1) / MF_SB * MF_SB; maxe > 0 && k0 >= 0; k0 -= MF_SB) {
+                const unsigned nt = nblk(std::min(MF_SB, maxe - k0), MF_NB);
+                mf_bwd_tri_kernel<NS><<<dim3(nt, ny, sz), 256, 0, s>>>(lst, m->d_meta, S, k0, m->fact, m->inv, m->d_fdof,
+                                                                       m->sy, m->sx);
+                if (k0 == 0) continue;
+                if (mf_wide_tiles(k0, ny, sz))
+                    mf_bwd_update_kernel<NS, 2><<<dim3(k0 / 64, ny, sz), 256, 0, s>>>(lst, m->d_meta, S, k0, m->fact,
+                                                                                   m->d_fdof, m->sx, m->sy);
+                else
+                    mf_bwd_update_kernel<NS, 1><<<dim3(k0 / 32, ny, sz), 256, 0, s>>>(lst, m->d_meta, S, k0, m->fact,
+                                                                                   m->d_fdof, m->sx, m->sy);
+            }
+        }
+        EMFEM_LAUNCH("multifrontal backward");
+    }
+    return EMFEM_OK;
+}
+
 // M^-1 r for S right-hand sides (n, S) FP64 DOF-major -> x (FP64), zero on DOFs outside every front.
 int mf_apply(emfem_mf_s* m, int S, const double2* r, double2* x, cudaStream_t s) {
     EMFEM_REQUIRE(m->factored, "emfem_mf: solve before a successful factorization");
@@ -1045,74 +1016,8 @@ int mf_apply(emfem_mf_s* m, int S, const double2* r, double2* x, cudaStream_t s)
         set_error("emfem_mf: %d right-hand sides exceed the reserved %d (emfem_mf_reserve)", S, m->S);
         return EMFEM_ERR_INVALID_ARG;
     }
-    const int nl = (int)m->levels.size();
-    EMFEM_CUDA(cudaMemsetAsync(m->sx, 0, sizeof(float2) * m->n * S, s));
-    for (int L = 0; L < nl; L++) {
-        const int nfl = (int)m->levels[L].size();
-        const int* lst = m->d_lst + m->lvl_off[L];
-        long long maxn = m->lvl_max_n[L], maxb = m->lvl_max_b[L];
-        for (int y0 = 0; y0 < nfl; y0 += 65535) {
-            const int ny = std::min(65535, nfl - y0);
-            dim3 g(nblk(maxn * S, MF_CHUNK), ny);
-            mf_fwd_gather_kernel<<<g, 256, 0, s>>>(lst + y0, m->d_meta, S, m->d_fdof, m->d_scale, r, m->sw);
-            dim3 ge(nblk(maxb * S, MF_CHUNK), ny);
-            mf_fwd_ea_kernel<<<ge, 256, 0, s>>>(lst + y0, m->d_meta, S, 0, m->d_ea, m->suv, m->sw);
-            mf_fwd_ea_kernel<<<ge, 256, 0, s>>>(lst + y0, m->d_meta, S, 1, m->d_ea, m->suv, m->sw);
-            const unsigned sz = (unsigned)((S + 7) / 8);
-            for (int k0 = 0; k0 < m->lvl_max_e[L]; k0 += MF_SB) {
-                if (ny < 148)   // a few large fronts: the serial step chain, so overlap its copies
-                    mf_fwd_block_kernel<2, MF_BLOCK_NT_FEW><<<ny, MF_BLOCK_NT_FEW, MF_BLOCK_SMEM2, s>>>(
-                        lst + y0, m->d_meta, S, k0, m->fact, m->inv, m->sw);
-                else
-                    mf_fwd_block_kernel<1, 256><<<ny, 256, MF_BLOCK_SMEM, s>>>(lst + y0, m->d_meta, S, k0, m->fact, m->inv, m->sw);
-                dim3 gu(nblk(maxn - k0, 32 * MF_RPL), ny, sz);   // rows [k1, n) of a front: at most n - k0
-                mf_fwd_update_kernel<<<gu, 256, 0, s>>>(lst + y0, m->d_meta, S, k0, m->fact, m->sw);
-            }
-            mf_fwd_finish_kernel<<<g, 256, 0, s>>>(lst + y0, m->d_meta, S, m->sw, m->sy, m->suv);
-        }
-        EMFEM_LAUNCH("multifrontal forward");
-    }
-    for (int L = nl - 1; L >= 0; L--) {
-        const int nfl = (int)m->levels[L].size();
-        const int* lst = m->d_lst + m->lvl_off[L];
-        long long maxn = m->lvl_max_n[L];
-        long long maxe = m->lvl_max_e[L];
-        for (int y0 = 0; y0 < nfl; y0 += 65535) {
-            const int ny = std::min(65535, nfl - y0);
-            dim3 g(nblk(maxn * S, MF_CHUNK), ny);
-            mf_bwd_gather_kernel<<<g, 256, 0, s>>>(lst + y0, m->d_meta, S, m->d_fdof, m->sy, m->sx, m->sw);
-            const unsigned sz = (unsigned)((S + 7) / 8);
-            const long long nsplit = (m->lvl_max_ob[L] + MF_CW - 1) / MF_CW;
-            if (nsplit > 1 && nfl < 148) {
-                const unsigned nrg = nblk(maxe, 32 * MF_RPL);
-                dim3 gb(nrg * (unsigned)nsplit, ny, sz);
-                mf_bwd_bnd_split_kernel<<<gb, 256, 0, s>>>(lst + y0, m->d_meta, S, (int)nrg, m->lvl_wv[L], m->fact,
-                                                          m->sw, m->spart);
-                dim3 gs(nblk(maxe * S, MF_CHUNK), ny);
-                mf_bwd_bnd_sum_kernel<<<gs, 256, 0, s>>>(lst + y0, m->d_meta, S, (int)nsplit, m->lvl_wv[L], m->spart,
-                                                        m->sw);
-            } else {
-                dim3 gb(nblk(maxe, 32 * MF_RPL), ny, sz);
-                mf_bwd_bnd_kernel<<<gb, 256, 0, s>>>(lst + y0, m->d_meta, S, m->fact, m->sw);
-            }
-            const int nblocks = (int)((maxe + MF_SB - 1) / MF_SB);
-            for (int bi = nblocks - 1; bi >= 0; bi--) {
-                const int k0 = bi * MF_SB;
-                if (ny < 148)
-                    mf_bwd_block_kernel<2, MF_BLOCK_NT_FEW><<<ny, MF_BLOCK_NT_FEW, MF_BLOCK_SMEM2, s>>>(
-                        lst + y0, m->d_meta, S, k0, m->fact, m->inv, m->sw);
-                else
-                    mf_bwd_block_kernel<1, 256><<<ny, 256, MF_BLOCK_SMEM, s>>>(lst + y0, m->d_meta, S, k0, m->fact, m->inv, m->sw);
-                if (k0 > 0) {
-                    dim3 gu(nblk(k0, 32 * MF_RPL), ny, sz);
-                    mf_bwd_update_kernel<<<gu, 256, 0, s>>>(lst + y0, m->d_meta, S, k0, m->fact, m->sw);
-                }
-            }
-            dim3 gf(nblk(maxe * S, MF_CHUNK), ny);
-            mf_bwd_finish_kernel<<<gf, 256, 0, s>>>(lst + y0, m->d_meta, S, m->d_fdof, m->sw, m->sx);
-        }
-        EMFEM_LAUNCH("multifrontal backward");
-    }
+    EMFEM_TRY(S >= 16 ? mf_sweep_tree<16>(m, S, r, s) : S > 4 ? mf_sweep_tree<8>(m, S, r, s)
+              : S > 2 ? mf_sweep_tree<4>(m, S, r, s) : S == 2 ? mf_sweep_tree<2>(m, S, r, s) : mf_sweep_tree<1>(m, S, r, s));
     mf_out_kernel<<<grid_for(m->n * S, 256), 256, 0, s>>>(m->n, S, m->d_free, m->d_scale, m->sx, x);
     EMFEM_LAUNCH("mf_out_kernel");
     return EMFEM_OK;
@@ -1149,6 +1054,11 @@ static int mf_factor_levels(emfem_mf_s* m, const double2* K_vals, cudaStream_t s
                 mf_trail_kernel<T><<<dim3((unsigned)std::max(1LL, nt * nt), ny), 256, 0, s>>>(lst, m->d_meta, k, ws);
             }
             mf_compact_kernel<T><<<dim3(nblk(maxn * maxn, MF_CHUNK), ny), 256, 0, s>>>(lst, m->d_meta, ws, m->fact, upd);
+            if (m->lvl_max_e[L] > MF_NB) {
+                const int nbb = std::min(MF_NBB, (int)nblk(m->lvl_max_e[L], MF_NB));
+                mf_block_inverse_kernel<T><<<dim3(2 * nbb, nblk(m->lvl_max_e[L], MF_SB), ny), 256, sizeof(MfInvSmem<T>), s>>>(
+                    lst, m->d_meta, ws, invc, m->fact);
+            }
             rc = check_cuda(cudaGetLastError(), "multifrontal factor level");
         }
     }
@@ -1185,7 +1095,7 @@ int emfem_mf_create(emfem_handle h, int64_t n, int n_fronts, const int32_t* e, c
     m->levels.assign(nl, {});
     for (int v = 0; v < n_fronts; v++) m->levels[level[v]].push_back(v);
     // offsets
-    long long fact = 0, inv = 0, pivo = 0, eao = 0, y = 0;
+    long long fact = 0, inv = 0, pivo = 0, eao = 0;
     for (int v = 0; v < n_fronts; v++) {
         FrontMeta& f = m->meta[v];
         f.e = e[v]; f.b = b[v]; f.n = e[v] + b[v]; f.parent = parent[v];
@@ -1196,7 +1106,6 @@ int emfem_mf_create(emfem_handle h, int64_t n, int n_fronts, const int32_t* e, c
         f.fact = fact; fact += (long long)f.n * f.e + (long long)f.e * f.b;
         f.inv = inv; inv += (long long)((f.e + MF_NB - 1) / MF_NB) * 2 * MF_NB * MF_NB;
         f.piv = pivo; pivo += f.e;
-        f.y = y; y += f.e;
     }
     for (int v = 0; v < n_fronts; v++) {
         int p = parent[v];
@@ -1208,7 +1117,7 @@ int emfem_mf_create(emfem_handle h, int64_t n, int n_fronts, const int32_t* e, c
         if (level[p] <= level[v]) { delete m; set_error("emfem_mf_create: parent below child"); return EMFEM_ERR_INVALID_ARG; }
     }
     // per-level workspace and solve-buffer offsets; update store by first-fit over the level schedule
-    long long ws_max = 0, wv_max = 0;
+    long long ws_max = 0;
     std::map<long long, long long> freel;   // offset -> size
     long long upd_top = 0;
     auto alloc = [&](long long sz) -> long long {
@@ -1234,30 +1143,32 @@ int emfem_mf_create(emfem_handle h, int64_t n, int n_fronts, const int32_t* e, c
             if (pv->first + pv->second == it->first) { pv->second += it->second; freel.erase(it); }
         }
     };
-    long long uv = 0;
+    long long wv = 0, yo = 0;
     m->lvl_max_e.assign(nl, 0); m->lvl_max_n.assign(nl, 0); m->lvl_max_asm.assign(nl, 0); m->lvl_max_b.assign(nl, 0);
-    m->lvl_wv.assign(nl, 0); m->lvl_max_ob.assign(nl, 0);
+    m->lvl_y0.assign(nl, 0); m->lvl_yl.assign(nl, 0); m->lvl_max_ob.assign(nl, 0); m->lvl_split.assign(nl, 1);
     for (int L = 0; L < nl; L++) {
-        long long wso = 0, wvo = 0;
+        long long wso = 0;
+        m->lvl_y0[L] = yo;
         for (int v : m->levels[L]) {
             FrontMeta& f = m->meta[v];
             f.ws = wso; wso += (long long)f.n * f.n;
-            f.wv = wvo; wvo += f.n;
-            f.uv = uv; uv += f.b;
+            f.wv = wv; wv += f.n;
+            f.y = yo; yo += f.e;
             m->lvl_max_e[L] = std::max(m->lvl_max_e[L], f.e);
             m->lvl_max_n[L] = std::max(m->lvl_max_n[L], f.n);
             m->lvl_max_asm[L] = std::max(m->lvl_max_asm[L], f.asm1 - f.asm0);
             long long cb = 0;
             for (int c : f.child) if (c >= 0) cb = std::max<long long>(cb, m->meta[c].b);
             m->lvl_max_b[L] = std::max(m->lvl_max_b[L], cb);
-            m->lvl_max_ob[L] = std::max<long long>(m->lvl_max_ob[L], f.b);
+            m->lvl_max_ob[L] = std::max(m->lvl_max_ob[L], f.b);
         }
         ws_max = std::max(ws_max, wso);
-        wv_max = std::max(wv_max, wvo);
-        m->lvl_wv[L] = wvo;
-        // levels of few fronts (the top of the tree) split their long boundary products over CTAs
-        const long long nsplit = (m->lvl_max_ob[L] + MF_CW - 1) / MF_CW;
-        if (nsplit > 1 && m->levels[L].size() < 148) m->part_n = std::max(m->part_n, nsplit * wvo);
+        m->lvl_yl[L] = yo - m->lvl_y0[L];
+        // levels of few fronts (the top of the tree) split their boundary products until every SM has four CTAs
+        const long long tiles = (m->lvl_max_e[L] + 31) / 32 * (long long)m->levels[L].size();
+        const long long most = (m->lvl_max_ob[L] + MF_KC - 1) / MF_KC;
+        if (tiles > 0) m->lvl_split[L] = (int)std::max(1LL, std::min(most, (4 * 148 + tiles - 1) / tiles));
+        if (m->lvl_split[L] > 1) m->part_n = std::max(m->part_n, m->lvl_split[L] * m->lvl_yl[L]);
         // the level's fronts get their update blocks; their children's are freed once the level assembled
         for (int v : m->levels[L]) {
             FrontMeta& f = m->meta[v];
@@ -1268,7 +1179,8 @@ int emfem_mf_create(emfem_handle h, int64_t n, int n_fronts, const int32_t* e, c
                 if (c >= 0) release(m->meta[c].upd, (long long)m->meta[c].b * m->meta[c].b);
     }
     m->fact_n = fact; m->inv_n = inv; m->piv_n = pivo; m->ws_n = ws_max; m->upd_n = upd_top;
-    m->wv_n = wv_max; m->uv_n = uv; m->y_n = y;
+    m->wv_n = wv; m->y_n = yo;
+    if (wv >= (1LL << 31)) { delete m; set_error("emfem_mf_create: %lld front rows exceed int32", wv); return EMFEM_ERR_INVALID_ARG; }
     for (int v = 0; v < n_fronts; v++) {
         double E = e[v], B = b[v];
         m->flops += 8.0 * (E * E * E / 3 + E * E * B + E * B * B);
@@ -1324,18 +1236,20 @@ int emfem_mf_create(emfem_handle h, int64_t n, int n_fronts, const int32_t* e, c
     mk((void**)&m->upd, sizeof(float2) * upd_top);
     mk((void**)&m->d_npert, sizeof(int));
     mk((void**)&m->d_scale, sizeof(double) * n);
+    mk((void**)&m->d_cmap, sizeof(int) * 2 * wv);
     if (rc != EMFEM_OK) { mf_free(m); delete m; return rc; }
-    rc = check_cuda(cudaFuncSetAttribute(mf_fwd_block_kernel<1, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)MF_BLOCK_SMEM), "cudaFuncSetAttribute");
+    rc = check_cuda(cudaFuncSetAttribute(mf_block_inverse_kernel<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)sizeof(MfInvSmem<float2>)), "cudaFuncSetAttribute");
     if (rc == EMFEM_OK)
-        rc = check_cuda(cudaFuncSetAttribute(mf_bwd_block_kernel<1, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)MF_BLOCK_SMEM), "cudaFuncSetAttribute");
-    if (rc == EMFEM_OK)
-        rc = check_cuda(cudaFuncSetAttribute(mf_fwd_block_kernel<2, MF_BLOCK_NT_FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)MF_BLOCK_SMEM2), "cudaFuncSetAttribute");
-    if (rc == EMFEM_OK)
-        rc = check_cuda(cudaFuncSetAttribute(mf_bwd_block_kernel<2, MF_BLOCK_NT_FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)MF_BLOCK_SMEM2), "cudaFuncSetAttribute");
+        rc = check_cuda(cudaFuncSetAttribute(mf_block_inverse_kernel<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)sizeof(MfInvSmem<double2>)), "cudaFuncSetAttribute");
+    if (rc == EMFEM_OK) rc = check_cuda(cudaMemsetAsync(m->d_cmap, 0xff, sizeof(int) * 2 * wv, h->h.stream), "cudaMemsetAsync");
+    if (rc == EMFEM_OK) {
+        for (int v0 = 0; v0 < n_fronts; v0 += 65535)
+            mf_child_rows_kernel<<<dim3(4, std::min(65535, n_fronts - v0)), 256, 0, h->h.stream>>>(v0, n_fronts, m->d_meta,
+                                                                                                   m->d_ea, m->d_cmap, wv);
+        rc = check_cuda(cudaGetLastError(), "mf_child_rows_kernel");
+    }
     if (rc != EMFEM_OK) { mf_free(m); delete m; return rc; }
     *out = m;
     return EMFEM_OK;
