@@ -111,7 +111,7 @@ struct FrontMeta {        // per front, device
     int e, b, n, parent;
     int child[2];
     long long fdof, ea, asm0, asm1;   // offsets into fdof / ea / asm arrays
-    long long fact, inv, piv;         // factor store offsets (float2 / float2 / int)
+    long long fact, inv;              // factor store offsets (float2)
     long long ws, upd;                // level workspace (float2) / update store (float2) offsets
     long long wv, y;                  // solve buffers: the front's rows of w, its own rows of y
 };
@@ -185,181 +185,227 @@ __global__ void mf_ea_kernel(const int* __restrict__ lst, const FrontMeta* __res
     }
 }
 
+// Index order of non-negative values as unsigned words, for the pivot search (redux instructions).
+__device__ __forceinline__ unsigned mf_max_key(float v, unsigned all, bool in) {
+    const unsigned k = in ? __float_as_uint(v) : 0u;
+    const unsigned mx = __reduce_max_sync(all, k);          // every lane takes part, candidate or not
+    return __ballot_sync(all, in && k == mx);
+}
+__device__ __forceinline__ unsigned mf_max_key(double v, unsigned all, bool in) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    const unsigned hi = in ? (unsigned)(b >> 32) : 0u;
+    const unsigned mh = __reduce_max_sync(all, hi);
+    const bool top = in && hi == mh;
+    const unsigned lo = top ? (unsigned)b : 0u;
+    const unsigned ml = __reduce_max_sync(all, lo);
+    return __ballot_sync(all, top && lo == ml);
+}
+__device__ __forceinline__ float mf_shfl(float v, int l) { return __shfl_sync(0xffffffffu, v, l); }
+__device__ __forceinline__ double mf_shfl(double v, int l) { return __shfl_sync(0xffffffffu, v, l); }
+
 // LU with partial pivoting of the 32 x 32 diagonal block at step k, plus the explicit inverses of its
-// unit-lower L and upper U.  One warp per front; lane = column (or row in the pivot search).  The
-// inverses go to inv (complex64, read by the solves) and, for a complex128 factorization, also to invc
-// (complex128, read by the panel kernel); for complex64 invc is inv.
+// unit-lower L and upper U.  One CTA per front.  It is a serial step of every front's chain, bound by latency:
+// warp 0 factors with a row per lane in registers (rows exchange places in `pos`, not in the registers; the
+// pivot search is two or three redux instructions), then warp 0 forms the inverse of U and warp 1 that of L,
+// a column per lane, adding each solved entry to all entries that need it (independent sums instead of one
+// dot product after the other).  64 us a step with the block in shared memory, 45 us now (cavity of 82 944
+// tets).  The inverses go to inv (complex64, read by the solves) and, for a complex128 factorization, also to
+// invc (complex128, read by the panel kernel); for complex64 invc is inv.
 template <typename T>
-__global__ void __launch_bounds__(32) mf_diag_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm, int k,
+__global__ void __launch_bounds__(64) mf_diag_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm, int k,
                                                      T* __restrict__ ws, float2* __restrict__ inv, T* __restrict__ invc,
-                                                     int* __restrict__ piv, int* __restrict__ nperturbed) {
+                                                     int* __restrict__ nperturbed) {
     typedef typename CxT<T>::R R;
     __shared__ T D[MF_NB][MF_NB + 1];
     __shared__ T X[MF_NB][MF_NB + 1];
+    __shared__ T dinv[MF_NB];
+    __shared__ int sq[MF_NB];
     const FrontMeta& f = fm[lst[blockIdx.x]];
     if (k >= f.e) return;
     const int kb = min(MF_NB, f.e - k);
-    const int lane = threadIdx.x;
+    const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
     const long long ld = f.n;
     T* W = ws + f.ws + k + (long long)k * ld;
     const T zero = CxT<T>::make(0.0, 0.0);
-    R bmax = 0;
-    for (int c = 0; c < kb; c++) {
-        T v = lane < kb ? W[lane + (long long)c * ld] : zero;
-        D[lane][c] = v;
-        bmax = max(bmax, cabs2(v));
+    if (wl == 0) {
+        const unsigned all = 0xffffffffu;
+        T a[MF_NB];
+        R bmax = 0;
+#pragma unroll
+        for (int c = 0; c < MF_NB; c++) {
+            a[c] = (lane < kb && c < kb) ? W[lane + (long long)c * ld] : zero;
+            bmax = max(bmax, cabs2(a[c]));
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) bmax = max(bmax, __shfl_xor_sync(all, bmax, o));
+        const R floor2 = max(bmax, (R)1e-30) * (R)1e-12;      // (1e-6 of the block's largest entry)^2
+        int pos = lane, pert = 0;
+#pragma unroll
+        for (int j = 0; j < MF_NB; j++) {
+            if (j >= kb) break;
+            // pivot: largest |row[j]| among the rows at positions >= j (ties: smallest position)
+            const unsigned cand = mf_max_key(cabs2(a[j]), all, pos >= j && pos < kb);
+            const int br = (int)__reduce_min_sync(all, (cand >> lane) & 1 ? (unsigned)pos : 64u);
+            const int bl = __ffs(__ballot_sync(all, pos == br)) - 1;
+            pos = pos == br ? j : (pos == j ? br : pos);
+            T d;
+            d.x = mf_shfl(a[j].x, bl);
+            d.y = mf_shfl(a[j].y, bl);
+            if (cabs2(d) < floor2) {
+                const R v = sqrt(cabs2(d)), fl = sqrt(floor2);
+                d = v > 0 ? CxT<T>::make(d.x / v * fl, d.y / v * fl) : CxT<T>::make(fl, 0.0);
+                if (lane == bl) a[j] = d;
+                pert++;
+            }
+            const T pinv = cinv(d);
+            const bool low = pos > j && pos < kb;
+            if (low) a[j] = cmul(a[j], pinv);
+#pragma unroll
+            for (int c = j + 1; c < MF_NB; c++) {
+                T u;
+                u.x = mf_shfl(a[c].x, bl);
+                u.y = mf_shfl(a[c].y, bl);
+                if (low) cfms(a[c], a[j], u);
+            }
+        }
+        if (lane == 0 && pert) atomicAdd(nperturbed, pert);
+        sq[pos] = lane;
+#pragma unroll
+        for (int c = 0; c < MF_NB; c++) D[pos][c] = a[c];
+        __syncwarp();
+        if (lane < kb) dinv[lane] = cinv(D[lane][lane]);
     }
-    for (int o = 16; o > 0; o >>= 1) bmax = max(bmax, __shfl_xor_sync(0xffffffffu, bmax, o));
-    const R floor2 = max(bmax, (R)1e-30) * (R)1e-12;      // (1e-6 of the block's largest entry)^2
+    __syncthreads();
+    if (wl == 1) {                                  // write L\U back while the inverses are formed
+        for (int c = 0; c < kb; c++)
+            if (lane < kb) W[lane + (long long)c * ld] = D[lane][c];
+    }
+    {
+        // column `lane` of the inverse; t[i] collects the sum that entry i needs
+        T t[MF_NB];
+#pragma unroll
+        for (int i = 0; i < MF_NB; i++) t[i] = zero;
+        if (wl == 0) {
+#pragma unroll
+            for (int i = MF_NB - 1; i >= 0; i--) {
+                T x = zero;
+                if (i < kb && lane < kb && i <= lane) {
+                    x = dinv[i];
+                    if (i < lane) { const T q = cmul(t[i], x); x = CxT<T>::make(-q.x, -q.y); }
+                }
+                if (i < kb) {
+#pragma unroll
+                    for (int r = 0; r < i; r++) cfma(t[r], D[r][i], x);
+                }
+                t[i] = x;
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < MF_NB; i++) {
+                T x = zero;
+                if (i < kb && lane < kb && i >= lane) x = i == lane ? CxT<T>::make(1.0, 0.0) : CxT<T>::make(-t[i].x, -t[i].y);
+                if (i < kb) {
+#pragma unroll
+                    for (int r = i + 1; r < MF_NB; r++) cfma(t[r], D[r][i], x);
+                }
+                t[i] = x;
+            }
+        }
+        // the block's row swaps folded into the inverse of L: position i holds row sq[i], so column sq[c] of
+        // Linv P is column c of Linv
+        const int col = wl == 0 ? lane : sq[lane];
+        __syncthreads();                            // both warps are done with L\U: D takes the inverse of U
+#pragma unroll
+        for (int i = 0; i < MF_NB; i++) (wl == 0 ? D : X)[i][col] = t[i];
+    }
     __syncwarp();
-    int* P = piv + f.piv + k;
-    int pert = 0;
-    for (int j = 0; j < kb; j++) {
-        // pivot: largest |D[r][j]| for r >= j (ties: smallest r)
-        R best = (lane >= j && lane < kb) ? cabs2(D[lane][j]) : (R)-1;
-        int br = lane;
-        for (int o = 16; o > 0; o >>= 1) {
-            R ob = __shfl_xor_sync(0xffffffffu, best, o);
-            int orr = __shfl_xor_sync(0xffffffffu, br, o);
-            if (ob > best || (ob == best && orr < br)) { best = ob; br = orr; }
-        }
-        if (lane == 0) P[j] = br;
-        if (br != j && lane < kb) {
-            T t = D[j][lane];
-            D[j][lane] = D[br][lane];
-            D[br][lane] = t;
-        }
-        __syncwarp();
-        if (lane == 0 && cabs2(D[j][j]) < floor2) {
-            T d = D[j][j];
-            R a = sqrt(cabs2(d));
-            R fl = sqrt(floor2);
-            D[j][j] = a > 0 ? CxT<T>::make(d.x / a * fl, d.y / a * fl) : CxT<T>::make(fl, 0.0);
-            pert++;
-        }
-        __syncwarp();
-        T pinv = cinv(D[j][j]);
-        if (lane > j && lane < kb) D[lane][j] = cmul(D[lane][j], pinv);
-        __syncwarp();
-        if (lane > j && lane < kb) {
-            T u = D[j][lane];
-            for (int r = j + 1; r < kb; r++) cfms(D[r][lane], D[r][j], u);
-        }
-        __syncwarp();
-    }
-    if (lane == 0 && pert) atomicAdd(nperturbed, pert);
-    // write L\U back
-    for (int c = 0; c < kb; c++)
-        if (lane < kb) W[lane + (long long)c * ld] = D[lane][c];
-    const long long ib = f.inv + (long long)(k / MF_NB) * 2 * MF_NB * MF_NB;   // Linv then Uinv, column-major 32x32
-    float2* Li = inv + ib;
-    float2* Ui = Li + MF_NB * MF_NB;
-    T* Lc = invc + ib;
-    T* Uc = Lc + MF_NB * MF_NB;
+    // Linv P, then Uinv: column-major 32 x 32 each
+    const long long ib = f.inv + (long long)(k / MF_NB) * 2 * MF_NB * MF_NB + (wl == 0 ? MF_NB * MF_NB : 0);
     constexpr bool wide = sizeof(T) != sizeof(float2);
-    // Uinv: lane = column c of X = U^-1 (back substitution, own column only)
-    {
-        int c = lane;
-        for (int i = 0; i < MF_NB; i++) X[i][c] = zero;
-        if (c < kb) {
-            X[c][c] = cinv(D[c][c]);
-            for (int i = c - 1; i >= 0; i--) {
-                T s = zero;
-                for (int t = i + 1; t <= c; t++) cfma(s, D[i][t], X[t][c]);
-                T q = cmul(s, cinv(D[i][i]));
-                X[i][c] = CxT<T>::make(-q.x, -q.y);
-            }
-        }
-    }
-    __syncwarp();
     for (int c = 0; c < MF_NB; c++) {
-        Ui[lane + c * MF_NB] = to_c64(X[lane][c]);
-        if (wide) Uc[lane + c * MF_NB] = X[lane][c];
-    }
-    __syncwarp();
-    // Linv: lane = column c of Y = L^-1 (unit lower, forward substitution)
-    {
-        int c = lane;
-        for (int i = 0; i < MF_NB; i++) X[i][c] = zero;
-        if (c < kb) {
-            X[c][c] = CxT<T>::make(1.0, 0.0);
-            for (int i = c + 1; i < kb; i++) {
-                T s = zero;
-                for (int t = c; t < i; t++) cfma(s, D[i][t], X[t][c]);
-                X[i][c] = CxT<T>::make(-s.x, -s.y);
-            }
-        }
-    }
-    __syncwarp();
-    // the block's row swaps folded into the inverse: w' = P w (swaps j = 0..kb-1 in order) has
-    // w'[i] = w[q[i]], so y = Linv w' = (Linv P) w with column q[i] of Linv P = column i of Linv
-    int q[MF_NB];
-#pragma unroll
-    for (int i = 0; i < MF_NB; i++) q[i] = i;
-    for (int j = 0; j < kb; j++) {
-        int r = P[j];
-        int a = 0, b2 = 0;
-#pragma unroll
-        for (int i = 0; i < MF_NB; i++) { if (i == j) a = q[i]; if (i == r) b2 = q[i]; }
-#pragma unroll
-        for (int i = 0; i < MF_NB; i++) { if (i == j) q[i] = b2; if (i == r) q[i] = a; }
-    }
-#pragma unroll
-    for (int i = 0; i < MF_NB; i++) {
-        Li[lane + q[i] * MF_NB] = to_c64(X[lane][i]);
-        if (wide) Lc[lane + q[i] * MF_NB] = X[lane][i];
+        const T v = (wl == 0 ? D : X)[lane][c];
+        inv[ib + lane + c * MF_NB] = to_c64(v);
+        if (wide) invc[ib + lane + c * MF_NB] = v;
     }
 }
 
-// Block row (columns >= k + kb): row swaps, then L^-1; block column (rows >= k + kb): times U^-1.
-// Items 0 .. m-1 are columns, m .. 2m-1 rows (m = n - k - kb).
-template <typename T>
+// Block row (columns >= k + kb): row swaps and L^-1; block column (rows >= k + kb): times U^-1.  A CTA takes a
+// tile of TW columns (the first nt of grid.x) or rows, staged in shared memory with coalesced loads, as a
+// small product with the 32 x 32 inverse, 2 x TW / 16 results per thread.  One row or column per thread
+// read the block row with a stride of the front and ran on a fraction of the SMs: 58 us a step on the
+// 82 944-tet cavity, 21 us now.
+template <typename T, int TW>
 __global__ void __launch_bounds__(256) mf_panel_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm, int k,
-                                                       T* __restrict__ ws, const T* __restrict__ invc,
-                                                       const int* __restrict__ piv) {
-    __shared__ T Li[MF_NB * MF_NB];
-    __shared__ T Ui[MF_NB * MF_NB];
+                                                       int nt, T* __restrict__ ws, const T* __restrict__ invc) {
+    __shared__ T A[MF_NB][MF_NB + 1];                // inverse: [t][i] (block row) or [t][c] (block column)
+    __shared__ T V[MF_NB][TW + 1];                   // tile: [t][column] or [t][row]
     const FrontMeta& f = fm[lst[blockIdx.y]];
     if (k >= f.e) return;
-    const int kb = min(MF_NB, f.e - k);
-    const long long m = f.n - k - kb;
-    long long item = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if ((long long)blockIdx.x * blockDim.x >= 2 * m) return;
-    const T* L = invc + f.inv + (long long)(k / MF_NB) * 2 * MF_NB * MF_NB;
-    for (int t = threadIdx.x; t < MF_NB * MF_NB; t += blockDim.x) { Li[t] = L[t]; Ui[t] = L[MF_NB * MF_NB + t]; }
-    __syncthreads();
-    if (item >= 2 * m) return;
+    const int kb = min(MF_NB, f.e - k), m = f.n - k - kb;
+    const bool rowblk = (int)blockIdx.x < nt;
+    const int x0 = ((int)blockIdx.x - (rowblk ? 0 : nt)) * TW;
+    if (x0 >= m) return;
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     const long long ld = f.n;
     T* W = ws + f.ws;
     const T zero = CxT<T>::make(0.0, 0.0);
-    T v[MF_NB];
-    if (item < m) {
-        long long c = k + kb + item;
-        T* col = W + k + c * ld;
+    const T* L = invc + f.inv + (long long)(k / MF_NB) * 2 * MF_NB * MF_NB + (rowblk ? 0 : MF_NB * MF_NB);
+    constexpr int NJ = TW / 16;
+    if (rowblk) {
+        T* C = W + k + (long long)(k + kb + x0) * ld;      // kb rows x (up to) TW columns
+        for (int q = tid; q < MF_NB * MF_NB; q += 256) A[q / MF_NB][q % MF_NB] = L[q];          // Li[i + t * 32]
+        for (int q = tid; q < MF_NB * TW; q += 256) {
+            const int t = q % MF_NB, c = q / MF_NB;
+            V[t][c] = (t < kb && x0 + c < m) ? C[t + c * ld] : zero;
+        }
+        __syncthreads();
+        T o[2][NJ];
 #pragma unroll
-        for (int i = 0; i < MF_NB; i++) v[i] = i < kb ? col[i] : zero;
+        for (int j = 0; j < NJ; j++) o[0][j] = o[1][j] = zero;
+#pragma unroll 8
+        for (int t = 0; t < MF_NB; t++) {
+            const T a0 = A[t][tx], a1 = A[t][tx + 16];
 #pragma unroll
-        for (int i = 0; i < MF_NB; i++) {
-            if (i < kb) {
-                T s = zero;
-#pragma unroll
-                for (int t = 0; t < MF_NB; t++) cfma(s, Li[i + t * MF_NB], v[t]);   // (Linv P) times the column
-                col[i] = s;
+            for (int j = 0; j < NJ; j++) {
+                const T v = V[t][ty + 16 * j];
+                cfma(o[0][j], a0, v);                 // (Linv P) times the column
+                cfma(o[1][j], a1, v);
             }
         }
+#pragma unroll
+        for (int j = 0; j < NJ; j++) {
+            const int c = ty + 16 * j;
+            if (x0 + c >= m) continue;
+            if (tx < kb) C[tx + c * ld] = o[0][j];
+            if (tx + 16 < kb) C[tx + 16 + c * ld] = o[1][j];
+        }
     } else {
-        long long r = k + kb + (item - m);
-        T* row = W + r + (long long)k * ld;
+        T* C = W + (k + kb + x0) + (long long)k * ld;      // (up to) TW rows x kb columns
+        for (int q = tid; q < MF_NB * MF_NB; q += 256) A[q % MF_NB][q / MF_NB] = L[q];          // Ui[t + c * 32]
+        for (int q = tid; q < MF_NB * TW; q += 256) {
+            const int r = q % TW, t = q / TW;
+            V[t][r] = (t < kb && x0 + r < m) ? C[r + t * ld] : zero;
+        }
+        __syncthreads();
+        T o[2][NJ];
 #pragma unroll
-        for (int i = 0; i < MF_NB; i++) v[i] = i < kb ? row[(long long)i * ld] : zero;
+        for (int j = 0; j < NJ; j++) o[0][j] = o[1][j] = zero;
+#pragma unroll 8
+        for (int t = 0; t < MF_NB; t++) {
+            const T a0 = A[t][ty], a1 = A[t][ty + 16];
 #pragma unroll
-        for (int c = 0; c < MF_NB; c++) {
-            if (c < kb) {
-                T s = zero;
-#pragma unroll
-                for (int t = 0; t < MF_NB; t++) cfma(s, v[t], Ui[t + c * MF_NB]);
-                row[(long long)c * ld] = s;
+            for (int j = 0; j < NJ; j++) {
+                const T v = V[t][tx + 16 * j];
+                cfma(o[0][j], v, a0);
+                cfma(o[1][j], v, a1);
             }
+        }
+#pragma unroll
+        for (int j = 0; j < NJ; j++) {
+            const int r = tx + 16 * j;
+            if (x0 + r >= m) continue;
+            if (ty < kb) C[r + ty * ld] = o[0][j];
+            if (ty + 16 < kb) C[r + (ty + 16) * ld] = o[1][j];
         }
     }
 }
@@ -885,13 +931,12 @@ struct emfem_mf_s {
     double* d_scale = nullptr;                    // equilibration D^-1/2 of the current factorization
     float2* fact = nullptr;
     float2* inv = nullptr;
-    int* piv = nullptr;
     void* ws = nullptr;                           // level workspace, complex64 or (wide) complex128
     void* upd = nullptr;                          // update store, same precision as ws
     void* invc = nullptr;                         // complex128 copies of the inverse blocks (wide only)
     bool wide = false;                            // fronts factored in complex128
     int* d_npert = nullptr;
-    long long fact_n = 0, inv_n = 0, piv_n = 0, ws_n = 0, upd_n = 0;
+    long long fact_n = 0, inv_n = 0, ws_n = 0, upd_n = 0;
     long long wv_n = 0, y_n = 0;                  // solve buffer rows
     std::vector<long long> lvl_y0, lvl_yl;        // per level: first row of y and rows of y (its fronts' own rows)
     std::vector<int> lvl_max_ob;                  // per level: largest boundary
@@ -910,7 +955,7 @@ struct emfem_mf_s {
 };
 
 static void mf_free(emfem_mf_s* m) {
-    void* ps[] = {m->d_meta, m->d_lst, m->d_fdof, m->d_ea, m->d_slot, m->d_off, m->d_free, m->d_scale, m->fact, m->inv, m->piv,
+    void* ps[] = {m->d_meta, m->d_lst, m->d_fdof, m->d_ea, m->d_slot, m->d_off, m->d_free, m->d_scale, m->fact, m->inv,
                   m->ws, m->upd, m->invc, m->d_npert, m->d_cmap, m->sw, m->sy, m->sx, m->spart};
     for (void* p : ps)
         if (p) cudaFree(p);
@@ -1046,10 +1091,12 @@ static int mf_factor_levels(emfem_mf_s* m, const double2* K_vals, cudaStream_t s
             for (int c = 0; c < 2; c++)
                 mf_ea_kernel<T><<<dim3(nblk(maxb * maxb, MF_CHUNK), ny), 256, 0, s>>>(lst, m->d_meta, c, m->d_ea, upd, ws);
             for (int k = 0; k < m->lvl_max_e[L]; k += MF_NB) {
-                mf_diag_kernel<T><<<ny, 32, 0, s>>>(lst, m->d_meta, k, ws, m->inv, invc, m->piv, m->d_npert);
+                mf_diag_kernel<T><<<ny, 64, 0, s>>>(lst, m->d_meta, k, ws, m->inv, invc, m->d_npert);
                 long long mm = maxn - k - 1;
                 if (mm < 1) mm = 1;
-                mf_panel_kernel<T><<<dim3(nblk(2 * mm, 256), ny), 256, 0, s>>>(lst, m->d_meta, k, ws, invc, m->piv);
+                constexpr int TW = sizeof(T) == sizeof(float2) ? 64 : 32;     // tiles within static shared memory
+                const unsigned npt = nblk(mm, TW);
+                mf_panel_kernel<T, TW><<<dim3(2 * npt, ny), 256, 0, s>>>(lst, m->d_meta, k, (int)npt, ws, invc);
                 long long nt = (mm + MF_TILE - 1) / MF_TILE;
                 mf_trail_kernel<T><<<dim3((unsigned)std::max(1LL, nt * nt), ny), 256, 0, s>>>(lst, m->d_meta, k, ws);
             }
@@ -1095,7 +1142,7 @@ int emfem_mf_create(emfem_handle h, int64_t n, int n_fronts, const int32_t* e, c
     m->levels.assign(nl, {});
     for (int v = 0; v < n_fronts; v++) m->levels[level[v]].push_back(v);
     // offsets
-    long long fact = 0, inv = 0, pivo = 0, eao = 0;
+    long long fact = 0, inv = 0, eao = 0;
     for (int v = 0; v < n_fronts; v++) {
         FrontMeta& f = m->meta[v];
         f.e = e[v]; f.b = b[v]; f.n = e[v] + b[v]; f.parent = parent[v];
@@ -1105,7 +1152,6 @@ int emfem_mf_create(emfem_handle h, int64_t n, int n_fronts, const int32_t* e, c
         f.asm0 = asm_ptr ? asm_ptr[v] : 0; f.asm1 = asm_ptr ? asm_ptr[v + 1] : 0;
         f.fact = fact; fact += (long long)f.n * f.e + (long long)f.e * f.b;
         f.inv = inv; inv += (long long)((f.e + MF_NB - 1) / MF_NB) * 2 * MF_NB * MF_NB;
-        f.piv = pivo; pivo += f.e;
     }
     for (int v = 0; v < n_fronts; v++) {
         int p = parent[v];
@@ -1178,7 +1224,7 @@ int emfem_mf_create(emfem_handle h, int64_t n, int n_fronts, const int32_t* e, c
             for (int c : m->meta[v].child)
                 if (c >= 0) release(m->meta[c].upd, (long long)m->meta[c].b * m->meta[c].b);
     }
-    m->fact_n = fact; m->inv_n = inv; m->piv_n = pivo; m->ws_n = ws_max; m->upd_n = upd_top;
+    m->fact_n = fact; m->inv_n = inv; m->ws_n = ws_max; m->upd_n = upd_top;
     m->wv_n = wv; m->y_n = yo;
     if (wv >= (1LL << 31)) { delete m; set_error("emfem_mf_create: %lld front rows exceed int32", wv); return EMFEM_ERR_INVALID_ARG; }
     for (int v = 0; v < n_fronts; v++) {
@@ -1231,7 +1277,6 @@ int emfem_mf_create(emfem_handle h, int64_t n, int n_fronts, const int32_t* e, c
     };
     mk((void**)&m->fact, sizeof(float2) * fact);
     mk((void**)&m->inv, sizeof(float2) * inv);
-    mk((void**)&m->piv, sizeof(int) * pivo);
     mk((void**)&m->ws, sizeof(float2) * ws_max);
     mk((void**)&m->upd, sizeof(float2) * upd_top);
     mk((void**)&m->d_npert, sizeof(int));
@@ -1259,7 +1304,7 @@ int emfem_mf_info(emfem_mf m, size_t* device_bytes, double* flops, int* n_levels
     EMFEM_REQUIRE(m, "emfem_mf_info: bad handle");
     if (device_bytes)
         *device_bytes = sizeof(float2) * (m->fact_n + m->inv_n) + (m->wide ? sizeof(double2) : sizeof(float2)) *
-                        (m->ws_n + m->upd_n) + (m->wide ? sizeof(double2) * m->inv_n : 0) + sizeof(int) * m->piv_n +
+                        (m->ws_n + m->upd_n) + (m->wide ? sizeof(double2) * m->inv_n : 0) + sizeof(int) * 2 * m->wv_n +
                         sizeof(double) * m->n;
     if (flops) *flops = m->flops;
     if (n_levels) *n_levels = (int)m->levels.size();
