@@ -410,79 +410,125 @@ __global__ void __launch_bounds__(256) mf_panel_kernel(const int* __restrict__ l
     }
 }
 
-// Trailing update C -= A B on 64 x 64 tiles: A = W[k+kb.., k..k+kb), B = W[k..k+kb, k+kb..).  The k
-// extent runs in stages of KH columns (32 for complex64: one stage; 16 for complex128, whose tiles
-// would otherwise exceed the static shared-memory limit).
-template <typename T>
-__global__ void __launch_bounds__(256) mf_trail_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm, int k,
-                                                       T* __restrict__ ws) {
-    constexpr int KH = sizeof(T) == sizeof(float2) ? MF_NB : MF_NB / 2;
-    __shared__ T As[KH][MF_TILE + 1];
-    __shared__ T Bs[KH][MF_TILE + 1];
-    const FrontMeta& f = fm[lst[blockIdx.y]];
-    if (k >= f.e) return;
-    const int kb = min(MF_NB, f.e - k);
-    const long long m = f.n - k - kb;
-    const long long nt = (m + MF_TILE - 1) / MF_TILE;
-    if ((long long)blockIdx.x >= nt * nt) return;
-    const long long ti = blockIdx.x % nt, tj = blockIdx.x / nt;
-    const long long r0 = k + kb + ti * MF_TILE, c0 = k + kb + tj * MF_TILE;
-    const long long ld = f.n;
-    T* W = ws + f.ws;
-    const int tid = threadIdx.x;
-    const int tx = tid % 16, ty = tid / 16;
+// Update C -= A B of one tile of TM x 64 entries: A = W[rows, ka .. ka + kw), B = W[ka .. ka + kw, columns).
+// 256 threads, TM / 16 x 4 accumulators each; the k extent runs in stages of KS columns, NSTG of them in
+// flight by asynchronous copies, and the tile's C entries come straight into the accumulators meanwhile.
+// Every entry is updated in ascending k, so how the k extent is cut into calls does not change a bit.
+template <typename T> struct MfTile { static constexpr int KS = sizeof(T) == sizeof(float2) ? 16 : 8, NSTG = 3; };
+template <typename T, int TM>
+struct MfTileSmem {
+    T a[MfTile<T>::NSTG][MfTile<T>::KS][TM + 1];
+    T b[MfTile<T>::NSTG][MfTile<T>::KS][MF_TILE + 1];
+};
+template <typename T, int TM>
+__device__ __forceinline__ void mf_tile_update(MfTileSmem<T, TM>& sm, T* W, int ld, int r0, int r1, int c0, int c1, int ka, int kw) {
+    constexpr int KS = MfTile<T>::KS, NSTG = MfTile<T>::NSTG, NI = TM / 16;
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     const T zero = CxT<T>::make(0.0, 0.0);
-    T acc[4][4];
-    for (int k2 = 0; k2 < kb; k2 += KH) {
-        if (k2) __syncthreads();                  // the previous stage's tiles are consumed
-        // A tile (64 rows x KH) and B tile (KH x 64 cols) by asynchronous copies; out-of-range parts zeroed
-        for (int t = tid; t < KH * MF_TILE; t += 256) {
-            int rr = t % MF_TILE, kk = t / MF_TILE;
-            long long r = r0 + rr;
-            if (k2 + kk < kb && r < f.n) cp_async_c(&As[kk][rr], &W[r + (long long)(k + k2 + kk) * ld]);
-            else As[kk][rr] = zero;
-            int kk2 = t % KH, cc = t / KH;
-            long long c = c0 + cc;
-            if (k2 + kk2 < kb && c < f.n) cp_async_c(&Bs[kk2][cc], &W[(k + k2 + kk2) + c * ld]);
-            else Bs[kk2][cc] = zero;
-        }
-        if (k2 == 0) {
-            // the thread's 16 C entries go straight into its accumulators while the tiles are in flight
+    const int nst = (kw + KS - 1) / KS;
+    const int ar = tid % TM, ak = tid / TM, bk = tid % KS, bc = tid / KS;       // the thread's share of a stage
+    const T* A = W + r0 + ar + (long long)(ka + ak) * ld;
+    const T* B = W + ka + bk + (long long)(c0 + bc) * ld;
+    auto stage = [&](int st) {
+        if (st < nst) {
+            const int k0 = st * KS, slot = st % NSTG;
+            const T* pa = A + (long long)k0 * ld;
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                long long c = c0 + ty + 16 * j;
+            for (int u = 0; u < KS * TM / 256; u++) {
+                const int kk = ak + u * (256 / TM);
+                if (k0 + kk < kw && r0 + ar < r1) cp_async_c(&sm.a[slot][kk][ar], pa + (long long)(u * (256 / TM)) * ld);
+                else sm.a[slot][kk][ar] = zero;
+            }
+            const T* pb = B + k0;
 #pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    long long r = r0 + tx + 16 * i;
-                    acc[i][j] = (r < f.n && c < f.n) ? W[r + c * ld] : zero;
-                }
+            for (int u = 0; u < KS * MF_TILE / 256; u++) {
+                const int cc = bc + u * (256 / KS);
+                if (k0 + bk < kw && c0 + cc < c1) cp_async_c(&sm.b[slot][bk][cc], pb + (long long)(u * (256 / KS)) * ld);
+                else sm.b[slot][bk][cc] = zero;
             }
         }
-        cp_async_wait_all();
-        __syncthreads();
-        const int kn = min(KH, kb - k2);
-        for (int kk = 0; kk < kn; kk++) {
-            T a[4], b[4];
+        cp_async_commit();
+    };
 #pragma unroll
-            for (int i = 0; i < 4; i++) a[i] = As[kk][tx + 16 * i];
+    for (int st = 0; st < NSTG - 1; st++) stage(st);
+    T acc[NI][4];
 #pragma unroll
-            for (int j = 0; j < 4; j++) b[j] = Bs[kk][ty + 16 * j];
+    for (int j = 0; j < 4; j++) {
+        const int c = c0 + ty + 16 * j;
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+        for (int i = 0; i < NI; i++) {
+            const int r = r0 + tx + 16 * i;
+            acc[i][j] = (r < r1 && c < c1) ? W[r + (long long)c * ld] : zero;
+        }
+    }
+    for (int st = 0; st < nst; st++) {
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(NSTG - 2) : "memory");
+        __syncthreads();                       // stage st has landed, stage st - 1 is consumed
+        stage(st + NSTG - 1);
+        const int slot = st % NSTG;
 #pragma unroll
-                for (int j = 0; j < 4; j++) cfms(acc[i][j], a[i], b[j]);
+        for (int kk = 0; kk < KS; kk++) {
+            T av[NI], bv[4];
+#pragma unroll
+            for (int i = 0; i < NI; i++) av[i] = sm.a[slot][kk][tx + 16 * i];
+#pragma unroll
+            for (int j = 0; j < 4; j++) bv[j] = sm.b[slot][kk][ty + 16 * j];
+#pragma unroll
+            for (int i = 0; i < NI; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) cfms(acc[i][j], av[i], bv[j]);
         }
     }
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-        long long c = c0 + ty + 16 * j;
-        if (c >= f.n) continue;
+        const int c = c0 + ty + 16 * j;
+        if (c >= c1) continue;
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            long long r = r0 + tx + 16 * i;
-            if (r < f.n) W[r + c * ld] = acc[i][j];
+        for (int i = 0; i < NI; i++) {
+            const int r = r0 + tx + 16 * i;
+            if (r < r1) W[r + (long long)c * ld] = acc[i][j];
         }
     }
+}
+
+// The trailing update is cut in two: eliminating a step of 32 columns updates only the columns and rows of
+// its outer block (MF_OB columns), which the block's next steps need, and the rest of the front is updated
+// once per outer block with rank MF_OB.  C is then read and written once per MF_OB eliminated columns
+// instead of once per 32: with rank 32 a tile moved 96 KB for a million flops, a quarter of DRAM's rate at half
+// of the FMA pipe's, and the tiles' pipeline never filled.  Same sums in the same order.
+constexpr int MF_OB = 128;
+
+// Step k: strips of the outer block [ks, ke): columns [k + kb, ke) of all rows below k + kb (tiles x < nr), and
+// rows [k + kb, ke) of the columns from ke on.
+template <typename T>
+__global__ void __launch_bounds__(256) mf_strip_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm, int k,
+                                                       int ob, int nr, T* __restrict__ ws) {
+    extern __shared__ __align__(16) unsigned char mf_smem[];
+    MfTileSmem<T, 64>& sm = *reinterpret_cast<MfTileSmem<T, 64>*>(mf_smem);
+    const FrontMeta& f = fm[lst[blockIdx.y]];
+    const int k1 = k + MF_NB, ke = min(ob + MF_OB, f.e);
+    if (k1 >= ke) return;                        // the outer block's last step: nothing left inside it
+    const int half = blockIdx.x & 1, t = blockIdx.x >> 1;      // the strip is at most 96 wide: two tiles
+    const bool cols = t < nr;
+    const int along = (cols ? k1 : ke) + (cols ? t : t - nr) * 64, across = k1 + half * 64;
+    if (along >= f.n || across >= ke) return;
+    if (cols) mf_tile_update<T, 64>(sm, ws + f.ws, f.n, along, f.n, across, ke, k, MF_NB);
+    else mf_tile_update<T, 64>(sm, ws + f.ws, f.n, across, ke, along, f.n, k, MF_NB);
+}
+
+// Rank-(ke - ob) update of everything below and right of the outer block [ob, ke)
+template <typename T, int TM>
+__global__ void __launch_bounds__(256, TM > 64 || sizeof(T) > 8 ? 2 : 3) mf_trail_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm,
+                                                                         int ob, T* __restrict__ ws) {
+    extern __shared__ __align__(16) unsigned char mf_smem[];
+    MfTileSmem<T, TM>& sm = *reinterpret_cast<MfTileSmem<T, TM>*>(mf_smem);
+    const FrontMeta& f = fm[lst[blockIdx.y]];
+    if (ob >= f.e) return;
+    const int ke = min(ob + MF_OB, f.e), m = f.n - ke;
+    const int nr = (m + TM - 1) / TM, nc = (m + MF_TILE - 1) / MF_TILE;
+    if ((int)blockIdx.x >= nr * nc) return;
+    const int ti = blockIdx.x % nr, tj = blockIdx.x / nr;
+    mf_tile_update<T, TM>(sm, ws + f.ws, f.n, ke + ti * TM, f.n, ke + tj * MF_TILE, f.n, ob, ke - ob);
 }
 
 // Factor columns (n x e) and U block row (e x b), rounded to complex64, and the Schur complement (b x b,
@@ -1069,6 +1115,12 @@ int mf_apply(emfem_mf_s* m, int S, const double2* r, double2* x, cudaStream_t s)
 }
 }  // namespace emfem
 
+// Tiles of 128 rows (8 x 4 accumulators: fewer shared-memory reads per multiply-add) where they still give every
+// SM four of them, else of 64; complex128 accumulators of that size would not fit the registers.
+static bool mf_tall_tiles(long long mt, int ny) {
+    return (mt + 127) / 128 * ((mt + 63) / 64) * ny >= 4 * 148;
+}
+
 // The level loop of one factorization, fronts in workspace precision T.
 template <typename T>
 static int mf_factor_levels(emfem_mf_s* m, const double2* K_vals, cudaStream_t s) {
@@ -1090,15 +1142,31 @@ static int mf_factor_levels(emfem_mf_s* m, const double2* K_vals, cudaStream_t s
                 lst, m->d_meta, K_vals, m->d_slot, m->d_off, m->d_fdof, m->d_scale, ws);
             for (int c = 0; c < 2; c++)
                 mf_ea_kernel<T><<<dim3(nblk(maxb * maxb, MF_CHUNK), ny), 256, 0, s>>>(lst, m->d_meta, c, m->d_ea, upd, ws);
-            for (int k = 0; k < m->lvl_max_e[L]; k += MF_NB) {
+            const int maxe = m->lvl_max_e[L];
+            for (int k = 0; k < maxe; k += MF_NB) {
+                const int ob = k / MF_OB * MF_OB;
                 mf_diag_kernel<T><<<ny, 64, 0, s>>>(lst, m->d_meta, k, ws, m->inv, invc, m->d_npert);
-                long long mm = maxn - k - 1;
-                if (mm < 1) mm = 1;
+                const long long mm = std::max(1LL, maxn - k - 1);
                 constexpr int TW = sizeof(T) == sizeof(float2) ? 64 : 32;     // tiles within static shared memory
                 const unsigned npt = nblk(mm, TW);
                 mf_panel_kernel<T, TW><<<dim3(2 * npt, ny), 256, 0, s>>>(lst, m->d_meta, k, (int)npt, ws, invc);
-                long long nt = (mm + MF_TILE - 1) / MF_TILE;
-                mf_trail_kernel<T><<<dim3((unsigned)std::max(1LL, nt * nt), ny), 256, 0, s>>>(lst, m->d_meta, k, ws);
+                if (k + MF_NB < std::min(ob + MF_OB, maxe)) {
+                    const unsigned nr = nblk(mm, 64);
+                    mf_strip_kernel<T><<<dim3(4 * nr, ny), 256, sizeof(MfTileSmem<T, 64>), s>>>(lst, m->d_meta, k, ob, (int)nr, ws);
+                    continue;
+                }
+                // fronts of the level that ended inside the outer block are updated with their own rank here too
+                const long long mt = std::max(1LL, maxn - ob - 1), nc = (mt + MF_TILE - 1) / MF_TILE;
+                bool tall = false;
+                if constexpr (sizeof(T) == sizeof(float2)) {
+                    tall = mf_tall_tiles(mt, ny);
+                    if (tall)
+                    mf_trail_kernel<T, 128><<<dim3((unsigned)((mt + 127) / 128 * nc), ny), 256, sizeof(MfTileSmem<T, 128>), s>>>(
+                        lst, m->d_meta, ob, ws);
+                }
+                if (!tall)
+                    mf_trail_kernel<T, 64><<<dim3((unsigned)(nc * nc), ny), 256, sizeof(MfTileSmem<T, 64>), s>>>(lst, m->d_meta,
+                                                                                                               ob, ws);
             }
             mf_compact_kernel<T><<<dim3(nblk(maxn * maxn, MF_CHUNK), ny), 256, 0, s>>>(lst, m->d_meta, ws, m->fact, upd);
             if (m->lvl_max_e[L] > MF_NB) {
@@ -1288,6 +1356,21 @@ int emfem_mf_create(emfem_handle h, int64_t n, int n_fronts, const int32_t* e, c
     if (rc == EMFEM_OK)
         rc = check_cuda(cudaFuncSetAttribute(mf_block_inverse_kernel<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)sizeof(MfInvSmem<double2>)), "cudaFuncSetAttribute");
+    if (rc == EMFEM_OK)
+        rc = check_cuda(cudaFuncSetAttribute(mf_strip_kernel<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)sizeof(MfTileSmem<float2, 64>)), "cudaFuncSetAttribute");
+    if (rc == EMFEM_OK)
+        rc = check_cuda(cudaFuncSetAttribute(mf_strip_kernel<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)sizeof(MfTileSmem<double2, 64>)), "cudaFuncSetAttribute");
+    if (rc == EMFEM_OK)
+        rc = check_cuda(cudaFuncSetAttribute(mf_trail_kernel<float2, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)sizeof(MfTileSmem<float2, 64>)), "cudaFuncSetAttribute");
+    if (rc == EMFEM_OK)
+        rc = check_cuda(cudaFuncSetAttribute(mf_trail_kernel<float2, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)sizeof(MfTileSmem<float2, 128>)), "cudaFuncSetAttribute");
+    if (rc == EMFEM_OK)
+        rc = check_cuda(cudaFuncSetAttribute(mf_trail_kernel<double2, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)sizeof(MfTileSmem<double2, 64>)), "cudaFuncSetAttribute");
     if (rc == EMFEM_OK) rc = check_cuda(cudaMemsetAsync(m->d_cmap, 0xff, sizeof(int) * 2 * wv, h->h.stream), "cudaMemsetAsync");
     if (rc == EMFEM_OK) {
         for (int v0 = 0; v0 < n_fronts; v0 += 65535)
