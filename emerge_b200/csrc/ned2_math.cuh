@@ -149,12 +149,11 @@ EMFEM_HD void matinv3(const cd M[9], cd out[9]) {
     for (int i = 0; i < 9; i++) out[i] = cdiv(out[i], det);
 }
 
-// Compute the invariants of one tet into inv[INV_NDOUBLE].
-//   xs,ys,zs: vertex coordinates in the tet's own order; ids: global node ids;
-//   elen: edge lengths in tet_to_edge order; ur, er: row-major 3x3.
-EMFEM_HD void tet_invariants(const double xs[4], const double ys[4], const double zs[4], const int64_t ids[4],
-                             const double elen[6], const cd ur[9], const cd er[9], double* inv) {
-    double G[4][3];
+// Barycentric-gradient numerators G_i (6V grad L_i up to a common sign) and 6V of a tet.
+EMFEM_HD double tet_cofactors(const double xs[4], const double ys[4], const double zs[4], double G[4][3]) {
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
     for (int i = 0; i < 4; i++) {
         int j = i == 0 ? 1 : 0;
         int k = i <= 1 ? 2 : 1;
@@ -167,7 +166,16 @@ EMFEM_HD void tet_invariants(const double xs[4], const double ys[4], const doubl
     double u0 = xs[1] - xs[0], u1 = ys[1] - ys[0], u2 = zs[1] - zs[0];
     double v0 = xs[2] - xs[0], v1 = ys[2] - ys[0], v2 = zs[2] - zs[0];
     double w0 = xs[3] - xs[0], w1 = ys[3] - ys[0], w2 = zs[3] - zs[0];
-    double V6 = fabs(u0 * (v1 * w2 - v2 * w1) + u1 * (v2 * w0 - v0 * w2) + u2 * (v0 * w1 - v1 * w0));
+    return fabs(u0 * (v1 * w2 - v2 * w1) + u1 * (v2 * w0 - v0 * w2) + u2 * (v0 * w1 - v1 * w0));
+}
+
+// Compute the invariants of one tet into inv[INV_NDOUBLE].
+//   xs,ys,zs: vertex coordinates in the tet's own order; ids: global node ids;
+//   elen: edge lengths in tet_to_edge order; ur, er: row-major 3x3.
+EMFEM_HD void tet_invariants(const double xs[4], const double ys[4], const double zs[4], const int64_t ids[4],
+                             const double elen[6], const cd ur[9], const cd er[9], double* inv) {
+    double G[4][3];
+    const double V6 = tet_cofactors(xs, ys, zs, G);
     inv[INV_SD] = 1.0 / (V6 * V6 * V6);
     inv[INV_SF] = 1.0 / V6;
     for (int i = 0; i < 4; i++) for (int j = i + 1; j < 4; j++) {
@@ -225,10 +233,40 @@ struct InvView {
     EMFEM_HD double L(int e) const { return g(INV_L + e); }
 };
 
-// The same accessors over one tet's record in the array-of-structs buffer (records of INV_STRIDE doubles,
-// 16-byte aligned): on the device every complex invariant is one 16-byte load instead of two 8-byte
-// ones, with the same values (so the same results) as InvView.
-struct InvRec {
+// ---- the same blocks with the tet's vertices in ascending global order -------------------------------------
+// In that order every edge and face has its vertices ascending (no orientation to decode per block), the six
+// edges are the six vertex pairs in canonical order, and a block's index sets are small constants.  A record
+// (array of structs, 960 bytes) holds, for the sorted tet: P[a][b] / (6V) / 7! and Q[p][q] / (6V)^3 / 5! (so that the
+// volume coefficients are the integers prod k_i!), the distances and edge lengths by vertex pair, and the sorted
+// slot of each of the tet's ten local entities.
+constexpr int REC_P = 0;          // 16 complex
+constexpr int REC_Q = 32;         // 36 complex
+constexpr int REC_DS = 104;       // 6 vertex-pair distances
+constexpr int REC_L = 110;        // 6 edge lengths, by vertex pair
+constexpr int REC_SLOT = 116;     // sorted slot of local entity s in bits 4 s .. 4 s + 3 (a 64-bit integer)
+constexpr int REC_NDOUBLE = 117;
+constexpr int REC_STRIDE = 120;
+
+EMFEM_HD int canon_p(int e) { return (0x211000 >> (4 * e)) & 15; }            // vertices of canonical edge e
+EMFEM_HD int canon_q(int e) { return (0x332321 >> (4 * e)) & 15; }
+EMFEM_HD int canon_fv(int f, int k) { return ((k == 0 ? 0x1000 : k == 1 ? 0x2211 : 0x3332) >> (4 * f)) & 15; }
+EMFEM_HD int canon_fp(int f, int k) {      // vertex pairs (0, 1), (0, 2), (1, 2) of canonical face f
+    return ((k == 0 ? 0x3100 : k == 1 ? 0x4221 : 0x5543) >> (4 * f)) & 15;
+}
+
+// Sorted slots of the ten local entities (see REC_SLOT) for vertex ranks r[4].
+EMFEM_HD unsigned long long canon_slots(const int r[4]) {
+    unsigned long long m = 0;
+    for (int e = 0; e < 6; e++) m |= (unsigned long long)pair_index(r[tet_edge_p(e)], r[tet_edge_q(e)]) << (4 * e);
+    for (int f = 0; f < 4; f++) {
+        const int missing = 6 - (r[tet_face_v(f, 0)] + r[tet_face_v(f, 1)] + r[tet_face_v(f, 2)]);
+        m |= (unsigned long long)(9 - missing) << (4 * (6 + f));             // faces 012, 013, 023, 123
+    }
+    return m;
+}
+
+// Record accessors: complex values as one 16-byte load where the record is 16-byte aligned.
+struct RecGlobal {
     const double* base;
     EMFEM_HD double g(int f) const { return base[f]; }
     EMFEM_HD cd c(int f) const {
@@ -239,17 +277,113 @@ struct InvRec {
         return mk(base[f], base[f + 1]);
 #endif
     }
-    EMFEM_HD cd P(int a, int b) const { return c(INV_P + 2 * (4 * a + b)); }
-    EMFEM_HD cd Q(int a, int b, int cc, int d) const {
-        int p = pair_index(a, b), q = pair_index(cc, d);
-        double s = ((a < b) == (cc < d)) ? 1.0 : -1.0;
-        cd v = c(INV_Q + 2 * (6 * p + q));
-        return mk(s * v.x, s * v.y);
-    }
-    EMFEM_HD double Ds(int a, int b) const { return g(INV_DS + pair_index(a, b)); }
-    EMFEM_HD double L(int e) const { return g(INV_L + e); }
 };
-static_assert(INV_STRIDE % 2 == 0 && INV_P % 2 == 0 && INV_Q % 2 == 0, "complex invariants are 16-byte aligned");
+struct RecShared {
+    const double* base;
+    EMFEM_HD double g(int f) const { return base[f]; }
+    EMFEM_HD cd c(int f) const { return mk(base[f], base[f + 1]); }
+};
+static_assert(REC_STRIDE % 2 == 0 && REC_P % 2 == 0 && REC_Q % 2 == 0, "complex invariants are 16-byte aligned");
+
+// prod k_i! of four vertices as a double: equal pairs only (the sets below never hold one vertex four times
+// unless both of its pairs are given)
+EMFEM_HD double two_if(bool c) { return c ? 2.0 : 1.0; }
+EMFEM_HD double six_if(bool c) { return c ? 6.0 : 2.0; }       // {x, x, y, z}: x once more among y, z
+EMFEM_HD double pairs2(bool same) { return same ? 24.0 : 4.0; }   // {x, x, y, y}
+EMFEM_HD void fma_c(cd& s, double k, cd v) { s.x = fma(k, v.x, s.x); s.y = fma(k, v.y, s.y); }
+
+// Pair block of sorted slots sx, sy (0..5 edges, 6..9 faces), scaled as pair_block's.
+template <class IV>
+EMFEM_HD void canon_block(const IV& I, int sx, int sy, cd d[4], cd f[4]) {
+    const bool xe = sx < 6, ye = sy < 6;
+    if (xe && ye) {
+        const int a = canon_p(sx), b = canon_q(sx), c = canon_p(sy), e = canon_q(sy);
+        const cd q = I.c(REC_Q + 2 * (6 * sx + sy));
+        const cd pac = I.c(REC_P + 2 * (4 * a + c)), pad = I.c(REC_P + 2 * (4 * a + e));
+        const cd pbc = I.c(REC_P + 2 * (4 * b + c)), pbd = I.c(REC_P + 2 * (4 * b + e));
+        const double L = I.g(REC_L + sx) * I.g(REC_L + sy);
+        const bool ac = a == c, ad = a == e, bc = b == c, bd = b == e;
+        const cd q9 = (9.0 * L) * q;
+        d[0] = two_if(ac) * q9; d[1] = two_if(ad) * q9; d[2] = two_if(bc) * q9; d[3] = two_if(bd) * q9;
+        const double abcd = two_if(ac || ad) * two_if(bc || bd);
+        const double abcc = six_if(ac || bc), abdd = six_if(ad || bd), aacd = six_if(ac || ad), bbcd = six_if(bc || bd);
+        const cd uac = L * pac, uad = -L * pad, ubc = -L * pbc, ubd = L * pbd;
+        f[0] = abcd * uac; fma_c(f[0], abcc, uad); fma_c(f[0], aacd, ubc); fma_c(f[0], pairs2(ac), ubd);
+        f[1] = abdd * uac; fma_c(f[1], abcd, uad); fma_c(f[1], pairs2(ad), ubc); fma_c(f[1], aacd, ubd);
+        f[2] = bbcd * uac; fma_c(f[2], pairs2(bc), uad); fma_c(f[2], abcd, ubc); fma_c(f[2], abcc, ubd);
+        f[3] = pairs2(bd) * uac; fma_c(f[3], bbcd, uad); fma_c(f[3], abdd, ubc); fma_c(f[3], abcd, ubd);
+    } else if (xe != ye) {
+        // edge-face block; a face row uses the transposed edge-face block (curlcurl.py:321-328)
+        const int es = xe ? sx : sy, fs = (xe ? sy : sx) - 6;
+        const int a = canon_p(es), b = canon_q(es), c = canon_fv(fs, 0), e = canon_fv(fs, 1), g = canon_fv(fs, 2);
+        const int pcd = canon_fp(fs, 0), pcf = canon_fp(fs, 1), pdf = canon_fp(fs, 2);
+        const cd qcd = I.c(REC_Q + 2 * (6 * es + pcd)), qcf = I.c(REC_Q + 2 * (6 * es + pcf)), qdf = I.c(REC_Q + 2 * (6 * es + pdf));
+        const cd pac = I.c(REC_P + 2 * (4 * a + c)), pad = I.c(REC_P + 2 * (4 * a + e)), paf = I.c(REC_P + 2 * (4 * a + g));
+        const cd pbc = I.c(REC_P + 2 * (4 * b + c)), pbd = I.c(REC_P + 2 * (4 * b + e)), pbf = I.c(REC_P + 2 * (4 * b + g));
+        const double L1 = I.g(REC_L + es), k0 = L1 * I.g(REC_DS + pcf), k1 = L1 * I.g(REC_DS + pcd);
+        const bool ac = a == c, ad = a == e, af = a == g, bc = b == c, bd = b == e, bf = b == g;
+        const cd q3f = 3.0 * qcf, q3d = 3.0 * qdf, q3c = 3.0 * qcd;
+        auto curl = [&](bool xc, bool xd, bool xf, cd& lo, cd& hi) {      // sums with L_x: x one of the edge's vertices
+            const double vc = two_if(xc), vd = two_if(xd), vf = two_if(xf);
+            const cd s = vd * q3f, t = vc * q3d, u = vf * q3c;
+            lo = k0 * mk(-2.0 * s.x - t.x - u.x, -2.0 * s.y - t.y - u.y);
+            hi = k1 * mk(2.0 * u.x + s.x - t.x, 2.0 * u.y + s.y - t.y);
+        };
+        cd e00, e01, e10, e11;
+        curl(ac, ad, af, e00, e01);
+        curl(bc, bd, bf, e10, e11);
+        const double abcd = two_if(ac || ad) * two_if(bc || bd), abdf = two_if(ad || af) * two_if(bd || bf);
+        const double abcf = two_if(ac || af) * two_if(bc || bf);
+        const double aacd = six_if(ac || ad), aadf = six_if(ad || af), aacf = six_if(ac || af);
+        const double bbcd = six_if(bc || bd), bbdf = six_if(bd || bf), bbcf = six_if(bc || bf);
+        cd g00 = abcd * paf; fma_c(g00, -abdf, pac); fma_c(g00, -aacd, pbf); fma_c(g00, aadf, pbc);
+        cd g01 = abdf * pac; fma_c(g01, -abcf, pad); fma_c(g01, -aadf, pbc); fma_c(g01, aacf, pbd);
+        cd g10 = bbcd * paf; fma_c(g10, -bbdf, pac); fma_c(g10, -abcd, pbf); fma_c(g10, abdf, pbc);
+        cd g11 = bbdf * pac; fma_c(g11, -bbcf, pad); fma_c(g11, -abdf, pbc); fma_c(g11, abcf, pbd);
+        d[0] = e00; d[3] = e11;
+        d[1] = xe ? e01 : e10; d[2] = xe ? e10 : e01;
+        f[0] = k0 * g00; f[3] = k1 * g11;
+        f[1] = xe ? k1 * g01 : k0 * g10; f[2] = xe ? k0 * g10 : k1 * g01;
+    } else {
+        const int fx = sx - 6, fy = sy - 6;
+        const int a = canon_fv(fx, 0), b = canon_fv(fx, 1), e = canon_fv(fx, 2);
+        const int c = canon_fv(fy, 0), dd = canon_fv(fy, 1), g = canon_fv(fy, 2);
+        const int pab = canon_fp(fx, 0), pae = canon_fp(fx, 1), pbe = canon_fp(fx, 2);
+        const int pcd = canon_fp(fy, 0), pcf = canon_fp(fy, 1), pdf = canon_fp(fy, 2);
+        const double Lac1 = I.g(REC_DS + pae), Lab1 = I.g(REC_DS + pab), Lac2 = I.g(REC_DS + pcf), Lab2 = I.g(REC_DS + pcd);
+        // curl of L_r W_su against the column's first and second function, s and u the row's other vertices
+        auto curl = [&](int r, int psu, cd& lo, cd& hi) {
+            const cd cf = I.c(REC_Q + 2 * (6 * psu + pcf)), df = I.c(REC_Q + 2 * (6 * psu + pdf)), cdq = I.c(REC_Q + 2 * (6 * psu + pcd));
+            const double vc = two_if(r == c), vd = two_if(r == dd), vf = two_if(r == g);
+            const cd s = vd * cf, t = vc * df, u = vf * cdq;
+            lo = mk(2.0 * s.x + t.x + u.x, 2.0 * s.y + t.y + u.y);
+            hi = mk(t.x - 2.0 * u.x - s.x, t.y - 2.0 * u.y - s.y);
+        };
+        cd b0, b1, a0, a1, e0, e1;
+        curl(b, pae, b0, b1);
+        curl(a, pbe, a0, a1);
+        curl(e, pab, e0, e1);
+        d[0] = (Lac1 * Lac2) * mk(2.0 * b0.x + a0.x + e0.x, 2.0 * b0.y + a0.y + e0.y);
+        d[1] = (Lac1 * Lab2) * mk(2.0 * b1.x + a1.x + e1.x, 2.0 * b1.y + a1.y + e1.y);
+        d[2] = (Lab1 * Lac2) * mk(a0.x - 2.0 * e0.x - b0.x, a0.y - 2.0 * e0.y - b0.y);
+        d[3] = (Lab1 * Lab2) * mk(a1.x - 2.0 * e1.x - b1.x, a1.y - 2.0 * e1.y - b1.y);
+        const cd pef = I.c(REC_P + 2 * (4 * e + g)), pec = I.c(REC_P + 2 * (4 * e + c)), ped = I.c(REC_P + 2 * (4 * e + dd));
+        const cd paf = I.c(REC_P + 2 * (4 * a + g)), pac = I.c(REC_P + 2 * (4 * a + c)), pad = I.c(REC_P + 2 * (4 * a + dd));
+        const cd pbf = I.c(REC_P + 2 * (4 * b + g)), pbc = I.c(REC_P + 2 * (4 * b + c)), pbd = I.c(REC_P + 2 * (4 * b + dd));
+        const bool ac = a == c, ad = a == dd, af = a == g, bc = b == c, bd = b == dd, bf = b == g, ec = e == c, ed = e == dd, ef = e == g;
+        // prod k_i! of {x, y, u, v}, x != y, u != v
+        const double abcd = two_if(ac || ad) * two_if(bc || bd), abdf = two_if(ad || af) * two_if(bd || bf);
+        const double bcdf = two_if(bc || bd || bf), bedf = two_if(bd || bf) * two_if(ed || ef);
+        const double abcf = two_if(ac || af) * two_if(bc || bf), becf = two_if(bc || bf) * two_if(ec || ef);
+        const double eacd = two_if(ec || ed) * two_if(ac || ad), eadf = two_if(ed || ef) * two_if(ad || af);
+        const double eacf = two_if(ec || ef) * two_if(ac || af);
+        cd m0 = abcd * pef; fma_c(m0, -abdf, pec); fma_c(m0, -bcdf, paf); fma_c(m0, bedf, pac);
+        cd m1 = abdf * pec; fma_c(m1, -abcf, ped); fma_c(m1, -bedf, pac); fma_c(m1, becf, pad);
+        cd m2 = bcdf * paf; fma_c(m2, -bedf, pac); fma_c(m2, -eacd, pbf); fma_c(m2, eadf, pbc);
+        cd m3 = bedf * pac; fma_c(m3, -becf, pad); fma_c(m3, -eadf, pbc); fma_c(m3, eacf, pbd);
+        f[0] = (Lac1 * Lac2) * m0; f[1] = (Lac1 * Lab2) * m1; f[2] = (Lab1 * Lac2) * m2; f[3] = (Lab1 * Lab2) * m3;
+    }
+}
 
 // Volume coefficient table: vc[A*125 + B*25 + C*5 + D] = prod k_i! / (sum k_i + 3)!,
 // letters 1..4 name vertices, 0 = absent (curlcurl.py:64-92).

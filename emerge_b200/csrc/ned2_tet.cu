@@ -6,7 +6,8 @@
 //   * Plan (once per mesh): for every entity, its incident tets sorted ascending, the sorted set
 //     S_X of first-kind DOFs of those tets (row X's columns are S_X then S_X + H; row X + H has the
 //     same columns), and for every (X, t) incidence the position in S_X of each of t's 10 entities.
-//   * Numeric: per-tet invariants (ned2_math.cuh) are computed once per tet; then one thread per
+//   * Numeric: per-tet records (ned2_math.cuh, vertices in ascending global order) are computed once per tet;
+//     then one thread per
 //     (X, k) — row pair of X, column pair of S_X[k] — sums the 2x2 D/F pair blocks of X's incident
 //     tets in ascending tet order and writes its 4 E and 4 B CSR values once.  No atomics, no COO
 //     buffer; the pattern equals SciPy's tocsr() of the reference COO (sorted rows, zeros kept).
@@ -27,40 +28,133 @@ __device__ __forceinline__ cd load_c(const double2* p, long long i) {
     return mk(v.x, v.y);
 }
 
-__global__ void __launch_bounds__(128) tet_invariants_kernel(
+// Sorted-vertex records (ned2_math.cuh, REC_*) of all tets, eight lanes per tet: lanes 0-5 hold one column of Q
+// (and one edge length and one distance), lanes 6 and 7 two columns of P each, so a record leaves the warp
+// in runs of 96 contiguous bytes and a mesh of a few thousand tets still fills the chip.  One thread per tet
+// computed all 52 complex values one after the other and stored them 960 bytes apart: 13.1 us at 6 000 tets and
+// 385 us at 384 000; 8.0 and 450 now (369 MB written, 184 MB read).
+__device__ __forceinline__ void sort_swap(bool c, double a[3], double b[3], int64_t& ia, int64_t& ib) {
+    const int64_t t = c ? ib : ia;
+    ib = c ? ia : ib;
+    ia = t;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const double u = c ? b[k] : a[k];
+        b[k] = c ? a[k] : b[k];
+        a[k] = u;
+    }
+}
+
+__global__ void __launch_bounds__(128) tet_records_kernel(
     long long nt, long long nn, long long ne, const double* __restrict__ nodes,
     const int64_t* __restrict__ tets, const int64_t* __restrict__ t2e, const double* __restrict__ elen,
-    const double2* __restrict__ ur, const double2* __restrict__ er, double* __restrict__ inv, int* status) {
-    long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const double2* __restrict__ ur, const double2* __restrict__ er, double* __restrict__ rec, int* status) {
+    const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x, t = gt >> 3;
+    const int l = threadIdx.x & 7;
     if (t >= nt) return;
-    int64_t ids[4];
-    double xs[4], ys[4], zs[4], el[6];
+    int64_t ids[4], sid[4];
+    double X[4][3];
     bool bad = false, finite = true;
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         int64_t v = tets[i * nt + t];
         if (v < 0 || v >= nn) { bad = true; v = 0; }
-        ids[i] = v;
-        xs[i] = nodes[v]; ys[i] = nodes[nn + v]; zs[i] = nodes[2 * nn + v];
-        finite &= isfinite(xs[i]) && isfinite(ys[i]) && isfinite(zs[i]);
-    }
+        ids[i] = sid[i] = v;
 #pragma unroll
-    for (int e = 0; e < 6; e++) {
-        int64_t id = t2e[e * nt + t];
-        if (id < 0 || id >= ne) { bad = true; id = 0; }
-        el[e] = elen[id];
-        finite &= isfinite(el[e]);
+        for (int k = 0; k < 3; k++) X[i][k] = nodes[k * nn + v];
+        finite &= isfinite(X[i][0]) && isfinite(X[i][1]) && isfinite(X[i][2]);
     }
-    if (bad) flag(status, DEV_BAD_INDEX);
-    cd U[9], E[9];
+    // material tensors: er for the columns of P, ur for those of Q
+    cd M[9];
+    const double2* src = l < 6 ? ur : er;
 #pragma unroll
     for (int k = 0; k < 9; k++) {
-        U[k] = load_c(ur, k * nt + t); E[k] = load_c(er, k * nt + t);
-        finite &= isfinite(U[k].x) && isfinite(U[k].y) && isfinite(E[k].x) && isfinite(E[k].y);
+        M[k] = load_c(src, k * nt + t);
+        finite &= isfinite(M[k].x) && isfinite(M[k].y);
     }
-    double* out = inv + t * INV_STRIDE;
-    tet_invariants(xs, ys, zs, ids, el, U, E, out);
-    if (!(out[INV_SF] < 1e300)) flag(status, DEV_DEGENERATE);
+    double el = 0.0;
+    if (l < 6) {
+        int64_t id = t2e[l * nt + t];
+        if (id < 0 || id >= ne) { bad = true; id = 0; }
+        el = elen[id];
+        finite &= isfinite(el);
+    }
+    int r[4];                               // rank of each local vertex by its global id
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        r[i] = 0;
+#pragma unroll
+        for (int j = 0; j < 4; j++) r[i] += ids[j] < ids[i] ? 1 : 0;
+    }
+    sort_swap(sid[1] < sid[0], X[0], X[1], sid[0], sid[1]);
+    sort_swap(sid[3] < sid[2], X[2], X[3], sid[2], sid[3]);
+    sort_swap(sid[2] < sid[0], X[0], X[2], sid[0], sid[2]);
+    sort_swap(sid[3] < sid[1], X[1], X[3], sid[1], sid[3]);
+    sort_swap(sid[2] < sid[1], X[1], X[2], sid[1], sid[2]);
+    const double xs[4] = {X[0][0], X[1][0], X[2][0], X[3][0]};
+    const double ys[4] = {X[0][1], X[1][1], X[2][1], X[3][1]};
+    const double zs[4] = {X[0][2], X[1][2], X[2][2], X[3][2]};
+    double G[4][3];
+    const double V6 = tet_cofactors(xs, ys, zs, G);
+    const double sF = 1.0 / V6, sD = 1.0 / (V6 * V6 * V6);
+    double* out = rec + t * REC_STRIDE;
+    if (l < 6) {
+        cd Ms[9];
+        matinv3(M, Ms);
+        double C[6][3], cq[3], dq = 0.0;
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = i + 1; j < 4; j++) {
+                const int p = pair_index(i, j);
+                C[p][0] = G[i][1] * G[j][2] - G[i][2] * G[j][1];
+                C[p][1] = G[i][2] * G[j][0] - G[i][0] * G[j][2];
+                C[p][2] = G[i][0] * G[j][1] - G[i][1] * G[j][0];
+                if (p == l || p == 0) {
+                    const double dx = xs[i] - xs[j], dy = ys[i] - ys[j], dz = zs[i] - zs[j];
+                    cq[0] = C[p][0]; cq[1] = C[p][1]; cq[2] = C[p][2];
+                    dq = dx * dx + dy * dy + dz * dz;
+                }
+            }
+        out[REC_DS + l] = sqrt(dq);
+        cd mx[3];
+        const double sc = sD / 120.0;
+#pragma unroll
+        for (int i = 0; i < 3; i++) mx[i] = sc * (Ms[3 * i] * cq[0] + Ms[3 * i + 1] * cq[1] + Ms[3 * i + 2] * cq[2]);
+        double2* Q = reinterpret_cast<double2*>(out + REC_Q);
+#pragma unroll
+        for (int p = 0; p < 6; p++) {
+            const cd v = C[p][0] * mx[0] + C[p][1] * mx[1] + C[p][2] * mx[2];
+            Q[6 * p + l] = make_double2(v.x, v.y);
+        }
+        // local edge l joins vertices of these ranks
+        int rp = 0, rq = 0;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            if (i == tet_edge_p(l)) rp = r[i];
+            if (i == tet_edge_q(l)) rq = r[i];
+        }
+        out[REC_L + pair_index(rp, rq)] = el;
+    } else {
+        double2* P = reinterpret_cast<double2*>(out + REC_P);
+        const double sc = sF / 5040.0;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int b = 2 * (l - 6) + h;
+            const double g0 = l == 6 ? G[h][0] : G[2 + h][0], g1 = l == 6 ? G[h][1] : G[2 + h][1], g2 = l == 6 ? G[h][2] : G[2 + h][2];
+            cd eG[3];
+#pragma unroll
+            for (int i = 0; i < 3; i++) eG[i] = sc * (M[3 * i] * g0 + M[3 * i + 1] * g1 + M[3 * i + 2] * g2);
+#pragma unroll
+            for (int a = 0; a < 4; a++) {
+                const cd v = G[a][0] * eG[0] + G[a][1] * eG[1] + G[a][2] * eG[2];
+                P[4 * a + b] = make_double2(v.x, v.y);
+            }
+        }
+        if (l == 6) reinterpret_cast<unsigned long long*>(out)[REC_SLOT] = canon_slots(r);
+    }
+    if (bad) flag(status, DEV_BAD_INDEX);
+    if (!(sF < 1e300)) flag(status, DEV_DEGENERATE);
     if (!finite) flag(status, DEV_NONFINITE);
 }
 
@@ -339,18 +433,16 @@ __global__ void export_indices_kernel(long long H, long long sum_m, const int* _
 // pair block, column-entity major so every warp evaluates one edge/face block type; results staged
 // in shared memory.  Phase 2: one thread per output (X, k) sums its tets' staged blocks in
 // ascending tet order and writes the 4 E and 4 B CSR values of its column pair.
-constexpr int INV_SMEM_STRIDE = 121;  // odd stride in doubles: lanes of a warp hit distinct banks
+constexpr int REC_SMEM_STRIDE = 117;  // odd stride in doubles: lanes of a warp hit distinct banks
 
 template <int CH, bool SINV>
 struct ChunkSmem {
     static constexpr size_t stage = (size_t)(CH + 1) * 10 * 8 * 16;
-    static constexpr size_t inv = SINV ? (size_t)CH * INV_SMEM_STRIDE * 8 : 0;
-    static constexpr size_t vtab = 625 * 8;
+    static constexpr size_t inv = SINV ? (size_t)CH * REC_SMEM_STRIDE * 8 : 0;
     static constexpr size_t rec = (size_t)CH * 16;
     static constexpr size_t code = (size_t)CH * 4;
     static constexpr size_t off_inv = stage;
-    static constexpr size_t off_vtab = off_inv + inv;
-    static constexpr size_t off_rec = (off_vtab + vtab + 15) & ~(size_t)15;
+    static constexpr size_t off_rec = (off_inv + inv + 15) & ~(size_t)15;
     static constexpr size_t off_code = off_rec + rec;
     static constexpr size_t off_ent = off_code + code;              // (CH + 1) mptr, (CH + 1) inc_ptr
     static constexpr size_t total = off_ent + (size_t)(2 * CH + 2) * 4;
@@ -367,13 +459,11 @@ __global__ void __launch_bounds__(NT, MINB) assemble_chunk_kernel(
     typedef ChunkSmem<CH, SINV> L;
     extern __shared__ __align__(16) unsigned char smem[];
     double2* stage = reinterpret_cast<double2*>(smem);                 // [q][sy][CH + 1] (padded rows)
-    double* sinv = reinterpret_cast<double*>(smem + L::off_inv);       // [CH][INV_SMEM_STRIDE]
-    double* vtab = reinterpret_cast<double*>(smem + L::off_vtab);      // 625
+    double* sinv = reinterpret_cast<double*>(smem + L::off_inv);       // [CH][REC_SMEM_STRIDE]
     uint4* srec = reinterpret_cast<uint4*>(smem + L::off_rec);         // CH
     uint32_t* scode = reinterpret_cast<uint32_t*>(smem + L::off_code); // CH
     int* smptr = reinterpret_cast<int*>(smem + L::off_ent);             // chunk entities' mptr, X0..X1
     int* sinc = smptr + CH + 1;                                          // chunk entities' inc_ptr - i0
-    load_vtab(vtab);
     const int X0 = chunk_ptr[blockIdx.x], X1 = chunk_ptr[blockIdx.x + 1];
     const int i0 = inc_ptr[X0], ninc = inc_ptr[X1] - i0;
     const int nent = X1 - X0;  // <= CH: every entity has at least one incidence
@@ -390,14 +480,13 @@ __global__ void __launch_bounds__(NT, MINB) assemble_chunk_kernel(
         // one warp per incidence: lanes copy consecutive doubles of the tet's record
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
         for (int li = warp; li < ninc; li += NT / 32) {
-            const double* src = inv + (long long)(scode[li] >> 4) * INV_STRIDE;
-            double* dst = sinv + li * INV_SMEM_STRIDE;
+            const double* src = inv + (long long)(scode[li] >> 4) * REC_STRIDE;
+            double* dst = sinv + li * REC_SMEM_STRIDE;
 #pragma unroll
-            for (int f = lane; f < INV_NDOUBLE; f += 32) dst[f] = src[f];
+            for (int f = lane; f < REC_NDOUBLE; f += 32) dst[f] = src[f];
         }
+        __syncthreads();
     }
-    __syncthreads();
-    VTab T{vtab};
     const int npad = (ninc + 31) & ~31;
     const int nwork = LM ? 10 * ninc : 10 * npad;
     for (int w = threadIdx.x; w < nwork; w += NT) {
@@ -409,15 +498,13 @@ __global__ void __launch_bounds__(NT, MINB) assemble_chunk_kernel(
             sy = w / npad; li = w - sy * npad;
             if (li >= ninc) continue;
         }
-        int sx = (int)((srec[li].z >> 16) & 0xff);  // byte 10 of the record
+        const uint32_t code = scode[li];
+        const double* base = SINV ? sinv + li * REC_SMEM_STRIDE : inv + (long long)(code >> 4) * REC_STRIDE;
+        const unsigned long long slots = *reinterpret_cast<const unsigned long long*>(base + REC_SLOT);
+        const int cx = (int)(slots >> (4 * (code & 15))) & 15, cy = (int)(slots >> (4 * sy)) & 15;
         cd d[4], f[4];
-        if constexpr (SINV) {
-            const InvView I{sinv + li * INV_SMEM_STRIDE, 1};
-            pair_block(I, unpack_rank((int)I.g(INV_RANK)), T, sx, sy, d, f);
-        } else {
-            const InvRec I{inv + (long long)(scode[li] >> 4) * INV_STRIDE};
-            pair_block(I, unpack_rank((int)I.g(INV_RANK)), T, sx, sy, d, f);
-        }
+        if constexpr (SINV) canon_block(RecShared{base}, cx, cy, d, f);
+        else canon_block(RecGlobal{base}, cx, cy, d, f);
 #pragma unroll
         for (int q = 0; q < 4; q++) {
             stage[(q * 10 + sy) * (CH + 1) + li] = make_double2(d[q].x, d[q].y);
@@ -432,15 +519,18 @@ __global__ void __launch_bounds__(NT, MINB) assemble_chunk_kernel(
         int lo = 0, hi = nent;  // largest e in [0, nent) with smptr[e] <= j
         while (hi - lo > 1) { int mid = (lo + hi) >> 1; if (smptr[mid] <= j) lo = mid; else hi = mid; }
         const int mb = smptr[lo], k = j - mb, m = smptr[lo + 1] - mb;
+        const unsigned k4 = (unsigned)k * 0x01010101u;
         double2 acc[8];
 #pragma unroll
         for (int q = 0; q < 8; q++) acc[q] = make_double2(0.0, 0.0);
         for (int li = sinc[lo]; li < sinc[lo + 1]; li++) {
-            uint4 r4 = srec[li];
-            uint32_t wds[4] = {r4.x, r4.y, r4.z, r4.w};
+            // the local entity of this incidence's tet whose column position is k (bytes 0-9 of its record)
+            const uint4 r4 = srec[li];
+            const unsigned m0 = __vcmpeq4(r4.x, k4), m1 = __vcmpeq4(r4.y, k4), m2 = __vcmpeq4(r4.z, k4) & 0xffffu;
             int sy = -1;
-#pragma unroll
-            for (int q = 0; q < 10; q++) if ((int)((wds[q >> 2] >> (8 * (q & 3))) & 0xff) == k) sy = q;
+            if (m0) sy = (__ffs(m0) - 1) >> 3;
+            else if (m1) sy = 4 + ((__ffs(m1) - 1) >> 3);
+            else if (m2) sy = 8 + ((__ffs(m2) - 1) >> 3);
             if (sy < 0) continue;
 #pragma unroll
             for (int q = 0; q < 8; q++) {
@@ -527,7 +617,7 @@ struct emfem_plan_s {
     uint8_t* rec = nullptr;        // 16 * 10 nt
     int* mptr = nullptr;           // H + 1
     int* S = nullptr;              // sum_m
-    double* inv = nullptr;         // INV_STRIDE * nt (array of structs)
+    double* inv = nullptr;         // REC_STRIDE * nt: the tets' records (array of structs)
     int* chunk_ptr[N_ASM_VARIANTS] = {nullptr};   // per variant: n_chunks + 1 entity boundaries
     int n_chunks[N_ASM_VARIANTS] = {0};
     int variant = 0;                                 // kernel variant used by emfem_plan_assemble
@@ -596,7 +686,7 @@ int emfem_plan_create(emfem_handle h, int64_t n_tets, int64_t n_edges, int64_t n
     PTRY(check_cuda(cudaMalloc(&p->inc_code, 10 * n_tets * sizeof(uint32_t)), "cudaMalloc(inc_code)"));
     PTRY(check_cuda(cudaMalloc(&p->rec, 10 * n_tets * (size_t)INC_REC), "cudaMalloc(rec)"));
     PTRY(check_cuda(cudaMalloc(&p->mptr, (H + 1) * sizeof(int)), "cudaMalloc(mptr)"));
-    PTRY(check_cuda(cudaMalloc(&p->inv, (size_t)INV_STRIDE * n_tets * sizeof(double)), "cudaMalloc(inv)"));
+    PTRY(check_cuda(cudaMalloc(&p->inv, (size_t)REC_STRIDE * n_tets * sizeof(double)), "cudaMalloc(inv)"));
     PTRY(check_cuda(cudaMalloc(&cnt, H * sizeof(int)), "cudaMalloc(cnt)"));
     PTRY(check_cuda(cudaMalloc(&cursor, H * sizeof(int)), "cudaMalloc(cursor)"));
     PTRY(check_cuda(cudaMalloc(&scratch, nscr * sizeof(int)), "cudaMalloc(scan)"));
@@ -723,10 +813,10 @@ int emfem_plan_assemble(emfem_plan p, int64_t n_nodes, int64_t n_edges, const do
                   "emfem_plan_assemble: null argument");
     EMFEM_REQUIRE(n_edges == p->ne, "emfem_plan_assemble: n_edges differs from the plan's");
     cudaStream_t s = p->h->stream;
-    tet_invariants_kernel<<<grid_for(p->nt, 128), 128, 0, s>>>(p->nt, n_nodes, n_edges, nodes, tets, tet_to_edge,
-                                                                edge_lengths, (const double2*)ur, (const double2*)er,
-                                                                p->inv, p->h->dev_status);
-    EMFEM_LAUNCH("tet_invariants_kernel");
+    tet_records_kernel<<<grid_for(8 * p->nt, 128), 128, 0, s>>>(p->nt, n_nodes, n_edges, nodes, tets, tet_to_edge,
+                                                                 edge_lengths, (const double2*)ur, (const double2*)er,
+                                                                 p->inv, p->h->dev_status);
+    EMFEM_LAUNCH("tet_records_kernel");
     const int v = p->variant;
     launch_asm_variant(v, (unsigned)p->n_chunks[v], s, p->chunk_ptr[v], p->H, p->mptr, p->inc_ptr, p->inc_code,
                        (const uint4*)p->rec, p->inv, (double2*)E_vals, (double2*)B_vals);
