@@ -1020,6 +1020,41 @@ __global__ void patch_add_kernel(long long np, const int* __restrict__ slot, con
     K[s].y += gr * v.y + gi * v.x;
 }
 
+// Columns of a batched vector moved to a batch of another width (column c of the narrower one holds column
+// m[c] of the wider one, -1: zero).
+struct ColMap { signed char m[64]; };
+template <typename T>
+__global__ void pack_columns_kernel(long long rows, int from, int to, ColMap map, const T* __restrict__ src, T* __restrict__ dst) {
+    long long g = (long long)blockIdx.x * VB + threadIdx.x;
+    if (g >= rows * to) return;
+    const int c = map.m[g % to];
+    T v;
+    v.x = v.y = 0;
+    if (c >= 0) v = src[g / to * from + c];
+    dst[g] = v;
+}
+template <typename T>
+__global__ void unpack_columns_kernel(long long rows, int from, int to, ColMap map, const T* __restrict__ src, T* __restrict__ dst) {
+    long long g = (long long)blockIdx.x * VB + threadIdx.x;
+    if (g >= rows * from) return;
+    const int c = map.m[g % from];
+    if (c >= 0) dst[g / from * to + c] = src[g];
+}
+// the same for the inverse 2 x 2 pair blocks, four values per pair and system
+template <typename T>
+__global__ void pack_blocks_kernel(long long h, int from, int to, ColMap map, const T* __restrict__ src, T* __restrict__ dst) {
+    long long g = (long long)blockIdx.x * VB + threadIdx.x;
+    if (g >= h * to) return;
+    const int c = map.m[g % to];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        T v;
+        v.x = v.y = 0;
+        if (c >= 0) v = src[(g / to * from + c) * 4 + k];
+        dst[g * 4 + k] = v;
+    }
+}
+
 static int pow2_at_least(int v) {
     int p = 1;
     while (p < v) p <<= 1;
@@ -1028,7 +1063,7 @@ static int pow2_at_least(int v) {
 
 // ---- workspace layout ----------------------------------------------------------------------
 struct Layout {
-    size_t off_state, off_gamma, off_k0, off_partial, off_patchmap, off_scale, off_gpair;
+    size_t off_state, off_gamma, off_k0, off_partial, off_patchmap, off_scale, off_gpair, off_k0c, off_gammac;
     size_t off_x, off_b, off_r64, off_Ax;                  // FP64 vectors (n, S)
     size_t off_v[8];                                       // Krylov vectors of the inner precision
     size_t off_minv;
@@ -1050,6 +1085,8 @@ static Layout make_layout(long long n, long long nnz, long long npatch, int S, i
     L.off_patchmap = o; o = align256(o + sizeof(int) * n);
     L.off_scale = o; o = align256(o + sizeof(double) * S * G);
     L.off_gpair = o; o = align256(o + sizeof(int) * (G + 1));
+    L.off_k0c = o; o = align256(o + sizeof(double) * S);
+    L.off_gammac = o; o = align256(o + sizeof(double) * 2 * S * (nports > 0 ? nports : 1));
     L.off_x = o; o = align256(o + vec64);
     L.off_b = o; o = align256(o + vec64);
     L.off_r64 = o; o = align256(o + vec64);
@@ -1144,33 +1181,165 @@ struct Krylov {
         return check_cuda(cudaGetLastError(), "krylov iteration");
     }
 
-    // one eager iteration (loads every kernel before capture), then `chunk` iterations captured once
-    // and replayed until no system is active or the iteration cap is reached
-    int run(int chunk) {
-        EMFEM_TRY(iteration());
-        cudaGraph_t graph = nullptr;
-        cudaGraphExec_t exec = nullptr;
-        EMFEM_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-        int st_cap = EMFEM_OK;
-        for (int k = 0; k < chunk && st_cap == EMFEM_OK; k++) st_cap = iteration();
-        cudaError_t e = cudaStreamEndCapture(s, &graph);
-        if (st_cap != EMFEM_OK) { if (graph) cudaGraphDestroy(graph); return st_cap; }
-        EMFEM_CUDA(e);
-        EMFEM_CUDA(cudaGraphInstantiate(&exec, graph, 0));
-        std::vector<SysState> host((size_t)G * S);
-        int rounds = (maxit + chunk - 1) / chunk + 1;
-        int rc = EMFEM_OK;
-        for (int it = 0; it < rounds; it++) {
-            if ((rc = check_cuda(cudaGraphLaunch(exec, s), "cudaGraphLaunch")) != EMFEM_OK) break;
-            if ((rc = check_cuda(cudaMemcpyAsync(host.data(), st, sizeof(SysState) * host.size(), cudaMemcpyDeviceToHost, s), "copy state")) != EMFEM_OK) break;
-            if ((rc = check_cuda(cudaStreamSynchronize(s), "sync")) != EMFEM_OK) break;
-            bool any = false;
-            for (size_t k = 0; k < host.size(); k++) any |= host[k].active != 0;
-            if (!any) break;
+    // ---- narrowing the batch (FP64 BiCGStab on one group) ----
+    // Systems converge at different iterations, and a column that has stopped still takes its lanes and its
+    // share of every gather.  When the active systems fit half the columns, their vectors, preconditioner
+    // and scalars move to a batch of that width; a stopped system's solution goes back to its own column of
+    // xfull.  Vectors of a narrower batch live in the two halves of the workspace by turns: `wide` holds what an
+    // iteration recomputes (five vectors of the full batch), `held` the carried ones (three), each with a
+    // separate place for the block inverses.
+    T* xfull = nullptr;                       // (n, S0): non-null enables narrowing
+    T *wide = nullptr, *held = nullptr, *minv_wide = nullptr, *minv_held = nullptr;
+    double *k0c = nullptr, *gammac = nullptr; // narrowed batch's per-system scalars (device)
+    std::vector<double> hk0, hgamma;          // per-system scalars of the full batch (host)
+    int S0 = 0;                               // width of the full batch
+    std::vector<int> col;                     // column of the full batch that each column holds, -1: none
+    std::vector<SysState> done;               // states by column of the full batch
+    bool in_wide = false;
+    // Below this many vector entries an iteration is bound by its launches, not by its width.
+    static constexpr long long NARROW_MIN = 1 << 18;
+
+    int pack(const T* src, T* dst, long long rows, int from, int to, const ColMap& m) {
+        pack_columns_kernel<T><<<grid_for(rows * to, VB), VB, 0, s>>>(rows, from, to, m, src, dst);
+        return check_cuda(cudaGetLastError(), "pack_columns_kernel");
+    }
+    // the solutions of the current columns into their columns of xfull
+    int flush() {
+        if (x == xfull) return EMFEM_OK;
+        ColMap m;
+        for (int c = 0; c < S; c++) m.m[c] = (signed char)col[c];
+        unpack_columns_kernel<T><<<grid_for(n * (long long)S, VB), VB, 0, s>>>(n, S, S0, m, x, xfull);
+        return check_cuda(cudaGetLastError(), "unpack_columns_kernel");
+    }
+    int narrow(const std::vector<SysState>& host, int to) {
+        EMFEM_TRY(flush());
+        ColMap m;
+        std::vector<int> ncol(to, -1);
+        std::vector<SysState> nst(to, SysState{});
+        int c = 0;
+        for (int k = 0; k < S; k++)
+            if (host[k].active) { m.m[c] = (signed char)k; ncol[c] = col[k]; nst[c] = host[k]; c++; }
+        for (int k = c; k < to; k++) m.m[k] = -1;
+        T* o = in_wide ? held : wide;
+        const size_t step = ((size_t)n * to + 15) & ~(size_t)15;
+        T* nx = o;
+        EMFEM_TRY(pack(x, nx, n, S, to, m));
+        T* nr = o + step;
+        EMFEM_TRY(pack(r, nr, n, S, to, m));
+        T* nv[6];
+        for (int q = 0; q < 6; q++) {
+            nv[q] = o + (2 + q) * step;
+            if (q < 3) EMFEM_TRY(pack(v[q], nv[q], n, S, to, m));      // r_hat, p, v; the others are recomputed
         }
-        cudaGraphExecDestroy(exec);
-        cudaGraphDestroy(graph);
-        return rc;
+        T* nm = in_wide ? minv_held : minv_wide;
+        if (bj()) {
+            pack_blocks_kernel<T><<<grid_for(h * (long long)to, VB), VB, 0, s>>>(h, S, to, m, minv, nm);
+            EMFEM_TRY(check_cuda(cudaGetLastError(), "pack_blocks_kernel"));
+        }
+        if (aux) {
+            T* na = (T*)aux_dinv_buffer(aux, to);      // ends before the wider batch's begins (to <= S / 2)
+            EMFEM_TRY(pack(adinv, na, aux->na, S, to, m));
+            adinv = na;
+        }
+        std::vector<double> pk(to, 0.0), pg_(2 * (size_t)to * (op.n_ports > 0 ? op.n_ports : 1), 0.0);
+        for (int k = 0; k < c; k++) {
+            pk[k] = hk0[ncol[k]];
+            for (int q = 0; q < 2 * op.n_ports; q++) pg_[2 * (size_t)k * op.n_ports + q] = hgamma[2 * (size_t)ncol[k] * op.n_ports + q];
+        }
+        EMFEM_CUDA(cudaMemcpyAsync(k0c, pk.data(), sizeof(double) * pk.size(), cudaMemcpyHostToDevice, s));
+        EMFEM_CUDA(cudaMemcpyAsync(gammac, pg_.data(), sizeof(double) * pg_.size(), cudaMemcpyHostToDevice, s));
+        EMFEM_CUDA(cudaMemcpyAsync(st, nst.data(), sizeof(SysState) * to, cudaMemcpyHostToDevice, s));
+        EMFEM_CUDA(cudaStreamSynchronize(s));
+        x = nx; r = nr; minv = nm; col = ncol; S = to; nsys = c;
+        for (int q = 0; q < 6; q++) v[q] = nv[q];
+        op.S = to; op.k0sq = k0c; op.gamma = gammac;
+        in_wide = !in_wide;
+        return EMFEM_OK;
+    }
+
+    int read_states(std::vector<SysState>& host, cudaStream_t on) {
+        EMFEM_CUDA(cudaMemcpyAsync(host.data(), st, sizeof(SysState) * host.size(), cudaMemcpyDeviceToHost, on));
+        EMFEM_CUDA(cudaStreamSynchronize(on));
+        return EMFEM_OK;
+    }
+    static int count_active(const std::vector<SysState>& host) {
+        int n_act = 0;
+        for (const SysState& q : host) n_act += q.active != 0;
+        return n_act;
+    }
+
+    // One eager iteration (loads every kernel before capture), then `chunk` iterations captured once and
+    // replayed until no system is active, the iteration cap is reached or the batch is narrowed.  With `ahead`
+    // the next replay is queued before the flags of the one before are read (on a second stream), so the GPU
+    // does not wait for the host; the replay queued last finds every system stopped.
+    int run(int chunk) {
+        const bool narrowing = xfull && method == 1 && G == 1;
+        const bool ahead = mf == nullptr;      // an LU application does not skip stopped systems
+        if (narrowing) {
+            S0 = S;
+            col.resize(S);
+            for (int k = 0; k < S; k++) col[k] = k;
+            done.assign(S, SysState{});
+        }
+        cudaStream_t side = nullptr;
+        cudaEvent_t ev = nullptr;
+        int rc = EMFEM_OK;
+        if (ahead) {
+            rc = check_cuda(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking), "cudaStreamCreate");
+            if (rc == EMFEM_OK) rc = check_cuda(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming), "cudaEventCreate");
+        }
+        int left = (maxit + chunk - 1) / chunk + 1;
+        while (rc == EMFEM_OK && left > 0) {
+            std::vector<SysState> host((size_t)G * S);
+            cudaGraph_t graph = nullptr;
+            cudaGraphExec_t exec = nullptr;
+            if ((rc = iteration()) != EMFEM_OK) break;
+            if ((rc = check_cuda(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture")) != EMFEM_OK) break;
+            for (int k = 0; k < chunk && rc == EMFEM_OK; k++) rc = iteration();
+            const cudaError_t e = cudaStreamEndCapture(s, &graph);
+            if (rc == EMFEM_OK) rc = check_cuda(e, "cudaStreamEndCapture");
+            if (rc == EMFEM_OK) rc = check_cuda(cudaGraphInstantiate(&exec, graph, 0), "cudaGraphInstantiate");
+            int to = 0, active = 1;
+            if (ahead && rc == EMFEM_OK) { rc = check_cuda(cudaGraphLaunch(exec, s), "cudaGraphLaunch"); left--; }
+            while (rc == EMFEM_OK) {
+                if (ahead) {
+                    if ((rc = check_cuda(cudaEventRecord(ev, s), "cudaEventRecord")) != EMFEM_OK) break;
+                    if (left > 0) { if ((rc = check_cuda(cudaGraphLaunch(exec, s), "cudaGraphLaunch")) != EMFEM_OK) break; }
+                    left--;
+                    if ((rc = check_cuda(cudaStreamWaitEvent(side, ev, 0), "cudaStreamWaitEvent")) != EMFEM_OK) break;
+                    if ((rc = read_states(host, side)) != EMFEM_OK) break;
+                } else {
+                    if ((rc = check_cuda(cudaGraphLaunch(exec, s), "cudaGraphLaunch")) != EMFEM_OK) break;
+                    left--;
+                    if ((rc = read_states(host, s)) != EMFEM_OK) break;
+                }
+                active = count_active(host);
+                if (active == 0 || left <= 0) break;
+                if (narrowing && S > 1 && n * (long long)S >= NARROW_MIN && 2 * pow2_at_least(active) <= S) {
+                    to = pow2_at_least(active);
+                    break;
+                }
+            }
+            // the replay queued ahead may have stopped more systems: read the states again when all is done
+            if (rc == EMFEM_OK) rc = read_states(host, s);
+            if (exec) cudaGraphExecDestroy(exec);
+            if (graph) cudaGraphDestroy(graph);
+            if (rc != EMFEM_OK) break;
+            if (narrowing)
+                for (int k = 0; k < S; k++) if (col[k] >= 0) done[col[k]] = host[k];
+            active = count_active(host);
+            if (active == 0 || !to) break;
+            rc = narrow(host, pow2_at_least(active));
+        }
+        if (rc == EMFEM_OK && narrowing && S != S0) {
+            rc = flush();
+            if (rc == EMFEM_OK)
+                rc = check_cuda(cudaMemcpyAsync(st, done.data(), sizeof(SysState) * S0, cudaMemcpyHostToDevice, s), "copy state");
+        }
+        const int rs = check_cuda(cudaStreamSynchronize(s), "sync");
+        if (ev) cudaEventDestroy(ev);
+        if (side) cudaStreamDestroy(side);
+        return rc != EMFEM_OK ? rc : rs;
     }
 };
 
@@ -1389,6 +1558,12 @@ static int krylov_impl(emfem_handle hd, int method, int64_t n, int64_t nnz, cons
             STRY(aux_setup_dinv<double2>(aux, S, nsys, k0dev, gdev, k.adinv, s));
         }
         k.mf = mf;
+        if (method == 1 && G == 1) {
+            k.xfull = x64; k.k0c = (double*)(ws + L.off_k0c); k.gammac = (double*)(ws + L.off_gammac);
+            k.hk0 = hk0; k.hgamma = hg;
+            k.wide = k.v[3]; k.held = k.v[0];
+            k.minv_wide = Ax; k.minv_held = (double2*)(ws + L.off_minv);
+        }
         // the recurrence tolerance is half the requested one so the FP64 true residual meets it
         reduce_update_kernel<<<G * S, VB, 0, s>>>(partial, (int)nbv, S, 2, st, UPD_INIT, maxit, 0.5 * tol, nsys, G,
                                               vec_pairs(S), gpair);

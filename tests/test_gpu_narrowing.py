@@ -1,0 +1,36 @@
+"""A batch whose systems converge at different iterations is narrowed while it runs; every system must come back
+in its own column, with its own status and iteration count."""
+import numpy as np
+import pytest
+import torch
+
+from emerge_b200 import problems
+from emerge_b200.sweep import FrequencySweep
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("nsys,precond,maxit", [(13, "aux", 20000), (32, "aux", 20000), (16, "none", 40), (7, "aux", 150)])
+def test_narrowed_batch_equals_single_solves(cuda, nsys, precond, maxit):
+    P = problems.waveguide(nx=10, ny=5, nz=20)            # n * nsys beyond the width from which batches are narrowed
+    sw = FrequencySweep(P)
+    assert sw.n * nsys >= 1 << 18
+    freqs = np.linspace(7.2e9, 12.5e9, nsys)
+    systems = [(float(f), k % 2) for k, f in enumerate(freqs)]
+    b = sw.rhs(systems)
+    b[:, 2] = 0                                            # one system that is solved before it starts
+    k0, gam = sw.k0sq(freqs), sw.gammas(freqs)
+    tol = 1e-9
+    res = sw.solve_rhs(k0, b, gam, tol=tol, maxit=maxit, precond=precond)
+    assert res.iters[2] == 0 and res.status[2] == 0 and torch.count_nonzero(res.x[:, 2]) == 0
+    y = sw.apply(systems, res.x)
+    bm = b * sw.mask[:, None]
+    nb = torch.linalg.norm(bm, dim=0)
+    rel = (torch.linalg.norm(bm - y, dim=0) / torch.where(nb > 0, nb, torch.ones_like(nb))).cpu().numpy()
+    np.testing.assert_allclose(rel, res.relres, rtol=1e-3, atol=1e-13)
+    if maxit >= 20000:
+        assert (res.status == 0).all() and (rel <= tol).all()
+        assert len(set(res.iters.tolist())) > 3            # the systems stop at different iterations
+    else:
+        live = np.arange(nsys) != 2
+        assert (res.status[live] == 1).any() and (res.iters <= maxit).all()
