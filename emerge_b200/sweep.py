@@ -663,20 +663,25 @@ class FrequencySweep:
         """y = K_f x for each system (FP64; PEC rows/cols eliminated)."""
         nsys = len(systems)
         freqs = [f for f, _ in systems]
-        k0 = torch.from_numpy(self.k0sq(freqs)).to(self.device)
-        g = self.gammas(freqs)
-        gam = torch.from_numpy(np.ascontiguousarray(np.stack([g.real, g.imag], axis=-1).reshape(-1))).to(self.device)
         S = 1 << (nsys - 1).bit_length()          # the kernel takes a power-of-two batch
+        g = self.gammas(freqs)
+        # per-system scalars in one host-to-device copy (a pageable one waits for the device): k0^2, then the
+        # gammas, padding columns repeating the last system
+        sc = np.empty(S * (1 + 2 * self.n_ports))
+        sc[:nsys] = self.k0sq(freqs)
+        gs = sc[S:].reshape(S, self.n_ports, 2)
+        gs[:nsys, :, 0], gs[:nsys, :, 1] = g.real, g.imag
+        sc[nsys:S] = sc[nsys - 1]
+        gs[nsys:] = gs[nsys - 1:nsys]
+        scd = torch.from_numpy(sc).to(self.device)
         if S != nsys:
-            pad = S - nsys
-            x = torch.cat([x, torch.zeros((x.shape[0], pad), dtype=x.dtype, device=x.device)], dim=1)
-            k0 = torch.cat([k0, k0[-1:].repeat(pad)])
-            gam = torch.cat([gam, gam[-2 * self.n_ports:].repeat(pad)]) if self.n_ports else gam
+            x = torch.cat([x, torch.zeros((x.shape[0], S - nsys), dtype=x.dtype, device=x.device)], dim=1)
+        x = x.contiguous()
         y = torch.empty_like(x)
         h = Handle.get(self.device)
         check(lib().emfem_sweep_spmv(h.h, self.n, ptr(self.plan.indptr), ptr(self.plan.indices), ptr(self.E),
-                                     ptr(self.B), S, ptr(k0), self.patch_rows.numel(), ptr(self.patch_rows),
+                                     ptr(self.B), S, ptr(scd), self.patch_rows.numel(), ptr(self.patch_rows),
                                      ptr(self.patch_rowptr), ptr(self.patch_cols), ptr(self.patch_vals),
-                                     ptr(self.patch_port), self.n_ports, ptr(gam), ptr(self.mask), ptr(x.contiguous()),
+                                     ptr(self.patch_port), self.n_ports, ptr(scd[S:]), ptr(self.mask), ptr(x),
                                      ptr(y)), "emfem_sweep_spmv")
         return y[:, :nsys] if S != nsys else y
