@@ -387,87 +387,173 @@ __global__ void aux_prolong_kernel(long long n, int S, const int* __restrict__ g
 }
 
 // ---- network forward ------------------------------------------------------------------------
-// One warp per (aux node y, system s); lane c holds channel c.  Layer l (0-based):
+// Rows are (aux node y, system s).  Layer l (0-based):
 //   in_y   = l == 0 ? x_y w_in[t_y] : H_l[y]            (complex channels, real weights)
 //   m_y    = inv_deg_y * sum_{j in N(y)} in_j
 //   out_y  = in_y W_l[t_y] + m_y U_l[t_y]               (t = type: 0 vertex, 1 edge)
 // Layer 0 recomputes in_j = x_j w_in[t_j] on the fly.  The last layer optionally writes
 // za_y = x_y + sum_c out_y[c] w_out[t_y][c].
-template <typename TX>
-__global__ void __launch_bounds__(AB) mpnn_layer_kernel(long long na, int S, int layer, const float* __restrict__ P,
-                                                        const int* __restrict__ nptr, const int* __restrict__ nbr,
-                                                        const float* __restrict__ inv_deg, const uint8_t* __restrict__ atype,
-                                                        const TX* __restrict__ x, const float2* __restrict__ Hin,
-                                                        float2* __restrict__ Hout, TX* __restrict__ za) {
-    __shared__ float sW[2][NN_C][NN_C + 1], sU[2][NN_C][NN_C + 1];
-    __shared__ float sWin[2][NN_C], sWout[2][NN_C];
-    for (int k = threadIdx.x; k < 2 * NN_C * NN_C; k += blockDim.x) {
-        int t = k / (NN_C * NN_C), r = (k / NN_C) % NN_C, c = k % NN_C;
-        sW[t][r][c] = P[nn_off_W(layer) + k];
-        sU[t][r][c] = P[nn_off_U(layer) + k];
+// A warp takes NN_R rows at a time: it gathers in_y and m_y of each with lanes over channels, leaves them in shared
+// memory, and multiplies with lanes over output channels, so that a weight read serves NN_R rows and a row's
+// values arrive as broadcasts of four floats (shuffles of one row at a time bound it before: 74 us a layer
+// at 75 768 rows, 46 now).
+constexpr int NN_R = 8;
+constexpr int NN_T = 128;                // threads per block: 4 warps and their tiles fit static shared memory
+
+// types of the tile's first and last row; nodes are ordered by type, so equal ones mean one type throughout
+__device__ __forceinline__ int2 tile_types(const uint8_t* atype, long long w0, long long total, int S) {
+    const long long w1 = w0 + NN_R - 1 < total ? w0 + NN_R - 1 : total - 1;
+    return make_int2(atype[w0 / S], atype[w1 / S]);
+}
+
+// o[r] (+)= row r of s times the (w, u) pairs of its type; s[r][k] = (a.x, a.y, b.x, b.y)
+__device__ __forceinline__ void tile_product(const float4 (*s)[NN_C], const float2 (*wu)[NN_C][NN_C], int t, int lane, float2* o) {
+#pragma unroll 8
+    for (int k = 0; k < NN_C; k++) {
+        const float2 w = wu[t][k][lane];
+#pragma unroll
+        for (int r = 0; r < NN_R; r++) {
+            const float4 v = s[r][k];
+            o[r].x += v.x * w.x + v.z * w.y;
+            o[r].y += v.y * w.x + v.w * w.y;
+        }
     }
-    for (int k = threadIdx.x; k < 2 * NN_C; k += blockDim.x) {
+}
+
+template <typename TX>
+__global__ void __launch_bounds__(NN_T) mpnn_layer_kernel(long long na, int S, int layer, const float* __restrict__ P,
+                                                          const int* __restrict__ nptr, const int* __restrict__ nbr,
+                                                          const float* __restrict__ inv_deg, const uint8_t* __restrict__ atype,
+                                                          const TX* __restrict__ x, const float2* __restrict__ Hin,
+                                                          float2* __restrict__ Hout, float2* __restrict__ Mout,
+                                                          TX* __restrict__ za) {
+    __shared__ float2 sWU[2][NN_C][NN_C];
+    __shared__ float4 sA[NN_T / 32][NN_R][NN_C];
+    __shared__ float sWin[2][NN_C], sWout[2][NN_C];
+    for (int k = threadIdx.x; k < 2 * NN_C * NN_C; k += NN_T)
+        (&sWU[0][0][0])[k] = make_float2(P[nn_off_W(layer) + k], P[nn_off_U(layer) + k]);
+    for (int k = threadIdx.x; k < 2 * NN_C; k += NN_T) {
         sWin[k / NN_C][k % NN_C] = P[nn_off_win() + k];
         sWout[k / NN_C][k % NN_C] = P[nn_off_wout() + k];
     }
     __syncthreads();
-    int lane = threadIdx.x & 31;
-    long long nw = (long long)gridDim.x * (blockDim.x >> 5);
-    for (long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < na * S; w += nw) {
-    long long y = w / S;
-    int s = (int)(w % S);
-    int t = atype[y];
-    float2 in, m = make_float2(0.f, 0.f);
-    if (layer == 0) {
-        TX xv = x[w];
-        in = make_float2((float)xv.x * sWin[t][lane], (float)xv.y * sWin[t][lane]);
-        for (int k = nptr[y]; k < nptr[y + 1]; k++) {
-            long long j = nbr[k];
-            TX xj = x[j * S + s];
-            float wj = sWin[atype[j]][lane];
-            m.x += (float)xj.x * wj;
-            m.y += (float)xj.y * wj;
+    const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
+    const long long total = na * S, ntiles = (total + NN_R - 1) / NN_R;
+    for (long long tile = (long long)blockIdx.x * (NN_T / 32) + wl; tile < ntiles; tile += (long long)gridDim.x * (NN_T / 32)) {
+        const long long w0 = tile * NN_R;
+        const int2 tt = tile_types(atype, w0, total, S);
+        float2 in[NN_R], m[NN_R];
+        if (S % NN_R == 0) {                 // the tile's rows are systems of one node: its neighbours are read once
+            const long long y = w0 / S, so = w0 - y * S;
+            const int k1 = nptr[y + 1];
+#pragma unroll
+            for (int r = 0; r < NN_R; r++) {
+                m[r] = make_float2(0.f, 0.f);
+                if (layer == 0) {
+                    const TX xv = x[w0 + r];
+                    in[r] = make_float2((float)xv.x * sWin[tt.x][lane], (float)xv.y * sWin[tt.x][lane]);
+                } else {
+                    in[r] = Hin[(w0 + r) * NN_C + lane];
+                }
+            }
+            for (int k = nptr[y]; k < k1; k++) {
+                const long long j = nbr[k], wj = j * S + so;
+                if (layer == 0) {
+                    const float wv = sWin[atype[j]][lane];
+#pragma unroll
+                    for (int r = 0; r < NN_R; r++) {
+                        const TX xj = x[wj + r];
+                        m[r].x += (float)xj.x * wv;
+                        m[r].y += (float)xj.y * wv;
+                    }
+                } else {
+#pragma unroll
+                    for (int r = 0; r < NN_R; r++) {
+                        const float2 hj = Hin[(wj + r) * NN_C + lane];
+                        m[r].x += hj.x;
+                        m[r].y += hj.y;
+                    }
+                }
+            }
+            const float idg = inv_deg[y];
+#pragma unroll
+            for (int r = 0; r < NN_R; r++) { m[r].x *= idg; m[r].y *= idg; }
+        } else {
+#pragma unroll
+            for (int r = 0; r < NN_R; r++) {
+                in[r] = m[r] = make_float2(0.f, 0.f);
+                const long long w = w0 + r;
+                if (w >= total) continue;
+                const long long y = w / S;
+                const int s = (int)(w % S);
+                if (layer == 0) {
+                    const TX xv = x[w];
+                    const float wv = sWin[atype[y]][lane];
+                    in[r] = make_float2((float)xv.x * wv, (float)xv.y * wv);
+                } else {
+                    in[r] = Hin[w * NN_C + lane];
+                }
+                for (int k = nptr[y]; k < nptr[y + 1]; k++) {
+                    const long long j = nbr[k];
+                    if (layer == 0) {
+                        const TX xj = x[j * S + s];
+                        const float wv = sWin[atype[j]][lane];
+                        m[r].x += (float)xj.x * wv;
+                        m[r].y += (float)xj.y * wv;
+                    } else {
+                        const float2 hj = Hin[(j * S + s) * NN_C + lane];
+                        m[r].x += hj.x;
+                        m[r].y += hj.y;
+                    }
+                }
+                const float idg = inv_deg[y];
+                m[r].x *= idg; m[r].y *= idg;
+            }
         }
-    } else {
-        in = Hin[w * NN_C + lane];
-        for (int k = nptr[y]; k < nptr[y + 1]; k++) {
-            float2 hj = Hin[((long long)nbr[k] * S + s) * NN_C + lane];
-            m.x += hj.x;
-            m.y += hj.y;
+        __syncwarp();                        // the previous tile's values are consumed
+#pragma unroll
+        for (int r = 0; r < NN_R; r++) sA[wl][r][lane] = make_float4(in[r].x, in[r].y, m[r].x, m[r].y);
+        __syncwarp();
+        float2 o[NN_R];
+#pragma unroll
+        for (int r = 0; r < NN_R; r++) o[r] = make_float2(0.f, 0.f);
+        tile_product(sA[wl], sWU, tt.x, lane, o);
+        if (tt.y != tt.x) {                  // the tile where the node types meet: rows of the second type again
+            float2 o1[NN_R];
+#pragma unroll
+            for (int r = 0; r < NN_R; r++) o1[r] = make_float2(0.f, 0.f);
+            tile_product(sA[wl], sWU, tt.y, lane, o1);
+#pragma unroll
+            for (int r = 0; r < NN_R; r++) if (w0 + r < total && atype[(w0 + r) / S] == tt.y) o[r] = o1[r];
         }
-    }
-    float idg = inv_deg[y];
-    m.x *= idg; m.y *= idg;
-    float2 o = make_float2(0.f, 0.f);
-#pragma unroll 8
-    for (int k = 0; k < NN_C; k++) {
-        float ix = __shfl_sync(0xffffffffu, in.x, k), iy = __shfl_sync(0xffffffffu, in.y, k);
-        float mx = __shfl_sync(0xffffffffu, m.x, k), my = __shfl_sync(0xffffffffu, m.y, k);
-        float wv = sW[t][k][lane], uv = sU[t][k][lane];
-        o.x += ix * wv + mx * uv;
-        o.y += iy * wv + my * uv;
-    }
-    if (Hout) Hout[w * NN_C + lane] = o;
-    if (za) {
-        float zr = o.x * sWout[t][lane], zi = o.y * sWout[t][lane];
-        for (int off = 16; off > 0; off >>= 1) {
-            zr += __shfl_down_sync(0xffffffffu, zr, off);
-            zi += __shfl_down_sync(0xffffffffu, zi, off);
+#pragma unroll
+        for (int r = 0; r < NN_R; r++) {
+            const long long w = w0 + r;
+            if (w >= total) break;
+            if (Hout) Hout[w * NN_C + lane] = o[r];
+            if (Mout) Mout[w * NN_C + lane] = m[r];
+            if (za) {
+                const float wo = sWout[atype[w / S]][lane];
+                float zr = o[r].x * wo, zi = o[r].y * wo;
+                for (int off = 16; off > 0; off >>= 1) {
+                    zr += __shfl_down_sync(0xffffffffu, zr, off);
+                    zi += __shfl_down_sync(0xffffffffu, zi, off);
+                }
+                if (lane == 0) {
+                    TX xv = x[w], q;
+                    q.x = xv.x + zr;
+                    q.y = xv.y + zi;
+                    za[w] = q;
+                }
+            }
         }
-        if (lane == 0) {
-            TX xv = x[w], r;
-            r.x = xv.x + zr;
-            r.y = xv.y + zi;
-            za[w] = r;
-        }
-    }
     }
 }
 
-// persistent grid for the warp-per-row network kernels: the weights are staged once per block
-static unsigned warp_grid(long long rows) {
-    long long blocks = (rows + (AB / 32) - 1) / (AB / 32);
-    long long cap = 148LL * 8;
+// persistent grid for the tile-per-warp network kernels: the weights are staged once per block
+static unsigned tile_grid(long long rows) {
+    long long blocks = (rows + NN_R * (NN_T / 32) - 1) / (NN_R * (NN_T / 32));
+    long long cap = 148LL * 6;
     return (unsigned)(blocks < cap ? (blocks > 0 ? blocks : 1) : cap);
 }
 
@@ -668,19 +754,21 @@ int mpnn_forward_tc(const emfem_aux_s* a, int S, const float* P, const TX* x, fl
     return check_cuda(cudaGetLastError(), "mpnn_layer_tc_kernel");
 }
 
-// Hstore non-null: every layer's output is kept (training); else layers alternate H0/H1 and the
+// Hstore non-null: every layer's output and, after them, every layer's m are kept (training); else layers alternate H0/H1 and the
 // last layer writes only za.
 template <typename TX>
 int mpnn_forward(const emfem_aux_s* a, int S, const float* P, const TX* x, float2* H0, float2* H1, float2* Hstore,
                  TX* za, cudaStream_t s) {
     long long na = a->na;
-    unsigned grid = warp_grid(na * S);
+    unsigned grid = tile_grid(na * S);
     const float2* hin = nullptr;
     for (int l = 0; l < NN_L; l++) {
         float2* hout = Hstore ? Hstore + (size_t)l * na * S * NN_C : ((l % 2 == 0) ? H0 : H1);
         bool last = l == NN_L - 1;
-        mpnn_layer_kernel<TX><<<grid, AB, 0, s>>>(na, S, l, P, a->inc_ptr, a->inc, a->inv_deg, a->atype, x, hin,
-                                                  (last && !Hstore) ? nullptr : hout, last ? za : nullptr);
+        mpnn_layer_kernel<TX><<<grid, NN_T, 0, s>>>(na, S, l, P, a->inc_ptr, a->inc, a->inv_deg, a->atype, x, hin,
+                                                  (last && !Hstore) ? nullptr : hout,
+                                                  Hstore ? Hstore + (size_t)(NN_L + l) * na * S * NN_C : nullptr,
+                                                  last ? za : nullptr);
         hin = hout;
     }
     return check_cuda(cudaGetLastError(), "mpnn_layer_kernel");
@@ -695,68 +783,79 @@ int mpnn_forward(const emfem_aux_s* a, int S, const float* P, const TX* x, float
 // rows into one partial row, then the partial rows are added in block order.
 constexpr int WG_BLOCKS = 296;
 
-__global__ void __launch_bounds__(AB) mpnn_bwd_dm_kernel(long long na, int S, int layer, const float* __restrict__ P,
-                                                         const float* __restrict__ inv_deg,
-                                                         const uint8_t* __restrict__ atype,
-                                                         const float2* __restrict__ dOut, float2* __restrict__ dM) {
-    __shared__ float sU[2][NN_C][NN_C + 1];
-    for (int k = threadIdx.x; k < 2 * NN_C * NN_C; k += blockDim.x) {
-        int t = k / (NN_C * NN_C), r = (k / NN_C) % NN_C, c = k % NN_C;
-        sU[t][r][c] = P[nn_off_U(layer) + k];
-    }
+// dM_y = inv_deg_y U[t_y] dOut_y and the local part of dIn_y, W[t_y] dOut_y, tile by tile as the forward layer
+__global__ void __launch_bounds__(NN_T) mpnn_bwd_local_kernel(long long na, int S, int layer, const float* __restrict__ P,
+                                                              const float* __restrict__ inv_deg,
+                                                              const uint8_t* __restrict__ atype,
+                                                              const float2* __restrict__ dOut, float2* __restrict__ dM,
+                                                              float2* __restrict__ dIn) {
+    __shared__ float2 sWU[2][NN_C][NN_C + 1];            // transposed: [type][output channel c][input channel k]
+    __shared__ float2 sD[NN_T / 32][NN_R][NN_C];
+    for (int q = threadIdx.x; q < 2 * NN_C * NN_C; q += NN_T)
+        sWU[q / (NN_C * NN_C)][q % NN_C][(q / NN_C) % NN_C] = make_float2(P[nn_off_W(layer) + q], P[nn_off_U(layer) + q]);
     __syncthreads();
-    int lane = threadIdx.x & 31;
-    long long nw = (long long)gridDim.x * (blockDim.x >> 5);
-    for (long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < na * S; w += nw) {
-        long long y = w / S;
-        int t = atype[y];
-        float2 d = dOut[w * NN_C + lane];
-        float2 o = make_float2(0.f, 0.f);
+    const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
+    const long long total = na * S, ntiles = (total + NN_R - 1) / NN_R;
+    for (long long tile = (long long)blockIdx.x * (NN_T / 32) + wl; tile < ntiles; tile += (long long)gridDim.x * (NN_T / 32)) {
+        const long long w0 = tile * NN_R;
+        const int2 tt = tile_types(atype, w0, total, S);
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < NN_R; r++)
+            sD[wl][r][lane] = w0 + r < total ? dOut[(w0 + r) * NN_C + lane] : make_float2(0.f, 0.f);
+        __syncwarp();
+        for (int t = tt.x; t <= tt.y; t++) {             // one type, or both where they meet
+            float2 ow[NN_R], ou[NN_R];
+#pragma unroll
+            for (int r = 0; r < NN_R; r++) ow[r] = ou[r] = make_float2(0.f, 0.f);
 #pragma unroll 8
-        for (int c = 0; c < NN_C; c++) {
-            float dx = __shfl_sync(0xffffffffu, d.x, c), dy = __shfl_sync(0xffffffffu, d.y, c);
-            float u = sU[t][lane][c];
-            o.x += u * dx;
-            o.y += u * dy;
+            for (int c = 0; c < NN_C; c++) {
+                const float2 w = sWU[t][c][lane];
+#pragma unroll
+                for (int r = 0; r < NN_R; r++) {
+                    const float2 d = sD[wl][r][c];
+                    ow[r].x += w.x * d.x; ow[r].y += w.x * d.y;
+                    ou[r].x += w.y * d.x; ou[r].y += w.y * d.y;
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < NN_R; r++) {
+                const long long w = w0 + r;
+                if (w >= total) break;
+                const long long y = w / S;
+                if (tt.x != tt.y && atype[y] != t) continue;
+                const float idg = inv_deg[y];
+                dIn[w * NN_C + lane] = ow[r];
+                dM[w * NN_C + lane] = make_float2(ou[r].x * idg, ou[r].y * idg);
+            }
         }
-        float idg = inv_deg[y];
-        dM[w * NN_C + lane] = make_float2(o.x * idg, o.y * idg);
     }
 }
 
-__global__ void __launch_bounds__(AB) mpnn_bwd_din_kernel(long long na, int S, int layer, const float* __restrict__ P,
-                                                          const int* __restrict__ nptr, const int* __restrict__ nbr,
-                                                          const uint8_t* __restrict__ atype,
-                                                          const float2* __restrict__ dOut, const float2* __restrict__ dM,
-                                                          float2* __restrict__ dIn) {
-    __shared__ float sW[2][NN_C][NN_C + 1];
-    for (int k = threadIdx.x; k < 2 * NN_C * NN_C; k += blockDim.x) {
-        int t = k / (NN_C * NN_C), r = (k / NN_C) % NN_C, c = k % NN_C;
-        sW[t][r][c] = P[nn_off_W(layer) + k];
+// dIn_y += sum of dM over y's neighbours, a thread per (row, channel)
+__global__ void __launch_bounds__(AB) mpnn_bwd_gather_kernel(long long na, int S, const int* __restrict__ nptr,
+                                                             const int* __restrict__ nbr, const float2* __restrict__ dM,
+                                                             float2* __restrict__ dIn) {
+    const long long w = ((long long)blockIdx.x * AB + threadIdx.x) >> 5;
+    if (w >= na * S) return;
+    const int lane = threadIdx.x & 31, s = (int)(w % S);
+    const long long y = w / S;
+    float2 o = dIn[w * NN_C + lane];
+    int k = nptr[y];
+    const int k1 = nptr[y + 1];
+    for (; k + 4 <= k1; k += 4) {            // four neighbours in flight, summed in order
+        float2 m[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) m[u] = dM[((long long)nbr[k + u] * S + s) * NN_C + lane];
+#pragma unroll
+        for (int u = 0; u < 4; u++) { o.x += m[u].x; o.y += m[u].y; }
     }
-    __syncthreads();
-    int lane = threadIdx.x & 31;
-    long long nw = (long long)gridDim.x * (blockDim.x >> 5);
-    for (long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < na * S; w += nw) {
-        long long y = w / S;
-        int s = (int)(w % S);
-        int t = atype[y];
-        float2 d = dOut[w * NN_C + lane];
-        float2 o = make_float2(0.f, 0.f);
-#pragma unroll 8
-        for (int c = 0; c < NN_C; c++) {
-            float dx = __shfl_sync(0xffffffffu, d.x, c), dy = __shfl_sync(0xffffffffu, d.y, c);
-            float wv = sW[t][lane][c];
-            o.x += wv * dx;
-            o.y += wv * dy;
-        }
-        for (int k = nptr[y]; k < nptr[y + 1]; k++) {
-            float2 m = dM[((long long)nbr[k] * S + s) * NN_C + lane];
-            o.x += m.x;
-            o.y += m.y;
-        }
-        dIn[w * NN_C + lane] = o;
+    for (; k < k1; k++) {
+        const float2 m = dM[((long long)nbr[k] * S + s) * NN_C + lane];
+        o.x += m.x;
+        o.y += m.y;
     }
+    dIn[w * NN_C + lane] = o;
 }
 
 template <typename TX>
@@ -770,70 +869,83 @@ __device__ __forceinline__ float2 layer_in(int layer, const float* sWin, const u
     return Hin[(j * S + s) * NN_C + k];
 }
 
-// partial row per block: [2 types][2 mats (W, U)][C][C]
+// Weight gradients of a layer: partial row per block in the gradient's layout, [W, U][2 types][C][C].  A block's
+// rows are staged WG_R at a time (in, m and dOut side by side); each half of its threads owns all 2 x 32 x 32 sums of the type
+// at hand, 4 x 4 per thread, and takes every other row, so a row costs a thread four 16-byte reads for 32
+// multiply-adds (one output row of four columns per thread and a branch on the type: 120 us a layer at
+// 75 768 rows, 40 now).  Rows are ordered by type: a block does its vertex rows, then its edge rows.
+constexpr int WG_R = 32;
 template <typename TX>
-__global__ void __launch_bounds__(AB) mpnn_bwd_wgrad_kernel(long long na, int S, int layer, const float* __restrict__ P,
-                                                            const int* __restrict__ nptr, const int* __restrict__ nbr,
-                                                            const float* __restrict__ inv_deg,
+__global__ void __launch_bounds__(AB) mpnn_bwd_wgrad_kernel(long long na, long long nn, int S, int layer, const float* __restrict__ P,
                                                             const uint8_t* __restrict__ atype, const TX* __restrict__ x,
-                                                            const float2* __restrict__ Hin,
+                                                            const float2* __restrict__ Hin, const float2* __restrict__ M,
                                                             const float2* __restrict__ dOut, float* __restrict__ partial) {
     __shared__ float sWin[2 * NN_C];
-    __shared__ float2 sIn[8][NN_C], sM[8][NN_C], sD[8][NN_C];
-    __shared__ int sT[8];
+    __shared__ __align__(16) float2 sIM[2][WG_R][NN_C];  // in, m
+    __shared__ __align__(16) float2 sD[WG_R][NN_C];
     for (int k = threadIdx.x; k < 2 * NN_C; k += blockDim.x) sWin[k] = P[nn_off_win() + k];
-    // thread owns outputs (k = tid / 8, c = 4 (tid % 8) .. +3) for both types and both matrices
-    int kk = threadIdx.x >> 3, c0 = (threadIdx.x & 7) * 4;
-    float accW[2][4], accU[2][4];
-    for (int t = 0; t < 2; t++)
-        for (int q = 0; q < 4; q++) accW[t][q] = accU[t][q] = 0.f;
-    long long rows = na * S;
-    long long per = (rows + gridDim.x - 1) / gridDim.x;
-    long long r0 = blockIdx.x * per, r1 = min(rows, r0 + per);
-    int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    __syncthreads();
-    for (long long base = r0; base < r1; base += 8) {
-        long long w = base + warp;
-        if (w < r1) {
-            long long y = w / S;
-            int s = (int)(w % S);
-            float2 in = layer_in<TX>(layer, sWin, atype, x, Hin, y, S, s, lane);
-            float2 m = make_float2(0.f, 0.f);
-            for (int k = nptr[y]; k < nptr[y + 1]; k++) {
-                float2 v = layer_in<TX>(layer, sWin, atype, x, Hin, nbr[k], S, s, lane);
-                m.x += v.x; m.y += v.y;
-            }
-            float idg = inv_deg[y];
-            sIn[warp][lane] = in;
-            sM[warp][lane] = make_float2(m.x * idg, m.y * idg);
-            sD[warp][lane] = dOut[w * NN_C + lane];
-            if (lane == 0) sT[warp] = atype[y];
-        } else {
-            sIn[warp][lane] = make_float2(0.f, 0.f);
-            sM[warp][lane] = make_float2(0.f, 0.f);
-            sD[warp][lane] = make_float2(0.f, 0.f);
-            if (lane == 0) sT[warp] = 0;
-        }
-        __syncthreads();
-        for (int r = 0; r < 8; r++) {
-            int t = sT[r];
-            float2 iv = sIn[r][kk], mv = sM[r][kk];
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                float2 d = sD[r][c0 + q];
-                float gw = iv.x * d.x + iv.y * d.y, gu = mv.x * d.x + mv.y * d.y;
-                if (t == 0) { accW[0][q] += gw; accU[0][q] += gu; }
-                else { accW[1][q] += gw; accU[1][q] += gu; }
-            }
-        }
-        __syncthreads();
-    }
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int hf = threadIdx.x >> 7, o = threadIdx.x & 127, mat = o >> 6, k0 = ((o >> 3) & 7) * 4, c0 = (o & 7) * 4;
+    const long long rows = na * S;
+    const long long per = (rows + gridDim.x - 1) / gridDim.x;
+    const long long r0 = blockIdx.x * per, r1 = min(rows, r0 + per);
     float* out = partial + (long long)blockIdx.x * 4 * NN_C * NN_C;
-    for (int t = 0; t < 2; t++)
-        for (int q = 0; q < 4; q++) {
-            out[(t * 2 + 0) * NN_C * NN_C + kk * NN_C + c0 + q] = accW[t][q];
-            out[(t * 2 + 1) * NN_C * NN_C + kk * NN_C + c0 + q] = accU[t][q];
+    for (int t = 0; t < 2; t++) {
+        const long long b0 = t == 0 ? r0 : max(r0, nn * S), b1 = t == 0 ? min(r1, nn * S) : r1;
+        float acc[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
+        for (long long base = b0; base < b1; base += WG_R) {
+            __syncthreads();
+#pragma unroll
+            for (int q = 0; q < WG_R / (AB / 32); q++) {
+                const int rr = warp + q * (AB / 32);
+                const long long w = base + rr;
+                float2 in = make_float2(0.f, 0.f), m = in, d = in;
+                if (w < b1) {
+                    const long long y = w / S;
+                    const int s = (int)(w % S);
+                    in = layer_in<TX>(layer, sWin, atype, x, Hin, y, S, s, lane);
+                    m = M[w * NN_C + lane];
+                    d = dOut[w * NN_C + lane];
+                }
+                sIM[0][rr][lane] = in;
+                sIM[1][rr][lane] = m;
+                sD[rr][lane] = d;
+            }
+            __syncthreads();
+#pragma unroll 4
+            for (int rr = hf; rr < WG_R; rr += 2) {
+                const float4 a0 = *reinterpret_cast<const float4*>(&sIM[mat][rr][k0]), a1 = *reinterpret_cast<const float4*>(&sIM[mat][rr][k0 + 2]);
+                const float4 d0 = *reinterpret_cast<const float4*>(&sD[rr][c0]), d1 = *reinterpret_cast<const float4*>(&sD[rr][c0 + 2]);
+                const float ax[4] = {a0.x, a0.z, a1.x, a1.z}, ay[4] = {a0.y, a0.w, a1.y, a1.w};
+                const float dx[4] = {d0.x, d0.z, d1.x, d1.z}, dy[4] = {d0.y, d0.w, d1.y, d1.w};
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+#pragma unroll
+                    for (int j = 0; j < 4; j++) acc[i][j] += ax[i] * dx[j] + ay[i] * dy[j];
+            }
         }
+        // the two halves' sums, first half first
+        __syncthreads();
+        float* red = reinterpret_cast<float*>(&sIM[0][0][0]);
+        if (hf == 1) {
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) red[(4 * i + j) * 128 + o] = acc[i][j];
+        }
+        __syncthreads();
+        if (hf == 0) {
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    out[((mat * 2 + t) * NN_C + k0 + i) * NN_C + c0 + j] = acc[i][j] + red[(4 * i + j) * 128 + o];
+        }
+    }
 }
 
 // dw_in[t][c] = sum Re(conj(x_y) dIn0_y[c]), dw_out[t][c] = sum Re(conj(out_L,y[c]) dza_y) over y of
@@ -870,14 +982,21 @@ __global__ void __launch_bounds__(AB) mpnn_bwd_vec_kernel(long long na, int S, c
     }
 }
 
-// out[c] = sum_r partial[r * stride + c] for c < count, rows added in order
-__global__ void partial_sum_kernel(int nrows, int stride, int count, const float* __restrict__ partial,
-                                   float* __restrict__ out) {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= count) return;
+// out[c] = sum_r partial[r * stride + c] for c < count: 32 columns per block, 8 groups of rows summed apart and
+// then in order
+__global__ void __launch_bounds__(AB) partial_sum_kernel(int nrows, int stride, int count, const float* __restrict__ partial,
+                                                         float* __restrict__ out) {
+    __shared__ float red[AB / 32][32];
+    const int lane = threadIdx.x & 31, g = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
     float v = 0.f;
-    for (int r = 0; r < nrows; r++) v += partial[(long long)r * stride + c];
-    out[c] = v;
+    if (c < count)
+        for (int r = g; r < nrows; r += AB / 32) v += partial[(long long)r * stride + c];
+    red[g][lane] = v;
+    __syncthreads();
+    if (g == 0 && c < count) {
+        for (int q = 1; q < AB / 32; q++) v += red[q][lane];
+        out[c] = v;
+    }
 }
 
 template <typename TX>
@@ -1225,7 +1344,7 @@ int emfem_mpnn_nparams(void) { return EMFEM_MPNN_NPARAMS; }
 int emfem_mpnn_workspace_floats(emfem_aux a, int nsys, int64_t* activation_floats, int64_t* scratch_floats) {
     EMFEM_REQUIRE(a && nsys >= 1, "emfem_mpnn_workspace_floats: bad argument");
     int64_t act = (int64_t)a->na * nsys * NN_C * 2;
-    if (activation_floats) *activation_floats = NN_L * act;
+    if (activation_floats) *activation_floats = 2 * NN_L * act;      // every layer's output and neighbour mean
     if (scratch_floats) *scratch_floats = 3 * act + (int64_t)WG_BLOCKS * 4 * NN_C * NN_C;
     return EMFEM_OK;
 }
@@ -1254,33 +1373,27 @@ int emfem_mpnn_backward(emfem_aux a, int nsys, const float* params, const void* 
     float2* dIn = dM + actn;
     float* partial = (float*)(dIn + actn);
     const float2* A = (const float2*)act;
-    unsigned gw = warp_grid(rows);
     mpnn_bwd_out_kernel<float2><<<grid_for(rows * NN_C, AB), AB, 0, s>>>(na, nsys, params, a->atype,
                                                                          (const float2*)dza, dOut);
     // w_out gradient from dza and the last layer's output, before dOut is overwritten
     mpnn_bwd_vec_kernel<float2><<<WG_BLOCKS, AB, 0, s>>>(na, nsys, a->atype, (const float2*)x, dOut,
                                                          A + (size_t)(NN_L - 1) * actn, (const float2*)dza, partial);
-    partial_sum_kernel<<<1, 2 * NN_C, 0, s>>>(WG_BLOCKS, 4 * NN_C, 2 * NN_C, partial + 2 * NN_C, grad + nn_off_wout());
+    partial_sum_kernel<<<2 * NN_C / 32, AB, 0, s>>>(WG_BLOCKS, 4 * NN_C, 2 * NN_C, partial + 2 * NN_C, grad + nn_off_wout());
     for (int l = NN_L - 1; l >= 0; l--) {
         const float2* Hin = l > 0 ? A + (size_t)(l - 1) * actn : nullptr;
-        mpnn_bwd_wgrad_kernel<float2><<<WG_BLOCKS, AB, 0, s>>>(na, nsys, l, params, a->inc_ptr, a->inc, a->inv_deg,
-                                                               a->atype, (const float2*)x, Hin, dOut, partial);
-        // partial rows are [t][mat][C][C]; grad holds W_l[t][C][C] then U_l[t][C][C]
-        for (int t = 0; t < 2; t++)
-            for (int mat = 0; mat < 2; mat++) {
-                float* dst = grad + (mat == 0 ? nn_off_W(l) : nn_off_U(l)) + t * NN_C * NN_C;
-                partial_sum_kernel<<<grid_for(NN_C * NN_C, AB), AB, 0, s>>>(
-                    WG_BLOCKS, 4 * NN_C * NN_C, NN_C * NN_C, partial + (t * 2 + mat) * NN_C * NN_C, dst);
-            }
-        mpnn_bwd_dm_kernel<<<gw, AB, 0, s>>>(na, nsys, l, params, a->inv_deg, a->atype, dOut, dM);
-        mpnn_bwd_din_kernel<<<gw, AB, 0, s>>>(na, nsys, l, params, a->inc_ptr, a->inc, a->atype, dOut, dM, dIn);
+        mpnn_bwd_wgrad_kernel<float2><<<WG_BLOCKS, AB, 0, s>>>(na, a->nn, nsys, l, params, a->atype, (const float2*)x, Hin,
+                                                               A + (size_t)(NN_L + l) * actn, dOut, partial);
+        partial_sum_kernel<<<4 * NN_C * NN_C / 32, AB, 0, s>>>(WG_BLOCKS, 4 * NN_C * NN_C, 4 * NN_C * NN_C, partial,
+                                                               grad + nn_off_W(l));
+        mpnn_bwd_local_kernel<<<tile_grid(rows), NN_T, 0, s>>>(na, nsys, l, params, a->inv_deg, a->atype, dOut, dM, dIn);
+        mpnn_bwd_gather_kernel<<<grid_for(rows * 32, AB), AB, 0, s>>>(na, nsys, a->inc_ptr, a->inc, dM, dIn);
         std::swap(dOut, dIn);   // dIn of layer l is dOut of layer l - 1
     }
     EMFEM_LAUNCH("mpnn backward");
     // dOut now holds dL/d in_0 = dL/d(x w_in) per channel: w_in gradient
     mpnn_bwd_vec_kernel<float2><<<WG_BLOCKS, AB, 0, s>>>(na, nsys, a->atype, (const float2*)x, dOut,
                                                          A + (size_t)(NN_L - 1) * actn, (const float2*)dza, partial);
-    partial_sum_kernel<<<1, 2 * NN_C, 0, s>>>(WG_BLOCKS, 4 * NN_C, 2 * NN_C, partial, grad + nn_off_win());
+    partial_sum_kernel<<<2 * NN_C / 32, AB, 0, s>>>(WG_BLOCKS, 4 * NN_C, 2 * NN_C, partial, grad + nn_off_win());
     EMFEM_LAUNCH("mpnn backward vectors");
     return EMFEM_OK;
 }

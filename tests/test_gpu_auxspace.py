@@ -134,6 +134,29 @@ def test_network_forward_backward_vs_oracle(guide):
     assert np.abs(z3 - z16[:, :3]).max() <= 1e-6 * np.abs(z16).max()
 
 
+@pytest.mark.parametrize("S", [1, 2, 5, 8, 16])
+def test_network_batch_widths_vs_oracle(guide, S):
+    """Tiles of the training kernels: rows of one node (S a multiple of 8), of several, the tile where vertex and
+    edge rows meet, and the remainder of the last tile."""
+    P, sw = guide
+    aux = sw.aux_space()
+    ex = aux.export()
+    ptr, nbr = ex["graph_ptr"].cpu().numpy(), ex["graph_nbr"].cpu().numpy()
+    atype = (np.arange(aux.n_aux) >= P.mesh.n_nodes).astype(np.uint8)
+    net = Network(aux, seed=4, init="random")
+    rng = np.random.default_rng(S)
+    x, d = ((rng.standard_normal((aux.n_aux, S)) + 1j * rng.standard_normal((aux.n_aux, S))).astype(np.complex64)
+            for _ in range(2))
+    za = net.forward(torch.from_numpy(x).to(aux.device)).cpu().numpy()
+    grad = net.backward(torch.from_numpy(d).to(aux.device)).cpu().numpy()
+    p = net.params.cpu().numpy().astype(np.float64)
+    zo, cache = oa.mpnn_forward(p, x.astype(np.complex128), ptr, nbr, atype)
+    go = oa.mpnn_backward(p, x.astype(np.complex128), ptr, nbr, atype, cache, d.astype(np.complex128))
+    # four layers of 64-term single-precision sums
+    assert np.abs(za - zo).max() <= 2e-5 * np.abs(zo).max()
+    assert np.abs(grad - go).max() <= 1e-4 * np.abs(go).max()
+
+
 def test_training_reduces_correction_loss_and_learned_solve_converges(guide, golden):
     P, sw = guide
     aux = sw.aux_space()
