@@ -204,128 +204,138 @@ __device__ __forceinline__ float mf_shfl(float v, int l) { return __shfl_sync(0x
 __device__ __forceinline__ double mf_shfl(double v, int l) { return __shfl_sync(0xffffffffu, v, l); }
 
 // LU with partial pivoting of the 32 x 32 diagonal block at step k, plus the explicit inverses of its
-// unit-lower L and upper U.  One CTA per front.  It is a serial step of every front's chain, bound by latency:
-// warp 0 factors with a row per lane in registers (rows exchange places in `pos`, not in the registers; the
-// pivot search is two or three redux instructions), then warp 0 forms the inverse of U and warp 1 that of L,
-// a column per lane, adding each solved entry to all entries that need it (independent sums instead of one
-// dot product after the other).  64 us a step with the block in shared memory, 45 us now (cavity of 82 944
-// tets).  The inverses go to inv (complex64, read by the solves) and, for a complex128 factorization, also to
-// invc (complex128, read by the panel kernel); for complex64 invc is inv.
+// unit-lower L and upper U.  One CTA per front: a serial step of every front's chain, bound by latency.  The block
+// lives in shared memory by columns, warp w owning columns w, w + 8, ..; every warp finds the pivot of column j
+// by itself (two or three redux instructions), rows keep their place and exchange their positions in `pos`, and
+// one barrier a step passes the updated columns on.  Warps 0-3 then form the inverse of L and 4-7 that of U,
+// eight columns per warp with a row per lane (32 steps of shuffles, no barrier).  Rolled loops: a warp with
+// the block in registers needs straight-line code that the instruction cache cannot hold (45 us a step on the
+// 82 944-tet cavity, as one warp in shared memory 64 us; now 20, complex128 27).  The inverses go to inv (complex64, read by
+// the solves) and, for a complex128 factorization, also to invc (complex128, read by the panel kernel); for
+// complex64 invc is inv.
 template <typename T>
-__global__ void __launch_bounds__(64) mf_diag_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm, int k,
-                                                     T* __restrict__ ws, float2* __restrict__ inv, T* __restrict__ invc,
-                                                     int* __restrict__ nperturbed) {
+__global__ void __launch_bounds__(256) mf_diag_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm, int k,
+                                                      T* __restrict__ ws, float2* __restrict__ inv, T* __restrict__ invc,
+                                                      int* __restrict__ nperturbed) {
     typedef typename CxT<T>::R R;
-    __shared__ T D[MF_NB][MF_NB + 1];
-    __shared__ T X[MF_NB][MF_NB + 1];
+    __shared__ T D[MF_NB][MF_NB + 1];            // [column][row]: the block, then U
+    __shared__ T L[MF_NB][MF_NB + 1];            // [column][row]: the multipliers
     __shared__ T dinv[MF_NB];
     __shared__ int sq[MF_NB];
     const FrontMeta& f = fm[lst[blockIdx.x]];
     if (k >= f.e) return;
+    const unsigned all = 0xffffffffu;
     const int kb = min(MF_NB, f.e - k);
     const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
     const long long ld = f.n;
     T* W = ws + f.ws + k + (long long)k * ld;
     const T zero = CxT<T>::make(0.0, 0.0);
-    if (wl == 0) {
-        const unsigned all = 0xffffffffu;
-        T a[MF_NB];
-        R bmax = 0;
 #pragma unroll
-        for (int c = 0; c < MF_NB; c++) {
-            a[c] = (lane < kb && c < kb) ? W[lane + (long long)c * ld] : zero;
-            bmax = max(bmax, cabs2(a[c]));
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) bmax = max(bmax, __shfl_xor_sync(all, bmax, o));
-        const R floor2 = max(bmax, (R)1e-30) * (R)1e-12;      // (1e-6 of the block's largest entry)^2
-        int pos = lane, pert = 0;
-#pragma unroll
-        for (int j = 0; j < MF_NB; j++) {
-            if (j >= kb) break;
-            // pivot: largest |row[j]| among the rows at positions >= j (ties: smallest position)
-            const unsigned cand = mf_max_key(cabs2(a[j]), all, pos >= j && pos < kb);
-            const int br = (int)__reduce_min_sync(all, (cand >> lane) & 1 ? (unsigned)pos : 64u);
-            const int bl = __ffs(__ballot_sync(all, pos == br)) - 1;
-            pos = pos == br ? j : (pos == j ? br : pos);
-            T d;
-            d.x = mf_shfl(a[j].x, bl);
-            d.y = mf_shfl(a[j].y, bl);
-            if (cabs2(d) < floor2) {
-                const R v = sqrt(cabs2(d)), fl = sqrt(floor2);
-                d = v > 0 ? CxT<T>::make(d.x / v * fl, d.y / v * fl) : CxT<T>::make(fl, 0.0);
-                if (lane == bl) a[j] = d;
-                pert++;
-            }
-            const T pinv = cinv(d);
-            const bool low = pos > j && pos < kb;
-            if (low) a[j] = cmul(a[j], pinv);
-#pragma unroll
-            for (int c = j + 1; c < MF_NB; c++) {
-                T u;
-                u.x = mf_shfl(a[c].x, bl);
-                u.y = mf_shfl(a[c].y, bl);
-                if (low) cfms(a[c], a[j], u);
-            }
-        }
-        if (lane == 0 && pert) atomicAdd(nperturbed, pert);
-        sq[pos] = lane;
-#pragma unroll
-        for (int c = 0; c < MF_NB; c++) D[pos][c] = a[c];
-        __syncwarp();
-        if (lane < kb) dinv[lane] = cinv(D[lane][lane]);
+    for (int q = 0; q < 4; q++) {
+        const int c = wl + 8 * q;
+        D[c][lane] = (lane < kb && c < kb) ? W[lane + (long long)c * ld] : zero;
+        L[c][lane] = zero;
     }
     __syncthreads();
-    if (wl == 1) {                                  // write L\U back while the inverses are formed
-        for (int c = 0; c < kb; c++)
-            if (lane < kb) W[lane + (long long)c * ld] = D[lane][c];
-    }
-    {
-        // column `lane` of the inverse; t[i] collects the sum that entry i needs
-        T t[MF_NB];
+    R bmax = 0;
 #pragma unroll
-        for (int i = 0; i < MF_NB; i++) t[i] = zero;
+    for (int c = 0; c < MF_NB; c++) bmax = max(bmax, cabs2(D[c][lane]));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) bmax = max(bmax, __shfl_xor_sync(all, bmax, o));
+    const R floor2 = max(bmax, (R)1e-30) * (R)1e-12;      // (1e-6 of the block's largest entry)^2
+    int pos = lane, pert = 0;
+    for (int j = 0; j < kb; j++) {
+        // pivot: largest |row[j]| among the rows at positions >= j (ties: smallest position)
+        const T aj = D[j][lane];
+        const unsigned cand = mf_max_key(cabs2(aj), all, pos >= j && pos < kb);
+        const unsigned key = (cand >> lane) & 1 ? (unsigned)pos : 64u;
+        const int br = (int)__reduce_min_sync(all, key);
+        const int bl = __ffs(__ballot_sync(all, pos == br)) - 1;
+        pos = pos == br ? j : (pos == j ? br : pos);
+        T d;
+        d.x = mf_shfl(aj.x, bl);
+        d.y = mf_shfl(aj.y, bl);
+        if (cabs2(d) < floor2) {
+            const R v = sqrt(cabs2(d)), fl = sqrt(floor2);
+            d = v > 0 ? CxT<T>::make(d.x / v * fl, d.y / v * fl) : CxT<T>::make(fl, 0.0);
+            pert++;
+        }
+        const T pinv = cinv(d);
+        const bool low = pos > j && pos < kb;
+        const T l = low ? cmul(aj, pinv) : zero;
         if (wl == 0) {
+            L[j][lane] = l;
+            if (lane == bl) dinv[j] = pinv;
+        }
 #pragma unroll
-            for (int i = MF_NB - 1; i >= 0; i--) {
-                T x = zero;
-                if (i < kb && lane < kb && i <= lane) {
-                    x = dinv[i];
-                    if (i < lane) { const T q = cmul(t[i], x); x = CxT<T>::make(-q.x, -q.y); }
-                }
-                if (i < kb) {
-#pragma unroll
-                    for (int r = 0; r < i; r++) cfma(t[r], D[r][i], x);
-                }
-                t[i] = x;
-            }
-        } else {
-#pragma unroll
-            for (int i = 0; i < MF_NB; i++) {
-                T x = zero;
-                if (i < kb && lane < kb && i >= lane) x = i == lane ? CxT<T>::make(1.0, 0.0) : CxT<T>::make(-t[i].x, -t[i].y);
-                if (i < kb) {
-#pragma unroll
-                    for (int r = i + 1; r < MF_NB; r++) cfma(t[r], D[r][i], x);
-                }
-                t[i] = x;
+        for (int q = 0; q < 4; q++) {
+            const int c = wl + 8 * q;
+            if (c > j) {
+                const T u = D[c][bl];
+                if (low) cfms(D[c][lane], l, u);
             }
         }
-        // the block's row swaps folded into the inverse of L: position i holds row sq[i], so column sq[c] of
-        // Linv P is column c of Linv
-        const int col = wl == 0 ? lane : sq[lane];
-        __syncthreads();                            // both warps are done with L\U: D takes the inverse of U
-#pragma unroll
-        for (int i = 0; i < MF_NB; i++) (wl == 0 ? D : X)[i][col] = t[i];
+        __syncthreads();                          // column j + 1 is up to date for every warp; column j is read
+        if (lane == bl && wl == (j & 7)) D[j][lane] = d;          // the pivot as used
     }
-    __syncwarp();
-    // Linv P, then Uinv: column-major 32 x 32 each
-    const long long ib = f.inv + (long long)(k / MF_NB) * 2 * MF_NB * MF_NB + (wl == 0 ? MF_NB * MF_NB : 0);
+    if (threadIdx.x == 0 && pert) atomicAdd(nperturbed, pert);
+    if (wl == 0) sq[pos] = lane;
+    __syncthreads();
+    // rows in pivot order: entry (position i, column c) is L below the diagonal, D on and above it
+    const int src = sq[lane];
+    T row[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const int c = wl + 8 * q;
+        row[q] = lane > c ? L[c][src] : D[c][src];
+        if (lane < kb && c < kb) W[lane + (long long)c * ld] = row[q];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const int c = wl + 8 * q;
+        D[c][lane] = row[q];
+    }
+    __syncthreads();
+    const bool upper = wl >= 4;
+    const int c0 = (wl & 3) * 8;
+    T x[8];
+#pragma unroll
+    for (int q = 0; q < 8; q++) x[q] = CxT<T>::make(lane == c0 + q && lane < kb ? 1.0 : 0.0, 0.0);
+    if (!upper) {
+        for (int t = 0; t < kb; t++) {
+            const T m = lane > t ? D[t][lane] : zero;
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                T v;
+                v.x = mf_shfl(x[q].x, t);
+                v.y = mf_shfl(x[q].y, t);
+                cfms(x[q], m, v);
+            }
+        }
+    } else {
+        for (int t = kb - 1; t >= 0; t--) {
+            const T m = lane < t ? D[t][lane] : zero, di = dinv[t];
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                T v;
+                v.x = mf_shfl(x[q].x, t);
+                v.y = mf_shfl(x[q].y, t);
+                v = cmul(v, di);
+                if (lane == t) x[q] = v;
+                cfms(x[q], m, v);
+            }
+        }
+    }
+    // Linv P, then Uinv: column-major 32 x 32 each.  The block's row swaps are folded into the inverse of L: position
+    // i holds row sq[i], so column sq[c] of Linv P is column c of Linv.
+    const long long ib = f.inv + (long long)(k / MF_NB) * 2 * MF_NB * MF_NB + (upper ? MF_NB * MF_NB : 0);
     constexpr bool wide = sizeof(T) != sizeof(float2);
-    for (int c = 0; c < MF_NB; c++) {
-        const T v = (wl == 0 ? D : X)[lane][c];
-        inv[ib + lane + c * MF_NB] = to_c64(v);
-        if (wide) invc[ib + lane + c * MF_NB] = v;
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+        const int c = upper ? c0 + q : sq[c0 + q];
+        inv[ib + lane + c * MF_NB] = to_c64(x[q]);
+        if (wide) invc[ib + lane + c * MF_NB] = x[q];
     }
 }
 
@@ -333,7 +343,7 @@ __global__ void __launch_bounds__(64) mf_diag_kernel(const int* __restrict__ lst
 // tile of TW columns (the first nt of grid.x) or rows, staged in shared memory with coalesced loads, as a
 // small product with the 32 x 32 inverse, 2 x TW / 16 results per thread.  One row or column per thread
 // read the block row with a stride of the front and ran on a fraction of the SMs: 58 us a step on the
-// 82 944-tet cavity, 21 us now.
+// 82 944-tet cavity, 21 now.
 template <typename T, int TW>
 __global__ void __launch_bounds__(256) mf_panel_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm, int k,
                                                        int nt, T* __restrict__ ws, const T* __restrict__ invc) {
@@ -734,7 +744,7 @@ __global__ void mf_fwd_gather_kernel(const int* __restrict__ lst, const FrontMet
 constexpr int MF_KC = MF_SB;
 template <int NS>
 struct MfProdSmem {
-    float2 x[MF_KC][NS];
+    alignas(16) float2 x[MF_KC][NS];
     float2 red[8][NS < 4 ? NS : 4][64];
 };
 
@@ -761,11 +771,19 @@ __device__ __forceinline__ void mf_product(MfProdSmem<NS>& sm, int c0, int c1, i
             float2 mv[RPL];
 #pragma unroll
             for (int i = 0; i < RPL; i++) mv[i] = mat(i, cb + c);
+            if constexpr (NS > 1) {          // two right-hand sides per 16-byte read
 #pragma unroll
-            for (int q = 0; q < NS; q++) {
-                const float2 xv = sm.x[c][q];
+                for (int q = 0; q < NS; q += 2) {
+                    const float4 xv = *reinterpret_cast<const float4*>(&sm.x[c][q]);
 #pragma unroll
-                for (int i = 0; i < RPL; i++) cfma(acc[i][q], mv[i], xv);
+                    for (int i = 0; i < RPL; i++) {
+                        cfma(acc[i][q], mv[i], make_float2(xv.x, xv.y));
+                        cfma(acc[i][q + 1], mv[i], make_float2(xv.z, xv.w));
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < RPL; i++) cfma(acc[i][0], mv[i], sm.x[c][0]);
             }
         }
     }
@@ -817,7 +835,7 @@ __global__ void __launch_bounds__(256) mf_fwd_tri_kernel(const int* __restrict__
 
 // rows [k1, n): w[r] -= L[r, k0:k1] y[k0:k1]
 template <int NS, int RPL>
-__global__ void __launch_bounds__(256) mf_fwd_update_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm,
+__global__ void __launch_bounds__(256, NS * RPL > 16 ? 2 : 3) mf_fwd_update_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm,
                                                             int S, int k0, const float2* __restrict__ fact,
                                                             const float2* __restrict__ y, float2* __restrict__ w) {
     __shared__ MfProdSmem<NS> sm;
@@ -845,7 +863,7 @@ __global__ void __launch_bounds__(256) mf_fwd_update_kernel(const int* __restric
 // DOFs).  Levels of few fronts split the columns over nsplit CTAs of cw columns; their sums go to part and
 // mf_bwd_bnd_sum_kernel subtracts them in order.
 template <int NS, int RPL>
-__global__ void __launch_bounds__(256) mf_bwd_bnd_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm, int S,
+__global__ void __launch_bounds__(256, NS * RPL > 16 ? 2 : 3) mf_bwd_bnd_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm, int S,
                                                          int nrt, int nsplit, int cw, long long y0, long long yl,
                                                          const float2* __restrict__ fact, const int* __restrict__ fdof,
                                                          const float2* __restrict__ xs, float2* __restrict__ y,
@@ -915,7 +933,7 @@ __global__ void __launch_bounds__(256) mf_bwd_tri_kernel(const int* __restrict__
 
 // rows [0, k0): y[r] -= U[r, k0:k1] x[k0:k1]
 template <int NS, int RPL>
-__global__ void __launch_bounds__(256) mf_bwd_update_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm,
+__global__ void __launch_bounds__(256, NS * RPL > 16 ? 2 : 3) mf_bwd_update_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm,
                                                             int S, int k0, const float2* __restrict__ fact,
                                                             const int* __restrict__ fdof, const float2* __restrict__ xs,
                                                             float2* __restrict__ y) {
@@ -1145,7 +1163,7 @@ static int mf_factor_levels(emfem_mf_s* m, const double2* K_vals, cudaStream_t s
             const int maxe = m->lvl_max_e[L];
             for (int k = 0; k < maxe; k += MF_NB) {
                 const int ob = k / MF_OB * MF_OB;
-                mf_diag_kernel<T><<<ny, 64, 0, s>>>(lst, m->d_meta, k, ws, m->inv, invc, m->d_npert);
+                mf_diag_kernel<T><<<ny, 256, 0, s>>>(lst, m->d_meta, k, ws, m->inv, invc, m->d_npert);
                 const long long mm = std::max(1LL, maxn - k - 1);
                 constexpr int TW = sizeof(T) == sizeof(float2) ? 64 : 32;     // tiles within static shared memory
                 const unsigned npt = nblk(mm, TW);
