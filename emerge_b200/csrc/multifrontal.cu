@@ -160,28 +160,31 @@ __global__ void mf_asm_kernel(const int* __restrict__ lst, const FrontMeta* __re
     }
 }
 
+// Extend-add of one child slot: a warp per column of the child's Schur complement (walking flat entries spent
+// its time on 64-bit divisions: 290 us a launch on the 82 944-tet cavity, 260 now).
 template <typename T>
-__global__ void mf_ea_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm, int cslot,
-                             const int* __restrict__ ea, const T* __restrict__ upd, T* __restrict__ ws) {
+__global__ void __launch_bounds__(256) mf_ea_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm, int cslot,
+                                                    const int* __restrict__ ea, const T* __restrict__ upd, T* __restrict__ ws) {
     const FrontMeta& f = fm[lst[blockIdx.y]];
-    int c = f.child[cslot];
+    const int c = f.child[cslot];
     if (c < 0) return;
     const FrontMeta& g = fm[c];
-    long long nb = g.b;
-    long long tot = nb * nb;
-    long long i0 = (long long)blockIdx.x * MF_CHUNK;
-    if (i0 >= tot) return;
-    long long i1 = min(i0 + MF_CHUNK, tot);
+    const int nb = g.b, j = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (j >= nb) return;
     const int* map = ea + g.ea;
-    const T* U = upd + g.upd;
-    T* W = ws + f.ws;
-    long long ld = f.n;
-    for (long long idx = i0 + threadIdx.x; idx < i1; idx += blockDim.x) {
-        long long i = idx % nb, j = idx / nb;
-        T u = U[idx];
-        T* dst = W + map[i] + (long long)map[j] * ld;
-        dst->x += u.x;
-        dst->y += u.y;
+    const T* U = upd + g.upd + (long long)j * nb;
+    T* W = ws + f.ws + (long long)map[j] * f.n;
+    for (int i0 = threadIdx.x & 31; i0 < nb; i0 += 128) {
+        T u[4], w[4];
+        int r[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) r[q] = i0 + 32 * q < nb ? map[i0 + 32 * q] : -1;
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            if (r[q] >= 0) { u[q] = U[i0 + 32 * q]; w[q] = W[r[q]]; }
+#pragma unroll
+        for (int q = 0; q < 4; q++)            // a column's rows are distinct
+            if (r[q] >= 0) { w[q].x += u[q].x; w[q].y += u[q].y; W[r[q]] = w[q]; }
     }
 }
 
@@ -543,24 +546,28 @@ __global__ void __launch_bounds__(256, TM > 64 || sizeof(T) > 8 ? 2 : 3) mf_trai
 
 // Factor columns (n x e) and U block row (e x b), rounded to complex64, and the Schur complement (b x b,
 // workspace precision) out of the workspace.
+// (a warp per column: walking flat entries spent its time on 64-bit divisions, 611 us a launch on the 82 944-tet
+// cavity, 469 now)
 template <typename T>
-__global__ void mf_compact_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm,
-                                  const T* __restrict__ ws, float2* __restrict__ fact, T* __restrict__ upd) {
+__global__ void __launch_bounds__(256) mf_compact_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm,
+                                                         const T* __restrict__ ws, float2* __restrict__ fact, T* __restrict__ upd) {
     const FrontMeta& f = fm[lst[blockIdx.y]];
-    const long long n = f.n, e = f.e, b = f.b;
-    long long i0 = (long long)blockIdx.x * MF_CHUNK;
-    if (i0 >= n * n) return;
-    long long i1 = min(i0 + MF_CHUNK, n * n);
-    const T* W = ws + f.ws;
+    const int n = f.n, e = f.e, j = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (j >= n) return;
+    const T* W = ws + f.ws + (long long)j * n;
     float2* F = fact + f.fact;
-    T* U = upd + f.upd;
-    for (long long idx = i0 + threadIdx.x; idx < i1; idx += blockDim.x) {
-        long long i = idx % n, j = idx / n;
-        T v = W[idx];
-        if (j < e) F[idx] = to_c64(v);
-        else if (i < e) F[n * e + i + (j - e) * e] = to_c64(v);
-        else U[(i - e) + (j - e) * b] = v;
+    if (j < e) {
+        F += (long long)j * n;
+#pragma unroll 4
+        for (int i = lane; i < n; i += 32) F[i] = to_c64(W[i]);
+        return;
     }
+    F += (long long)n * e + (long long)(j - e) * e;
+#pragma unroll 4
+    for (int i = lane; i < e; i += 32) F[i] = to_c64(W[i]);
+    T* U = upd + f.upd + (long long)(j - e) * f.b;
+#pragma unroll 4
+    for (int i = lane; i < f.b; i += 32) U[i] = W[e + i];
 }
 
 // Inverses of the 256 x 256 diagonal blocks of L and U, written over the factor store's copy of those blocks.
@@ -826,9 +833,9 @@ __global__ void __launch_bounds__(256) mf_fwd_tri_kernel(const int* __restrict__
     const bool live = r < f.e;
     const long long n = f.n;
     mf_product<NS, 1>(sm, k0, min(r0 + MF_NB, f.e), ns, [&](int c) { return X + (long long)c * S; },
-                      [&](int, int c) {
-                          if (!live) return make_float2(0.f, 0.f);
-                          return c < r0 ? F[c * n] : D[(c - r0) * MF_NB];
+                      [&](int, int c) {       // one load from a selected address: loads behind a branch are not batched
+                          const float2* p = c < r0 ? F + c * n : D + (c - r0) * MF_NB;
+                          return live ? *p : make_float2(0.f, 0.f);
                       },
                       [&](int t, int q, float2 v) { if (r0 + t < f.e) Y[(long long)(r0 + t) * S + q] = v; });
 }
@@ -925,8 +932,8 @@ __global__ void __launch_bounds__(256) mf_bwd_tri_kernel(const int* __restrict__
     const long long n = f.n;
     mf_product<NS, 1>(sm, r0, min(k0 + MF_SB, f.e), ns, [&](int c) { return X + (long long)c * S; },
                       [&](int, int c) {
-                          if (!live) return make_float2(0.f, 0.f);
-                          return c < r0 + MF_NB ? D[(c - r0) * MF_NB] : F[c * n];
+                          const float2* p = c < r0 + MF_NB ? D + (c - r0) * MF_NB : F + c * n;
+                          return live ? *p : make_float2(0.f, 0.f);
                       },
                       [&](int t, int q, float2 v) { if (r0 + t < f.e) xs[(long long)d[r0 + t] * S + s0 + q] = v; });
 }
@@ -1159,7 +1166,7 @@ static int mf_factor_levels(emfem_mf_s* m, const double2* K_vals, cudaStream_t s
             mf_asm_kernel<T><<<dim3(nblk(m->lvl_max_asm[L], MF_CHUNK), ny), 256, 0, s>>>(
                 lst, m->d_meta, K_vals, m->d_slot, m->d_off, m->d_fdof, m->d_scale, ws);
             for (int c = 0; c < 2; c++)
-                mf_ea_kernel<T><<<dim3(nblk(maxb * maxb, MF_CHUNK), ny), 256, 0, s>>>(lst, m->d_meta, c, m->d_ea, upd, ws);
+                mf_ea_kernel<T><<<dim3(nblk(maxb, 8), ny), 256, 0, s>>>(lst, m->d_meta, c, m->d_ea, upd, ws);
             const int maxe = m->lvl_max_e[L];
             for (int k = 0; k < maxe; k += MF_NB) {
                 const int ob = k / MF_OB * MF_OB;
@@ -1186,7 +1193,7 @@ static int mf_factor_levels(emfem_mf_s* m, const double2* K_vals, cudaStream_t s
                     mf_trail_kernel<T, 64><<<dim3((unsigned)(nc * nc), ny), 256, sizeof(MfTileSmem<T, 64>), s>>>(lst, m->d_meta,
                                                                                                                ob, ws);
             }
-            mf_compact_kernel<T><<<dim3(nblk(maxn * maxn, MF_CHUNK), ny), 256, 0, s>>>(lst, m->d_meta, ws, m->fact, upd);
+            mf_compact_kernel<T><<<dim3(nblk(maxn, 8), ny), 256, 0, s>>>(lst, m->d_meta, ws, m->fact, upd);
             if (m->lvl_max_e[L] > MF_NB) {
                 const int nbb = std::min(MF_NBB, (int)nblk(m->lvl_max_e[L], MF_NB));
                 mf_block_inverse_kernel<T><<<dim3(2 * nbb, nblk(m->lvl_max_e[L], MF_SB), ny), 256, sizeof(MfInvSmem<T>), s>>>(
