@@ -755,45 +755,53 @@ struct MfProdSmem {
     float2 red[8][NS < 4 ? NS : 4][64];
 };
 
-// XOf(c): pointer to the NS values of column c;  MAt(i, c): entry (row rl + 32 i of the tile, column c);
-// Out(row of the tile, q, value)
-template <int NS, int RPL, typename XOf, typename MAt, typename Out>
-__device__ __forceinline__ void mf_product(MfProdSmem<NS>& sm, int c0, int c1, int ns, XOf xof, MAt mat, Out out) {
-    const int rl = threadIdx.x & 31, g = threadIdx.x >> 5;
-    float2 acc[RPL][NS];
+// Columns [c0, c0 + nc) of x into shared memory: XOf(c) points at column c's values, ns of them real
+template <int NS, typename XOf>
+__device__ __forceinline__ void mf_stage_x(MfProdSmem<NS>& sm, int c0, int nc, int ns, XOf xof) {
+    for (int t = threadIdx.x; t < nc * NS; t += 256) {
+        const int c = t / NS, q = t % NS;
+        sm.x[c][q] = q < ns ? xof(c0 + c)[q] : make_float2(0.f, 0.f);
+    }
+}
+
+// acc += staged columns [0, nc) times M: MAt(i, c) is entry (row rl + 32 i of the tile, staged column c).  A warp
+// takes every eighth column, U of them at once with the columns past the end masked: a plain unrolled loop runs
+// its remainder one load latency per column (block-inverse kernels of one front, whose column counts are
+// no multiples of 64: 18 us a launch at one or eight right-hand sides, 5 and 7 now)
+template <int NS, int RPL, int U, typename MAt>
+__device__ __forceinline__ void mf_accumulate(const MfProdSmem<NS>& sm, float2 (*acc)[NS], int nc, MAt mat) {
+    for (int c0 = threadIdx.x >> 5; c0 < nc; c0 += 8 * U) {
+        float2 mv[U][RPL];
 #pragma unroll
-    for (int i = 0; i < RPL; i++)
+        for (int u = 0; u < U; u++)
 #pragma unroll
-        for (int q = 0; q < NS; q++) acc[i][q] = make_float2(0.f, 0.f);
-    for (int cb = c0; cb < c1; cb += MF_KC) {
-        const int nc = min(MF_KC, c1 - cb);
-        if (cb > c0) __syncthreads();
-        for (int t = threadIdx.x; t < nc * NS; t += 256) {
-            const int c = t / NS, q = t % NS;
-            sm.x[c][q] = q < ns ? xof(cb + c)[q] : make_float2(0.f, 0.f);
-        }
-        __syncthreads();
-#pragma unroll 8
-        for (int c = g; c < nc; c += 8) {
-            float2 mv[RPL];
+            for (int i = 0; i < RPL; i++) mv[u][i] = c0 + 8 * u < nc ? mat(i, c0 + 8 * u) : make_float2(0.f, 0.f);
 #pragma unroll
-            for (int i = 0; i < RPL; i++) mv[i] = mat(i, cb + c);
+        for (int u = 0; u < U; u++) {
+            const int c = c0 + 8 * u;
+            if (c >= nc) break;              // the same for the whole warp
             if constexpr (NS > 1) {          // two right-hand sides per 16-byte read
 #pragma unroll
                 for (int q = 0; q < NS; q += 2) {
                     const float4 xv = *reinterpret_cast<const float4*>(&sm.x[c][q]);
 #pragma unroll
                     for (int i = 0; i < RPL; i++) {
-                        cfma(acc[i][q], mv[i], make_float2(xv.x, xv.y));
-                        cfma(acc[i][q + 1], mv[i], make_float2(xv.z, xv.w));
+                        cfma(acc[i][q], mv[u][i], make_float2(xv.x, xv.y));
+                        cfma(acc[i][q + 1], mv[u][i], make_float2(xv.z, xv.w));
                     }
                 }
             } else {
 #pragma unroll
-                for (int i = 0; i < RPL; i++) cfma(acc[i][0], mv[i], sm.x[c][0]);
+                for (int i = 0; i < RPL; i++) cfma(acc[i][0], mv[u][i], sm.x[c][0]);
             }
         }
     }
+}
+
+// The warps' sums in order, Out(row of the tile, right-hand side, value)
+template <int NS, int RPL, typename Out>
+__device__ __forceinline__ void mf_finish(MfProdSmem<NS>& sm, float2 (*acc)[NS], int ns, Out out) {
+    const int rl = threadIdx.x & 31, g = threadIdx.x >> 5;
     constexpr int QB = NS < 4 ? NS : 4;
 #pragma unroll
     for (int q0 = 0; q0 < NS; q0 += QB) {
@@ -814,6 +822,19 @@ __device__ __forceinline__ void mf_product(MfProdSmem<NS>& sm, int c0, int c1, i
     }
 }
 
+template <int NS, int RPL, typename XOf, typename MAt, typename Out>
+__device__ __forceinline__ void mf_product(MfProdSmem<NS>& sm, int c0, int c1, int ns, XOf xof, MAt mat, Out out) {
+    float2 acc[RPL][NS] = {};
+    for (int cb = c0; cb < c1; cb += MF_KC) {
+        const int nc = min(MF_KC, c1 - cb);
+        if (cb > c0) __syncthreads();
+        mf_stage_x(sm, cb, nc, ns, xof);
+        __syncthreads();
+        mf_accumulate<NS, RPL, 8>(sm, acc, nc, [&](int i, int c) { return mat(i, cb + c); });
+    }
+    mf_finish<NS, RPL>(sm, acc, ns, out);
+}
+
 // y[k0 .. k1) = G w[k0 .. k1), G the inverse of the 256-block of L: 32 rows per CTA, off-diagonal blocks from
 // the factor store, the diagonal one from the inverse store
 template <int NS>
@@ -832,12 +853,16 @@ __global__ void __launch_bounds__(256) mf_fwd_tri_kernel(const int* __restrict__
     float2* Y = y + f.y * S + s0;
     const bool live = r < f.e;
     const long long n = f.n;
-    mf_product<NS, 1>(sm, k0, min(r0 + MF_NB, f.e), ns, [&](int c) { return X + (long long)c * S; },
-                      [&](int, int c) {       // one load from a selected address: loads behind a branch are not batched
-                          const float2* p = c < r0 ? F + c * n : D + (c - r0) * MF_NB;
-                          return live ? *p : make_float2(0.f, 0.f);
-                      },
-                      [&](int t, int q, float2 v) { if (r0 + t < f.e) Y[(long long)(r0 + t) * S + q] = v; });
+    const int co = r0 - k0;              // staged columns: the block row's off-diagonal part, then its diagonal block
+    const int nc = min(r0 + MF_NB, f.e) - k0;
+    float2 acc[1][NS] = {};
+    mf_stage_x(sm, k0, nc, ns, [&](int c) { return X + (long long)c * S; });
+    __syncthreads();
+    mf_accumulate<NS, 1, 16>(sm, acc, nc, [&](int, int c) {
+        const float2* p = c < co ? F + (k0 + c) * n : D + (c - co) * MF_NB;
+        return live ? *p : make_float2(0.f, 0.f);
+    });
+    mf_finish<NS, 1>(sm, acc, ns, [&](int t, int q, float2 v) { if (r0 + t < f.e) Y[(long long)(r0 + t) * S + q] = v; });
 }
 
 // rows [k1, n): w[r] -= L[r, k0:k1] y[k0:k1]
@@ -930,12 +955,15 @@ __global__ void __launch_bounds__(256) mf_bwd_tri_kernel(const int* __restrict__
     const int* d = fdof + f.fdof;
     const bool live = r < f.e;
     const long long n = f.n;
-    mf_product<NS, 1>(sm, r0, min(k0 + MF_SB, f.e), ns, [&](int c) { return X + (long long)c * S; },
-                      [&](int, int c) {
-                          const float2* p = c < r0 + MF_NB ? D + (c - r0) * MF_NB : F + c * n;
-                          return live ? *p : make_float2(0.f, 0.f);
-                      },
-                      [&](int t, int q, float2 v) { if (r0 + t < f.e) xs[(long long)d[r0 + t] * S + s0 + q] = v; });
+    const int ce = min(k0 + MF_SB, f.e) - r0, cd = min(MF_NB, ce);
+    float2 acc[1][NS] = {};
+    mf_stage_x(sm, r0, ce, ns, [&](int c) { return X + (long long)c * S; });
+    __syncthreads();
+    mf_accumulate<NS, 1, 16>(sm, acc, ce, [&](int, int c) {
+        const float2* p = c < cd ? D + c * MF_NB : F + (r0 + c) * n;
+        return live ? *p : make_float2(0.f, 0.f);
+    });
+    mf_finish<NS, 1>(sm, acc, ns, [&](int t, int q, float2 v) { if (r0 + t < f.e) xs[(long long)d[r0 + t] * S + s0 + q] = v; });
 }
 
 // rows [0, k0): y[r] -= U[r, k0:k1] x[k0:k1]
