@@ -728,10 +728,10 @@ def main():
                          "frac": achieved / hbm, "traffic": ASM_TRAFFIC_PER_TET * nt,
                          "traffic_note": "bytes per launch of assemble_chunk_kernel: dram read+write per tet from the "
                                          "ncu capture at 82 944 tets (profiles/assemble_chunk_kernel_cavity24.md) "
-                                         "scaled by tets; the invariants kernel adds ~1.4 KB/tet",
+                                         "scaled by tets; the records kernel adds ~1.4 KB/tet",
                          "peak_kind": peak_kind,
                          "alg_bytes_per_tet": alg_bytes_per_tet,
-                         "kernels": "tet_invariants_kernel+assemble_chunk_kernel"},
+                         "kernels": "tet_records_kernel+assemble_chunk_kernel"},
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(d2h),
                     "api": "emerge_b200.assembly.tet_mass_stiffness_matrices (host numpy in, SciPy CSR out)"},
             "gpu_launches": 2 * args.steps,

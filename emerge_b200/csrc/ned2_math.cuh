@@ -278,11 +278,25 @@ struct RecGlobal {
 #endif
     }
 };
-struct RecShared {
+// The fields one block kind needs, staged in shared memory (even offsets, records an odd number of 16-byte
+// words apart): C_OFF and G_OFF are subtracted from the field numbers of complex and real fields.
+template <int C_OFF, int G_OFF>
+struct RecStaged {
     const double* base;
-    EMFEM_HD double g(int f) const { return base[f]; }
-    EMFEM_HD cd c(int f) const { return mk(base[f], base[f + 1]); }
+    EMFEM_HD double g(int f) const { return base[f - G_OFF]; }
+    EMFEM_HD cd c(int f) const {
+#if defined(__CUDA_ARCH__)
+        const double2 v = *reinterpret_cast<const double2*>(base + f - C_OFF);
+        return mk(v.x, v.y);
+#else
+        return mk(base[f - C_OFF], base[f - C_OFF + 1]);
+#endif
+    }
 };
+// curl-curl: Q, then the real fields from REC_DS on; mass: P, then the same real fields
+typedef RecStaged<REC_Q, REC_Q> RecCurl;
+typedef RecStaged<REC_P, REC_DS - 32> RecMass;
+constexpr int REC_CURL_STRIDE = 86, REC_MASS_STRIDE = 46;       // doubles
 static_assert(REC_STRIDE % 2 == 0 && REC_P % 2 == 0 && REC_Q % 2 == 0, "complex invariants are 16-byte aligned");
 
 // prod k_i! of four vertices as a double: equal pairs only (the sets below never hold one vertex four times
@@ -292,19 +306,66 @@ EMFEM_HD double six_if(bool c) { return c ? 6.0 : 2.0; }       // {x, x, y, z}: 
 EMFEM_HD double pairs2(bool same) { return same ? 24.0 : 4.0; }   // {x, x, y, y}
 EMFEM_HD void fma_c(cd& s, double k, cd v) { s.x = fma(k, v.x, s.x); s.y = fma(k, v.y, s.y); }
 
-// Pair block of sorted slots sx, sy (0..5 edges, 6..9 faces), scaled as pair_block's.
+// Pair blocks of sorted slots sx, sy (0..5 edges, 6..9 faces), scaled as pair_block's: the curl-curl block d needs
+// only Q of the record, the mass block f only P.
 template <class IV>
-EMFEM_HD void canon_block(const IV& I, int sx, int sy, cd d[4], cd f[4]) {
+EMFEM_HD void canon_curl(const IV& I, int sx, int sy, cd d[4]) {
     const bool xe = sx < 6, ye = sy < 6;
     if (xe && ye) {
         const int a = canon_p(sx), b = canon_q(sx), c = canon_p(sy), e = canon_q(sy);
-        const cd q = I.c(REC_Q + 2 * (6 * sx + sy));
+        const cd q9 = (9.0 * (I.g(REC_L + sx) * I.g(REC_L + sy))) * I.c(REC_Q + 2 * (6 * sx + sy));
+        d[0] = two_if(a == c) * q9; d[1] = two_if(a == e) * q9; d[2] = two_if(b == c) * q9; d[3] = two_if(b == e) * q9;
+    } else if (xe != ye) {
+        // edge-face block; a face row uses the transposed edge-face block (curlcurl.py:321-328)
+        const int es = xe ? sx : sy, fs = (xe ? sy : sx) - 6;
+        const int a = canon_p(es), b = canon_q(es), c = canon_fv(fs, 0), e = canon_fv(fs, 1), g = canon_fv(fs, 2);
+        const int pcd = canon_fp(fs, 0), pcf = canon_fp(fs, 1), pdf = canon_fp(fs, 2);
+        const cd qcd = I.c(REC_Q + 2 * (6 * es + pcd)), qcf = I.c(REC_Q + 2 * (6 * es + pcf)), qdf = I.c(REC_Q + 2 * (6 * es + pdf));
+        const double L3 = 3.0 * I.g(REC_L + es), k0 = L3 * I.g(REC_DS + pcf), k1 = L3 * I.g(REC_DS + pcd);
+        auto curl = [&](int x, cd& lo, cd& hi) {      // sums with L_x: x one of the edge's vertices
+            const double vc = two_if(x == c), vd = two_if(x == e), vf = two_if(x == g);
+            const cd s = vd * qcf, t = vc * qdf, u = vf * qcd;
+            lo = k0 * mk(-2.0 * s.x - t.x - u.x, -2.0 * s.y - t.y - u.y);
+            hi = k1 * mk(2.0 * u.x + s.x - t.x, 2.0 * u.y + s.y - t.y);
+        };
+        cd e00, e01, e10, e11;
+        curl(a, e00, e01);
+        curl(b, e10, e11);
+        d[0] = e00; d[3] = e11;
+        d[1] = xe ? e01 : e10; d[2] = xe ? e10 : e01;
+    } else {
+        const int fx = sx - 6, fy = sy - 6;
+        const int c = canon_fv(fy, 0), dd = canon_fv(fy, 1), g = canon_fv(fy, 2);
+        const int pab = canon_fp(fx, 0), pae = canon_fp(fx, 1), pbe = canon_fp(fx, 2);
+        const int pcd = canon_fp(fy, 0), pcf = canon_fp(fy, 1), pdf = canon_fp(fy, 2);
+        // curl of L_r W_su against the column's first and second function, s and u the row's other vertices
+        auto curl = [&](int r, int psu, cd& lo, cd& hi) {
+            const cd cf = I.c(REC_Q + 2 * (6 * psu + pcf)), df = I.c(REC_Q + 2 * (6 * psu + pdf)), cdq = I.c(REC_Q + 2 * (6 * psu + pcd));
+            const cd s = two_if(r == dd) * cf, t = two_if(r == c) * df, u = two_if(r == g) * cdq;
+            lo = mk(2.0 * s.x + t.x + u.x, 2.0 * s.y + t.y + u.y);
+            hi = mk(t.x - 2.0 * u.x - s.x, t.y - 2.0 * u.y - s.y);
+        };
+        cd b0, b1, a0, a1, e0, e1;
+        curl(canon_fv(fx, 1), pae, b0, b1);
+        curl(canon_fv(fx, 0), pbe, a0, a1);
+        curl(canon_fv(fx, 2), pab, e0, e1);
+        const double Lac1 = I.g(REC_DS + pae), Lab1 = I.g(REC_DS + pab), Lac2 = I.g(REC_DS + pcf), Lab2 = I.g(REC_DS + pcd);
+        d[0] = (Lac1 * Lac2) * mk(2.0 * b0.x + a0.x + e0.x, 2.0 * b0.y + a0.y + e0.y);
+        d[1] = (Lac1 * Lab2) * mk(2.0 * b1.x + a1.x + e1.x, 2.0 * b1.y + a1.y + e1.y);
+        d[2] = (Lab1 * Lac2) * mk(a0.x - 2.0 * e0.x - b0.x, a0.y - 2.0 * e0.y - b0.y);
+        d[3] = (Lab1 * Lab2) * mk(a1.x - 2.0 * e1.x - b1.x, a1.y - 2.0 * e1.y - b1.y);
+    }
+}
+
+template <class IV>
+EMFEM_HD void canon_mass(const IV& I, int sx, int sy, cd f[4]) {
+    const bool xe = sx < 6, ye = sy < 6;
+    if (xe && ye) {
+        const int a = canon_p(sx), b = canon_q(sx), c = canon_p(sy), e = canon_q(sy);
         const cd pac = I.c(REC_P + 2 * (4 * a + c)), pad = I.c(REC_P + 2 * (4 * a + e));
         const cd pbc = I.c(REC_P + 2 * (4 * b + c)), pbd = I.c(REC_P + 2 * (4 * b + e));
         const double L = I.g(REC_L + sx) * I.g(REC_L + sy);
         const bool ac = a == c, ad = a == e, bc = b == c, bd = b == e;
-        const cd q9 = (9.0 * L) * q;
-        d[0] = two_if(ac) * q9; d[1] = two_if(ad) * q9; d[2] = two_if(bc) * q9; d[3] = two_if(bd) * q9;
         const double abcd = two_if(ac || ad) * two_if(bc || bd);
         const double abcc = six_if(ac || bc), abdd = six_if(ad || bd), aacd = six_if(ac || ad), bbcd = six_if(bc || bd);
         const cd uac = L * pac, uad = -L * pad, ubc = -L * pbc, ubd = L * pbd;
@@ -313,25 +374,12 @@ EMFEM_HD void canon_block(const IV& I, int sx, int sy, cd d[4], cd f[4]) {
         f[2] = bbcd * uac; fma_c(f[2], pairs2(bc), uad); fma_c(f[2], abcd, ubc); fma_c(f[2], abcc, ubd);
         f[3] = pairs2(bd) * uac; fma_c(f[3], bbcd, uad); fma_c(f[3], abdd, ubc); fma_c(f[3], abcd, ubd);
     } else if (xe != ye) {
-        // edge-face block; a face row uses the transposed edge-face block (curlcurl.py:321-328)
         const int es = xe ? sx : sy, fs = (xe ? sy : sx) - 6;
         const int a = canon_p(es), b = canon_q(es), c = canon_fv(fs, 0), e = canon_fv(fs, 1), g = canon_fv(fs, 2);
-        const int pcd = canon_fp(fs, 0), pcf = canon_fp(fs, 1), pdf = canon_fp(fs, 2);
-        const cd qcd = I.c(REC_Q + 2 * (6 * es + pcd)), qcf = I.c(REC_Q + 2 * (6 * es + pcf)), qdf = I.c(REC_Q + 2 * (6 * es + pdf));
         const cd pac = I.c(REC_P + 2 * (4 * a + c)), pad = I.c(REC_P + 2 * (4 * a + e)), paf = I.c(REC_P + 2 * (4 * a + g));
         const cd pbc = I.c(REC_P + 2 * (4 * b + c)), pbd = I.c(REC_P + 2 * (4 * b + e)), pbf = I.c(REC_P + 2 * (4 * b + g));
-        const double L1 = I.g(REC_L + es), k0 = L1 * I.g(REC_DS + pcf), k1 = L1 * I.g(REC_DS + pcd);
+        const double L1 = I.g(REC_L + es), k0 = L1 * I.g(REC_DS + canon_fp(fs, 1)), k1 = L1 * I.g(REC_DS + canon_fp(fs, 0));
         const bool ac = a == c, ad = a == e, af = a == g, bc = b == c, bd = b == e, bf = b == g;
-        const cd q3f = 3.0 * qcf, q3d = 3.0 * qdf, q3c = 3.0 * qcd;
-        auto curl = [&](bool xc, bool xd, bool xf, cd& lo, cd& hi) {      // sums with L_x: x one of the edge's vertices
-            const double vc = two_if(xc), vd = two_if(xd), vf = two_if(xf);
-            const cd s = vd * q3f, t = vc * q3d, u = vf * q3c;
-            lo = k0 * mk(-2.0 * s.x - t.x - u.x, -2.0 * s.y - t.y - u.y);
-            hi = k1 * mk(2.0 * u.x + s.x - t.x, 2.0 * u.y + s.y - t.y);
-        };
-        cd e00, e01, e10, e11;
-        curl(ac, ad, af, e00, e01);
-        curl(bc, bd, bf, e10, e11);
         const double abcd = two_if(ac || ad) * two_if(bc || bd), abdf = two_if(ad || af) * two_if(bd || bf);
         const double abcf = two_if(ac || af) * two_if(bc || bf);
         const double aacd = six_if(ac || ad), aadf = six_if(ad || af), aacf = six_if(ac || af);
@@ -340,36 +388,17 @@ EMFEM_HD void canon_block(const IV& I, int sx, int sy, cd d[4], cd f[4]) {
         cd g01 = abdf * pac; fma_c(g01, -abcf, pad); fma_c(g01, -aadf, pbc); fma_c(g01, aacf, pbd);
         cd g10 = bbcd * paf; fma_c(g10, -bbdf, pac); fma_c(g10, -abcd, pbf); fma_c(g10, abdf, pbc);
         cd g11 = bbdf * pac; fma_c(g11, -bbcf, pad); fma_c(g11, -abdf, pbc); fma_c(g11, abcf, pbd);
-        d[0] = e00; d[3] = e11;
-        d[1] = xe ? e01 : e10; d[2] = xe ? e10 : e01;
         f[0] = k0 * g00; f[3] = k1 * g11;
         f[1] = xe ? k1 * g01 : k0 * g10; f[2] = xe ? k0 * g10 : k1 * g01;
     } else {
         const int fx = sx - 6, fy = sy - 6;
         const int a = canon_fv(fx, 0), b = canon_fv(fx, 1), e = canon_fv(fx, 2);
         const int c = canon_fv(fy, 0), dd = canon_fv(fy, 1), g = canon_fv(fy, 2);
-        const int pab = canon_fp(fx, 0), pae = canon_fp(fx, 1), pbe = canon_fp(fx, 2);
-        const int pcd = canon_fp(fy, 0), pcf = canon_fp(fy, 1), pdf = canon_fp(fy, 2);
-        const double Lac1 = I.g(REC_DS + pae), Lab1 = I.g(REC_DS + pab), Lac2 = I.g(REC_DS + pcf), Lab2 = I.g(REC_DS + pcd);
-        // curl of L_r W_su against the column's first and second function, s and u the row's other vertices
-        auto curl = [&](int r, int psu, cd& lo, cd& hi) {
-            const cd cf = I.c(REC_Q + 2 * (6 * psu + pcf)), df = I.c(REC_Q + 2 * (6 * psu + pdf)), cdq = I.c(REC_Q + 2 * (6 * psu + pcd));
-            const double vc = two_if(r == c), vd = two_if(r == dd), vf = two_if(r == g);
-            const cd s = vd * cf, t = vc * df, u = vf * cdq;
-            lo = mk(2.0 * s.x + t.x + u.x, 2.0 * s.y + t.y + u.y);
-            hi = mk(t.x - 2.0 * u.x - s.x, t.y - 2.0 * u.y - s.y);
-        };
-        cd b0, b1, a0, a1, e0, e1;
-        curl(b, pae, b0, b1);
-        curl(a, pbe, a0, a1);
-        curl(e, pab, e0, e1);
-        d[0] = (Lac1 * Lac2) * mk(2.0 * b0.x + a0.x + e0.x, 2.0 * b0.y + a0.y + e0.y);
-        d[1] = (Lac1 * Lab2) * mk(2.0 * b1.x + a1.x + e1.x, 2.0 * b1.y + a1.y + e1.y);
-        d[2] = (Lab1 * Lac2) * mk(a0.x - 2.0 * e0.x - b0.x, a0.y - 2.0 * e0.y - b0.y);
-        d[3] = (Lab1 * Lab2) * mk(a1.x - 2.0 * e1.x - b1.x, a1.y - 2.0 * e1.y - b1.y);
         const cd pef = I.c(REC_P + 2 * (4 * e + g)), pec = I.c(REC_P + 2 * (4 * e + c)), ped = I.c(REC_P + 2 * (4 * e + dd));
         const cd paf = I.c(REC_P + 2 * (4 * a + g)), pac = I.c(REC_P + 2 * (4 * a + c)), pad = I.c(REC_P + 2 * (4 * a + dd));
         const cd pbf = I.c(REC_P + 2 * (4 * b + g)), pbc = I.c(REC_P + 2 * (4 * b + c)), pbd = I.c(REC_P + 2 * (4 * b + dd));
+        const double Lac1 = I.g(REC_DS + canon_fp(fx, 1)), Lab1 = I.g(REC_DS + canon_fp(fx, 0));
+        const double Lac2 = I.g(REC_DS + canon_fp(fy, 1)), Lab2 = I.g(REC_DS + canon_fp(fy, 0));
         const bool ac = a == c, ad = a == dd, af = a == g, bc = b == c, bd = b == dd, bf = b == g, ec = e == c, ed = e == dd, ef = e == g;
         // prod k_i! of {x, y, u, v}, x != y, u != v
         const double abcd = two_if(ac || ad) * two_if(bc || bd), abdf = two_if(ad || af) * two_if(bd || bf);
