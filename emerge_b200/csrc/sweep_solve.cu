@@ -132,12 +132,13 @@ __device__ __forceinline__ void block_store2(double2 v0, double2 v1, int ncomp, 
 // per lane, and the 32 / L groups of lanes take every (32 / L)-th entry, so that a read of a matrix entry
 // serves NR systems and a batch of one system still has 32 entries in flight.  Entries travel by asynchronous
 // copies, DEPTH stages of 32 / L entries deep: as many bytes in flight held in registers leave too few
-// warps (115 against 75 us at S = 32 below; depths 3 to 5 are alike, 8 costs the second block of an SM, and
+// warps (115 against 75 us at S = 32 with one entry a stage; 8 stages cost the second block of an SM, and
 // one system, whose row is three stages, is fastest with 2).  E - k0^2 B is formed per entry (2 + 4
 // multiply-adds per system instead of 8).
 // Measured (one launch, us, before: a thread per row and system): 6 000-tet guide, S = 1 / 4 / 16 / 32:
-// 37 / 30 / 69 / 98 -> 14 / 23 / 51 / 75; 82 944-tet cavity: 283 / 379 / 1058 / 1340 -> 205 / 290 / 613 / 921
+// 37 / 30 / 69 / 98 -> 14 / 18 / 40 / 64; 82 944-tet cavity: 283 / 379 / 1058 / 1340 -> 205 / 254 / 483 / 793
 // (the last at 0.9 TB/s of matrix and 6.4 TB/s of gathered x; FP64 multiply-adds are half of its time).
+
 // Sum over the lane groups, halving the values a lane holds while it can: afterwards a lane holds row
 // (lane & 16) and max(1, 2 NR L / 32) systems of the lane, the first of them the returned one.
 template <int L, int NR>
@@ -178,12 +179,19 @@ __device__ __forceinline__ void cp_async8z(void* dst, const void* src, bool ok) 
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src), "r"(n) : "memory");
 }
 
-// Pipeline stages of a warp: 32 / L entries each, their x values and the two rows' E and B.
+// Pipeline stages of a warp: UE entries per lane group each, their x values and the two rows' E and B.  More entries
+// a stage spread its bookkeeping (which took the issue slots of the narrow batches), more shared memory a warp
+// costs resident warps.  Measured on the 6 000- and 82 944-tet meshes, us for one entry in four stages / two entries /
+// four entries in two stages: S = 4 22.9 290 / 18.4 254 (three stages) / 19.1 286; S = 8 37.6 467 / 27.2 341 (three) /
+// 24.0 305; S = 16 50.7 613 / 39.6 483 (three) / 40.4 532; S = 32 74.2 921 / 64.2 793 (three) / 86.7 1099.
 template <typename R, int L, int NR, bool HASB>
 struct SpmvStage {
-    static constexpr int DEPTH = L == 1 ? 2 : 4;
-    typename V2<R>::T x[32 / L][L * NR];
-    double2 eb[HASB ? 4 : 2][32 / L];        // E row 0, E row 1, B row 0, B row 1
+    static constexpr bool FOUR = L == 8 && NR == 1;
+    static constexpr int UE = L == 1 ? 1 : FOUR ? 4 : 2;
+    static constexpr int GE = 32 / L * UE;
+    static constexpr int DEPTH = L <= 2 || FOUR ? 2 : 3;
+    typename V2<R>::T x[GE][L * NR];
+    double2 eb[HASB ? 4 : 2][GE];            // E row 0, E row 1, B row 0, B row 1
 };
 
 template <typename R, int L, int NR, bool HASB>
@@ -194,7 +202,7 @@ __global__ void __launch_bounds__(VB, NR == 1 ? 4 : NR == 2 ? 3 : 2) spmv_kernel
     typedef SpmvStage<R, L, NR, HASB> Stage;
     constexpr int G = 32 / L;                       // entry groups of a warp
     constexpr int NV = 2 * NR > G ? 2 * NR / G : 1; // values of a lane after the reduction
-    constexpr int D = Stage::DEPTH;
+    constexpr int D = Stage::DEPTH, UE = Stage::UE, GE = Stage::GE, CPC = 32 / GE;   // CPC stages per 32 indices
     constexpr int XC = L * NR * (int)sizeof(T) / 16;      // 16-byte chunks of an entry's x values (0: 8 bytes)
     extern __shared__ __align__(16) unsigned char spmv_sm[];
     const int S = a.S;
@@ -233,43 +241,43 @@ __global__ void __launch_bounds__(VB, NR == 1 ? 4 : NR == 2 ? 3 : 2) spmv_kernel
 #pragma unroll
         for (int q = 0; q < 2 * NR; q++) acc[q] = make_double2(0.0, 0.0);
         const int nm = n0 > n1 ? n0 : n1;
-        const int nst = (nm + G - 1) / G;
+        const int nst = (nm + GE - 1) / GE;
         // 32 column indices of each row per coalesced load, the next ones in flight while these are used
         int ia = -1, ib = -1;
         int ia2 = lane < n0 ? a.indices[j0 + lane] : -1, ib2 = lane < n1 ? a.indices[j1 + lane] : -1;
         bool paired = true;                          // the rows' columns agree so far
         auto issue = [&](int t) {
             if (t < nst) {
-                if (t % L == 0) {
+                if (t % CPC == 0) {
                     ia = ia2; ib = ib2;
-                    const int kn = t * G + 32 + lane;
+                    const int kn = t * GE + 32 + lane;
                     ia2 = kn < n0 ? a.indices[j0 + kn] : -1;
                     ib2 = kn < n1 ? a.indices[j1 + kn] : -1;
                     paired = paired && __all_sync(0xffffffffu, ia == ib);
                 }
                 Stage& sg = st[t % D];
-                const int kc = (t % L) * G;          // first entry of the stage inside the 32 of the chunk
+                const int kc = (t % CPC) * GE;       // first entry of the stage inside the 32 of the chunk
                 if (XC > 0) {
 #pragma unroll
-                    for (int q = 0; q < (G * XC + 31) / 32; q++) {
+                    for (int q = 0; q < (GE * XC + 31) / 32; q++) {
                         const int ch = lane + 32 * q, en = ch / (XC > 0 ? XC : 1), c = __shfl_sync(0xffffffffu, ia, (kc + en) & 31);
-                        if (G * XC >= 32 || ch < G * XC)
+                        if (GE * XC >= 32 || ch < GE * XC)
                             cp_async16z(reinterpret_cast<char*>(&sg.x[0][0]) + 16 * ch,
                                         reinterpret_cast<const char*>(x + (long long)(c < 0 ? 0 : c) * S + sb) + 16 * (ch % (XC > 0 ? XC : 1)), c >= 0);
                     }
                 } else {
                     const int c = __shfl_sync(0xffffffffu, ia, (kc + lane) & 31);
-                    if (lane < G) cp_async8z(&sg.x[lane][0], x + (long long)(c < 0 ? 0 : c) * S, c >= 0);
+                    if (lane < GE) cp_async8z(&sg.x[lane][0], x + (long long)(c < 0 ? 0 : c) * S, c >= 0);
                 }
-                constexpr int NE = (HASB ? 4 : 2) * G;
+                constexpr int NE = (HASB ? 4 : 2) * GE;
 #pragma unroll
                 for (int q = 0; q < (NE + 31) / 32; q++) {
-                    const int e = lane + 32 * q, which = e / G, kk = t * G + e % G;
+                    const int e = lane + 32 * q, which = e / GE, kk = t * GE + e % GE;
                     if (NE % 32 == 0 || e < NE) {
                         const bool second = which & 1;
                         const bool ok = kk < (second ? n1 : n0);
                         const double2* src = (which & 2 ? Bv : Ev) + (second ? j1 : j0) + (ok ? kk : 0);
-                        cp_async16z(&sg.eb[which][e % G], src, ok);
+                        cp_async16z(&sg.eb[which][e % GE], src, ok);
                     }
                 }
             }
@@ -282,34 +290,38 @@ __global__ void __launch_bounds__(VB, NR == 1 ? 4 : NR == 2 ? 3 : 2) spmv_kernel
             asm volatile("cp.async.wait_group %0;\n" ::"n"(D - 1) : "memory");
             __syncwarp();
             const Stage& sg = st[t % D];
-            T xa[NR];
 #pragma unroll
-            for (int r = 0; r < NR; r++) xa[r] = sg.x[g][sl + r * L];
-            const double2 e0 = sg.eb[0][g], e1 = sg.eb[1][g];
-            double2 b0, b1;
-            if (HASB) { b0 = sg.eb[2][g]; b1 = sg.eb[3][g]; }
+            for (int u = 0; u < UE; u++) {
+                const int en = u * G + g;
+                T xa[NR];
 #pragma unroll
-            for (int r = 0; r < NR; r++) {
-                const double xr = xa[r].x, xi = xa[r].y;
-                const double kr = HASB ? fma(-k2[r], b0.x, e0.x) : e0.x;
-                const double ki = HASB ? fma(-k2[r], b0.y, e0.y) : e0.y;
-                acc[r].x = fma(kr, xr, fma(-ki, xi, acc[r].x));
-                acc[r].y = fma(kr, xi, fma(ki, xr, acc[r].y));
-            }
-            if (!paired) {                           // the second row's own columns
-                const int kk = t * G + g;
-                const int cb = kk < n1 ? a.indices[j1 + kk] : -1;
-                const T* xc = x + (long long)(cb >= 0 ? cb : 0) * S + s0;
+                for (int r = 0; r < NR; r++) xa[r] = sg.x[en][sl + r * L];
+                const double2 e0 = sg.eb[0][en], e1 = sg.eb[1][en];
+                double2 b0, b1;
+                if (HASB) { b0 = sg.eb[2][en]; b1 = sg.eb[3][en]; }
 #pragma unroll
-                for (int r = 0; r < NR; r++) xa[r] = cb >= 0 ? xc[r * L] : mk2<R>(0, 0);
-            }
+                for (int r = 0; r < NR; r++) {
+                    const double xr = xa[r].x, xi = xa[r].y;
+                    const double kr = HASB ? fma(-k2[r], b0.x, e0.x) : e0.x;
+                    const double ki = HASB ? fma(-k2[r], b0.y, e0.y) : e0.y;
+                    acc[r].x = fma(kr, xr, fma(-ki, xi, acc[r].x));
+                    acc[r].y = fma(kr, xi, fma(ki, xr, acc[r].y));
+                }
+                if (!paired) {                           // the second row's own columns
+                    const int kk = t * GE + en;
+                    const int cb = kk < n1 ? a.indices[j1 + kk] : -1;
+                    const T* xc = x + (long long)(cb >= 0 ? cb : 0) * S + s0;
 #pragma unroll
-            for (int r = 0; r < NR; r++) {
-                const double xr = xa[r].x, xi = xa[r].y;
-                const double kr = HASB ? fma(-k2[r], b1.x, e1.x) : e1.x;
-                const double ki = HASB ? fma(-k2[r], b1.y, e1.y) : e1.y;
-                acc[NR + r].x = fma(kr, xr, fma(-ki, xi, acc[NR + r].x));
-                acc[NR + r].y = fma(kr, xi, fma(ki, xr, acc[NR + r].y));
+                    for (int r = 0; r < NR; r++) xa[r] = cb >= 0 ? xc[r * L] : mk2<R>(0, 0);
+                }
+#pragma unroll
+                for (int r = 0; r < NR; r++) {
+                    const double xr = xa[r].x, xi = xa[r].y;
+                    const double kr = HASB ? fma(-k2[r], b1.x, e1.x) : e1.x;
+                    const double ki = HASB ? fma(-k2[r], b1.y, e1.y) : e1.y;
+                    acc[NR + r].x = fma(kr, xr, fma(-ki, xi, acc[NR + r].x));
+                    acc[NR + r].y = fma(kr, xi, fma(ki, xr, acc[NR + r].y));
+                }
             }
             __syncwarp();
         }
