@@ -721,14 +721,41 @@ __global__ void mf_child_rows_kernel(int v0, int nf, const FrontMeta* __restrict
         M[ea[g.ea + i]] = (int)(g.wv + g.e + i);
 }
 
+// The kernels of an application are a chain of some 250 short dependent launches, so each is launched before its
+// predecessor has ended (programmatic stream serialization): it loads what the factorization left (maps and the
+// first factor columns), waits for the predecessor, and only then touches the vectors, past L1, which may hold lines
+// from before the predecessor's stores.  Every block waits, also one with nothing to do: a kernel that ended
+// earlier would let its successor pass the one before.
+__device__ __forceinline__ void mf_chain_start() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+__device__ __forceinline__ void mf_chain_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+__device__ __forceinline__ float2 mf_vec(const float2* p) {
+    float2 v;
+    asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];\n" : "=f"(v.x), "=f"(v.y) : "l"(p) : "memory");
+    return v;
+}
+template <typename... P, typename... A>
+static void mf_chain(void (*kernel)(P...), dim3 grid, cudaStream_t s, A... args) {
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = grid;
+    c.blockDim = dim3(256);
+    c.stream = s;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+
 // w (the front's rows, S per row): own rows from the right-hand side, plus both children's update rows
 __global__ void mf_fwd_gather_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm, int S,
                                      const int* __restrict__ fdof, const double* __restrict__ scale,
                                      const int* __restrict__ cmap, long long rows, const double2* __restrict__ rhs,
                                      float2* __restrict__ w) {
+    mf_chain_start();
     const FrontMeta& f = fm[lst[blockIdx.y]];
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (long long)f.n * S) return;
+    if (idx >= (long long)f.n * S) { mf_chain_wait(); return; }
     const int i = (int)(idx / S), s = (int)(idx % S);
     const int a = cmap[f.wv + i], b = cmap[rows + f.wv + i];
     float2 v = make_float2(0.f, 0.f);
@@ -738,8 +765,9 @@ __global__ void mf_fwd_gather_kernel(const int* __restrict__ lst, const FrontMet
         const double sc = scale[d];
         v = make_float2((float)(r.x * sc), (float)(r.y * sc));
     }
-    if (a >= 0) { const float2 u = w[(long long)a * S + s]; v.x += u.x; v.y += u.y; }
-    if (b >= 0) { const float2 u = w[(long long)b * S + s]; v.x += u.x; v.y += u.y; }
+    mf_chain_wait();
+    if (a >= 0) { const float2 u = mf_vec(w + (long long)a * S + s); v.x += u.x; v.y += u.y; }
+    if (b >= 0) { const float2 u = mf_vec(w + (long long)b * S + s); v.x += u.x; v.y += u.y; }
     w[f.wv * S + idx] = v;
 }
 
@@ -760,7 +788,7 @@ template <int NS, typename XOf>
 __device__ __forceinline__ void mf_stage_x(MfProdSmem<NS>& sm, int c0, int nc, int ns, XOf xof) {
     for (int t = threadIdx.x; t < nc * NS; t += 256) {
         const int c = t / NS, q = t % NS;
-        sm.x[c][q] = q < ns ? xof(c0 + c)[q] : make_float2(0.f, 0.f);
+        sm.x[c][q] = q < ns ? mf_vec(xof(c0 + c) + q) : make_float2(0.f, 0.f);
     }
 }
 
@@ -768,14 +796,17 @@ __device__ __forceinline__ void mf_stage_x(MfProdSmem<NS>& sm, int c0, int nc, i
 // takes every eighth column, U of them at once with the columns past the end masked: a plain unrolled loop runs
 // its remainder one load latency per column (block-inverse kernels of one front, whose column counts are
 // no multiples of 64: 18 us a launch at one or eight right-hand sides, 5 and 7 now)
+template <int RPL, int U, typename MAt>
+__device__ __forceinline__ void mf_load(float2 (*mv)[RPL], int c0, int nc, MAt mat) {
+#pragma unroll
+    for (int u = 0; u < U; u++)
+#pragma unroll
+        for (int i = 0; i < RPL; i++) mv[u][i] = c0 + 8 * u < nc ? mat(i, c0 + 8 * u) : make_float2(0.f, 0.f);
+}
+// mv: this warp's first columns, loaded
 template <int NS, int RPL, int U, typename MAt>
-__device__ __forceinline__ void mf_accumulate(const MfProdSmem<NS>& sm, float2 (*acc)[NS], int nc, MAt mat) {
-    for (int c0 = threadIdx.x >> 5; c0 < nc; c0 += 8 * U) {
-        float2 mv[U][RPL];
-#pragma unroll
-        for (int u = 0; u < U; u++)
-#pragma unroll
-            for (int i = 0; i < RPL; i++) mv[u][i] = c0 + 8 * u < nc ? mat(i, c0 + 8 * u) : make_float2(0.f, 0.f);
+__device__ __forceinline__ void mf_accumulate(const MfProdSmem<NS>& sm, float2 (*acc)[NS], float2 (*mv)[RPL], int nc, MAt mat) {
+    for (int c0 = threadIdx.x >> 5; c0 < nc;) {
 #pragma unroll
         for (int u = 0; u < U; u++) {
             const int c = c0 + 8 * u;
@@ -795,6 +826,8 @@ __device__ __forceinline__ void mf_accumulate(const MfProdSmem<NS>& sm, float2 (
                 for (int i = 0; i < RPL; i++) cfma(acc[i][0], mv[u][i], sm.x[c][0]);
             }
         }
+        c0 += 8 * U;
+        if (c0 < nc) mf_load<RPL, U>(mv, c0, nc, mat);
     }
 }
 
@@ -825,12 +858,17 @@ __device__ __forceinline__ void mf_finish(MfProdSmem<NS>& sm, float2 (*acc)[NS],
 template <int NS, int RPL, typename XOf, typename MAt, typename Out>
 __device__ __forceinline__ void mf_product(MfProdSmem<NS>& sm, int c0, int c1, int ns, XOf xof, MAt mat, Out out) {
     float2 acc[RPL][NS] = {};
+    if (c0 >= c1) mf_chain_wait();
     for (int cb = c0; cb < c1; cb += MF_KC) {
         const int nc = min(MF_KC, c1 - cb);
-        if (cb > c0) __syncthreads();
+        auto at = [&](int i, int c) { return mat(i, cb + c); };
+        float2 mv[8][RPL];
+        mf_load<RPL, 8>(mv, threadIdx.x >> 5, nc, at);
+        if (cb == c0) mf_chain_wait();
+        else __syncthreads();
         mf_stage_x(sm, cb, nc, ns, xof);
         __syncthreads();
-        mf_accumulate<NS, RPL, 8>(sm, acc, nc, [&](int i, int c) { return mat(i, cb + c); });
+        mf_accumulate<NS, RPL, 8>(sm, acc, mv, nc, at);
     }
     mf_finish<NS, RPL>(sm, acc, ns, out);
 }
@@ -843,9 +881,10 @@ __global__ void __launch_bounds__(256) mf_fwd_tri_kernel(const int* __restrict__
                                                          const float2* __restrict__ inv, const float2* __restrict__ w,
                                                          float2* __restrict__ y) {
     __shared__ MfProdSmem<NS> sm;
+    mf_chain_start();
     const FrontMeta& f = fm[lst[blockIdx.y]];
     const int r0 = k0 + blockIdx.x * MF_NB;
-    if (r0 >= f.e) return;
+    if (r0 >= f.e) { mf_chain_wait(); return; }
     const int s0 = blockIdx.z * NS, ns = min(NS, S - s0), r = r0 + (threadIdx.x & 31);
     const float2* F = fact + f.fact + r;
     const float2* D = inv + f.inv + (long long)(r0 / MF_NB) * 2 * MF_NB * MF_NB + (threadIdx.x & 31);
@@ -856,12 +895,16 @@ __global__ void __launch_bounds__(256) mf_fwd_tri_kernel(const int* __restrict__
     const int co = r0 - k0;              // staged columns: the block row's off-diagonal part, then its diagonal block
     const int nc = min(r0 + MF_NB, f.e) - k0;
     float2 acc[1][NS] = {};
-    mf_stage_x(sm, k0, nc, ns, [&](int c) { return X + (long long)c * S; });
-    __syncthreads();
-    mf_accumulate<NS, 1, 16>(sm, acc, nc, [&](int, int c) {
+    auto at = [&](int, int c) {
         const float2* p = c < co ? F + (k0 + c) * n : D + (c - co) * MF_NB;
         return live ? *p : make_float2(0.f, 0.f);
-    });
+    };
+    float2 mv[16][1];
+    mf_load<1, 16>(mv, threadIdx.x >> 5, nc, at);
+    mf_chain_wait();
+    mf_stage_x(sm, k0, nc, ns, [&](int c) { return X + (long long)c * S; });
+    __syncthreads();
+    mf_accumulate<NS, 1, 16>(sm, acc, mv, nc, at);
     mf_finish<NS, 1>(sm, acc, ns, [&](int t, int q, float2 v) { if (r0 + t < f.e) Y[(long long)(r0 + t) * S + q] = v; });
 }
 
@@ -871,11 +914,12 @@ __global__ void __launch_bounds__(256, NS * RPL > 16 ? 2 : 3) mf_fwd_update_kern
                                                             int S, int k0, const float2* __restrict__ fact,
                                                             const float2* __restrict__ y, float2* __restrict__ w) {
     __shared__ MfProdSmem<NS> sm;
+    mf_chain_start();
     const FrontMeta& f = fm[lst[blockIdx.y]];
-    if (k0 >= f.e) return;
+    if (k0 >= f.e) { mf_chain_wait(); return; }
     const int k1 = min(k0 + MF_SB, f.e);
     const int r0 = k1 + blockIdx.x * 32 * RPL;
-    if (r0 >= f.n) return;
+    if (r0 >= f.n) { mf_chain_wait(); return; }
     const int s0 = blockIdx.z * NS, ns = min(NS, S - s0), r = r0 + (threadIdx.x & 31);
     const float2* F = fact + f.fact + r;
     const float2* X = y + f.y * S + s0;
@@ -886,8 +930,8 @@ __global__ void __launch_bounds__(256, NS * RPL > 16 ? 2 : 3) mf_fwd_update_kern
                         [&](int t, int q, float2 v) {
                             if (r0 + t >= n) return;
                             float2* p = W + (long long)(r0 + t) * S + q;
-                            p->x -= v.x;
-                            p->y -= v.y;
+                            const float2 o = mf_vec(p);
+                            *p = make_float2(o.x - v.x, o.y - v.y);
                         });
 }
 
@@ -901,9 +945,10 @@ __global__ void __launch_bounds__(256, NS * RPL > 16 ? 2 : 3) mf_bwd_bnd_kernel(
                                                          const float2* __restrict__ xs, float2* __restrict__ y,
                                                          float2* __restrict__ part) {
     __shared__ MfProdSmem<NS> sm;
+    mf_chain_start();
     const FrontMeta& f = fm[lst[blockIdx.y]];
     const int r0 = (blockIdx.x % nrt) * 32 * RPL, sp = blockIdx.x / nrt;
-    if (f.b == 0 || r0 >= f.e) return;
+    if (f.b == 0 || r0 >= f.e) { mf_chain_wait(); return; }
     const int s0 = blockIdx.z * NS, ns = min(NS, S - s0), r = r0 + (threadIdx.x & 31);
     const long long e = f.e;
     const float2* M = fact + f.fact + (long long)f.n * e + r;
@@ -917,25 +962,27 @@ __global__ void __launch_bounds__(256, NS * RPL > 16 ? 2 : 3) mf_bwd_bnd_kernel(
                             if (r0 + t >= e) return;
                             float2* p = Y + (long long)(r0 + t) * S + q;
                             if (nsplit > 1) { *p = v; return; }
-                            p->x -= v.x;
-                            p->y -= v.y;
+                            const float2 o = mf_vec(p);
+                            *p = make_float2(o.x - v.x, o.y - v.y);
                         });
 }
 
 __global__ void mf_bwd_bnd_sum_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm, int S, int nsplit,
                                       long long y0, long long yl, const float2* __restrict__ part, float2* __restrict__ y) {
+    mf_chain_start();
     const FrontMeta& f = fm[lst[blockIdx.y]];
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    mf_chain_wait();
     if (f.b == 0 || idx >= (long long)f.e * S) return;
     float2 t = make_float2(0.f, 0.f);
     for (int sp = 0; sp < nsplit; sp++) {
-        const float2 v = part[((long long)sp * yl + f.y - y0) * S + idx];
+        const float2 v = mf_vec(part + ((long long)sp * yl + f.y - y0) * S + idx);
         t.x += v.x;
         t.y += v.y;
     }
     float2* p = y + f.y * S + idx;
-    p->x -= t.x;
-    p->y -= t.y;
+    const float2 o = mf_vec(p);
+    *p = make_float2(o.x - t.x, o.y - t.y);
 }
 
 // x[k0 .. k1) = H y[k0 .. k1), H the inverse of the 256-block of U, into the solution (DOF order)
@@ -945,9 +992,10 @@ __global__ void __launch_bounds__(256) mf_bwd_tri_kernel(const int* __restrict__
                                                          const float2* __restrict__ inv, const int* __restrict__ fdof,
                                                          const float2* __restrict__ y, float2* __restrict__ xs) {
     __shared__ MfProdSmem<NS> sm;
+    mf_chain_start();
     const FrontMeta& f = fm[lst[blockIdx.y]];
     const int r0 = k0 + blockIdx.x * MF_NB;
-    if (r0 >= f.e) return;
+    if (r0 >= f.e) { mf_chain_wait(); return; }
     const int s0 = blockIdx.z * NS, ns = min(NS, S - s0), r = r0 + (threadIdx.x & 31);
     const float2* F = fact + f.fact + r;
     const float2* D = inv + f.inv + (long long)(r0 / MF_NB) * 2 * MF_NB * MF_NB + MF_NB * MF_NB + (threadIdx.x & 31);
@@ -957,12 +1005,16 @@ __global__ void __launch_bounds__(256) mf_bwd_tri_kernel(const int* __restrict__
     const long long n = f.n;
     const int ce = min(k0 + MF_SB, f.e) - r0, cd = min(MF_NB, ce);
     float2 acc[1][NS] = {};
-    mf_stage_x(sm, r0, ce, ns, [&](int c) { return X + (long long)c * S; });
-    __syncthreads();
-    mf_accumulate<NS, 1, 16>(sm, acc, ce, [&](int, int c) {
+    auto at = [&](int, int c) {
         const float2* p = c < cd ? D + c * MF_NB : F + (r0 + c) * n;
         return live ? *p : make_float2(0.f, 0.f);
-    });
+    };
+    float2 mv[16][1];
+    mf_load<1, 16>(mv, threadIdx.x >> 5, ce, at);
+    mf_chain_wait();
+    mf_stage_x(sm, r0, ce, ns, [&](int c) { return X + (long long)c * S; });
+    __syncthreads();
+    mf_accumulate<NS, 1, 16>(sm, acc, mv, ce, at);
     mf_finish<NS, 1>(sm, acc, ns, [&](int t, int q, float2 v) { if (r0 + t < f.e) xs[(long long)d[r0 + t] * S + s0 + q] = v; });
 }
 
@@ -973,8 +1025,9 @@ __global__ void __launch_bounds__(256, NS * RPL > 16 ? 2 : 3) mf_bwd_update_kern
                                                             const int* __restrict__ fdof, const float2* __restrict__ xs,
                                                             float2* __restrict__ y) {
     __shared__ MfProdSmem<NS> sm;
+    mf_chain_start();
     const FrontMeta& f = fm[lst[blockIdx.y]];
-    if (k0 >= f.e) return;
+    if (k0 >= f.e) { mf_chain_wait(); return; }
     const int k1 = min(k0 + MF_SB, f.e), r0 = blockIdx.x * 32 * RPL;      // k0 is a multiple of 256: whole tiles
     const int s0 = blockIdx.z * NS, ns = min(NS, S - s0), r = r0 + (threadIdx.x & 31);
     const float2* F = fact + f.fact + r;
@@ -986,8 +1039,8 @@ __global__ void __launch_bounds__(256, NS * RPL > 16 ? 2 : 3) mf_bwd_update_kern
                         [&](int i, int c) { return F[32 * i + c * n]; },
                         [&](int t, int q, float2 v) {
                             float2* p = Y + (long long)(r0 + t) * S + q;
-                            p->x -= v.x;
-                            p->y -= v.y;
+                            const float2 o = mf_vec(p);
+                            *p = make_float2(o.x - v.x, o.y - v.y);
                         });
 }
 
@@ -1091,6 +1144,7 @@ template <int NS>
 static int mf_sweep_tree(emfem_mf_s* m, int S, const double2* r, cudaStream_t s) {
     const int nl = (int)m->levels.size();
     const unsigned sz = (unsigned)((S + NS - 1) / NS);
+    bool first = true;
     for (int L = 0; L < nl; L++) {
         const int nfl = (int)m->levels[L].size();
         const long long maxn = m->lvl_max_n[L];
@@ -1098,18 +1152,21 @@ static int mf_sweep_tree(emfem_mf_s* m, int S, const double2* r, cudaStream_t s)
         for (int y0 = 0; y0 < nfl; y0 += 65535) {
             const int ny = std::min(65535, nfl - y0);
             const int* lst = m->d_lst + m->lvl_off[L] + y0;
-            mf_fwd_gather_kernel<<<dim3(nblk(maxn * S, 256), ny), 256, 0, s>>>(lst, m->d_meta, S, m->d_fdof, m->d_scale,
-                                                                              m->d_cmap, m->wv_n, r, m->sw);
+            // the first launch waits for all before it: the right-hand side and, after a factorization, the factors
+            const dim3 gg(nblk(maxn * S, 256), ny);
+            if (first)
+                mf_fwd_gather_kernel<<<gg, 256, 0, s>>>(lst, m->d_meta, S, m->d_fdof, m->d_scale, m->d_cmap, m->wv_n, r, m->sw);
+            else
+                mf_chain(mf_fwd_gather_kernel, gg, s, lst, m->d_meta, S, m->d_fdof, m->d_scale, m->d_cmap, m->wv_n, r, m->sw);
+            first = false;
             for (int k0 = 0; k0 < maxe; k0 += MF_SB) {
                 const unsigned nt = nblk(std::min(MF_SB, maxe - k0), MF_NB);
-                mf_fwd_tri_kernel<NS><<<dim3(nt, ny, sz), 256, 0, s>>>(lst, m->d_meta, S, k0, m->fact, m->inv, m->sw, m->sy);
+                mf_chain(mf_fwd_tri_kernel<NS>, dim3(nt, ny, sz), s, lst, m->d_meta, S, k0, m->fact, m->inv, m->sw, m->sy);
                 const long long rows = maxn - k0;            // rows [k1, n) of a front: at most n - k0
                 if (mf_wide_tiles(rows, ny, sz))
-                    mf_fwd_update_kernel<NS, 2><<<dim3(nblk(rows, 64), ny, sz), 256, 0, s>>>(lst, m->d_meta, S, k0, m->fact,
-                                                                                         m->sy, m->sw);
+                    mf_chain(mf_fwd_update_kernel<NS, 2>, dim3(nblk(rows, 64), ny, sz), s, lst, m->d_meta, S, k0, m->fact, m->sy, m->sw);
                 else
-                    mf_fwd_update_kernel<NS, 1><<<dim3(nblk(rows, 32), ny, sz), 256, 0, s>>>(lst, m->d_meta, S, k0, m->fact,
-                                                                                         m->sy, m->sw);
+                    mf_chain(mf_fwd_update_kernel<NS, 1>, dim3(nblk(rows, 32), ny, sz), s, lst, m->d_meta, S, k0, m->fact, m->sy, m->sw);
             }
         }
         EMFEM_LAUNCH("multifrontal forward");
@@ -1124,28 +1181,28 @@ static int mf_sweep_tree(emfem_mf_s* m, int S, const double2* r, cudaStream_t s)
             if (m->lvl_max_ob[L] > 0) {
                 if (mf_wide_tiles(maxe, ny * nsplit, sz)) {
                     const int nrt = (int)nblk(maxe, 64);
-                    mf_bwd_bnd_kernel<NS, 2><<<dim3(nrt * nsplit, ny, sz), 256, 0, s>>>(
-                        lst, m->d_meta, S, nrt, nsplit, cw, m->lvl_y0[L], m->lvl_yl[L], m->fact, m->d_fdof, m->sx, m->sy, m->spart);
+                    mf_chain(mf_bwd_bnd_kernel<NS, 2>, dim3(nrt * nsplit, ny, sz), s, lst, m->d_meta, S, nrt, nsplit, cw,
+                             m->lvl_y0[L], m->lvl_yl[L], m->fact, m->d_fdof, m->sx, m->sy, m->spart);
                 } else {
                     const int nrt = (int)nblk(maxe, 32);
-                    mf_bwd_bnd_kernel<NS, 1><<<dim3(nrt * nsplit, ny, sz), 256, 0, s>>>(
-                        lst, m->d_meta, S, nrt, nsplit, cw, m->lvl_y0[L], m->lvl_yl[L], m->fact, m->d_fdof, m->sx, m->sy, m->spart);
+                    mf_chain(mf_bwd_bnd_kernel<NS, 1>, dim3(nrt * nsplit, ny, sz), s, lst, m->d_meta, S, nrt, nsplit, cw,
+                             m->lvl_y0[L], m->lvl_yl[L], m->fact, m->d_fdof, m->sx, m->sy, m->spart);
                 }
                 if (nsplit > 1)
-                    mf_bwd_bnd_sum_kernel<<<dim3(nblk((long long)maxe * S, 256), ny), 256, 0, s>>>(
-                        lst, m->d_meta, S, nsplit, m->lvl_y0[L], m->lvl_yl[L], m->spart, m->sy);
+                    mf_chain(mf_bwd_bnd_sum_kernel, dim3(nblk((long long)maxe * S, 256), ny), s, lst, m->d_meta, S, nsplit,
+                             m->lvl_y0[L], m->lvl_yl[L], m->spart, m->sy);
             }
             for (int k0 = (maxe - 1) / MF_SB * MF_SB; maxe > 0 && k0 >= 0; k0 -= MF_SB) {
                 const unsigned nt = nblk(std::min(MF_SB, maxe - k0), MF_NB);
-                mf_bwd_tri_kernel<NS><<<dim3(nt, ny, sz), 256, 0, s>>>(lst, m->d_meta, S, k0, m->fact, m->inv, m->d_fdof,
-                                                                       m->sy, m->sx);
+                mf_chain(mf_bwd_tri_kernel<NS>, dim3(nt, ny, sz), s, lst, m->d_meta, S, k0, m->fact, m->inv, m->d_fdof,
+                         m->sy, m->sx);
                 if (k0 == 0) continue;
                 if (mf_wide_tiles(k0, ny, sz))
-                    mf_bwd_update_kernel<NS, 2><<<dim3(k0 / 64, ny, sz), 256, 0, s>>>(lst, m->d_meta, S, k0, m->fact,
-                                                                                   m->d_fdof, m->sx, m->sy);
+                    mf_chain(mf_bwd_update_kernel<NS, 2>, dim3(k0 / 64, ny, sz), s, lst, m->d_meta, S, k0, m->fact,
+                             m->d_fdof, m->sx, m->sy);
                 else
-                    mf_bwd_update_kernel<NS, 1><<<dim3(k0 / 32, ny, sz), 256, 0, s>>>(lst, m->d_meta, S, k0, m->fact,
-                                                                                   m->d_fdof, m->sx, m->sy);
+                    mf_chain(mf_bwd_update_kernel<NS, 1>, dim3(k0 / 32, ny, sz), s, lst, m->d_meta, S, k0, m->fact,
+                             m->d_fdof, m->sx, m->sy);
             }
         }
         EMFEM_LAUNCH("multifrontal backward");
