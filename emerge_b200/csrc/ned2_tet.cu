@@ -458,14 +458,13 @@ __global__ void export_indices_kernel(long long H, long long sum_m, const int* _
 }
 
 // ---------------------------------------------------------------- fused numeric assembly
-// One CTA per chunk of consecutive entities of one kind (all edges or all faces) holding at most
-// CH incidences.  Phase 0: the chunk's incidence records and the invariants of their tets are
-// copied to shared memory with coalesced loads.  Phase 1: one thread per (incidence, column entity)
-// pair block, column-entity major so every warp evaluates one edge/face block type; results staged
-// in shared memory.  Phase 2: one thread per output (X, k) sums its tets' staged blocks in
-// ascending tet order and writes the 4 CSR values of its column pair.  blockIdx.y 0 does E, 1 does B: they share no
-// arithmetic, and half the stage and half the registers let twice the warps hide the latency of the record
-// gathers, which is what bounds the kernel.
+// One CTA per chunk of consecutive entities of one kind (all edges or all faces) holding at most CH incidences, and
+// per matrix: blockIdx.y 0 does E, 1 does B, which share no arithmetic.  Phase 0: the chunk's incidence records
+// (and, in the staged variants, the part of the tets' records the matrix needs) to shared memory.  Phase 1: one
+// thread per (incidence, column entity) pair block, results staged in shared memory.  Phase 2: one thread per
+// output (X, k) sums its tets' staged blocks in ascending tet order and writes the 4 CSR values of its column
+// pair.  The latency of the record gathers bounds it; with E and B in one thread half as many warps were resident
+// (82 944-tet profile: 18 warps an SM).  384 000 tets, this kernel: 2.22 ms together, 2.13 ms apart.
 template <int CH, bool SINV>
 struct ChunkSmem {
     static constexpr size_t stage = (size_t)CH * 10 * 4 * 16;
