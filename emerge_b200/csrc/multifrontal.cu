@@ -61,10 +61,7 @@ __device__ __forceinline__ void cp_async8(void* dst_smem, const void* src) {
     unsigned d = (unsigned)__cvta_generic_to_shared(dst_smem);
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
 }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-// wait until at most one committed group is still in flight
-__device__ __forceinline__ void cp_async_wait_1() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
 __device__ __forceinline__ float2 cinv(float2 a) {
     float d = 1.0f / cabs2(a);
     return make_float2(a.x * d, -a.y * d);
