@@ -243,6 +243,7 @@ __global__ void __launch_bounds__(256) mf_diag_kernel(const int* __restrict__ ls
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) bmax = max(bmax, __shfl_xor_sync(all, bmax, o));
     const R floor2 = max(bmax, (R)1e-30) * (R)1e-12;      // (1e-6 of the block's largest entry)^2
+    __syncthreads();                              // every warp has the same floor before any column changes
     int pos = lane, pert = 0;
     for (int j = 0; j < kb; j++) {
         // pivot: largest |row[j]| among the rows at positions >= j (ties: smallest position)
