@@ -1075,7 +1075,7 @@ static int pow2_at_least(int v) {
 
 // ---- workspace layout ----------------------------------------------------------------------
 struct Layout {
-    size_t off_state, off_gamma, off_k0, off_partial, off_patchmap, off_scale, off_gpair, off_k0c, off_gammac;
+    size_t off_state, off_snap, off_gamma, off_k0, off_partial, off_patchmap, off_scale, off_gpair, off_k0c, off_gammac;
     size_t off_x, off_b, off_r64, off_Ax;                  // FP64 vectors (n, S)
     size_t off_v[8];                                       // Krylov vectors of the inner precision
     size_t off_minv;
@@ -1091,6 +1091,7 @@ static Layout make_layout(long long n, long long nnz, long long npatch, int S, i
     size_t vec64 = (size_t)n * S * sizeof(double2);
     size_t vecw = (size_t)n * S * (precision ? sizeof(float2) : sizeof(double2));
     L.off_state = o; o = align256(o + sizeof(SysState) * 2 * S * G);
+    L.off_snap = o; o = align256(o + sizeof(SysState) * 2 * S * G);
     L.off_gamma = o; o = align256(o + sizeof(double) * 2 * S * G * (nports > 0 ? nports : 1));
     L.off_k0 = o; o = align256(o + sizeof(double) * S * G);
     L.off_partial = o; o = align256(o + sizeof(double2) * 3 * nb * S);
@@ -1123,6 +1124,7 @@ struct Krylov {
     T* v[7] = {nullptr};       // work vectors
     double2* partial = nullptr;
     SysState* st = nullptr;
+    SysState* snap = nullptr;       // two copies of st, read by the host while the next replay runs
     cudaStream_t s = nullptr;
     // grouped systems: G groups of S systems, group of every DOF pair, group pair ranges
     int G = 1;
@@ -1269,8 +1271,8 @@ struct Krylov {
         return EMFEM_OK;
     }
 
-    int read_states(std::vector<SysState>& host, cudaStream_t on) {
-        EMFEM_CUDA(cudaMemcpyAsync(host.data(), st, sizeof(SysState) * host.size(), cudaMemcpyDeviceToHost, on));
+    int read_states(std::vector<SysState>& host, const SysState* from, cudaStream_t on) {
+        EMFEM_CUDA(cudaMemcpyAsync(host.data(), from, sizeof(SysState) * host.size(), cudaMemcpyDeviceToHost, on));
         EMFEM_CUDA(cudaStreamSynchronize(on));
         return EMFEM_OK;
     }
@@ -1282,8 +1284,10 @@ struct Krylov {
 
     // One eager iteration (loads every kernel before capture), then `chunk` iterations captured once and
     // replayed until no system is active, the iteration cap is reached or the batch is narrowed.  With `ahead`
-    // the next replay is queued before the flags of the one before are read (on a second stream), so the GPU
-    // does not wait for the host; the replay queued last finds every system stopped.
+    // the next replay is queued before the flags of the one before are read, so the GPU does not wait for the
+    // host; the replay queued last finds every system stopped.  The host reads (on a second stream) a copy of the
+    // states taken between two replays, two copies by turns, so what it decides depends on iteration counts
+    // alone and not on how far the replay in flight has come.
     int run(int chunk) {
         const bool narrowing = xfull && method == 1 && G == 1;
         const bool ahead = mf == nullptr;      // an LU application does not skip stopped systems
@@ -1294,11 +1298,12 @@ struct Krylov {
             done.assign(S, SysState{});
         }
         cudaStream_t side = nullptr;
-        cudaEvent_t ev = nullptr;
+        cudaEvent_t ev[2] = {nullptr, nullptr};
         int rc = EMFEM_OK;
         if (ahead) {
             rc = check_cuda(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking), "cudaStreamCreate");
-            if (rc == EMFEM_OK) rc = check_cuda(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming), "cudaEventCreate");
+            for (int q = 0; q < 2 && rc == EMFEM_OK; q++)
+                rc = check_cuda(cudaEventCreateWithFlags(&ev[q], cudaEventDisableTiming), "cudaEventCreate");
         }
         int left = (maxit + chunk - 1) / chunk + 1;
         while (rc == EMFEM_OK && left > 0) {
@@ -1311,19 +1316,26 @@ struct Krylov {
             const cudaError_t e = cudaStreamEndCapture(s, &graph);
             if (rc == EMFEM_OK) rc = check_cuda(e, "cudaStreamEndCapture");
             if (rc == EMFEM_OK) rc = check_cuda(cudaGraphInstantiate(&exec, graph, 0), "cudaGraphInstantiate");
-            int to = 0, active = 1;
-            if (ahead && rc == EMFEM_OK) { rc = check_cuda(cudaGraphLaunch(exec, s), "cudaGraphLaunch"); left--; }
+            int to = 0, active = 1, cur = 0;
+            // one replay, then its states into copy q
+            auto replay = [&](int q) -> int {
+                EMFEM_CUDA(cudaGraphLaunch(exec, s));
+                left--;
+                if (!ahead) return EMFEM_OK;
+                EMFEM_CUDA(cudaMemcpyAsync(snap + q * host.size(), st, sizeof(SysState) * host.size(), cudaMemcpyDeviceToDevice, s));
+                EMFEM_CUDA(cudaEventRecord(ev[q], s));
+                return EMFEM_OK;
+            };
+            if (ahead && rc == EMFEM_OK) rc = replay(0);
             while (rc == EMFEM_OK) {
                 if (ahead) {
-                    if ((rc = check_cuda(cudaEventRecord(ev, s), "cudaEventRecord")) != EMFEM_OK) break;
-                    if (left > 0) { if ((rc = check_cuda(cudaGraphLaunch(exec, s), "cudaGraphLaunch")) != EMFEM_OK) break; }
-                    left--;
-                    if ((rc = check_cuda(cudaStreamWaitEvent(side, ev, 0), "cudaStreamWaitEvent")) != EMFEM_OK) break;
-                    if ((rc = read_states(host, side)) != EMFEM_OK) break;
+                    if (left > 0) { if ((rc = replay(1 - cur)) != EMFEM_OK) break; }
+                    if ((rc = check_cuda(cudaStreamWaitEvent(side, ev[cur], 0), "cudaStreamWaitEvent")) != EMFEM_OK) break;
+                    if ((rc = read_states(host, snap + cur * host.size(), side)) != EMFEM_OK) break;
+                    cur = 1 - cur;
                 } else {
-                    if ((rc = check_cuda(cudaGraphLaunch(exec, s), "cudaGraphLaunch")) != EMFEM_OK) break;
-                    left--;
-                    if ((rc = read_states(host, s)) != EMFEM_OK) break;
+                    if ((rc = replay(0)) != EMFEM_OK) break;
+                    if ((rc = read_states(host, st, s)) != EMFEM_OK) break;
                 }
                 active = count_active(host);
                 if (active == 0 || left <= 0) break;
@@ -1333,7 +1345,7 @@ struct Krylov {
                 }
             }
             // the replay queued ahead may have stopped more systems: read the states again when all is done
-            if (rc == EMFEM_OK) rc = read_states(host, s);
+            if (rc == EMFEM_OK) rc = read_states(host, st, s);
             if (exec) cudaGraphExecDestroy(exec);
             if (graph) cudaGraphDestroy(graph);
             if (rc != EMFEM_OK) break;
@@ -1349,7 +1361,7 @@ struct Krylov {
                 rc = check_cuda(cudaMemcpyAsync(st, done.data(), sizeof(SysState) * S0, cudaMemcpyHostToDevice, s), "copy state");
         }
         const int rs = check_cuda(cudaStreamSynchronize(s), "sync");
-        if (ev) cudaEventDestroy(ev);
+        for (cudaEvent_t q : ev) if (q) cudaEventDestroy(q);
         if (side) cudaStreamDestroy(side);
         return rc != EMFEM_OK ? rc : rs;
     }
@@ -1557,7 +1569,7 @@ static int krylov_impl(emfem_handle hd, int method, int64_t n, int64_t nnz, cons
         k.method = method; k.op = op64; k.n = n; k.h = n / 2; k.S = S; k.precond = precond; k.maxit = maxit; k.nsys = nsys;
         k.x = x64; k.r = (double2*)(ws + L.off_r64); k.minv = (double2*)(ws + L.off_minv);
         for (int q = 0; q < 7; q++) k.v[q] = (double2*)(ws + L.off_v[q]);
-        k.partial = partial; k.st = st; k.s = s;
+        k.partial = partial; k.st = st; k.snap = (SysState*)(ws + L.off_snap); k.s = s;
         k.op.skip = st;
         k.G = G; k.pg = G > 1 ? pair_group : nullptr; k.gpair = gpair;
         if (k.bj()) {
@@ -1593,7 +1605,7 @@ static int krylov_impl(emfem_handle hd, int method, int64_t n, int64_t nnz, cons
         float2* d32 = (float2*)(ws + L.off_v[7]);
         k.x = d32; k.r = r32; k.minv = (float2*)(ws + L.off_minv);
         for (int q = 0; q < 6; q++) k.v[q] = (float2*)(ws + L.off_v[q]);
-        k.partial = partial; k.st = st; k.s = s;
+        k.partial = partial; k.st = st; k.snap = (SysState*)(ws + L.off_snap); k.s = s;
         k.op.skip = st;
         k.G = G; k.pg = G > 1 ? pair_group : nullptr; k.gpair = gpair;
         const int* pgk = k.pg;

@@ -34,3 +34,15 @@ def test_narrowed_batch_equals_single_solves(cuda, nsys, precond, maxit):
     else:
         live = np.arange(nsys) != 2
         assert (res.status[live] == 1).any() and (res.iters <= maxit).all()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_repeated_solves_give_the_same_bits(cuda, precision):
+    """When the batch narrows is decided from the iteration counts, not from how far the host has come."""
+    sw = FrequencySweep(problems.waveguide(nx=10, ny=5, nz=20))
+    systems = [(float(f), k % 2) for k, f in enumerate(np.linspace(7.2e9, 12.5e9, 16))]
+    assert sw.n * len(systems) >= 1 << 18
+    runs = [sw.solve(systems, tol=1e-8, maxit=20000, precond="aux", precision=precision) for _ in range(4)]
+    assert (runs[0].status == 0).all()
+    for r in runs[1:]:
+        assert torch.equal(r.x, runs[0].x) and np.array_equal(r.iters, runs[0].iters)
