@@ -320,8 +320,8 @@ __global__ void __launch_bounds__(AB) aux_restrict_kernel(long long na, int S, c
         for (int u = 0; u < U; u++)
 #pragma unroll
             for (int r = 0; r < NR; r++) {
-                ar[r] += gv[u] * (double)vv[u][r].x;
-                ai[r] += gv[u] * (double)vv[u][r].y;
+                ar[r] = fma(gv[u], (double)vv[u][r].x, ar[r]);
+                ai[r] = fma(gv[u], (double)vv[u][r].y, ai[r]);
             }
     }
 #pragma unroll
@@ -338,8 +338,9 @@ __global__ void __launch_bounds__(AB) aux_restrict_kernel(long long na, int S, c
         TX o;
         if (dinv) {
             TX d = dinv[y * S + s];
-            o.x = ar[r] * (double)d.x - ai[r] * (double)d.y;
-            o.y = ar[r] * (double)d.y + ai[r] * (double)d.x;
+            // written out: left to itself the compiler contracts these differently from one NR to the next
+            o.x = fma(ar[r], (double)d.x, -(ai[r] * (double)d.y));
+            o.y = fma(ar[r], (double)d.y, ai[r] * (double)d.x);
         } else {
             o.x = ar[r]; o.y = ai[r];
         }

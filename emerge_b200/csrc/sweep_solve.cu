@@ -85,39 +85,34 @@ __device__ __forceinline__ double nrm2(T a) { return (double)a.x * a.x + (double
 
 enum DotMode { DOT_NONE = 0, DOT_XY = 1, DOT_CONJW_Y = 2, DOT_CONJY_W_YY = 3 };
 
-// DOF pairs (i, i + n/2) per block of the kernels below.  Every dot product is summed block by block, so
-// these depend on the batch size only: a mesh's groups of pairs (multiples of 256) are cut alike alone and
-// inside a grouped solve.
+// DOF pairs (i, i + n/2) per partial of the dot products below, for a batch of S systems.  They depend on the width
+// that the batch began with only (`cut` below): a mesh's groups of pairs (multiples of 256) are cut alike alone and
+// inside a grouped solve, and a batch that is narrowed while it runs keeps its cut.
 __host__ __device__ constexpr int spmv_pairs(int S) { return S >= 16 ? 16 : 8; }
 __host__ __device__ constexpr int vec_pairs(int S) { return S >= 16 ? 512 / S : VB / S; }
 
-// Block-level fixed-order tree reduction of up to three components per thread (two complex, one
-// real); thread s < S stores component c of this block at partial[(c * S + s) * nblocks + block], so the
-// partials of one system are contiguous.
-__device__ __forceinline__ void block_store3(double2 v0, double2 v1, double v2, int ncomp, int S, double2* partial) {
+// Fixed-order tree reduction of two components per thread.  A thread holds slot (threadIdx.x / S) of system
+// threadIdx.x % S; VB / cut slots make one partial, so a block writes cut / S of the nb partials of every system, at
+// partial[(c * S + s) * nb + p] for component c: the partials of one system are contiguous.
+__device__ __forceinline__ void block_store2(double2 v0, double2 v1, int ncomp, int S, int cut, long long nb, double2* partial) {
     __shared__ double2 r0[VB], r1[VB];
-    __shared__ double r2[VB];
+    const int W = VB / cut, slot = threadIdx.x / S, w = slot % W, s = threadIdx.x % S;
     r0[threadIdx.x] = v0;
     r1[threadIdx.x] = v1;
-    r2[threadIdx.x] = v2;
     __syncthreads();
-    for (int off = VB / 2; off >= S; off >>= 1) {
-        if (threadIdx.x < off) {
-            r0[threadIdx.x].x += r0[threadIdx.x + off].x; r0[threadIdx.x].y += r0[threadIdx.x + off].y;
-            r1[threadIdx.x].x += r1[threadIdx.x + off].x; r1[threadIdx.x].y += r1[threadIdx.x + off].y;
-            r2[threadIdx.x] += r2[threadIdx.x + off];
+    for (int off = W / 2; off > 0; off >>= 1) {
+        if (w < off) {
+            const int o = threadIdx.x + off * S;
+            r0[threadIdx.x].x += r0[o].x; r0[threadIdx.x].y += r0[o].y;
+            r1[threadIdx.x].x += r1[o].x; r1[threadIdx.x].y += r1[o].y;
         }
         __syncthreads();
     }
-    if (threadIdx.x < S) {
-        const long long nb = gridDim.x;
-        partial[threadIdx.x * nb + blockIdx.x] = r0[threadIdx.x];
-        if (ncomp > 1) partial[(S + threadIdx.x) * nb + blockIdx.x] = r1[threadIdx.x];
-        if (ncomp > 2) partial[(2 * S + threadIdx.x) * nb + blockIdx.x] = make_double2(r2[threadIdx.x], 0.0);
+    const long long p = (long long)blockIdx.x * (cut / S) + slot / W;
+    if (w == 0 && p < nb) {
+        partial[s * nb + p] = r0[threadIdx.x];
+        if (ncomp > 1) partial[(S + s) * nb + p] = r1[threadIdx.x];
     }
-}
-__device__ __forceinline__ void block_store2(double2 v0, double2 v1, int ncomp, int S, double2* partial) {
-    block_store3(v0, v1, 0.0, ncomp, S, partial);
 }
 
 // y = A x for all systems, a warp per DOF pair (rows i and i + n/2); optional dot-product epilogue (DotMode).
@@ -197,7 +192,7 @@ struct SpmvStage {
 template <typename R, int L, int NR, bool HASB>
 __global__ void __launch_bounds__(VB, NR == 1 ? 4 : NR == 2 ? 3 : 2) spmv_kernel(
     OpArgs a, const typename V2<R>::T* __restrict__ x, typename V2<R>::T* __restrict__ y, double2* __restrict__ partial,
-    int dotmode, const typename V2<R>::T* __restrict__ w) {
+    int dotmode, const typename V2<R>::T* __restrict__ w, int ppb) {
     typedef typename V2<R>::T T;
     typedef SpmvStage<R, L, NR, HASB> Stage;
     constexpr int G = 32 / L;                       // entry groups of a warp
@@ -210,7 +205,6 @@ __global__ void __launch_bounds__(VB, NR == 1 ? 4 : NR == 2 ? 3 : 2) spmv_kernel
     Stage* st = reinterpret_cast<Stage*>(spmv_sm) + wl * D;
     const int g = lane / L, sl = lane % L, sb = blockIdx.y * (L * NR), s0 = sb + sl;
     const long long hh = (a.n + 1) / 2;
-    const int ppb = spmv_pairs(S);
     const double2* __restrict__ Ev = (const double2*)a.E;
     const double2* __restrict__ Bv = (const double2*)a.B;
     double2 c0[NV];
@@ -340,15 +334,16 @@ __global__ void __launch_bounds__(VB, NR == 1 ? 4 : NR == 2 ? 3 : 2) spmv_kernel
                     for (int r = 0; r < NR; r++) {
                         const T xv = xc[r * L];
                         const double* gm = a.gamma + 2 * ((base + s0 + r * L) * a.n_ports + q);
-                        const double kr = gm[0] * v.x - gm[1] * v.y, ki = gm[0] * v.y + gm[1] * v.x;
-                        acc[half * NR + r].x += kr * xv.x - ki * xv.y;
-                        acc[half * NR + r].y += kr * xv.y + ki * xv.x;
+                        const double kr = fma(gm[0], v.x, -(gm[1] * v.y)), ki = fma(gm[0], v.y, gm[1] * v.x);
+                        acc[half * NR + r].x = fma(kr, (double)xv.x, fma(-ki, (double)xv.y, acc[half * NR + r].x));
+                        acc[half * NR + r].y = fma(kr, (double)xv.y, fma(ki, (double)xv.x, acc[half * NR + r].y));
                     }
                 }
             }
         }
         const int r0 = pair_reduce<L, NR>(acc, lane);
         const bool hi = lane & 16;
+        // (sums are written out as fma: every instantiation then rounds alike, which a narrowed batch relies on)
         // lane groups that hold copies of a value already written by another group have a bit of L..8 set
         const bool own = NR > 1 || (lane & 15 & ~(L - 1)) == 0;
         if (own && (two || !hi)) {
@@ -359,19 +354,22 @@ __global__ void __launch_bounds__(VB, NR == 1 ? 4 : NR == 2 ? 3 : 2) spmv_kernel
                 const double yr = acc[q].x, yi = acc[q].y;
                 y[o] = mk2<R>((R)yr, (R)yi);
                 if (dotmode == DOT_XY) {
-                    T xi = x[o];
-                    c0[q].x += (double)xi.x * yr - (double)xi.y * yi;
-                    c0[q].y += (double)xi.x * yi + (double)xi.y * yr;
+                    const T xi = x[o];
+                    const double a0 = xi.x, a1 = xi.y;
+                    c0[q].x = fma(a0, yr, fma(-a1, yi, c0[q].x));
+                    c0[q].y = fma(a0, yi, fma(a1, yr, c0[q].y));
                 } else if (dotmode == DOT_CONJW_Y) {
-                    T wi = w[o];
-                    c0[q].x += (double)wi.x * yr + (double)wi.y * yi;
-                    c0[q].y += (double)wi.x * yi - (double)wi.y * yr;
+                    const T wi = w[o];
+                    const double a0 = wi.x, a1 = wi.y;
+                    c0[q].x = fma(a0, yr, fma(a1, yi, c0[q].x));
+                    c0[q].y = fma(a0, yi, fma(-a1, yr, c0[q].y));
                 } else if (dotmode == DOT_CONJY_W_YY) {
-                    T wi = w[o];
-                    c0[q].x += yr * wi.x + yi * wi.y;
-                    c0[q].y += yr * wi.y - yi * wi.x;
-                    c1[q] += yr * yr + yi * yi;
-                    c2[q] += nrm2(wi);
+                    const T wi = w[o];
+                    const double a0 = wi.x, a1 = wi.y;
+                    c0[q].x = fma(a0, yr, fma(a1, yi, c0[q].x));
+                    c0[q].y = fma(a1, yr, fma(-a0, yi, c0[q].y));
+                    c1[q] = fma(yr, yr, fma(yi, yi, c1[q]));
+                    c2[q] = fma(a0, a0, fma(a1, a1, c2[q]));
                 }
             }
         }
@@ -418,14 +416,15 @@ static unsigned vec_blocks(long long h, int S) { return grid_for(h, vec_pairs(S)
 
 template <typename R, bool HASB>
 static void launch_spmv_b(const OpArgs& a, const typename V2<R>::T* x, typename V2<R>::T* y, double2* partial, int dotmode,
-                          const typename V2<R>::T* w, cudaStream_t s) {
-    dim3 grid(spmv_blocks(a.n, a.S), a.S > 32 ? a.S / 32 : 1);
+                          const typename V2<R>::T* w, int cut, cudaStream_t s) {
+    const int ppb = spmv_pairs(cut);
+    dim3 grid(spmv_blocks(a.n, cut), a.S > 32 ? a.S / 32 : 1);
 #define EMFEM_SPMV(L, NR)                                                                                      \
     do {                                                                                                       \
         constexpr size_t sm = sizeof(SpmvStage<R, L, NR, HASB>) * SpmvStage<R, L, NR, HASB>::DEPTH * (VB / 32);                                                  \
         if (sm > 48 * 1024)                                                                                    \
             cudaFuncSetAttribute(spmv_kernel<R, L, NR, HASB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm); \
-        spmv_kernel<R, L, NR, HASB><<<grid, VB, sm, s>>>(a, x, y, partial, dotmode, w);                        \
+        spmv_kernel<R, L, NR, HASB><<<grid, VB, sm, s>>>(a, x, y, partial, dotmode, w, ppb);                   \
     } while (0)
     switch (a.S) {
     case 1: EMFEM_SPMV(1, 1); break;
@@ -439,9 +438,9 @@ static void launch_spmv_b(const OpArgs& a, const typename V2<R>::T* x, typename 
 }
 template <typename R>
 static void launch_spmv(const OpArgs& a, const typename V2<R>::T* x, typename V2<R>::T* y, double2* partial, int dotmode,
-                        const typename V2<R>::T* w, cudaStream_t s) {
-    if (a.B) launch_spmv_b<R, true>(a, x, y, partial, dotmode, w, s);
-    else launch_spmv_b<R, false>(a, x, y, partial, dotmode, w, s);
+                        const typename V2<R>::T* w, int cut, cudaStream_t s) {
+    if (a.B) launch_spmv_b<R, true>(a, x, y, partial, dotmode, w, cut, s);
+    else launch_spmv_b<R, false>(a, x, y, partial, dotmode, w, cut, s);
 }
 
 // y[row] += sum_q gamma_q R_q x on the patch rows (a warp per patch row, lanes over (entry group, system)):
@@ -662,7 +661,7 @@ __global__ void __launch_bounds__(VB) cocg_init_kernel(long long h, int S, int p
         double2 a = dotu(rl, zl), b = dotu(rh, zh);
         rz.x += a.x + b.x; rz.y += a.y + b.y;
     }
-    block_store2(rz, rz, 1, S, partial);
+    block_store2(rz, rz, 1, S, S, gridDim.x, partial);
 }
 
 template <typename R>
@@ -698,7 +697,7 @@ __global__ void __launch_bounds__(VB) cocg_update_kernel(long long h, int S, int
         rz.x += a.x + b.x; rz.y += a.y + b.y;
         rr.x += nrm2(rv2[0]) + nrm2(rv2[1]);
     }
-    block_store2(rz, rr, 2, S, partial);
+    block_store2(rz, rr, 2, S, S, gridDim.x, partial);
 }
 
 template <typename R>
@@ -735,7 +734,7 @@ __global__ void __launch_bounds__(VB) bicg_init_kernel(long long h, int S, const
             c.x += nrm2(rv);
         }
     }
-    block_store2(c, c, 1, S, partial);
+    block_store2(c, c, 1, S, S, gridDim.x, partial);
 }
 
 // p = r + beta (p - omega v); p_hat = M^-1 p   (thread per DOF pair)
@@ -803,17 +802,18 @@ __global__ void __launch_bounds__(VB) bicg_s_kernel(long long h, int S, int prec
 
 // x += alpha p_hat + omega s_hat; r = s - omega t; partial (r_hat, r) and ||r||^2
 template <typename R>
-__global__ void __launch_bounds__(VB) bicg_x_kernel(long long h, int S, const int* __restrict__ pg,
+__global__ void __launch_bounds__(VB) bicg_x_kernel(long long h, int S, int cut, long long nb, const int* __restrict__ pg,
                                                     const SysState* __restrict__ st,
                                                     typename V2<R>::T* __restrict__ x, typename V2<R>::T* __restrict__ r,
                                                     const typename V2<R>::T* __restrict__ ph, const typename V2<R>::T* __restrict__ sh,
                                                     const typename V2<R>::T* __restrict__ t, const typename V2<R>::T* __restrict__ rh,
                                                     double2* __restrict__ partial) {
     typedef typename V2<R>::T T;
-    const int s = threadIdx.x % S;
+    const int s = threadIdx.x % S, slot = threadIdx.x / S, W = VB / cut;
+    const long long p = (long long)blockIdx.x * (cut / S) + slot / W;
     double2 c0 = make_double2(0, 0), c1 = c0;
-    for (int q = threadIdx.x / S; q < vec_pairs(S); q += VB / S) {
-        const long long i = (long long)blockIdx.x * vec_pairs(S) + q;
+    for (int q = slot % W; q < vec_pairs(cut); q += W) {
+        const long long i = p * vec_pairs(cut) + q;
         if (i >= h) break;
         const int sy = sys_of_row(pg, h, i, S, s);
         if (!st[sy].active) continue;
@@ -834,7 +834,7 @@ __global__ void __launch_bounds__(VB) bicg_x_kernel(long long h, int S, const in
             c1.x += nrm2(rv);
         }
     }
-    block_store2(c0, c1, 2, S, partial);
+    block_store2(c0, c1, 2, S, cut, nb, partial);
 }
 
 // ---- setup kernels -------------------------------------------------------------------
@@ -866,7 +866,7 @@ __global__ void __launch_bounds__(VB) residual_kernel(long long h, int S, const 
             r[g] = res;
         }
     }
-    block_store2(cb, cr, 2, S, partial);
+    block_store2(cb, cr, 2, S, S, gridDim.x, partial);
 }
 
 // Operator entry (row, col) of system s (E - k0^2 B + patch), used by the preconditioner setup.
@@ -1140,6 +1140,8 @@ struct Krylov {
     unsigned nb_all() const { return grid_for(n * (long long)S, VB); }
     unsigned nb_pair() const { return grid_for(h * (long long)S, VB); }
 
+    int cut = 1;                    // width that the batch began with: every sum is cut by it
+
     // restart BiCGStab's shadow residual only when (r_hat, r) is at the rounding level of the
     // vectors' precision (the dots accumulate in FP64); a looser FP32 threshold restarts so often
     // that the Krylov memory is lost
@@ -1148,11 +1150,12 @@ struct Krylov {
         reduce_update_kernel<<<G * S, VB, 0, s>>>(partial, (int)nblocks, S, ncomp, st, mode, maxit, restart_eps, nsys, G,
                                                   ppb, gpair);
     }
-    void reduce_spmv(int ncomp, int mode) { reduce(ncomp, spmv_blocks(n, S), spmv_pairs(S), mode); }
-    void reduce_vec(int ncomp, int mode) { reduce(ncomp, vec_blocks(h, S), vec_pairs(S), mode); }
-    void spmv(const T* in, T* out, int dotmode, const T* w) { launch_spmv<R>(op, in, out, partial, dotmode, w, s); }
+    void reduce_spmv(int ncomp, int mode) { reduce(ncomp, spmv_blocks(n, cut), spmv_pairs(cut), mode); }
+    void reduce_vec(int ncomp, int mode) { reduce(ncomp, vec_blocks(h, cut), vec_pairs(cut), mode); }
+    void spmv(const T* in, T* out, int dotmode, const T* w) { launch_spmv<R>(op, in, out, partial, dotmode, w, cut, s); }
 
     int start() {
+        cut = S;
         if (method == 0) {
             T *z = v[0], *p = v[1];
             cocg_init_kernel<R><<<vec_blocks(h, S), VB, 0, s>>>(h, S, precond, r, z, p, minv, partial);
@@ -1189,7 +1192,8 @@ struct Krylov {
             }
             spmv(sh, t, DOT_CONJY_W_YY, r);
             reduce_spmv(3, UPD_BICG_OMEGA);
-            bicg_x_kernel<R><<<vec_blocks(h, S), VB, 0, s>>>(h, S, pg, st, x, r, ph, sh, t, rh, partial);
+            const unsigned nb = vec_blocks(h, cut), per = cut / S;
+            bicg_x_kernel<R><<<(nb + per - 1) / per, VB, 0, s>>>(h, S, cut, nb, pg, st, x, r, ph, sh, t, rh, partial);
             reduce_vec(2, UPD_BICG_RHO);
         }
         return check_cuda(cudaGetLastError(), "krylov iteration");
@@ -1199,7 +1203,10 @@ struct Krylov {
     // Systems converge at different iterations, and a column that has stopped still takes its lanes and its
     // share of every gather.  When the active systems fit half the columns, their vectors, preconditioner
     // and scalars move to a batch of that width; a stopped system's solution goes back to its own column of
-    // xfull.  Vectors of a narrower batch live in the two halves of the workspace by turns: `wide` holds what an
+    // xfull.  No width from 8 columns on changes the order of a sum (dot products keep their cut; the SpMV and the
+    // aux restriction deal a row's entries out to four lane groups; the network and the LU treat a column by
+    // itself), so a system's bits do not depend on when it is moved, nor on whether it is: narrower than 8 a
+    // batch does not become, and one of 8 or fewer is left as it is.  Vectors of a narrower batch live in the two halves of the workspace by turns: `wide` holds what an
     // iteration recomputes (five vectors of the full batch), `held` the carried ones (three), each with a
     // separate place for the block inverses.
     T* xfull = nullptr;                       // (n, S0): non-null enables narrowing
@@ -1212,6 +1219,7 @@ struct Krylov {
     bool in_wide = false;
     // Below this many vector entries an iteration is bound by its launches, not by its width.
     static constexpr long long NARROW_MIN = 1 << 18;
+    static int width_for(int active) { return std::max(8, pow2_at_least(active)); }
 
     int pack(const T* src, T* dst, long long rows, int from, int to, const ColMap& m) {
         pack_columns_kernel<T><<<grid_for(rows * to, VB), VB, 0, s>>>(rows, from, to, m, src, dst);
@@ -1339,8 +1347,8 @@ struct Krylov {
                 }
                 active = count_active(host);
                 if (active == 0 || left <= 0) break;
-                if (narrowing && S > 1 && n * (long long)S >= NARROW_MIN && 2 * pow2_at_least(active) <= S) {
-                    to = pow2_at_least(active);
+                if (narrowing && n * (long long)S >= NARROW_MIN && 2 * width_for(active) <= S) {
+                    to = width_for(active);
                     break;
                 }
             }
@@ -1353,7 +1361,7 @@ struct Krylov {
                 for (int k = 0; k < S; k++) if (col[k] >= 0) done[col[k]] = host[k];
             active = count_active(host);
             if (active == 0 || !to) break;
-            rc = narrow(host, pow2_at_least(active));
+            rc = narrow(host, width_for(active));
         }
         if (rc == EMFEM_OK && narrowing && S != S0) {
             rc = flush();
@@ -1423,7 +1431,7 @@ int emfem_sweep_spmv(emfem_handle h, int64_t n, const int32_t* indptr, const int
     OpArgs a;
     build_op(a, n, nsys, indptr, indices, E_vals, B_vals, k0sq_dev, nullptr, patch_rowptr, patch_cols, patch_vals,
              patch_port, n_ports, gamma_dev, free_mask);
-    launch_spmv<double>(a, (const double2*)x, (double2*)y, nullptr, DOT_NONE, nullptr, h->h.stream);
+    launch_spmv<double>(a, (const double2*)x, (double2*)y, nullptr, DOT_NONE, nullptr, nsys, h->h.stream);
     EMFEM_LAUNCH("spmv_kernel");
     if (n_patch_rows > 0) {
         patch_rows_kernel<<<grid_for(n_patch_rows * 32, VB), VB, 0, h->h.stream>>>(n_patch_rows, patch_rows, a,
@@ -1558,7 +1566,7 @@ static int krylov_impl(emfem_handle hd, int method, int64_t n, int64_t nnz, cons
              patch_cols, patch_vals, patch_port, n_ports, gdev, free_mask);
     if (G > 1) op64.pg = pair_group;
     // initial residual r64 = b - A x0 and the outer state (||b||, tolerance, active)
-    launch_spmv<double>(op64, x64, Ax, nullptr, DOT_NONE, nullptr, s);
+    launch_spmv<double>(op64, x64, Ax, nullptr, DOT_NONE, nullptr, S, s);
     residual_kernel<<<nbv, VB, 0, s>>>(n / 2, S, free_mask, b64, Ax, r64, partial);
     reduce_update_kernel<<<G * S, VB, 0, s>>>(partial, (int)nbv, S, 2, st_outer, UPD_INIT, maxit, tol, nsys, G,
                                               vec_pairs(S), gpair);
@@ -1641,7 +1649,7 @@ static int krylov_impl(emfem_handle hd, int method, int64_t n, int64_t nnz, cons
             for (size_t q = 0; q < GSm; q++) if (ho[q].active) mx = std::max(mx, hin[q].iters);
             used += mx;
             add_scaled_f32_kernel<<<gv, VB, 0, s>>>(n, S, pgk, d32, scale, st_outer, x64);
-            launch_spmv<double>(op64, x64, Ax, nullptr, DOT_NONE, nullptr, s);
+            launch_spmv<double>(op64, x64, Ax, nullptr, DOT_NONE, nullptr, S, s);
             residual_kernel<<<nbv, VB, 0, s>>>(n / 2, S, free_mask, b64, Ax, r64, partial);
             // the inner state array is free now: reuse it to reduce ||b||^2, ||r||^2 of the new residual
             reduce_update_kernel<<<G * S, VB, 0, s>>>(partial, (int)nbv, S, 2, st, UPD_INIT, maxit, 1.0, S, G,
@@ -1684,7 +1692,7 @@ static int krylov_impl(emfem_handle hd, int method, int64_t n, int64_t nnz, cons
         const size_t GS = (size_t)G * S;
         std::vector<SysState> hs(GS);
         STRY(check_cuda(cudaMemcpyAsync(hs.data(), st, sizeof(SysState) * GS, cudaMemcpyDeviceToHost, s), "copy"));
-        launch_spmv<double>(op64, x64, Ax, nullptr, DOT_NONE, nullptr, s);
+        launch_spmv<double>(op64, x64, Ax, nullptr, DOT_NONE, nullptr, S, s);
         residual_kernel<<<nbv, VB, 0, s>>>(n / 2, S, free_mask, b64, Ax, r64, partial);
         reduce_update_kernel<<<G * S, VB, 0, s>>>(partial, (int)nbv, S, 2, st_outer, UPD_INIT, maxit, tol, S, G,
                                               vec_pairs(S), gpair);
@@ -1876,7 +1884,7 @@ extern "C" int emfem_sweep_spmv_noalloc(emfem_handle h, int64_t n, const int32_t
         OpArgs a;
         build_op(a, n, nsys, indptr, indices, E_vals, B_vals, k0sq_dev, pmap, patch_rowptr, patch_cols, patch_vals,
                  patch_port, n_ports, gamma_dev, free_mask);
-        launch_spmv<double>(a, (const double2*)x, (double2*)y, nullptr, DOT_NONE, nullptr, h->h.stream);
+        launch_spmv<double>(a, (const double2*)x, (double2*)y, nullptr, DOT_NONE, nullptr, nsys, h->h.stream);
         rc = check_cuda(cudaGetLastError(), "spmv_kernel");
     }
     if (prev != h->h.device) cudaSetDevice(prev);

@@ -81,6 +81,20 @@ def test_grouped_aux_sweep_matches_separate_aux_sweeps(cuda):
         assert torch.equal(alone.x, r.x) and np.array_equal(alone.iters, r.iters), (alone.iters, r.iters)
 
 
+def test_mesh_alone_and_in_a_batch_give_the_same_bits_at_narrowing_width(cuda):
+    """A mesh alone (one group) is large enough to be narrowed while it runs; in the batch of two it is not."""
+    Ps = [problems.waveguide(nx=10, ny=5, nz=20), problems.waveguide(nx=4, ny=2, nz=8, seed=1)]
+    freqs = np.linspace(7.2e9, 12.5e9, 16)
+    systems = [[(float(f), k % 2) for k, f in enumerate(freqs)]] * 2
+    bs = BatchSweep(Ps)
+    res = bs.solve(systems, tol=1e-8, maxit=20000, precond="aux")
+    alone = BatchSweep(Ps[:1])
+    assert alone.n * 16 >= 1 << 18
+    r = alone.solve(systems[:1], tol=1e-8, maxit=20000, precond="aux")[0]
+    assert (r.status == 0).all() and len(set(r.iters.tolist())) > 3
+    assert torch.equal(r.x, res[0].x) and np.array_equal(r.iters, res[0].iters)
+
+
 def test_grouped_learned_sweep_matches_separate_learned_sweeps(cuda):
     """precond="learned" over a batch: one network (weights per aux-node type) on the union's aux space."""
     from emerge_b200.auxspace import Network

@@ -46,3 +46,31 @@ def test_repeated_solves_give_the_same_bits(cuda, precision):
     assert (runs[0].status == 0).all()
     for r in runs[1:]:
         assert torch.equal(r.x, runs[0].x) and np.array_equal(r.iters, runs[0].iters)
+
+
+@pytest.mark.parametrize("nsys", [16, 32])
+@pytest.mark.parametrize("precond,maxit", [("block_jacobi", 200), ("aux", 150), ("learned", 60), ("lu", 12)])
+def test_bits_do_not_depend_on_the_other_columns(cuda, nsys, precond, maxit):
+    """Three systems among live neighbours (the batch keeps its width) and among columns that stop at once (it is
+    narrowed after the first replay): the same sums in the same order."""
+    from emerge_b200.auxspace import Network
+    sw = FrequencySweep(problems.waveguide(nx=10, ny=5, nz=20))
+    assert sw.n * nsys >= 1 << 18
+    freqs = np.linspace(8.2e9, 11.5e9, nsys)
+    systems = [(float(f), k % 2) for k, f in enumerate(freqs)]
+    kw = dict(tol=1e-13, maxit=maxit)
+    if precond == "learned":
+        net = Network(sw.aux_space(), seed=4, init="random")
+        net.params.mul_(0.5)
+        sw.set_network(net)
+    if precond == "lu":
+        kw["lu"] = sw.direct_solver().factor(float(freqs[nsys // 2]))
+    else:
+        kw["precond"] = precond
+    b = sw.rhs(systems)
+    live = [1, 6, nsys - 4]
+    alone = torch.zeros_like(b)
+    alone[:, live] = b[:, live]
+    full, few = (sw.solve_rhs(sw.k0sq(freqs), v, sw.gammas(freqs), **kw) for v in (b, alone))
+    assert torch.equal(full.x[:, live], few.x[:, live])
+    assert np.array_equal(full.iters[live], few.iters[live]) and (few.iters[live] > 2).all()
