@@ -17,8 +17,9 @@
 //   3. the factor columns, the U block row and the Schur complement are copied out of the level
 //      workspace (compact_kernel): factors to the factor store (rounded to complex64), the Schur
 //      complement to the update store (front precision) until the parent's level consumes it;
-//   4. the 256 x 256 diagonal blocks of the factor store are replaced by the blocks of their L and U
-//      inverses (block_inverse_kernel), so that the solves have no 32-step chains.
+//   4. the 256 x 256 diagonal blocks are kept as the inverses of their L and U (block_inverse_kernel), so
+//      that the solves have no 32-step chains.  The inverses are formed, stored and applied in FP64: their
+//      entries grow (rows are not exchanged across steps), and products with them cancel.
 // Pivoting stays inside each 32-row diagonal block (rows are never exchanged across blocks), so row swaps
 // touch only the block row; the solves apply them step by step.  A pivot smaller than 1e-6 of its block's
 // largest entry is raised to that floor and counted: the factorization is a preconditioner under an FP64
@@ -108,10 +109,27 @@ struct FrontMeta {        // per front, device
     int e, b, n, parent;
     int child[2];
     long long fdof, ea, asm0, asm1;   // offsets into fdof / ea / asm arrays
-    long long fact, inv;              // factor store offsets (float2)
+    long long fact, inv;              // factor store offset (float2), inverse store offset (double2)
     long long ws, upd;                // level workspace (float2) / update store (float2) offsets
     long long wv, y;                  // solve buffers: the front's rows of w, its own rows of y
 };
+
+// Stores of a front, 256 own columns [k0, k0 + w) at a time.
+// Factor store (complex64): per block w columns of the n - w rows outside its diagonal block, after all blocks
+// the e x b block row of U.
+__host__ __device__ __forceinline__ long long mf_fact_block(int n, int k0) { return (long long)k0 * (n - MF_SB); }
+__host__ __device__ inline long long mf_fact_rows_cols(int n, int e) {       // entries of the columns of all blocks
+    const int last = e / MF_SB * MF_SB, w = e - last;
+    return mf_fact_block(n, last) + (long long)w * (n - w);
+}
+// Inverse store (complex128): per block w columns of w + 32 entries.  Column c of the 32-column step j holds rows
+// [0, 32 j + 32) of the inverse of U, then from entry 32 j + 32 on rows 32 j and up of the inverse of L (with the
+// steps' row exchanges), so row r of the latter is entry r + 32.
+__host__ __device__ __forceinline__ long long mf_inv_block(int k0) { return (long long)k0 * (MF_SB + MF_NB); }
+__host__ __device__ inline long long mf_inv_entries(int e) {
+    const int last = e / MF_SB * MF_SB, w = e - last;
+    return mf_inv_block(last) + (long long)w * (w + MF_NB);
+}
 
 // ---------------------------------------------------------------- factorization kernels
 // Symmetric diagonal equilibration: the factorization runs on D^-1/2 K D^-1/2 with D = |diag K|, so every
@@ -210,12 +228,11 @@ __device__ __forceinline__ double mf_shfl(double v, int l) { return __shfl_sync(
 // one barrier a step passes the updated columns on.  Warps 0-3 then form the inverse of L and 4-7 that of U,
 // eight columns per warp with a row per lane (32 steps of shuffles, no barrier).  Rolled loops: a warp with
 // the block in registers needs straight-line code that the instruction cache cannot hold (45 us a step on the
-// 82 944-tet cavity, as one warp in shared memory 64 us; now 20, complex128 27).  The inverses go to inv (complex64, read by
-// the solves) and, for a complex128 factorization, also to invc (complex128, read by the panel kernel); for
-// complex64 invc is inv.
+// 82 944-tet cavity, as one warp in shared memory 64 us; now 20, complex128 27).  The inverses go to the diagonal
+// blocks of the inverse store, read by the panel and block inverse kernels and by the solves.
 template <typename T>
 __global__ void __launch_bounds__(256) mf_diag_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm, int k,
-                                                      T* __restrict__ ws, float2* __restrict__ inv, T* __restrict__ invc,
+                                                      T* __restrict__ ws, double2* __restrict__ inv,
                                                       int* __restrict__ nperturbed) {
     typedef typename CxT<T>::R R;
     __shared__ T D[MF_NB][MF_NB + 1];            // [column][row]: the block, then U
@@ -328,15 +345,14 @@ __global__ void __launch_bounds__(256) mf_diag_kernel(const int* __restrict__ ls
             }
         }
     }
-    // Linv P, then Uinv: column-major 32 x 32 each.  The block's row swaps are folded into the inverse of L: position
-    // i holds row sq[i], so column sq[c] of Linv P is column c of Linv.
-    const long long ib = f.inv + (long long)(k / MF_NB) * 2 * MF_NB * MF_NB + (upper ? MF_NB * MF_NB : 0);
-    constexpr bool wide = sizeof(T) != sizeof(float2);
+    // Linv P and Uinv.  The block's row swaps are folded into the inverse of L: position i holds row sq[i], so column
+    // sq[c] of Linv P is column c of Linv.
+    const int k0 = k / MF_SB * MF_SB, kl = k - k0, ldi = min(MF_SB, f.e - k0) + MF_NB;
+    double2* I = inv + f.inv + mf_inv_block(k0) + (long long)kl * ldi + kl + (upper ? 0 : MF_NB) + lane;
 #pragma unroll
     for (int q = 0; q < 8; q++) {
         const int c = upper ? c0 + q : sq[c0 + q];
-        inv[ib + lane + c * MF_NB] = to_c64(x[q]);
-        if (wide) invc[ib + lane + c * MF_NB] = x[q];
+        if (lane < kb && c < kb) I[(long long)c * ldi] = make_double2(x[q].x, x[q].y);
     }
 }
 
@@ -347,7 +363,7 @@ __global__ void __launch_bounds__(256) mf_diag_kernel(const int* __restrict__ ls
 // 82 944-tet cavity, 21 now.
 template <typename T, int TW>
 __global__ void __launch_bounds__(256) mf_panel_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm, int k,
-                                                       int nt, T* __restrict__ ws, const T* __restrict__ invc) {
+                                                       int nt, T* __restrict__ ws, const double2* __restrict__ inv) {
     __shared__ T A[MF_NB][MF_NB + 1];                // inverse: [t][i] (block row) or [t][c] (block column)
     __shared__ T V[MF_NB][TW + 1];                   // tile: [t][column] or [t][row]
     const FrontMeta& f = fm[lst[blockIdx.y]];
@@ -360,11 +376,17 @@ __global__ void __launch_bounds__(256) mf_panel_kernel(const int* __restrict__ l
     const long long ld = f.n;
     T* W = ws + f.ws;
     const T zero = CxT<T>::make(0.0, 0.0);
-    const T* L = invc + f.inv + (long long)(k / MF_NB) * 2 * MF_NB * MF_NB + (rowblk ? 0 : MF_NB * MF_NB);
+    const int k0 = k / MF_SB * MF_SB, kl = k - k0, ldi = min(MF_SB, f.e - k0) + MF_NB;
+    const double2* I = inv + f.inv + mf_inv_block(k0) + (long long)kl * ldi + kl + (rowblk ? MF_NB : 0);
     constexpr int NJ = TW / 16;
+    for (int q = tid; q < MF_NB * MF_NB; q += 256) {
+        const int i = q % MF_NB, c = q / MF_NB;                // entry (i, c) of the step's inverse
+        T v = zero;
+        if (i < kb && c < kb) { const double2 d = I[i + c * ldi]; v = CxT<T>::make(d.x, d.y); }
+        if (rowblk) A[c][i] = v; else A[i][c] = v;
+    }
     if (rowblk) {
         T* C = W + k + (long long)(k + kb + x0) * ld;      // kb rows x (up to) TW columns
-        for (int q = tid; q < MF_NB * MF_NB; q += 256) A[q / MF_NB][q % MF_NB] = L[q];          // Li[i + t * 32]
         for (int q = tid; q < MF_NB * TW; q += 256) {
             const int t = q % MF_NB, c = q / MF_NB;
             V[t][c] = (t < kb && x0 + c < m) ? C[t + c * ld] : zero;
@@ -392,7 +414,6 @@ __global__ void __launch_bounds__(256) mf_panel_kernel(const int* __restrict__ l
         }
     } else {
         T* C = W + (k + kb + x0) + (long long)k * ld;      // (up to) TW rows x kb columns
-        for (int q = tid; q < MF_NB * MF_NB; q += 256) A[q % MF_NB][q / MF_NB] = L[q];          // Ui[t + c * 32]
         for (int q = tid; q < MF_NB * TW; q += 256) {
             const int r = q % TW, t = q / TW;
             V[t][r] = (t < kb && x0 + r < m) ? C[r + t * ld] : zero;
@@ -542,8 +563,8 @@ __global__ void __launch_bounds__(256, TM > 64 || sizeof(T) > 8 ? 2 : 3) mf_trai
     mf_tile_update<T, TM>(sm, ws + f.ws, f.n, ke + ti * TM, f.n, ke + tj * MF_TILE, f.n, ob, ke - ob);
 }
 
-// Factor columns (n x e) and U block row (e x b), rounded to complex64, and the Schur complement (b x b,
-// workspace precision) out of the workspace.
+// Factor columns (their rows outside the 256-blocks) and U block row (e x b), rounded to complex64, and the Schur
+// complement (b x b, workspace precision) out of the workspace.
 // (a warp per column: walking flat entries spent its time on 64-bit divisions, 611 us a launch on the 82 944-tet
 // cavity, 469 now)
 template <typename T>
@@ -555,12 +576,15 @@ __global__ void __launch_bounds__(256) mf_compact_kernel(const int* __restrict__
     const T* W = ws + f.ws + (long long)j * n;
     float2* F = fact + f.fact;
     if (j < e) {
-        F += (long long)j * n;
+        const int k0 = j / MF_SB * MF_SB, w = min(MF_SB, e - k0);
+        F += mf_fact_block(n, k0) + (long long)(j - k0) * (n - w);
 #pragma unroll 4
-        for (int i = lane; i < n; i += 32) F[i] = to_c64(W[i]);
+        for (int i = lane; i < k0; i += 32) F[i] = to_c64(W[i]);
+#pragma unroll 4
+        for (int i = k0 + lane; i < n - w; i += 32) F[i] = to_c64(W[i + w]);
         return;
     }
-    F += (long long)n * e + (long long)(j - e) * e;
+    F += mf_fact_rows_cols(n, e) + (long long)(j - e) * e;
 #pragma unroll 4
     for (int i = lane; i < e; i += 32) F[i] = to_c64(W[i]);
     T* U = upd + f.upd + (long long)(j - e) * f.b;
@@ -568,25 +592,25 @@ __global__ void __launch_bounds__(256) mf_compact_kernel(const int* __restrict__
     for (int i = lane; i < f.b; i += 32) U[i] = W[e + i];
 }
 
-// Inverses of the 256 x 256 diagonal blocks of L and U, written over the factor store's copy of those blocks.
+// Inverses of the 256 x 256 diagonal blocks of L and U, below and above the steps' 32 x 32 inverses in the inverse store.
 // With the step's inverses A_j = Linv_j P_j (mf_diag_kernel) on the diagonal, block column j of the inverse
 // of the block-lower L is G_jj = A_j, G_ij = -A_i sum_{j <= t < i} L_it G_tj; that of U is H_jj = Uinv_j,
 // H_ij = -Uinv_i sum_{i < t <= j} U_it H_tj.  One CTA per (block column, L or U, 256-block, front): the
-// columns are independent, so nothing is serial but the at most 8 steps of one column.  Computed in the
-// front's precision from the workspace; the diagonal 32 x 32 blocks stay in the inverse store.
+// columns are independent, so nothing is serial but the at most 8 steps of one column.  FP64 for both front
+// precisions: a product with G is then as accurate as the 32-step substitution with L (complex64 inverses
+// were not: residual of one application 1.0e-4 -> 1.0e-3 on a 750-tet cavity, 0.12 -> 2.9 on a 3 696-tet
+// substrate at 1 GHz).
 constexpr int MF_NBB = MF_SB / MF_NB;
-template <typename T>
 struct MfInvSmem {
-    T x[MF_NBB][MF_NB][MF_NB + 1];       // the column's blocks, [block][row][column]
-    T a[MF_NB][MF_NB + 1];
-    T s[MF_NB][MF_NB + 1];
+    double2 x[MF_NBB][MF_NB][MF_NB + 1];       // the column's blocks, [block][row][column]
+    double2 a[MF_NB][MF_NB + 1];
+    double2 s[MF_NB][MF_NB + 1];
 };
 template <typename T>
 __global__ void __launch_bounds__(256) mf_block_inverse_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm,
-                                                               const T* __restrict__ ws, const T* __restrict__ invc,
-                                                               float2* __restrict__ fact) {
+                                                               const T* __restrict__ ws, double2* __restrict__ inv) {
     extern __shared__ __align__(16) unsigned char mf_smem[];
-    MfInvSmem<T>& sm = *reinterpret_cast<MfInvSmem<T>*>(mf_smem);
+    MfInvSmem& sm = *reinterpret_cast<MfInvSmem*>(mf_smem);
     const FrontMeta& f = fm[lst[blockIdx.z]];
     const int k0 = blockIdx.y * MF_SB;
     if (k0 >= f.e) return;
@@ -596,25 +620,33 @@ __global__ void __launch_bounds__(256) mf_block_inverse_kernel(const int* __rest
     if (j >= ns || (upper ? j == 0 : j == ns - 1)) return;       // no off-diagonal block in this column
     const long long n = f.n;
     const T* W = ws + f.ws + k0 + (long long)k0 * n;
-    const T* I = invc + f.inv + (long long)(k0 / MF_NB) * 2 * MF_NB * MF_NB;
-    float2* F = fact + f.fact + k0 + (long long)k0 * n;
+    double2* I = inv + f.inv + mf_inv_block(k0) + (upper ? 0 : MF_NB);
+    const int ldi = rows + MF_NB;
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;   // thread: rows tx, tx + 16, columns ty, ty + 16
-    const T zero = CxT<T>::make(0.0, 0.0);
-    for (int t = tid; t < MF_NB * MF_NB; t += 256)
-        sm.x[j][t % MF_NB][t / MF_NB] = I[(long long)j * 2 * MF_NB * MF_NB + (upper ? MF_NB * MF_NB : 0) + t];
+    const double2 zero = make_double2(0.0, 0.0);
+    auto block = [&](int i, int q) {                             // entry q of the inverse of step i
+        const int r = i * MF_NB + q % MF_NB, c = i * MF_NB + q / MF_NB;
+        return r < rows && c < rows ? I[r + (long long)c * ldi] : zero;
+    };
+    for (int t = tid; t < MF_NB * MF_NB; t += 256) sm.x[j][t % MF_NB][t / MF_NB] = block(j, t);
     __syncthreads();
     const int step = upper ? -1 : 1;
     for (int i = j + step; upper ? i >= 0 : i < ns; i += step) {
-        T acc[2][2] = {{zero, zero}, {zero, zero}};
+        double2 acc[2][2] = {{zero, zero}, {zero, zero}};
         for (int t = j; t != i; t += step) {
             for (int q = tid; q < MF_NB * MF_NB; q += 256) {
                 const int r = q % MF_NB, c = q / MF_NB;
-                sm.a[r][c] = (i * MF_NB + r < rows && t * MF_NB + c < rows) ? W[i * MF_NB + r + (long long)(t * MF_NB + c) * n] : zero;
+                double2 v = zero;
+                if (i * MF_NB + r < rows && t * MF_NB + c < rows) {
+                    const T l = W[i * MF_NB + r + (long long)(t * MF_NB + c) * n];
+                    v = make_double2(l.x, l.y);
+                }
+                sm.a[r][c] = v;
             }
             __syncthreads();
 #pragma unroll 8
             for (int k = 0; k < MF_NB; k++) {
-                const T a0 = sm.a[tx][k], a1 = sm.a[tx + 16][k], b0 = sm.x[t][k][ty], b1 = sm.x[t][k][ty + 16];
+                const double2 a0 = sm.a[tx][k], a1 = sm.a[tx + 16][k], b0 = sm.x[t][k][ty], b1 = sm.x[t][k][ty + 16];
                 cfma(acc[0][0], a0, b0); cfma(acc[0][1], a0, b1); cfma(acc[1][0], a1, b0); cfma(acc[1][1], a1, b1);
             }
             __syncthreads();
@@ -623,13 +655,12 @@ __global__ void __launch_bounds__(256) mf_block_inverse_kernel(const int* __rest
         for (int p = 0; p < 2; p++)
 #pragma unroll
             for (int q = 0; q < 2; q++) sm.s[tx + 16 * p][ty + 16 * q] = acc[p][q];
-        for (int q = tid; q < MF_NB * MF_NB; q += 256)
-            sm.a[q % MF_NB][q / MF_NB] = I[(long long)i * 2 * MF_NB * MF_NB + (upper ? MF_NB * MF_NB : 0) + q];
+        for (int q = tid; q < MF_NB * MF_NB; q += 256) sm.a[q % MF_NB][q / MF_NB] = block(i, q);
         __syncthreads();
-        T o[2][2] = {{zero, zero}, {zero, zero}};
+        double2 o[2][2] = {{zero, zero}, {zero, zero}};
 #pragma unroll 8
         for (int k = 0; k < MF_NB; k++) {
-            const T a0 = sm.a[tx][k], a1 = sm.a[tx + 16][k], b0 = sm.s[k][ty], b1 = sm.s[k][ty + 16];
+            const double2 a0 = sm.a[tx][k], a1 = sm.a[tx + 16][k], b0 = sm.s[k][ty], b1 = sm.s[k][ty + 16];
             cfms(o[0][0], a0, b0); cfms(o[0][1], a0, b1); cfms(o[1][0], a1, b0); cfms(o[1][1], a1, b1);
         }
 #pragma unroll
@@ -639,7 +670,7 @@ __global__ void __launch_bounds__(256) mf_block_inverse_kernel(const int* __rest
                 const int r = tx + 16 * p, c = ty + 16 * q;
                 sm.x[i][r][c] = o[p][q];
                 if (i * MF_NB + r < rows && j * MF_NB + c < rows)
-                    F[i * MF_NB + r + (long long)(j * MF_NB + c) * n] = to_c64(o[p][q]);
+                    I[i * MF_NB + r + (long long)(j * MF_NB + c) * ldi] = o[p][q];
             }
         __syncthreads();
     }
@@ -792,8 +823,7 @@ __device__ __forceinline__ void mf_stage_x(MfProdSmem<NS>& sm, int c0, int nc, i
 
 // acc += staged columns [0, nc) times M: MAt(i, c) is entry (row rl + 32 i of the tile, staged column c).  A warp
 // takes every eighth column, U of them at once with the columns past the end masked: a plain unrolled loop runs
-// its remainder one load latency per column (block-inverse kernels of one front, whose column counts are
-// no multiples of 64: 18 us a launch at one or eight right-hand sides, 5 and 7 now)
+// its remainder one load latency per column
 template <int RPL, int U, typename MAt>
 __device__ __forceinline__ void mf_load(float2 (*mv)[RPL], int c0, int nc, MAt mat) {
 #pragma unroll
@@ -871,39 +901,79 @@ __device__ __forceinline__ void mf_product(MfProdSmem<NS>& sm, int c0, int c1, i
     mf_finish<NS, RPL>(sm, acc, ns, out);
 }
 
-// y[k0 .. k1) = G w[k0 .. k1), G the inverse of the 256-block of L: 32 rows per CTA, off-diagonal blocks from
-// the factor store, the diagonal one from the inverse store
+// Products with the block inverses, FP64 inside (inverse entries and sums; x and the result are complex64): 32 rows per
+// CTA, a warp takes every eighth of the nc columns, 16 of them in flight.  M: entry (the CTA's first row, first
+// column), XOf(c) points at column c's x values, Out(row of the tile, right-hand side, value).  Latency bounds it at
+// the few-front levels: the FP64 multiply-adds of a whole application take 60 us of 2.4 ms at 24 576 tets.
+template <int NS>
+struct MfTriSmem {
+    double2 x[MF_SB][NS];
+    double2 red[8][NS < 4 ? NS : 4][MF_NB];
+};
+template <int NS, typename XOf, typename Out>
+__device__ __forceinline__ void mf_tri_product(MfTriSmem<NS>& sm, const double2* M, int ldm, int nr, int nc, int ns, XOf xof, Out out) {
+    constexpr int U = 16, QB = NS < 4 ? NS : 4;
+    const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
+    const double2 zero = make_double2(0.0, 0.0);
+    double2 acc[NS], mv[U];
+#pragma unroll
+    for (int q = 0; q < NS; q++) acc[q] = zero;
+    auto load = [&](int c0) {
+#pragma unroll
+        for (int u = 0; u < U; u++) mv[u] = lane < nr && c0 + 8 * u < nc ? M[lane + (long long)(c0 + 8 * u) * ldm] : zero;
+    };
+    load(g);
+    mf_chain_wait();
+    for (int t = threadIdx.x; t < nc * NS; t += 256) {
+        const int c = t / NS, q = t % NS;
+        const float2 v = q < ns ? mf_vec(xof(c) + q) : make_float2(0.f, 0.f);
+        sm.x[c][q] = make_double2(v.x, v.y);
+    }
+    __syncthreads();
+    for (int c0 = g; c0 < nc;) {
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int c = c0 + 8 * u;
+            if (c >= nc) break;              // the same for the whole warp
+#pragma unroll
+            for (int q = 0; q < NS; q++) cfma(acc[q], mv[u], sm.x[c][q]);
+        }
+        c0 += 8 * U;
+        if (c0 < nc) load(c0);
+    }
+#pragma unroll
+    for (int q0 = 0; q0 < NS; q0 += QB) {    // the warps' sums in order
+        if (q0) __syncthreads();
+#pragma unroll
+        for (int q = 0; q < QB; q++) sm.red[g][q][lane] = acc[q0 + q];
+        __syncthreads();
+        for (int t = threadIdx.x; t < MF_NB * QB; t += 256) {
+            const int q = t / MF_NB, r = t % MF_NB;
+            if (q0 + q >= ns || r >= nr) continue;
+            double2 v = zero;
+#pragma unroll
+            for (int gg = 0; gg < 8; gg++) { v.x += sm.red[gg][q][r].x; v.y += sm.red[gg][q][r].y; }
+            out(r, q0 + q, make_float2((float)v.x, (float)v.y));
+        }
+    }
+}
+
+// y[k0 .. k1) = G w[k0 .. k1), G the inverse of the 256-block of L
 template <int NS>
 __global__ void __launch_bounds__(256) mf_fwd_tri_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm,
-                                                         int S, int k0, const float2* __restrict__ fact,
-                                                         const float2* __restrict__ inv, const float2* __restrict__ w,
-                                                         float2* __restrict__ y) {
-    __shared__ MfProdSmem<NS> sm;
+                                                         int S, int k0, const double2* __restrict__ inv,
+                                                         const float2* __restrict__ w, float2* __restrict__ y) {
+    __shared__ MfTriSmem<NS> sm;
     mf_chain_start();
     const FrontMeta& f = fm[lst[blockIdx.y]];
     const int r0 = k0 + blockIdx.x * MF_NB;
     if (r0 >= f.e) { mf_chain_wait(); return; }
-    const int s0 = blockIdx.z * NS, ns = min(NS, S - s0), r = r0 + (threadIdx.x & 31);
-    const float2* F = fact + f.fact + r;
-    const float2* D = inv + f.inv + (long long)(r0 / MF_NB) * 2 * MF_NB * MF_NB + (threadIdx.x & 31);
-    const float2* X = w + f.wv * S + s0;
-    float2* Y = y + f.y * S + s0;
-    const bool live = r < f.e;
-    const long long n = f.n;
-    const int co = r0 - k0;              // staged columns: the block row's off-diagonal part, then its diagonal block
-    const int nc = min(r0 + MF_NB, f.e) - k0;
-    float2 acc[1][NS] = {};
-    auto at = [&](int, int c) {
-        const float2* p = c < co ? F + (k0 + c) * n : D + (c - co) * MF_NB;
-        return live ? *p : make_float2(0.f, 0.f);
-    };
-    float2 mv[16][1];
-    mf_load<1, 16>(mv, threadIdx.x >> 5, nc, at);
-    mf_chain_wait();
-    mf_stage_x(sm, k0, nc, ns, [&](int c) { return X + (long long)c * S; });
-    __syncthreads();
-    mf_accumulate<NS, 1, 16>(sm, acc, mv, nc, at);
-    mf_finish<NS, 1>(sm, acc, ns, [&](int t, int q, float2 v) { if (r0 + t < f.e) Y[(long long)(r0 + t) * S + q] = v; });
+    const int s0 = blockIdx.z * NS, ns = min(NS, S - s0), nr = min(MF_NB, f.e - r0), ldi = min(MF_SB, f.e - k0) + MF_NB;
+    const float2* X = w + (f.wv + k0) * S + s0;
+    float2* Y = y + (f.y + r0) * S + s0;
+    mf_tri_product<NS>(sm, inv + f.inv + mf_inv_block(k0) + (r0 - k0) + MF_NB, ldi, nr, r0 - k0 + nr, ns,
+                       [&](int c) { return X + (long long)c * S; },
+                       [&](int t, int q, float2 v) { Y[(long long)t * S + q] = v; });
 }
 
 // rows [k1, n): w[r] -= L[r, k0:k1] y[k0:k1]
@@ -919,12 +989,12 @@ __global__ void __launch_bounds__(256, NS * RPL > 16 ? 2 : 3) mf_fwd_update_kern
     const int r0 = k1 + blockIdx.x * 32 * RPL;
     if (r0 >= f.n) { mf_chain_wait(); return; }
     const int s0 = blockIdx.z * NS, ns = min(NS, S - s0), r = r0 + (threadIdx.x & 31);
-    const float2* F = fact + f.fact + r;
+    const long long n = f.n, ldf = n - (k1 - k0);
+    const float2* F = fact + f.fact + mf_fact_block(f.n, k0) + r - (k1 - k0);         // column c of the block at c ldf
     const float2* X = y + f.y * S + s0;
     float2* W = w + f.wv * S + s0;
-    const long long n = f.n;
     mf_product<NS, RPL>(sm, k0, k1, ns, [&](int c) { return X + (long long)c * S; },
-                        [&](int i, int c) { return r + 32 * i < n ? F[32 * i + c * n] : make_float2(0.f, 0.f); },
+                        [&](int i, int c) { return r + 32 * i < n ? F[32 * i + (c - k0) * ldf] : make_float2(0.f, 0.f); },
                         [&](int t, int q, float2 v) {
                             if (r0 + t >= n) return;
                             float2* p = W + (long long)(r0 + t) * S + q;
@@ -949,7 +1019,7 @@ __global__ void __launch_bounds__(256, NS * RPL > 16 ? 2 : 3) mf_bwd_bnd_kernel(
     if (f.b == 0 || r0 >= f.e) { mf_chain_wait(); return; }
     const int s0 = blockIdx.z * NS, ns = min(NS, S - s0), r = r0 + (threadIdx.x & 31);
     const long long e = f.e;
-    const float2* M = fact + f.fact + (long long)f.n * e + r;
+    const float2* M = fact + f.fact + mf_fact_rows_cols(f.n, f.e) + r;
     const int* d = fdof + f.fdof + e;
     const float2* X = xs + s0;
     const int c0 = min(sp * cw, f.b), c1 = nsplit > 1 ? min(c0 + cw, f.b) : f.b;
@@ -986,34 +1056,20 @@ __global__ void mf_bwd_bnd_sum_kernel(const int* __restrict__ lst, const FrontMe
 // x[k0 .. k1) = H y[k0 .. k1), H the inverse of the 256-block of U, into the solution (DOF order)
 template <int NS>
 __global__ void __launch_bounds__(256) mf_bwd_tri_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm,
-                                                         int S, int k0, const float2* __restrict__ fact,
-                                                         const float2* __restrict__ inv, const int* __restrict__ fdof,
-                                                         const float2* __restrict__ y, float2* __restrict__ xs) {
-    __shared__ MfProdSmem<NS> sm;
+                                                         int S, int k0, const double2* __restrict__ inv,
+                                                         const int* __restrict__ fdof, const float2* __restrict__ y,
+                                                         float2* __restrict__ xs) {
+    __shared__ MfTriSmem<NS> sm;
     mf_chain_start();
     const FrontMeta& f = fm[lst[blockIdx.y]];
     const int r0 = k0 + blockIdx.x * MF_NB;
     if (r0 >= f.e) { mf_chain_wait(); return; }
-    const int s0 = blockIdx.z * NS, ns = min(NS, S - s0), r = r0 + (threadIdx.x & 31);
-    const float2* F = fact + f.fact + r;
-    const float2* D = inv + f.inv + (long long)(r0 / MF_NB) * 2 * MF_NB * MF_NB + MF_NB * MF_NB + (threadIdx.x & 31);
-    const float2* X = y + f.y * S + s0;
-    const int* d = fdof + f.fdof;
-    const bool live = r < f.e;
-    const long long n = f.n;
-    const int ce = min(k0 + MF_SB, f.e) - r0, cd = min(MF_NB, ce);
-    float2 acc[1][NS] = {};
-    auto at = [&](int, int c) {
-        const float2* p = c < cd ? D + c * MF_NB : F + (r0 + c) * n;
-        return live ? *p : make_float2(0.f, 0.f);
-    };
-    float2 mv[16][1];
-    mf_load<1, 16>(mv, threadIdx.x >> 5, ce, at);
-    mf_chain_wait();
-    mf_stage_x(sm, r0, ce, ns, [&](int c) { return X + (long long)c * S; });
-    __syncthreads();
-    mf_accumulate<NS, 1, 16>(sm, acc, mv, ce, at);
-    mf_finish<NS, 1>(sm, acc, ns, [&](int t, int q, float2 v) { if (r0 + t < f.e) xs[(long long)d[r0 + t] * S + s0 + q] = v; });
+    const int s0 = blockIdx.z * NS, ns = min(NS, S - s0), nr = min(MF_NB, f.e - r0), ldi = min(MF_SB, f.e - k0) + MF_NB;
+    const float2* X = y + (f.y + r0) * S + s0;
+    const int* d = fdof + f.fdof + r0;
+    mf_tri_product<NS>(sm, inv + f.inv + mf_inv_block(k0) + (r0 - k0) + (long long)(r0 - k0) * ldi, ldi, nr,
+                       min(k0 + MF_SB, f.e) - r0, ns, [&](int c) { return X + (long long)c * S; },
+                       [&](int t, int q, float2 v) { xs[(long long)d[t] * S + s0 + q] = v; });
 }
 
 // rows [0, k0): y[r] -= U[r, k0:k1] x[k0:k1]
@@ -1028,13 +1084,13 @@ __global__ void __launch_bounds__(256, NS * RPL > 16 ? 2 : 3) mf_bwd_update_kern
     if (k0 >= f.e) { mf_chain_wait(); return; }
     const int k1 = min(k0 + MF_SB, f.e), r0 = blockIdx.x * 32 * RPL;      // k0 is a multiple of 256: whole tiles
     const int s0 = blockIdx.z * NS, ns = min(NS, S - s0), r = r0 + (threadIdx.x & 31);
-    const float2* F = fact + f.fact + r;
+    const long long ldf = f.n - (k1 - k0);
+    const float2* F = fact + f.fact + mf_fact_block(f.n, k0) + r;         // column c of the block at c ldf
     const float2* X = xs + s0;
     const int* d = fdof + f.fdof;
     float2* Y = y + f.y * S + s0;
-    const long long n = f.n;
     mf_product<NS, RPL>(sm, k0, k1, ns, [&](int c) { return X + (long long)d[c] * S; },
-                        [&](int i, int c) { return F[32 * i + c * n]; },
+                        [&](int i, int c) { return F[32 * i + (c - k0) * ldf]; },
                         [&](int t, int q, float2 v) {
                             float2* p = Y + (long long)(r0 + t) * S + q;
                             const float2 o = mf_vec(p);
@@ -1080,10 +1136,9 @@ struct emfem_mf_s {
     uint8_t* d_free = nullptr;                    // 1 where a DOF belongs to some front
     double* d_scale = nullptr;                    // equilibration D^-1/2 of the current factorization
     float2* fact = nullptr;
-    float2* inv = nullptr;
+    double2* inv = nullptr;                       // block inverses
     void* ws = nullptr;                           // level workspace, complex64 or (wide) complex128
     void* upd = nullptr;                          // update store, same precision as ws
-    void* invc = nullptr;                         // complex128 copies of the inverse blocks (wide only)
     bool wide = false;                            // fronts factored in complex128
     int* d_npert = nullptr;
     long long fact_n = 0, inv_n = 0, ws_n = 0, upd_n = 0;
@@ -1106,7 +1161,7 @@ struct emfem_mf_s {
 
 static void mf_free(emfem_mf_s* m) {
     void* ps[] = {m->d_meta, m->d_lst, m->d_fdof, m->d_ea, m->d_slot, m->d_off, m->d_free, m->d_scale, m->fact, m->inv,
-                  m->ws, m->upd, m->invc, m->d_npert, m->d_cmap, m->sw, m->sy, m->sx, m->spart};
+                  m->ws, m->upd, m->d_npert, m->d_cmap, m->sw, m->sy, m->sx, m->spart};
     for (void* p : ps)
         if (p) cudaFree(p);
 }
@@ -1141,7 +1196,8 @@ static bool mf_wide_tiles(long long rows, int ny, unsigned sz) { return (rows + 
 template <int NS>
 static int mf_sweep_tree(emfem_mf_s* m, int S, const double2* r, cudaStream_t s) {
     const int nl = (int)m->levels.size();
-    const unsigned sz = (unsigned)((S + NS - 1) / NS);
+    constexpr int NT = NS < 8 ? NS : 8;          // right-hand sides per CTA of the block-inverse products (48 KB of staging)
+    const unsigned sz = (unsigned)((S + NS - 1) / NS), szt = (unsigned)((S + NT - 1) / NT);
     bool first = true;
     for (int L = 0; L < nl; L++) {
         const int nfl = (int)m->levels[L].size();
@@ -1159,7 +1215,7 @@ static int mf_sweep_tree(emfem_mf_s* m, int S, const double2* r, cudaStream_t s)
             first = false;
             for (int k0 = 0; k0 < maxe; k0 += MF_SB) {
                 const unsigned nt = nblk(std::min(MF_SB, maxe - k0), MF_NB);
-                mf_chain(mf_fwd_tri_kernel<NS>, dim3(nt, ny, sz), s, lst, m->d_meta, S, k0, m->fact, m->inv, m->sw, m->sy);
+                mf_chain(mf_fwd_tri_kernel<NT>, dim3(nt, ny, szt), s, lst, m->d_meta, S, k0, m->inv, m->sw, m->sy);
                 const long long rows = maxn - k0;            // rows [k1, n) of a front: at most n - k0
                 if (mf_wide_tiles(rows, ny, sz))
                     mf_chain(mf_fwd_update_kernel<NS, 2>, dim3(nblk(rows, 64), ny, sz), s, lst, m->d_meta, S, k0, m->fact, m->sy, m->sw);
@@ -1192,8 +1248,7 @@ static int mf_sweep_tree(emfem_mf_s* m, int S, const double2* r, cudaStream_t s)
             }
             for (int k0 = (maxe - 1) / MF_SB * MF_SB; maxe > 0 && k0 >= 0; k0 -= MF_SB) {
                 const unsigned nt = nblk(std::min(MF_SB, maxe - k0), MF_NB);
-                mf_chain(mf_bwd_tri_kernel<NS>, dim3(nt, ny, sz), s, lst, m->d_meta, S, k0, m->fact, m->inv, m->d_fdof,
-                         m->sy, m->sx);
+                mf_chain(mf_bwd_tri_kernel<NT>, dim3(nt, ny, szt), s, lst, m->d_meta, S, k0, m->inv, m->d_fdof, m->sy, m->sx);
                 if (k0 == 0) continue;
                 if (mf_wide_tiles(k0, ny, sz))
                     mf_chain(mf_bwd_update_kernel<NS, 2>, dim3(k0 / 64, ny, sz), s, lst, m->d_meta, S, k0, m->fact,
@@ -1234,7 +1289,6 @@ template <typename T>
 static int mf_factor_levels(emfem_mf_s* m, const double2* K_vals, cudaStream_t s) {
     T* ws = (T*)m->ws;
     T* upd = (T*)m->upd;
-    T* invc = m->wide ? (T*)m->invc : (T*)m->inv;
     int rc = EMFEM_OK;
     const int nl = (int)m->levels.size();
     for (int L = 0; L < nl && rc == EMFEM_OK; L++) {
@@ -1253,11 +1307,11 @@ static int mf_factor_levels(emfem_mf_s* m, const double2* K_vals, cudaStream_t s
             const int maxe = m->lvl_max_e[L];
             for (int k = 0; k < maxe; k += MF_NB) {
                 const int ob = k / MF_OB * MF_OB;
-                mf_diag_kernel<T><<<ny, 256, 0, s>>>(lst, m->d_meta, k, ws, m->inv, invc, m->d_npert);
+                mf_diag_kernel<T><<<ny, 256, 0, s>>>(lst, m->d_meta, k, ws, m->inv, m->d_npert);
                 const long long mm = std::max(1LL, maxn - k - 1);
                 constexpr int TW = sizeof(T) == sizeof(float2) ? 64 : 32;     // tiles within static shared memory
                 const unsigned npt = nblk(mm, TW);
-                mf_panel_kernel<T, TW><<<dim3(2 * npt, ny), 256, 0, s>>>(lst, m->d_meta, k, (int)npt, ws, invc);
+                mf_panel_kernel<T, TW><<<dim3(2 * npt, ny), 256, 0, s>>>(lst, m->d_meta, k, (int)npt, ws, m->inv);
                 if (k + MF_NB < std::min(ob + MF_OB, maxe)) {
                     const unsigned nr = nblk(mm, 64);
                     mf_strip_kernel<T><<<dim3(4 * nr, ny), 256, sizeof(MfTileSmem<T, 64>), s>>>(lst, m->d_meta, k, ob, (int)nr, ws);
@@ -1279,8 +1333,8 @@ static int mf_factor_levels(emfem_mf_s* m, const double2* K_vals, cudaStream_t s
             mf_compact_kernel<T><<<dim3(nblk(maxn, 8), ny), 256, 0, s>>>(lst, m->d_meta, ws, m->fact, upd);
             if (m->lvl_max_e[L] > MF_NB) {
                 const int nbb = std::min(MF_NBB, (int)nblk(m->lvl_max_e[L], MF_NB));
-                mf_block_inverse_kernel<T><<<dim3(2 * nbb, nblk(m->lvl_max_e[L], MF_SB), ny), 256, sizeof(MfInvSmem<T>), s>>>(
-                    lst, m->d_meta, ws, invc, m->fact);
+                mf_block_inverse_kernel<T><<<dim3(2 * nbb, nblk(m->lvl_max_e[L], MF_SB), ny), 256, sizeof(MfInvSmem), s>>>(
+                    lst, m->d_meta, ws, m->inv);
             }
             rc = check_cuda(cudaGetLastError(), "multifrontal factor level");
         }
@@ -1326,8 +1380,8 @@ int emfem_mf_create(emfem_handle h, int64_t n, int n_fronts, const int32_t* e, c
         f.fdof = fdof_ptr[v];
         f.ea = eao; eao += b[v];
         f.asm0 = asm_ptr ? asm_ptr[v] : 0; f.asm1 = asm_ptr ? asm_ptr[v + 1] : 0;
-        f.fact = fact; fact += (long long)f.n * f.e + (long long)f.e * f.b;
-        f.inv = inv; inv += (long long)((f.e + MF_NB - 1) / MF_NB) * 2 * MF_NB * MF_NB;
+        f.fact = fact; fact += mf_fact_rows_cols(f.n, f.e) + (long long)f.e * f.b;
+        f.inv = inv; inv += mf_inv_entries(f.e);
     }
     for (int v = 0; v < n_fronts; v++) {
         int p = parent[v];
@@ -1452,7 +1506,7 @@ int emfem_mf_create(emfem_handle h, int64_t n, int n_fronts, const int32_t* e, c
         rc = check_cuda(cudaMalloc(dst, std::max<size_t>(bytes, 16)), "cudaMalloc");
     };
     mk((void**)&m->fact, sizeof(float2) * fact);
-    mk((void**)&m->inv, sizeof(float2) * inv);
+    mk((void**)&m->inv, sizeof(double2) * inv);
     mk((void**)&m->ws, sizeof(float2) * ws_max);
     mk((void**)&m->upd, sizeof(float2) * upd_top);
     mk((void**)&m->d_npert, sizeof(int));
@@ -1460,10 +1514,10 @@ int emfem_mf_create(emfem_handle h, int64_t n, int n_fronts, const int32_t* e, c
     mk((void**)&m->d_cmap, sizeof(int) * 2 * wv);
     if (rc != EMFEM_OK) { mf_free(m); delete m; return rc; }
     rc = check_cuda(cudaFuncSetAttribute(mf_block_inverse_kernel<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)sizeof(MfInvSmem<float2>)), "cudaFuncSetAttribute");
+                                         (int)sizeof(MfInvSmem)), "cudaFuncSetAttribute");
     if (rc == EMFEM_OK)
         rc = check_cuda(cudaFuncSetAttribute(mf_block_inverse_kernel<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)sizeof(MfInvSmem<double2>)), "cudaFuncSetAttribute");
+                                             (int)sizeof(MfInvSmem)), "cudaFuncSetAttribute");
     if (rc == EMFEM_OK)
         rc = check_cuda(cudaFuncSetAttribute(mf_strip_kernel<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)sizeof(MfTileSmem<float2, 64>)), "cudaFuncSetAttribute");
@@ -1494,8 +1548,8 @@ int emfem_mf_create(emfem_handle h, int64_t n, int n_fronts, const int32_t* e, c
 int emfem_mf_info(emfem_mf m, size_t* device_bytes, double* flops, int* n_levels) {
     EMFEM_REQUIRE(m, "emfem_mf_info: bad handle");
     if (device_bytes)
-        *device_bytes = sizeof(float2) * (m->fact_n + m->inv_n) + (m->wide ? sizeof(double2) : sizeof(float2)) *
-                        (m->ws_n + m->upd_n) + (m->wide ? sizeof(double2) * m->inv_n : 0) + sizeof(int) * 2 * m->wv_n +
+        *device_bytes = sizeof(float2) * m->fact_n + sizeof(double2) * m->inv_n + (m->wide ? sizeof(double2) : sizeof(float2)) *
+                        (m->ws_n + m->upd_n) + sizeof(int) * 2 * m->wv_n +
                         sizeof(double) * m->n;
     if (flops) *flops = m->flops;
     if (n_levels) *n_levels = (int)m->levels.size();
@@ -1510,23 +1564,22 @@ int emfem_mf_set_precision(emfem_mf m, int bits) {
     EMFEM_CUDA(cudaGetDevice(&prev));
     if (prev != m->h->device) EMFEM_CUDA(cudaSetDevice(m->h->device));
     EMFEM_CUDA(cudaStreamSynchronize(m->h->stream));
-    void* ps[] = {m->ws, m->upd, m->invc};
+    void* ps[] = {m->ws, m->upd};
     for (void* p : ps)
         if (p) cudaFree(p);
-    m->ws = m->upd = m->invc = nullptr;
+    m->ws = m->upd = nullptr;
     m->factored = false;
     const size_t el = wide ? sizeof(double2) : sizeof(float2);
     int rc = check_cuda(cudaMalloc(&m->ws, el * std::max(1LL, m->ws_n)), "cudaMalloc");
     if (rc == EMFEM_OK) rc = check_cuda(cudaMalloc(&m->upd, el * std::max(1LL, m->upd_n)), "cudaMalloc");
-    if (rc == EMFEM_OK && wide) rc = check_cuda(cudaMalloc(&m->invc, sizeof(double2) * std::max(1LL, m->inv_n)), "cudaMalloc");
     if (rc == EMFEM_OK) {
         m->wide = wide;
     } else {
         // leave a usable complex64 handle behind when the complex128 workspace does not fit
-        void* qs[] = {m->ws, m->upd, m->invc};
+        void* qs[] = {m->ws, m->upd};
         for (void* p : qs)
             if (p) cudaFree(p);
-        m->ws = m->upd = m->invc = nullptr;
+        m->ws = m->upd = nullptr;
         m->wide = false;
         if (cudaMalloc(&m->ws, sizeof(float2) * std::max(1LL, m->ws_n)) != cudaSuccess ||
             cudaMalloc(&m->upd, sizeof(float2) * std::max(1LL, m->upd_n)) != cudaSuccess)
