@@ -1596,11 +1596,8 @@ static int krylov_impl(emfem_handle hd, int method, int64_t n, int64_t nnz, cons
             k.wide = k.v[3]; k.held = k.v[0];
             k.minv_wide = Ax; k.minv_held = (double2*)(ws + L.off_minv);
         }
-        // the recurrence tolerance is half the requested one so the FP64 true residual meets it; an LU-preconditioned
-        // solve asked for nearly full precision goes to a tenth: its last iteration gains several digits anyway, and
-        // at low frequency the solution's error is some 300 times the residual
-        const double rtol = (mf && tol < 1e-10 ? 0.1 : 0.5) * tol;
-        reduce_update_kernel<<<G * S, VB, 0, s>>>(partial, (int)nbv, S, 2, st, UPD_INIT, maxit, rtol, nsys, G,
+        // the recurrence tolerance is half the requested one so the FP64 true residual meets it
+        reduce_update_kernel<<<G * S, VB, 0, s>>>(partial, (int)nbv, S, 2, st, UPD_INIT, maxit, 0.5 * tol, nsys, G,
                                               vec_pairs(S), gpair);
         STRY(check_cuda(cudaGetLastError(), "init state"));
         STRY(k.start());

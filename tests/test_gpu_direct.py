@@ -188,3 +188,16 @@ def test_auto_precision_sweep_converges_every_frequency(cuda):
         xs = _substrate_direct(P, freqs[j])
         x = r.x[:, j].cpu().numpy()
         assert np.linalg.norm(x - xs) <= 1e-8 * np.linalg.norm(xs), freqs[j]
+
+
+def test_lu_solve_stops_where_its_tolerance_is_met(cuda):
+    """One stopping rule at every tolerance: a residual that half the tolerance covers ends the solve."""
+    P = problems.substrate_box(nx=8, ny=6, nz=6)
+    sw = FrequencySweep(P)
+    f = 1e9
+    lu = sw.direct_solver().set_precision("c128").factor(f)
+    rel = [float(sw.solve_lu([(f, 0)], lu, tol=1e-15, maxit=k).relres[0]) for k in range(1, 9)]
+    ks = [k for k in range(8) if rel[k] < 4e-11]            # 2.2 times it lies below 1e-10
+    assert ks, rel
+    r = sw.solve_lu([(f, 0)], lu, tol=2.2 * rel[ks[0]], maxit=ks[0] + 1)
+    assert r.status[0] == 0 and r.iters[0] <= ks[0] + 1, (rel, r.status, r.iters)
