@@ -328,6 +328,7 @@ __global__ void __launch_bounds__(VB, NR == 1 ? 4 : NR == 2 ? 3 : 2) spmv_kernel
                 const int je = a.patch_rowptr[pr + 1];
                 for (int j = a.patch_rowptr[pr] + g; j < je; j += G) {
                     const int q = a.patch_port[j];
+                    if ((unsigned)q >= (unsigned)a.n_ports) continue;        // a port this call has no gamma for
                     const double2 v = Pv[j];
                     const T* xc = x + (long long)a.patch_cols[j] * S + s0;
 #pragma unroll
@@ -457,8 +458,10 @@ __global__ void __launch_bounds__(VB) patch_rows_kernel(long long np, const int*
     for (int s = lane % L; s < S; s += L) {
         double2 acc = make_double2(0.0, 0.0);
         for (int j = a.patch_rowptr[p] + g; j < a.patch_rowptr[p + 1]; j += G) {
+            const int q = a.patch_port[j];
+            if ((unsigned)q >= (unsigned)a.n_ports) continue;                // as in spmv_kernel
             const double2 v = Pv[j], xv = x[(long long)a.patch_cols[j] * S + s];
-            const double* gm = a.gamma + 2 * (s * a.n_ports + a.patch_port[j]);
+            const double* gm = a.gamma + 2 * (s * a.n_ports + q);
             const double kr = gm[0] * v.x - gm[1] * v.y, ki = gm[0] * v.y + gm[1] * v.x;
             acc.x += kr * xv.x - ki * xv.y;
             acc.y += kr * xv.y + ki * xv.x;
@@ -890,6 +893,7 @@ __device__ __forceinline__ double2 row_value(const OpArgs& a, long long row, lon
         for (int j = a.patch_rowptr[pr]; j < a.patch_rowptr[pr + 1]; j++) {
             if (a.patch_cols[j] != col) continue;
             int q = a.patch_port[j];
+            if ((unsigned)q >= (unsigned)a.n_ports) continue;                // as in spmv_kernel
             double gr = a.gamma[2 * (sy * a.n_ports + q)], gi = a.gamma[2 * (sy * a.n_ports + q) + 1];
             double2 pv = Pv[j];
             v.x += gr * pv.x - gi * pv.y;

@@ -154,7 +154,8 @@ int emfem_csr_compact_nonzero(emfem_handle h, int64_t n, const int32_t *indptr, 
  * (SolverSuperLU, src/emerge/_emerge/solver.py:535-572, reached through SolveRoutine.solve
  * :1241-1326).  A_s = E - k0sq[s] * B + sum_p gamma[s, p] * R_p, where B may be NULL (then
  * A_s = E + ...), and the Robin terms R_p are given as a small row-compressed "patch"
- * (patch_rows, patch_rowptr (n_patch_rows + 1), patch_cols, patch_vals, patch_port).  Rows and
+ * (patch_rows, patch_rowptr (n_patch_rows + 1), patch_cols, patch_vals, patch_port; entries of a port
+ * outside 0 .. n_ports - 1 do not count).  Rows and
  * columns where free_mask == 0 are eliminated exactly as SolveRoutine's submatrix A[ids, ids]
  * (their solution entries are zero).  Vectors are (n, nsys) c128, DOF-major (entry (i, s) at
  * i * nsys + s).  x holds the initial guess on entry (zero for the reference's behaviour) and the

@@ -1,5 +1,7 @@
 """The sweep SpMV on CSR matrices without the DOF-pair structure: odd sizes, empty and masked rows, rows
 longer than one index chunk, every batch width of the kernel's dispatch, with and without B."""
+import ctypes
+
 import numpy as np
 import pytest
 import scipy.sparse as sp
@@ -64,3 +66,49 @@ def test_spmv_matches_scipy(cuda, n, paired, S, has_b):
         err = np.abs(y.cpu().numpy() - ref)
         # at most 115 terms a row, a few roundings per term: 256 eps of the summed magnitudes
         assert (err <= 256 * np.finfo(float).eps * mag + 1e-300).all(), (err / (mag + 1e-300)).max()
+
+
+@pytest.mark.parametrize("S", [1, 8, 32])
+def test_patch_entries_of_other_ports_are_left_out(cuda, S):
+    """A call over the first n_ports ports of a patch that lists more: entries of the others do not count, in the
+    products and in the preconditioner blocks of a solve."""
+    n, nports = 64, 2
+    rng = np.random.default_rng(S)
+    A = sp.random(n, n, 0.2, random_state=5, format="csr") + sp.diags(np.full(n, 8.0))
+    A = (A + 1j * sp.diags(rng.random(n))).tocsr()
+    A.sort_indices()
+    prow = np.arange(0, n, 2)
+    pcols = np.stack([prow, prow, prow, prow], 1).reshape(-1)               # on the diagonal, four ports a row
+    pport = np.tile([0, 1, 5, -1], len(prow))
+    pvals = rng.standard_normal(len(pcols)) + 1j * rng.standard_normal(len(pcols))
+    gam = 0.5 * (rng.standard_normal((S, nports)) + 1j * rng.standard_normal((S, nports)))
+    x = rng.standard_normal((n, S)) + 1j * rng.standard_normal((n, S))
+    ref = A @ x
+    for i, j, q, v in zip(np.repeat(prow, 4), pcols, pport, pvals):
+        if 0 <= q < nports:
+            ref[i] += gam[:, q] * v * x[j]
+    d = lambda a, t: torch.from_numpy(np.ascontiguousarray(a)).to(cuda, t)
+    c128, i32 = torch.complex128, torch.int32
+    ip, ix, ev = d(A.indptr, i32), d(A.indices, i32), d(A.data, c128)
+    pr, pp, pc, pv, po = d(prow, i32), d(4 * np.arange(len(prow) + 1), i32), d(pcols, i32), d(pvals, c128), d(pport, i32)
+    k2, gd, md, xd = (d(np.ones(S), torch.float64), d(gam, c128), d(np.ones(n), torch.uint8), d(x, c128))
+    h = Handle.get(cuda)
+    for fn in (lib().emfem_sweep_spmv, lib().emfem_sweep_spmv_noalloc):
+        y = torch.empty_like(xd)
+        st = fn(h.h, n, ptr(ip), ptr(ix), ptr(ev), None, S, ptr(k2), len(prow), ptr(pr), ptr(pp), ptr(pc), ptr(pv),
+                ptr(po), nports, ptr(gd), ptr(md), ptr(xd), ptr(y))
+        assert st == 0, _lib.last_error()
+        np.testing.assert_allclose(y.cpu().numpy(), ref, rtol=0, atol=1e-12 * np.abs(ref).max())
+    sz = ctypes.c_size_t()
+    nnz = len(A.data)
+    assert lib().emfem_krylov_workspace_size(n, nnz, S, 0, ctypes.byref(sz)) == 0
+    ws = torch.empty(sz.value, dtype=torch.uint8, device=cuda)
+    ga = np.ascontiguousarray(np.stack([gam.real, gam.imag], -1).reshape(-1))
+    status, iters, rel = (ctypes.c_int * S)(), (ctypes.c_int * S)(), (ctypes.c_double * S)()
+    xs, b = torch.zeros_like(xd), d(ref, c128)
+    st = lib().emfem_krylov_solve(h.h, 1, n, nnz, ptr(ip), ptr(ix), ptr(ev), None, S, (ctypes.c_double * S)(*np.ones(S)),
+                                  len(prow), ptr(pr), ptr(pp), ptr(pc), ptr(pv), ptr(po), nports,
+                                  (ctypes.c_double * len(ga))(*ga), ptr(md), ptr(b), ptr(xs), 1e-12, 500, 1, 0, ptr(ws),
+                                  ws.numel(), status, iters, rel, None)
+    assert st == 0, _lib.last_error()
+    np.testing.assert_allclose(xs.cpu().numpy(), x, rtol=0, atol=1e-9 * np.abs(x).max())
