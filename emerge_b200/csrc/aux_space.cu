@@ -421,13 +421,88 @@ __device__ __forceinline__ void tile_product(const float4 (*s)[NN_C], const floa
     }
 }
 
+// in_y and m_y (see above) of a tile's rows, lanes over channels; t0: type of the tile's first row
+template <typename TX>
+__device__ __forceinline__ void tile_gather(long long w0, long long total, int S, int layer, int t0, int lane,
+                                            const float (*sWin)[NN_C], const int* __restrict__ nptr,
+                                            const int* __restrict__ nbr, const float* __restrict__ inv_deg,
+                                            const uint8_t* __restrict__ atype, const TX* __restrict__ x,
+                                            const float2* __restrict__ Hin, float2* in, float2* m) {
+    if (S % NN_R == 0) {                 // the tile's rows are systems of one node: its neighbours are read once
+        const long long y = w0 / S, so = w0 - y * S;
+        const int k1 = nptr[y + 1];
+#pragma unroll
+        for (int r = 0; r < NN_R; r++) {
+            m[r] = make_float2(0.f, 0.f);
+            if (layer == 0) {
+                const TX xv = x[w0 + r];
+                in[r] = make_float2((float)xv.x * sWin[t0][lane], (float)xv.y * sWin[t0][lane]);
+            } else {
+                in[r] = Hin[(w0 + r) * NN_C + lane];
+            }
+        }
+        for (int k = nptr[y]; k < k1; k++) {
+            const long long j = nbr[k], wj = j * S + so;
+            if (layer == 0) {
+                const float wv = sWin[atype[j]][lane];
+#pragma unroll
+                for (int r = 0; r < NN_R; r++) {
+                    const TX xj = x[wj + r];
+                    m[r].x += (float)xj.x * wv;
+                    m[r].y += (float)xj.y * wv;
+                }
+            } else {
+#pragma unroll
+                for (int r = 0; r < NN_R; r++) {
+                    const float2 hj = Hin[(wj + r) * NN_C + lane];
+                    m[r].x += hj.x;
+                    m[r].y += hj.y;
+                }
+            }
+        }
+        const float idg = inv_deg[y];
+#pragma unroll
+        for (int r = 0; r < NN_R; r++) { m[r].x *= idg; m[r].y *= idg; }
+    } else {
+#pragma unroll
+        for (int r = 0; r < NN_R; r++) {
+            in[r] = m[r] = make_float2(0.f, 0.f);
+            const long long w = w0 + r;
+            if (w >= total) continue;
+            const long long y = w / S;
+            const int s = (int)(w % S);
+            if (layer == 0) {
+                const TX xv = x[w];
+                const float wv = sWin[atype[y]][lane];
+                in[r] = make_float2((float)xv.x * wv, (float)xv.y * wv);
+            } else {
+                in[r] = Hin[w * NN_C + lane];
+            }
+            for (int k = nptr[y]; k < nptr[y + 1]; k++) {
+                const long long j = nbr[k];
+                if (layer == 0) {
+                    const TX xj = x[j * S + s];
+                    const float wv = sWin[atype[j]][lane];
+                    m[r].x += (float)xj.x * wv;
+                    m[r].y += (float)xj.y * wv;
+                } else {
+                    const float2 hj = Hin[(j * S + s) * NN_C + lane];
+                    m[r].x += hj.x;
+                    m[r].y += hj.y;
+                }
+            }
+            const float idg = inv_deg[y];
+            m[r].x *= idg; m[r].y *= idg;
+        }
+    }
+}
+
 template <typename TX>
 __global__ void __launch_bounds__(NN_T) mpnn_layer_kernel(long long na, int S, int layer, const float* __restrict__ P,
                                                           const int* __restrict__ nptr, const int* __restrict__ nbr,
                                                           const float* __restrict__ inv_deg, const uint8_t* __restrict__ atype,
                                                           const TX* __restrict__ x, const float2* __restrict__ Hin,
-                                                          float2* __restrict__ Hout, float2* __restrict__ Mout,
-                                                          TX* __restrict__ za) {
+                                                          float2* __restrict__ Hout, TX* __restrict__ za) {
     __shared__ float2 sWU[2][NN_C][NN_C];
     __shared__ float4 sA[NN_T / 32][NN_R][NN_C];
     __shared__ float sWin[2][NN_C], sWout[2][NN_C];
@@ -444,73 +519,7 @@ __global__ void __launch_bounds__(NN_T) mpnn_layer_kernel(long long na, int S, i
         const long long w0 = tile * NN_R;
         const int2 tt = tile_types(atype, w0, total, S);
         float2 in[NN_R], m[NN_R];
-        if (S % NN_R == 0) {                 // the tile's rows are systems of one node: its neighbours are read once
-            const long long y = w0 / S, so = w0 - y * S;
-            const int k1 = nptr[y + 1];
-#pragma unroll
-            for (int r = 0; r < NN_R; r++) {
-                m[r] = make_float2(0.f, 0.f);
-                if (layer == 0) {
-                    const TX xv = x[w0 + r];
-                    in[r] = make_float2((float)xv.x * sWin[tt.x][lane], (float)xv.y * sWin[tt.x][lane]);
-                } else {
-                    in[r] = Hin[(w0 + r) * NN_C + lane];
-                }
-            }
-            for (int k = nptr[y]; k < k1; k++) {
-                const long long j = nbr[k], wj = j * S + so;
-                if (layer == 0) {
-                    const float wv = sWin[atype[j]][lane];
-#pragma unroll
-                    for (int r = 0; r < NN_R; r++) {
-                        const TX xj = x[wj + r];
-                        m[r].x += (float)xj.x * wv;
-                        m[r].y += (float)xj.y * wv;
-                    }
-                } else {
-#pragma unroll
-                    for (int r = 0; r < NN_R; r++) {
-                        const float2 hj = Hin[(wj + r) * NN_C + lane];
-                        m[r].x += hj.x;
-                        m[r].y += hj.y;
-                    }
-                }
-            }
-            const float idg = inv_deg[y];
-#pragma unroll
-            for (int r = 0; r < NN_R; r++) { m[r].x *= idg; m[r].y *= idg; }
-        } else {
-#pragma unroll
-            for (int r = 0; r < NN_R; r++) {
-                in[r] = m[r] = make_float2(0.f, 0.f);
-                const long long w = w0 + r;
-                if (w >= total) continue;
-                const long long y = w / S;
-                const int s = (int)(w % S);
-                if (layer == 0) {
-                    const TX xv = x[w];
-                    const float wv = sWin[atype[y]][lane];
-                    in[r] = make_float2((float)xv.x * wv, (float)xv.y * wv);
-                } else {
-                    in[r] = Hin[w * NN_C + lane];
-                }
-                for (int k = nptr[y]; k < nptr[y + 1]; k++) {
-                    const long long j = nbr[k];
-                    if (layer == 0) {
-                        const TX xj = x[j * S + s];
-                        const float wv = sWin[atype[j]][lane];
-                        m[r].x += (float)xj.x * wv;
-                        m[r].y += (float)xj.y * wv;
-                    } else {
-                        const float2 hj = Hin[(j * S + s) * NN_C + lane];
-                        m[r].x += hj.x;
-                        m[r].y += hj.y;
-                    }
-                }
-                const float idg = inv_deg[y];
-                m[r].x *= idg; m[r].y *= idg;
-            }
-        }
+        tile_gather<TX>(w0, total, S, layer, tt.x, lane, sWin, nptr, nbr, inv_deg, atype, x, Hin, in, m);
         __syncwarp();                        // the previous tile's values are consumed
 #pragma unroll
         for (int r = 0; r < NN_R; r++) sA[wl][r][lane] = make_float4(in[r].x, in[r].y, m[r].x, m[r].y);
@@ -532,7 +541,6 @@ __global__ void __launch_bounds__(NN_T) mpnn_layer_kernel(long long na, int S, i
             const long long w = w0 + r;
             if (w >= total) break;
             if (Hout) Hout[w * NN_C + lane] = o[r];
-            if (Mout) Mout[w * NN_C + lane] = m[r];
             if (za) {
                 const float wo = sWout[atype[w / S]][lane];
                 float zr = o[r].x * wo, zi = o[r].y * wo;
@@ -755,8 +763,8 @@ int mpnn_forward_tc(const emfem_aux_s* a, int S, const float* P, const TX* x, fl
     return check_cuda(cudaGetLastError(), "mpnn_layer_tc_kernel");
 }
 
-// Hstore non-null: every layer's output and, after them, every layer's m are kept (training); else layers alternate H0/H1 and the
-// last layer writes only za.
+// Hstore non-null: every layer's output is kept (training); else layers alternate H0/H1 and the last layer writes
+// only za.
 template <typename TX>
 int mpnn_forward(const emfem_aux_s* a, int S, const float* P, const TX* x, float2* H0, float2* H1, float2* Hstore,
                  TX* za, cudaStream_t s) {
@@ -768,7 +776,6 @@ int mpnn_forward(const emfem_aux_s* a, int S, const float* P, const TX* x, float
         bool last = l == NN_L - 1;
         mpnn_layer_kernel<TX><<<grid, NN_T, 0, s>>>(na, S, l, P, a->inc_ptr, a->inc, a->inv_deg, a->atype, x, hin,
                                                   (last && !Hstore) ? nullptr : hout,
-                                                  Hstore ? Hstore + (size_t)(NN_L + l) * na * S * NN_C : nullptr,
                                                   last ? za : nullptr);
         hin = hout;
     }
@@ -783,6 +790,26 @@ int mpnn_forward(const emfem_aux_s* a, int S, const float* P, const TX* x, float
 // dIn gives dw_in.  Weight gradients: each of WG_BLOCKS blocks sums a fixed contiguous range of
 // rows into one partial row, then the partial rows are added in block order.
 constexpr int WG_BLOCKS = 296;
+
+// m of every row of a layer, formed again for its weight gradients (the forward keeps the layers' outputs only)
+template <typename TX>
+__global__ void __launch_bounds__(NN_T) mpnn_mean_kernel(long long na, int S, int layer, const float* __restrict__ P,
+                                                         const int* __restrict__ nptr, const int* __restrict__ nbr,
+                                                         const float* __restrict__ inv_deg, const uint8_t* __restrict__ atype,
+                                                         const TX* __restrict__ x, const float2* __restrict__ Hin,
+                                                         float2* __restrict__ M) {
+    __shared__ float sWin[2][NN_C];
+    for (int k = threadIdx.x; k < 2 * NN_C; k += NN_T) sWin[k / NN_C][k % NN_C] = P[nn_off_win() + k];
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const long long total = na * S, w0 = ((long long)blockIdx.x * (NN_T / 32) + (threadIdx.x >> 5)) * NN_R;
+    if (w0 >= total) return;
+    float2 in[NN_R], m[NN_R];
+    tile_gather<TX>(w0, total, S, layer, atype[w0 / S], lane, sWin, nptr, nbr, inv_deg, atype, x, Hin, in, m);
+#pragma unroll
+    for (int r = 0; r < NN_R; r++)
+        if (w0 + r < total) M[(w0 + r) * NN_C + lane] = m[r];
+}
 
 // dM_y = inv_deg_y U[t_y] dOut_y and the local part of dIn_y, W[t_y] dOut_y, tile by tile as the forward layer
 __global__ void __launch_bounds__(NN_T) mpnn_bwd_local_kernel(long long na, int S, int layer, const float* __restrict__ P,
@@ -1345,7 +1372,7 @@ int emfem_mpnn_nparams(void) { return EMFEM_MPNN_NPARAMS; }
 int emfem_mpnn_workspace_floats(emfem_aux a, int nsys, int64_t* activation_floats, int64_t* scratch_floats) {
     EMFEM_REQUIRE(a && nsys >= 1, "emfem_mpnn_workspace_floats: bad argument");
     int64_t act = (int64_t)a->na * nsys * NN_C * 2;
-    if (activation_floats) *activation_floats = 2 * NN_L * act;      // every layer's output and neighbour mean
+    if (activation_floats) *activation_floats = NN_L * act;
     if (scratch_floats) *scratch_floats = 3 * act + (int64_t)WG_BLOCKS * 4 * NN_C * NN_C;
     return EMFEM_OK;
 }
@@ -1382,8 +1409,10 @@ int emfem_mpnn_backward(emfem_aux a, int nsys, const float* params, const void* 
     partial_sum_kernel<<<2 * NN_C / 32, AB, 0, s>>>(WG_BLOCKS, 4 * NN_C, 2 * NN_C, partial + 2 * NN_C, grad + nn_off_wout());
     for (int l = NN_L - 1; l >= 0; l--) {
         const float2* Hin = l > 0 ? A + (size_t)(l - 1) * actn : nullptr;
+        mpnn_mean_kernel<float2><<<grid_for(rows, NN_R * (NN_T / 32)), NN_T, 0, s>>>(na, nsys, l, params, a->inc_ptr, a->inc,
+                                                                                     a->inv_deg, a->atype, (const float2*)x, Hin, dM);
         mpnn_bwd_wgrad_kernel<float2><<<WG_BLOCKS, AB, 0, s>>>(na, a->nn, nsys, l, params, a->atype, (const float2*)x, Hin,
-                                                               A + (size_t)(NN_L + l) * actn, dOut, partial);
+                                                               dM, dOut, partial);
         partial_sum_kernel<<<4 * NN_C * NN_C / 32, AB, 0, s>>>(WG_BLOCKS, 4 * NN_C * NN_C, 4 * NN_C * NN_C, partial,
                                                                grad + nn_off_W(l));
         mpnn_bwd_local_kernel<<<tile_grid(rows), NN_T, 0, s>>>(na, nsys, l, params, a->inv_deg, a->atype, dOut, dM, dIn);

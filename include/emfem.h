@@ -344,7 +344,7 @@ int emfem_aux_prolong(emfem_aux aux, int nsys, const void *za, const uint8_t *fr
  *   H_0 = x w_in[t];  H_{l+1,y} = H_{l,y} W_l[t_y] + (1/|N(y)|) sum_{j in N(y)} H_{l,j} U_l[t_y];
  *   za_y = x_y + H_{4,y} . w_out[t_y]           (linear in x, so M stays a fixed linear operator)
  * params (float): w_in[2][32] | (W_l[2][32][32] | U_l[2][32][32]) for l = 0..3 | w_out[2][32].
- * workspace_floats: sizes of act (forward output: all layers and their neighbour means) and scratch (backward).
+ * workspace_floats: sizes of act (forward output, all layers) and scratch (backward).
  * forward: za and act.  backward: grad (EMFEM_MPNN_NPARAMS floats, overwritten) of a real loss L
  *   given dza = dL/dRe(za) + i dL/dIm(za) (c64), from the act of the forward of the same x; the
  *   sums over nodes are fixed-order.  adam_step: one Adam update (bias-corrected, L2 weight decay

@@ -2,6 +2,8 @@
 gradient against the oracle's fit of the reference basis, the aux operator diagonals against SciPy,
 network gradients against the float64 oracle, the aux-preconditioned solve against the reference's
 SuperLU solution, and what training gains."""
+import ctypes
+
 import numpy as np
 import pytest
 import scipy.sparse as sp
@@ -9,6 +11,7 @@ import torch
 
 from oracle import auxspace as oa
 from emerge_b200 import problems
+from emerge_b200._lib import check, lib, ptr
 from emerge_b200.auxspace import AuxSpace, Network, make_pairs, train
 from emerge_b200.mesh import TetMesh, box_tet_mesh
 from emerge_b200.nedelec2 import Nedelec2
@@ -200,3 +203,26 @@ def test_training_reduces_correction_loss_and_learned_solve_converges(guide, gol
     assert (plain.status == 0).all()
     assert aux_j.iters.max() * 4 < plain.iters.max(), (aux_j.iters, plain.iters)
     sw.set_network(None)
+
+
+def test_training_activations_take_one_output_per_layer(cuda):
+    """act is (layers, n_aux, nsys, 32) complex64, as it was before the layers ran on tiles of rows: a caller that
+    sized it so is not overrun, and the backward pass needs no more."""
+    aux = AuxSpace(problems.waveguide(nx=4, ny=2, nz=5).mesh)
+    net = Network(aux, seed=3, init="random")
+    nsys, C, L = 3, 32, 4
+    a, s = ctypes.c_int64(), ctypes.c_int64()
+    check(lib().emfem_mpnn_workspace_floats(aux.handle, nsys, ctypes.byref(a), ctypes.byref(s)), "workspace")
+    assert a.value == L * aux.n_aux * nsys * C * 2
+    g = torch.Generator().manual_seed(5)
+    x, dz = (torch.complex(torch.randn(aux.n_aux, nsys, generator=g), torch.randn(aux.n_aux, nsys, generator=g)).to(cuda)
+             for _ in range(2))
+    act = torch.full((2 * a.value,), float("nan"), dtype=torch.float32, device=cuda)
+    scratch = torch.empty(s.value, dtype=torch.float32, device=cuda)
+    za, grad = torch.empty_like(x), torch.empty_like(net.params)
+    check(lib().emfem_mpnn_forward(aux.handle, nsys, ptr(net.params), ptr(x), ptr(act), ptr(za)), "forward")
+    check(lib().emfem_mpnn_backward(aux.handle, nsys, ptr(net.params), ptr(x), ptr(act), ptr(dz), ptr(grad), ptr(scratch)),
+          "backward")
+    assert torch.isfinite(act[:a.value]).all() and torch.isnan(act[a.value:]).all()
+    assert torch.equal(net.forward(x), za)
+    assert torch.equal(net.backward(dz).reshape(-1), grad.reshape(-1))
