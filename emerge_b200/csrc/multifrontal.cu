@@ -1153,6 +1153,7 @@ struct emfem_mf_s {
     int S = 0;
     float2 *sw = nullptr, *sy = nullptr, *sx = nullptr;
     double flops = 0.0;
+    bool unowned = false;                         // a front's boundary holds DOFs that no front eliminates (zero there)
     bool factored = false;
     bool lists = false;                           // assembly lists present (given or built)
     std::vector<int> h_pos, h_fpos;               // host copies used to build the lists on the device
@@ -1270,6 +1271,8 @@ int mf_apply(emfem_mf_s* m, int S, const double2* r, double2* x, cudaStream_t s)
         set_error("emfem_mf: %d right-hand sides exceed the reserved %d (emfem_mf_reserve)", S, m->S);
         return EMFEM_ERR_INVALID_ARG;
     }
+    // the solution of every eliminated DOF is written before it is read; a boundary DOF that none eliminates reads zero
+    if (m->unowned) EMFEM_CUDA(cudaMemsetAsync(m->sx, 0, sizeof(float2) * m->n * S, s));
     EMFEM_TRY(S >= 16 ? mf_sweep_tree<16>(m, S, r, s) : S > 4 ? mf_sweep_tree<8>(m, S, r, s)
               : S > 2 ? mf_sweep_tree<4>(m, S, r, s) : S == 2 ? mf_sweep_tree<2>(m, S, r, s) : mf_sweep_tree<1>(m, S, r, s));
     mf_out_kernel<<<grid_for(m->n * S, 256), 256, 0, s>>>(m->n, S, m->d_free, m->d_scale, m->sx, x);
@@ -1474,6 +1477,11 @@ int emfem_mf_create(emfem_handle h, int64_t n, int n_fronts, const int32_t* e, c
             int d = fdof[fdof_ptr[v] + i];
             if (d < 0 || d >= n) { delete m; set_error("emfem_mf_create: DOF %d out of range", d); return EMFEM_ERR_INVALID_ARG; }
             freed[d] = 1;
+        }
+    for (int v = 0; v < n_fronts && !m->unowned; v++)
+        for (int i = e[v]; i < e[v] + b[v]; i++) {
+            const int d = fdof[fdof_ptr[v] + i];
+            if (d < 0 || d >= n || !freed[d]) { m->unowned = true; break; }
         }
     long long nasm = asm_ptr ? asm_ptr[n_fronts] : 0;
     m->lists = asm_ptr != nullptr;

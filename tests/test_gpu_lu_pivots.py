@@ -11,15 +11,16 @@ from emerge_b200._lib import Handle, check, lib, ptr
 pytestmark = pytest.mark.gpu
 
 
-def _block_diagonal(nf, e, K):
-    """LU handle of nf unconnected fronts of e own DOFs, front v holding the dense K[v]."""
+def _fronts(nf, e, b, K):
+    """LU handle of nf unconnected fronts of e own and b boundary DOFs, front v holding the dense K[v]."""
     i32 = lambda a: np.ascontiguousarray(a, np.int32)
+    n = e + b
     ptrs = np.arange(nf + 1, dtype=np.int64)
-    slot = i32(np.arange(nf * e * e).reshape(nf, e, e).transpose(0, 2, 1))        # off = row + column * e
-    arrs = [i32(np.full(nf, e)), i32(np.zeros(nf)), i32(np.full(nf, -1)), i32(np.zeros(nf)), ptrs * e,
-            i32(np.arange(nf * e)), i32([0]), ptrs * e * e, slot, i32(np.tile(np.arange(e * e), nf))]
+    slot = i32(np.arange(nf * n * n).reshape(nf, n, n).transpose(0, 2, 1))        # off = row + column * n
+    arrs = [i32(np.full(nf, e)), i32(np.full(nf, b)), i32(np.full(nf, -1)), i32(np.zeros(nf)), ptrs * n,
+            i32(np.arange(nf * n)), i32(np.zeros(max(1, nf * b))), ptrs * n * n, slot, i32(np.tile(np.arange(n * n), nf))]
     m = ctypes.c_void_p()
-    check(lib().emfem_mf_create(Handle.get(K.device).h, nf * e, nf, *[a.ctypes.data_as(ctypes.c_void_p) for a in arrs],
+    check(lib().emfem_mf_create(Handle.get(K.device).h, nf * n, nf, *[a.ctypes.data_as(ctypes.c_void_p) for a in arrs],
                                 ctypes.byref(m)), "emfem_mf_create")
     return m
 
@@ -47,7 +48,7 @@ def test_raised_pivots_are_the_same_every_time(cuda, bits, tail):
     Kd = torch.from_numpy(K).to(cuda)
     b = rng.standard_normal((nf, e)) + 1j * rng.standard_normal((nf, e))
     bd = torch.from_numpy(b.reshape(-1, 1)).to(cuda)
-    m = _block_diagonal(nf, e, Kd)
+    m = _fronts(nf, e, 0, Kd)
     try:
         check(lib().emfem_mf_set_precision(m, bits), "emfem_mf_set_precision")
         check(lib().emfem_mf_reserve(m, 1), "emfem_mf_reserve")
@@ -65,6 +66,31 @@ def test_raised_pivots_are_the_same_every_time(cuda, bits, tail):
             ref = np.linalg.solve(K[v][np.ix_(live[v], live[v])], b[v, live[v]])
             # factors are complex64 in both precisions; the blocks' condition is below 3
             assert np.linalg.norm(x[v, live[v]] - ref) <= 32 * 6e-8 * 3 * np.linalg.norm(ref)
+    finally:
+        torch.cuda.synchronize()
+        lib().emfem_mf_destroy(m)
+
+
+def test_boundary_dofs_that_no_front_eliminates_are_zero(cuda):
+    """Fronts with a boundary and no parent: the solve takes the boundary as zero, also after solves of other widths."""
+    rng = np.random.default_rng(1)
+    nf, e, nb = 3, 70, 5
+    n = e + nb
+    K = np.eye(n) + 0.2 * (rng.standard_normal((nf, n, n)) + 1j * rng.standard_normal((nf, n, n))) / n ** 0.5
+    Kd = torch.from_numpy(K).to(cuda)
+    m = _fronts(nf, e, nb, Kd)
+    try:
+        check(lib().emfem_mf_factor(m, ptr(Kd), None), "emfem_mf_factor")
+        for nrhs in (16, 3, 1):
+            b = rng.standard_normal((nf, n, nrhs)) + 1j * rng.standard_normal((nf, n, nrhs))
+            bd = torch.from_numpy(b.reshape(nf * n, nrhs)).to(cuda)
+            xd = torch.empty_like(bd)
+            check(lib().emfem_mf_solve(m, nrhs, ptr(bd), ptr(xd)), "emfem_mf_solve")
+            x = xd.cpu().numpy().reshape(nf, n, nrhs)
+            assert (x[:, e:] == 0).all()
+            ref = np.linalg.solve(K[:, :e, :e], b[:, :e])
+            # complex64 factors of a matrix with condition below 10
+            assert np.linalg.norm(x[:, :e] - ref) <= n * 6e-8 * 10 * np.linalg.norm(ref)
     finally:
         torch.cuda.synchronize()
         lib().emfem_mf_destroy(m)
