@@ -92,6 +92,15 @@ class DeviceMesh:
         h.raise_on_device_status("emfem_mesh_check")
 
 
+# Revision of the assembly kernel variants: raised when their code changes, so that a tuning kept on disk never
+# chooses among kernels that it did not time.
+ASSEMBLY_KERNELS = 2
+
+
+def tune_key(gpu: str, n_tets: int, nnz: int) -> str:
+    return f"{gpu}|assemble|{n_tets}|{nnz}|kernels{ASSEMBLY_KERNELS}"
+
+
 class CsrPlan:
     """Device symbolic phase (``emfem_plan_*``): the CSR pattern of E/B and the row-owner map used
     by the fused assembly.  Pattern = union of all tet DOF pairs, sorted, zeros kept."""
@@ -156,12 +165,10 @@ class CsrPlan:
         """Autotune the assembly kernel variant (chunk capacity x CTA size) for this mesh on this GPU.
 
         Times every available variant with CUDA events on the current stream (one warm-up launch,
-        then ``reps`` launches) and keeps the fastest.  Results are cached as JSON keyed by GPU name
-        and mesh size (``~/.cache/emerge_b200/autotune.json`` unless ``cache`` is given)."""
+        then ``reps`` launches) and keeps the fastest.  Results are cached as JSON keyed by GPU name,
+        mesh size and the kernels' revision (``~/.cache/emerge_b200/autotune.json`` unless ``cache`` is given)."""
         path = cache or os.path.join(os.path.expanduser("~"), ".cache", "emerge_b200", "autotune.json")
-        nv = ctypes.c_int()
-        check(lib().emfem_plan_variants(self._p, ctypes.byref(nv), None), "emfem_plan_variants")
-        key = f"{torch.cuda.get_device_name(self.device)}|assemble|{self.dmesh.n_tets}|{self.nnz}|{nv.value}"
+        key = tune_key(torch.cuda.get_device_name(self.device), self.dmesh.n_tets, self.nnz)
         try:
             table = json.load(open(path))
         except (OSError, ValueError):

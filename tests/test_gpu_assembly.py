@@ -129,3 +129,21 @@ def test_drop_in_results_never_alias(cuda, small):
     np.testing.assert_array_equal(view, B1.data[5:9])
     assert not np.shares_memory(E1.data, E2.data) and not np.shares_memory(B1.data, B2.data)
     assert np.abs(B2.data - 2.0 * B1.data).max() <= 1e-12 * np.abs(B1.data).max()   # B is linear in er
+
+
+def test_tuning_kept_from_other_kernels_is_not_used(cuda, tmp_path):
+    """The tuning file is keyed by the kernels' revision: an entry without it chooses nothing."""
+    import json
+    P = problems.waveguide(nx=3, ny=2, nz=4)
+    dm = assembly.DeviceMesh(P.mesh, P.field)
+    plan = assembly.CsrPlan(dm)
+    er, ur = torch.from_numpy(P.er).to(cuda), torch.from_numpy(P.ur).to(cuda)
+    gpu = torch.cuda.get_device_name(plan.device)
+    path = tmp_path / "autotune.json"
+    old = f"{gpu}|assemble|{dm.n_tets}|{plan.nnz}|13"
+    path.write_text(json.dumps({old: {"variant": 6, "ms": {}}}))
+    entry = plan.tune(er, ur, reps=1, cache=str(path))
+    table = json.loads(path.read_text())
+    assert table[old]["variant"] == 6 and len(entry["ms"]) > 1
+    assert table[assembly.tune_key(gpu, dm.n_tets, plan.nnz)]["variant"] == entry["variant"] == plan.variant
+    assert plan.tune(er, ur, reps=1, cache=str(path)) == table[assembly.tune_key(gpu, dm.n_tets, plan.nnz)]
