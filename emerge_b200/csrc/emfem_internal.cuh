@@ -114,6 +114,8 @@ void* aux_dinv_buffer(const emfem_aux_s* a, int S);
 // Multifrontal LU (multifrontal.cu); the Krylov solver applies it as a right preconditioner.
 struct emfem_mf_s;
 namespace emfem {
-int mf_apply(emfem_mf_s* m, int S, const double2* r, double2* x, cudaStream_t s);
+// Columns of an (n, ld) batch that an LU application takes: all of them where count is ld, else m[0 .. count).
+struct MfCols { int ld, count; signed char m[64]; };
+int mf_apply(emfem_mf_s* m, const MfCols& cols, const double2* r, double2* x, cudaStream_t s);
 int mf_reserved(const emfem_mf_s* m);
 }  // namespace emfem

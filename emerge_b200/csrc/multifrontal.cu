@@ -779,7 +779,7 @@ static void mf_chain(void (*kernel)(P...), dim3 grid, cudaStream_t s, A... args)
 // w (the front's rows, S per row): own rows from the right-hand side, plus both children's update rows
 __global__ void mf_fwd_gather_kernel(const int* __restrict__ lst, const FrontMeta* __restrict__ fm, int S,
                                      const int* __restrict__ fdof, const double* __restrict__ scale,
-                                     const int* __restrict__ cmap, long long rows, const double2* __restrict__ rhs,
+                                     const int* __restrict__ cmap, long long rows, MfCols cols, const double2* __restrict__ rhs,
                                      float2* __restrict__ w) {
     mf_chain_start();
     const FrontMeta& f = fm[lst[blockIdx.y]];
@@ -790,7 +790,7 @@ __global__ void mf_fwd_gather_kernel(const int* __restrict__ lst, const FrontMet
     float2 v = make_float2(0.f, 0.f);
     if (i < f.e) {
         const int d = fdof[f.fdof + i];
-        const double2 r = rhs[(long long)d * S + s];
+        const double2 r = rhs[(long long)d * cols.ld + (cols.count == cols.ld ? s : cols.m[s])];
         const double sc = scale[d];
         v = make_float2((float)(r.x * sc), (float)(r.y * sc));
     }
@@ -1105,13 +1105,15 @@ __global__ void mf_fill_kernel(long long n, double v, double* __restrict__ x) {
 
 // x = D^-1/2 (scaled solution), zero outside every front
 __global__ void mf_out_kernel(long long n, int S, const uint8_t* __restrict__ freed, const double* __restrict__ scale,
-                              const float2* __restrict__ xs, double2* __restrict__ x) {
+                              const float2* __restrict__ xs, MfCols cols, double2* __restrict__ x) {
     long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= n * S) return;
-    const bool in = freed[g / S];
+    const long long i = g / S;
+    const int s = (int)(g % S);
+    const bool in = freed[i];
     const float2 v = in ? xs[g] : make_float2(0.f, 0.f);
-    const double sc = scale[g / S];
-    x[g] = in ? make_double2((double)v.x * sc, (double)v.y * sc) : make_double2(0.0, 0.0);
+    const double sc = scale[i];
+    x[i * cols.ld + (cols.count == cols.ld ? s : cols.m[s])] = in ? make_double2((double)v.x * sc, (double)v.y * sc) : make_double2(0.0, 0.0);
 }
 
 }  // namespace emfem
@@ -1195,7 +1197,8 @@ static bool mf_wide_tiles(long long rows, int ny, unsigned sz) { return (rows + 
 
 // Forward and backward pass over the tree, NS right-hand sides per CTA.
 template <int NS>
-static int mf_sweep_tree(emfem_mf_s* m, int S, const double2* r, cudaStream_t s) {
+static int mf_sweep_tree(emfem_mf_s* m, const MfCols& cols, const double2* r, cudaStream_t s) {
+    const int S = cols.count;
     const int nl = (int)m->levels.size();
     constexpr int NT = NS < 8 ? NS : 8;          // right-hand sides per CTA of the block-inverse products (48 KB of staging)
     const unsigned sz = (unsigned)((S + NS - 1) / NS), szt = (unsigned)((S + NT - 1) / NT);
@@ -1210,9 +1213,9 @@ static int mf_sweep_tree(emfem_mf_s* m, int S, const double2* r, cudaStream_t s)
             // the first launch waits for all before it: the right-hand side and, after a factorization, the factors
             const dim3 gg(nblk(maxn * S, 256), ny);
             if (first)
-                mf_fwd_gather_kernel<<<gg, 256, 0, s>>>(lst, m->d_meta, S, m->d_fdof, m->d_scale, m->d_cmap, m->wv_n, r, m->sw);
+                mf_fwd_gather_kernel<<<gg, 256, 0, s>>>(lst, m->d_meta, S, m->d_fdof, m->d_scale, m->d_cmap, m->wv_n, cols, r, m->sw);
             else
-                mf_chain(mf_fwd_gather_kernel, gg, s, lst, m->d_meta, S, m->d_fdof, m->d_scale, m->d_cmap, m->wv_n, r, m->sw);
+                mf_chain(mf_fwd_gather_kernel, gg, s, lst, m->d_meta, S, m->d_fdof, m->d_scale, m->d_cmap, m->wv_n, cols, r, m->sw);
             first = false;
             for (int k0 = 0; k0 < maxe; k0 += MF_SB) {
                 const unsigned nt = nblk(std::min(MF_SB, maxe - k0), MF_NB);
@@ -1264,8 +1267,10 @@ static int mf_sweep_tree(emfem_mf_s* m, int S, const double2* r, cudaStream_t s)
     return EMFEM_OK;
 }
 
-// M^-1 r for S right-hand sides (n, S) FP64 DOF-major -> x (FP64), zero on DOFs outside every front.
-int mf_apply(emfem_mf_s* m, int S, const double2* r, double2* x, cudaStream_t s) {
+// M^-1 r for columns of an (n, ld) FP64 batch, DOF-major -> the same columns of x (FP64), zero on DOFs outside every
+// front.  The width that the columns are taken at changes no sum.
+int mf_apply(emfem_mf_s* m, const MfCols& cols, const double2* r, double2* x, cudaStream_t s) {
+    const int S = cols.count;
     EMFEM_REQUIRE(m->factored, "emfem_mf: solve before a successful factorization");
     if (m->S < S) {
         set_error("emfem_mf: %d right-hand sides exceed the reserved %d (emfem_mf_reserve)", S, m->S);
@@ -1273,9 +1278,9 @@ int mf_apply(emfem_mf_s* m, int S, const double2* r, double2* x, cudaStream_t s)
     }
     // the solution of every eliminated DOF is written before it is read; a boundary DOF that none eliminates reads zero
     if (m->unowned) EMFEM_CUDA(cudaMemsetAsync(m->sx, 0, sizeof(float2) * m->n * S, s));
-    EMFEM_TRY(S >= 16 ? mf_sweep_tree<16>(m, S, r, s) : S > 4 ? mf_sweep_tree<8>(m, S, r, s)
-              : S > 2 ? mf_sweep_tree<4>(m, S, r, s) : S == 2 ? mf_sweep_tree<2>(m, S, r, s) : mf_sweep_tree<1>(m, S, r, s));
-    mf_out_kernel<<<grid_for(m->n * S, 256), 256, 0, s>>>(m->n, S, m->d_free, m->d_scale, m->sx, x);
+    EMFEM_TRY(S >= 16 ? mf_sweep_tree<16>(m, cols, r, s) : S > 4 ? mf_sweep_tree<8>(m, cols, r, s)
+              : S > 2 ? mf_sweep_tree<4>(m, cols, r, s) : S == 2 ? mf_sweep_tree<2>(m, cols, r, s) : mf_sweep_tree<1>(m, cols, r, s));
+    mf_out_kernel<<<grid_for(m->n * S, 256), 256, 0, s>>>(m->n, S, m->d_free, m->d_scale, m->sx, cols, x);
     EMFEM_LAUNCH("mf_out_kernel");
     return EMFEM_OK;
 }
@@ -1704,7 +1709,7 @@ int emfem_mf_reserve(emfem_mf m, int nrhs) {
 int emfem_mf_solve(emfem_mf m, int nrhs, const void* b, void* x) {
     EMFEM_REQUIRE(m && b && x && nrhs >= 1, "emfem_mf_solve: bad argument");
     EMFEM_TRY(mf_reserve(m, nrhs));
-    return mf_apply(m, nrhs, (const double2*)b, (double2*)x, m->h->stream);
+    return mf_apply(m, MfCols{nrhs, nrhs, {}}, (const double2*)b, (double2*)x, m->h->stream);
 }
 
 int emfem_mf_destroy(emfem_mf m) {
