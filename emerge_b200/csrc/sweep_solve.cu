@@ -1314,7 +1314,8 @@ struct Krylov {
     // alone and not on how far the replay in flight has come.
     int run(int chunk) {
         const bool narrowing = xfull && method == 1 && G == 1;
-        const bool ahead = mf == nullptr;      // an LU application does not skip stopped systems
+        // (an LU application and the network do not skip stopped systems: a replay for nothing costs more than the wait)
+        const bool ahead = !mf && precond != 4;
         if (narrowing) {
             S0 = S;
             col.resize(S);
