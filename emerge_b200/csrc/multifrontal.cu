@@ -10,10 +10,11 @@
 //      precision) and the Schur complements of its children (extend-add, one child slot after the other:
 //      no atomics);
 //   2. the first e columns of every front are eliminated in steps of 32: LU with partial pivoting inside
-//      the 32 x 32 diagonal block (diag_kernel, one warp per front, also forming the explicit inverses
-//      of its L and U), the block row (row swaps + L^-1) and block column (U^-1) of the panel
-//      (panel_kernel), and the rank-32 update of the trailing matrix (trail_kernel: 64 x 64 tiles,
-//      4 x 4 complex register tiles per thread), every kernel batched over the level's fronts;
+//      the 32 x 32 diagonal block (diag_kernel, one CTA of eight warps per front, also forming the explicit
+//      inverses of its L and U), the block row (row swaps + L^-1) and block column (U^-1) of the panel
+//      (panel_kernel), the update of the rest of the 128-column outer block (strip_kernel), and once per outer
+//      block the rank-128 update of the trailing matrix (trail_kernel: tiles of 128 x 64 or 64 x 64,
+//      8 x 4 or 4 x 4 complex accumulators per thread), every kernel batched over the level's fronts;
 //   3. the factor columns, the U block row and the Schur complement are copied out of the level
 //      workspace (compact_kernel): factors to the factor store (rounded to complex64), the Schur
 //      complement to the update store (front precision) until the parent's level consumes it;
@@ -21,12 +22,12 @@
 //      that the solves have no 32-step chains.  The inverses are formed, stored and applied in FP64: their
 //      entries grow (rows are not exchanged across steps), and products with them cancel.
 // Pivoting stays inside each 32-row diagonal block (rows are never exchanged across blocks), so row swaps
-// touch only the block row; the solves apply them step by step.  A pivot smaller than 1e-6 of its block's
+// touch only the block row; the step's inverse of L holds them for the solves.  A pivot smaller than 1e-6 of its block's
 // largest entry is raised to that floor and counted: the factorization is a preconditioner under an FP64
 // Krylov iteration, which removes such perturbations.
 //
-// Solves (M^-1 r for S right-hand sides, FP64 in and out, FP32 inside, scaled by D^-1/2 on the way in
-// and out) run the same tree: forward in level order (gather of the right-hand side and the children's
+// Solves (M^-1 r for S right-hand sides, FP64 in and out, FP32 inside but for the products with the block
+// inverses, scaled by D^-1/2 on the way in and out) run the same tree: forward in level order (gather of the right-hand side and the children's
 // update rows, then per 256 own rows the product with the block inverse and the update of the rows below),
 // backward in reverse (U12 product with the solved boundary, then per 256 own rows, from the last).
 #include "emfem_internal.cuh"
@@ -904,7 +905,7 @@ __device__ __forceinline__ void mf_product(MfProdSmem<NS>& sm, int c0, int c1, i
 // Products with the block inverses, FP64 inside (inverse entries and sums; x and the result are complex64): 32 rows per
 // CTA, a warp takes every eighth of the nc columns, 16 of them in flight.  M: entry (the CTA's first row, first
 // column), XOf(c) points at column c's x values, Out(row of the tile, right-hand side, value).  Latency bounds it at
-// the few-front levels: the FP64 multiply-adds of a whole application take 60 us of 2.4 ms at 24 576 tets.
+// the few-front levels: the FP64 multiply-adds of an application to 8 columns take 60 us at 24 576 tets.
 template <int NS>
 struct MfTriSmem {
     double2 x[MF_SB][NS];

@@ -62,8 +62,7 @@ EMFEM_HD int pair_index(int i, int j) {
     return lo == 0 ? hi - 1 : (lo == 1 ? hi + 1 : 5);
 }
 
-// Per-tet invariants.  The same struct is used in registers and, field by field, in the SoA
-// device buffer (see TetInvSoA).
+// Per-tet invariants of the element kernel (tet_element_kernel), in the tet's own vertex order.
 constexpr int INV_P = 0;          // 16 complex -> 32 doubles
 constexpr int INV_Q = 32;         // 36 complex -> 72 doubles
 constexpr int INV_DS = 104;       // 6 vertex-pair distances (canonical pair order)
@@ -72,7 +71,6 @@ constexpr int INV_SD = 116;       // 1/(6V)^3  (D scale: 6V from the coefficient
 constexpr int INV_SF = 117;       // 1/(6V)    (F scale)
 constexpr int INV_RANK = 118;     // vertex ranks packed as a double-encoded int (2 bits each)
 constexpr int INV_NDOUBLE = 119;
-constexpr int INV_STRIDE = 120;   // per-tet record length in the array-of-structs buffer (960 B)
 
 // Orientation of the tet's local entities from the rank (0..3) of each vertex's global id,
 // packed 2 bits per vertex (no per-thread arrays, so nothing spills to local memory).
@@ -415,19 +413,7 @@ EMFEM_HD void canon_mass(const IV& I, int sx, int sy, cd f[4]) {
 }
 
 // Volume coefficient table: vc[A*125 + B*25 + C*5 + D] = prod k_i! / (sum k_i + 3)!,
-// letters 1..4 name vertices, 0 = absent (curlcurl.py:64-92).
-EMFEM_HD void fill_volume_table(double* vc) {
-    const double fact[10] = {1, 1, 2, 6, 24, 120, 720, 5040, 40320, 362880};
-    for (int a = 0; a < 5; a++) for (int b = 0; b < 5; b++)
-    for (int c = 0; c < 5; c++) for (int d = 0; d < 5; d++) {
-        int cnt[7] = {0, 0, 0, 0, 0, 0, 0};
-        cnt[a]++; cnt[b]++; cnt[c]++; cnt[d]++;
-        double num = 1; int n = 0;
-        for (int i = 1; i < 7; i++) { num *= fact[cnt[i]]; n += cnt[i]; }
-        vc[((a * 5 + b) * 5 + c) * 5 + d] = num / fact[n + 3];
-    }
-}
-
+// letters 1..4 name vertices, 0 = absent (curlcurl.py:64-92; volume_coeff_closed).
 struct VTab {
     const double* vc;
     EMFEM_HD double v(int A, int B) const { return vc[(A * 5 + B) * 25]; }

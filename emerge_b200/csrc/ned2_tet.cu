@@ -584,8 +584,8 @@ __global__ void __launch_bounds__(NT, MINB) assemble_chunk_kernel(
     }
 }
 
-// Kernel variants: chunk capacity CH incidences, NT threads, min resident CTAs, invariants staged in
-// shared memory or read through L1.  The plan times them and keeps the fastest.
+// Kernel variants: chunk capacity CH incidences, NT threads, min resident CTAs, records staged in shared
+// memory or read through L1.  A plan takes the default below; CsrPlan.tune times them all and sets the fastest.
 struct AsmVariant { int ch; int nt; size_t smem; };
 #define EMFEM_ASM_VARIANTS(X)              \
     X(0, 32, 160, 5, true, true)           \

@@ -14,9 +14,9 @@
 // (ASM/curlcurl.py:348-357, e.g. VBCDE = VOLUME_COEFF_CACHE[B,C,D,F]), about 0.5 % of ||B||, and
 // COCG stalls near 1e-5 on it.  The default is therefore right-preconditioned BiCGStab
 // (van der Vorst 1992), the general-matrix member of the same BiCG family, with the same batched
-// operator and preconditioner.  Every reduction is a fixed-order tree, so runs are
-// bit-reproducible.  Iterations run in CUDA-graph chunks with all scalars on the device; the host
-// reads only the per-system active flags between chunks.
+// operator and preconditioner.  Every reduction is a fixed-order tree and the host decides by iteration
+// counts alone, so runs are bit-reproducible.  Iterations run in CUDA-graph chunks with all scalars on
+// the device; the host reads the per-system states between chunks.
 #include "emfem_internal.cuh"
 
 #include <vector>
@@ -971,11 +971,6 @@ __global__ void add_scaled_f32_kernel(long long n, int S, const int* __restrict_
     x[g].y += sc * (double)v.y;
 }
 
-__global__ void cast_values_kernel(long long nnz, const double2* __restrict__ src, float2* __restrict__ dst) {
-    long long g = (long long)blockIdx.x * VB + threadIdx.x;
-    if (g < nnz) dst[g] = make_float2((float)src[g].x, (float)src[g].y);
-}
-
 // inner state for one refinement step: unit-norm rhs, relative tolerance `itol`, active = outer active
 __global__ void inner_init_kernel(SysState* inner, const SysState* outer, int GS, double itol) {
     int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1631,7 +1626,7 @@ static int krylov_impl(emfem_handle hd, int method, int64_t n, int64_t nnz, cons
                                               vec_pairs(S), gpair);
         STRY(check_cuda(cudaGetLastError(), "init state"));
         STRY(k.start());
-        STRY(k.run(mf ? 2 : 16));     // an LU application is ~1000 launches: short captured chunks
+        STRY(k.run(mf ? 2 : 16));     // an LU solve takes a few iterations of two applications, some 250 launches each
     } else {
         OpArgs op32 = op64;  // FP64 values, FP32 vectors (see spmv_kernel)
         Krylov<float> k;
