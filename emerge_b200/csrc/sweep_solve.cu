@@ -189,8 +189,8 @@ struct SpmvStage {
     double2 eb[HASB ? 4 : 2][GE];            // E row 0, E row 1, B row 0, B row 1
 };
 
-template <typename R, int L, int NR, bool HASB>
-__global__ void __launch_bounds__(VB, NR == 1 ? 4 : NR == 2 ? 3 : 2) spmv_kernel(
+template <typename R, int L, int NR, bool HASB, int NT>
+__global__ void __launch_bounds__(NT, NT > VB ? 1 : NR == 1 ? 4 : NR == 2 ? 3 : 2) spmv_kernel(
     OpArgs a, const typename V2<R>::T* __restrict__ x, typename V2<R>::T* __restrict__ y, double2* __restrict__ partial,
     int dotmode, const typename V2<R>::T* __restrict__ w, int ppb) {
     typedef typename V2<R>::T T;
@@ -211,7 +211,34 @@ __global__ void __launch_bounds__(VB, NR == 1 ? 4 : NR == 2 ? 3 : 2) spmv_kernel
     double c1[NV], c2[NV];
 #pragma unroll
     for (int q = 0; q < NV; q++) { c0[q] = make_double2(0.0, 0.0); c1[q] = c2[q] = 0.0; }
-    for (int pw = wl; pw < ppb; pw += VB / 32) {
+    double2 acc[2 * NR];
+    long long late = -1;                            // NT > VB: row whose dot products wait for those of warp wl - 8
+    auto dots = [&](long long row, int r0) {
+#pragma unroll
+        for (int q = 0; q < NV; q++) {
+            const long long o = row * S + s0 + (r0 + q) * L;
+            const double yr = acc[q].x, yi = acc[q].y;
+            if (dotmode == DOT_XY) {
+                const T xi = x[o];
+                const double a0 = xi.x, a1 = xi.y;
+                c0[q].x = fma(a0, yr, fma(-a1, yi, c0[q].x));
+                c0[q].y = fma(a0, yi, fma(a1, yr, c0[q].y));
+            } else if (dotmode == DOT_CONJW_Y) {
+                const T wi = w[o];
+                const double a0 = wi.x, a1 = wi.y;
+                c0[q].x = fma(a0, yr, fma(a1, yi, c0[q].x));
+                c0[q].y = fma(a0, yi, fma(-a1, yr, c0[q].y));
+            } else if (dotmode == DOT_CONJY_W_YY) {
+                const T wi = w[o];
+                const double a0 = wi.x, a1 = wi.y;
+                c0[q].x = fma(a0, yr, fma(a1, yi, c0[q].x));
+                c0[q].y = fma(a1, yr, fma(-a0, yi, c0[q].y));
+                c1[q] = fma(yr, yr, fma(yi, yi, c1[q]));
+                c2[q] = fma(a0, a0, fma(a1, a1, c2[q]));
+            }
+        }
+    };
+    for (int pw = wl; pw < ppb; pw += NT / 32) {
         const long long i = (long long)blockIdx.x * ppb + pw;
         if (i >= hh) break;
         const int base = a.pg ? a.pg[i] * S : 0;
@@ -231,7 +258,6 @@ __global__ void __launch_bounds__(VB, NR == 1 ? 4 : NR == 2 ? 3 : 2) spmv_kernel
 #pragma unroll
             for (int r = 0; r < NR; r++) k2[r] = a.k0sq[base + s0 + r * L];
         }
-        double2 acc[2 * NR];
 #pragma unroll
         for (int q = 0; q < 2 * NR; q++) acc[q] = make_double2(0.0, 0.0);
         const int nm = n0 > n1 ? n0 : n1;
@@ -354,25 +380,9 @@ __global__ void __launch_bounds__(VB, NR == 1 ? 4 : NR == 2 ? 3 : 2) spmv_kernel
                 const long long o = row * S + s0 + (r0 + q) * L;
                 const double yr = acc[q].x, yi = acc[q].y;
                 y[o] = mk2<R>((R)yr, (R)yi);
-                if (dotmode == DOT_XY) {
-                    const T xi = x[o];
-                    const double a0 = xi.x, a1 = xi.y;
-                    c0[q].x = fma(a0, yr, fma(-a1, yi, c0[q].x));
-                    c0[q].y = fma(a0, yi, fma(a1, yr, c0[q].y));
-                } else if (dotmode == DOT_CONJW_Y) {
-                    const T wi = w[o];
-                    const double a0 = wi.x, a1 = wi.y;
-                    c0[q].x = fma(a0, yr, fma(a1, yi, c0[q].x));
-                    c0[q].y = fma(a0, yi, fma(-a1, yr, c0[q].y));
-                } else if (dotmode == DOT_CONJY_W_YY) {
-                    const T wi = w[o];
-                    const double a0 = wi.x, a1 = wi.y;
-                    c0[q].x = fma(a0, yr, fma(a1, yi, c0[q].x));
-                    c0[q].y = fma(a1, yr, fma(-a0, yi, c0[q].y));
-                    c1[q] = fma(yr, yr, fma(yi, yi, c1[q]));
-                    c2[q] = fma(a0, a0, fma(a1, a1, c2[q]));
-                }
             }
+            if (NT > VB && wl >= VB / 32) late = row;
+            else dots(row, r0);
         }
     }
     if (dotmode == DOT_NONE) return;
@@ -383,15 +393,32 @@ __global__ void __launch_bounds__(VB, NR == 1 ? 4 : NR == 2 ? 3 : 2) spmv_kernel
     WarpSums* r0s = reinterpret_cast<WarpSums*>(spmv_sm);
     WarpSums* r1s = r0s + VB / 32;
     const int rr0 = NR > 1 && L == 8 && (lane & 8) ? NR / 2 : 0;
+    if (NT > VB) {
+        // warp w takes over the sums of warp w - 8, as if it had done that warp's pair before its own
+        double2* c0s = reinterpret_cast<double2*>(spmv_sm) + threadIdx.x % VB;
+        double2* c1s = c0s + NV * VB;
+        if (wl < VB / 32) {
+#pragma unroll
+            for (int q = 0; q < NV; q++) { c0s[q * VB] = c0[q]; c1s[q * VB] = make_double2(c1[q], c2[q]); }
+        }
+        __syncthreads();
+        if (wl >= VB / 32) {
+#pragma unroll
+            for (int q = 0; q < NV; q++) { c0[q] = c0s[q * VB]; c1[q] = c1s[q * VB].x; c2[q] = c1s[q * VB].y; }
+            if (late >= 0) dots(late, rr0);
+        }
+        __syncthreads();
+    }
+    const int wo = NT > VB ? wl - VB / 32 : wl;      // the warp's place in the sums (negative: taken over)
 #pragma unroll
     for (int q = 0; q < NV; q++) {
         c0[q].x += __shfl_xor_sync(0xffffffffu, c0[q].x, 16);
         c0[q].y += __shfl_xor_sync(0xffffffffu, c0[q].y, 16);
         c1[q] += __shfl_xor_sync(0xffffffffu, c1[q], 16);
         c2[q] += __shfl_xor_sync(0xffffffffu, c2[q], 16);
-        if ((NR > 1 || (lane & 15 & ~(L - 1)) == 0) && !(lane & 16)) {
-            r0s[wl][lane % L + (rr0 + q) * L] = c0[q];
-            r1s[wl][lane % L + (rr0 + q) * L] = make_double2(c1[q], c2[q]);
+        if ((NR > 1 || (lane & 15 & ~(L - 1)) == 0) && !(lane & 16) && wo >= 0) {
+            r0s[wo][lane % L + (rr0 + q) * L] = c0[q];
+            r1s[wo][lane % L + (rr0 + q) * L] = make_double2(c1[q], c2[q]);
         }
     }
     __syncthreads();
@@ -420,20 +447,24 @@ static void launch_spmv_b(const OpArgs& a, const typename V2<R>::T* x, typename 
                           const typename V2<R>::T* w, int cut, cudaStream_t s) {
     const int ppb = spmv_pairs(cut);
     dim3 grid(spmv_blocks(a.n, cut), a.S > 32 ? a.S / 32 : 1);
-#define EMFEM_SPMV(L, NR)                                                                                      \
+#define EMFEM_SPMV(L, NR, NT)                                                                                  \
     do {                                                                                                       \
-        constexpr size_t sm = sizeof(SpmvStage<R, L, NR, HASB>) * SpmvStage<R, L, NR, HASB>::DEPTH * (VB / 32);                                                  \
+        constexpr size_t sm = sizeof(SpmvStage<R, L, NR, HASB>) * SpmvStage<R, L, NR, HASB>::DEPTH * (NT / 32); \
         if (sm > 48 * 1024)                                                                                    \
-            cudaFuncSetAttribute(spmv_kernel<R, L, NR, HASB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm); \
-        spmv_kernel<R, L, NR, HASB><<<grid, VB, sm, s>>>(a, x, y, partial, dotmode, w, ppb);                   \
+            cudaFuncSetAttribute(spmv_kernel<R, L, NR, HASB, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm); \
+        spmv_kernel<R, L, NR, HASB, NT><<<grid, NT, sm, s>>>(a, x, y, partial, dotmode, w, ppb);               \
     } while (0)
+    // 16 pairs a block are two a warp; where the blocks do not fill the SMs, 16 warps take one each, with the same sums
+    // (an iteration at 32 systems, 2 774 / 4 316 DOFs: 58.4 / 60.6 us with 8 warps, 49.0 / 50.3 with 16; a thread per row
+    // and system took 51.0 / 57.2)
+    const bool small = (long long)grid.x * grid.y <= 148;
     switch (a.S) {
-    case 1: EMFEM_SPMV(1, 1); break;
-    case 2: EMFEM_SPMV(2, 1); break;
-    case 4: EMFEM_SPMV(4, 1); break;
-    case 8: EMFEM_SPMV(8, 1); break;
-    case 16: EMFEM_SPMV(8, 2); break;
-    default: EMFEM_SPMV(8, 4); break;
+    case 1: EMFEM_SPMV(1, 1, VB); break;
+    case 2: EMFEM_SPMV(2, 1, VB); break;
+    case 4: EMFEM_SPMV(4, 1, VB); break;
+    case 8: EMFEM_SPMV(8, 1, VB); break;
+    case 16: if (small) EMFEM_SPMV(8, 2, 512); else EMFEM_SPMV(8, 2, VB); break;
+    default: if (small) EMFEM_SPMV(8, 4, 512); else EMFEM_SPMV(8, 4, VB); break;
     }
 #undef EMFEM_SPMV
 }
