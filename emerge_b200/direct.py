@@ -288,7 +288,8 @@ class DeviceLU:
     forms K_f = E − k0²B + Σ_p γ_p(k0) R_p on the device (``emfem_sweep_combine``; the Robin/port entries
     summed per CSR slot) and factors its equilibrated form.  ``precision`` is the arithmetic of the
     factorization: "c64" (complex64 fronts) or "c128" (complex128 fronts and update store, twice their
-    memory, about half the speed); the factors the solves read are complex64 either way.  ``solve``
+    memory, about half the speed); the factors the solves read are complex64 either way, the inverses
+    of their 256-row diagonal blocks complex128.  ``solve``
     applies (LU)⁻¹; the sweep uses it as the preconditioner of FP64 BiCGStab
     (:meth:`FrequencySweep.solve_lu`), also at neighbouring frequencies."""
 

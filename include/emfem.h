@@ -364,7 +364,8 @@ int emfem_adam_step(emfem_handle h, int64_t n, float *params, const float *grad,
  * Replaces the reference's direct solve, SolverSuperLU (src/emerge/_emerge/solver.py:535-572, SuperLU
  * with MMD ordering), for the sweep system on a CSR pattern.  The host builds the symbolic structure
  * (emerge_b200/direct.py: nested dissection of the mesh's tets, fronts, assembly lists); the library
- * factors and solves on the device in complex64 (fronts) with FP64 input and output.
+ * factors and solves on the device in complex64 (fronts) with FP64 input and output; the inverses of the
+ * 256-row diagonal blocks, which the solves apply, are formed and applied in FP64.
  * create (host arrays; allocates all device memory once): n_fronts fronts in postorder (children before
  *   parents, each front at most two children); e / b: eliminated and boundary DOFs per front (e + b <=
  *   46340); parent (-1 for the root), level (height, leaves 0; a parent's level exceeds its children's);
@@ -381,12 +382,13 @@ int emfem_adam_step(emfem_handle h, int64_t n, float *params, const float *grad,
  *   block's largest entry (pivoting is partial inside each 32-row diagonal block).  Synchronises the
  *   stream.
  * set_precision: bits = 64 (default) factors in complex64, 128 in complex128 (the level workspace and
- *   the update store double in size; the factor store stays complex64, rounded once at compaction).
+ *   the update store double in size; the factor store stays complex64, rounded once at compaction, and
+ *   the block inverses complex128 as they are for 64).
  *   Reallocates the workspace and drops the factorization; on an allocation failure the handle stays
  *   complex64 and the call returns the error.
  * reserve: solve buffers for up to nrhs right-hand sides (<= 256).
  * solve: x = (LU)^-1 b for nrhs right-hand sides, b and x (n, nrhs) c128 DOF-major, device; x is zero on
- *   DOFs that belong to no front (PEC).
+ *   DOFs that belong to no front (PEC), and on boundary DOFs that no front eliminates.
  * emfem_krylov_solve_lu: FP64 right-preconditioned BiCGStab of emfem_krylov_solve (same operator and
  *   arguments) with M = this factorization for every system; the factorization may belong to another
  *   frequency of the same mesh (a window of a sweep shares one).  Reserve the padded batch size

@@ -10,8 +10,9 @@ from emerge_b200.sweep import FrequencySweep
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("nsys,precond,maxit", [(13, "aux", 20000), (32, "aux", 20000), (16, "none", 40), (7, "aux", 150)])
-def test_narrowed_batch_equals_single_solves(cuda, nsys, precond, maxit):
+@pytest.mark.parametrize("nsys,precond,maxit", [(13, "aux", 20000), (32, "aux", 20000), (16, "none", 40), (24, "aux", 150),
+                                                (7, "aux", 150)])
+def test_narrowed_batch_solves_every_column(cuda, nsys, precond, maxit):
     P = problems.waveguide(nx=10, ny=5, nz=20)            # n * nsys beyond the width from which batches are narrowed
     sw = FrequencySweep(P)
     assert sw.n * nsys >= 1 << 18
